@@ -13,7 +13,7 @@
 // Autotuning (LITHO_BATCH_AUTOTUNE) times, per class, every candidate of
 //   conv grid N in {nextPow2(4N+1), 2x that} (the FFT plan of the SOCS stage),
 //   kernels per CTA in {2, 3, 4, 6, 8, 12} (the SOCS tile), and
-//   window column splits in {1, 2}
+//   window splits (of columns, plain form: of rows) in {1, 2}
 // with CUDA events on the context's stream and keeps the fastest; results are
 // cached on the context by (L, Nx, nk, images, precision).  The plan then
 // captures the whole sequence in a CUDA graph (LITHO_BATCH_GRAPH).
@@ -34,7 +34,7 @@ struct SubBatch {
 struct ClassRun {
   int L = 0;
   const litho_kernel_set* ks = nullptr;
-  int count = 0, maxM = 0;
+  int count = 0, maxBlocks = 0;
   float* images = nullptr;
   DevBuf win, band, tmbuf, wsum;
   int convN = 0, kpg = 1, colSplits = 1, part_stride = 1;  // convN == 0: the TCC band (band_tcc.cu)
@@ -113,7 +113,8 @@ static int run_class(litho_batch_plan* bp, int ci) {
   auto win_plan = [&](const SubBatch& s) {
     ImgGeom gw{s.mLx, s.mLy, c.L, c.L, Nx, Ny, c.ks->nk, c.convN};
     ImgPlan pw = make_plan(gw, s.count, ctx->sm_count);
-    pw.colSplits = std::min(c.colSplits, std::max(1, tc ? (s.mLx + 63) / 64 / 2 : (s.mLx + 63) / 64));
+    if (!tc) win_fold_plan(pw, ctx->sm_count);
+    pw.colSplits = std::min(c.colSplits, std::max(1, tc ? (s.mLx + 63) / 64 / 2 : win_fold_max_splits(gw)));
     pw.part_stride = c.part_stride;
     return pw;
   };
@@ -320,7 +321,11 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
     ClassRun& c = bp->classes[s.cls];
     s.first_in_class = c.count;
     c.count += s.count;
-    c.maxM = std::max(c.maxM, s.mLy);
+    // partials of one split: 128-row blocks (tensor cores) or column blocks (plain)
+    const ImgGeom gw{s.mLx, s.mLy, c.L, c.L, c.ks->Nx, c.ks->Ny, c.ks->nk, c.convN};
+    ImgPlan pw = make_plan(gw, s.count, ctx->sm_count);
+    if (precision != LITHO_PREC_MIXED) win_fold_plan(pw, ctx->sm_count);
+    c.maxBlocks = std::max(c.maxBlocks, pw.rowBlocks);
   }
   for (auto& c : bp->classes) image_floats += (size_t)c.count * c.L * c.L;
   int rc = bp->mask_pool.ensure(ctx, mask_floats * sizeof(float));
@@ -357,7 +362,7 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
   for (auto& c : bp->classes) {
     if (c.count == 0) continue;
     const int Nx = c.ks->Nx, Ny = c.ks->Ny, KY = 2 * Ny + 1;
-    c.part_stride = ((c.maxM + 127) / 128) * 2;  // row blocks x up to two column splits
+    c.part_stride = c.maxBlocks * 2;  // up to two splits
     rc = c.win.ensure(ctx, (size_t)c.count * c.part_stride * KY * (Nx + 1) * sizeof(float2));
     const int groups = std::max(c.ks->nk, c.ks->band_nc);  // the FFT form's kernel groups or the band chunks
     if (rc == LITHO_OK) rc = c.band.ensure(ctx, (size_t)c.count * groups * KY * (4 * Nx + 1) * sizeof(float2));

@@ -488,8 +488,7 @@ int litho_image_batch(litho_ctx* ctx, const litho_kernel_set* ks, const float* m
   }
   LITHO_RET(host_batch(ctx, g, batch, masks, ks, images, precision, img));
   LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  if (precision == LITHO_PREC_MIXED) LITHO_RET(tc_check_flag(ctx));
-  return LITHO_OK;
+  return tc_check_flag(ctx);
 }
 
 int litho_image(litho_ctx* ctx, const float* mask, int Lx, int Ly, const float* krn_r, const float* krn_i,

@@ -1,7 +1,7 @@
-// Row pairing of the FP32 interpolation kernel (imaging.cu, fi_out_kernel): with the
-// centred row coordinate y' = Y + (Fy-Ly)/2 - Fy/2, one set of sums over the band rows
-// serves the base row b = |y'| and gives rows y' = +b and y' = -b.  Plain C++ (host and
-// device), so the pairing is also checked on the CPU.
+// Row pairing of the FP32 transforms (fold.hpp, imaging_fold.cu): with the centred row
+// coordinate y' = Y + (Fy-Ly)/2 - Fy/2, one row of coefficients serves the base row b = |y'|
+// and its rows y' = +b and y' = -b.  Plain C++ (host and device), so the pairing is also
+// checked on the CPU.
 #pragma once
 
 #ifdef __CUDACC__

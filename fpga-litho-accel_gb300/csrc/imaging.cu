@@ -8,288 +8,27 @@
 // intensity is band-limited to |f| <= 2N, so this file computes exactly those
 // pieces and nothing else:
 //
-//   win_dft_kernel : W[v][u] = 1/(FxFy) sum_{y,x} m[y][x] e^{-2 pi i (u x'/Fx + v y'/Fy)}
-//                    (x' = x + (Fx-Lx)/2 - Fx/2).  A separable partial DFT: the
-//                    column stage is a 128 x Lx x (2Nx+1) FP32 contraction per CTA
-//                    with the mask chunks streamed through a cp.async ring in
-//                    shared memory, the row stage a small complex contraction in
-//                    the epilogue.  HBM: one read of the mask.
+//   win_fold_kernel: W[v][u] = 1/(FxFy) sum_{y,x} m[y][x] e^{-2 pi i (u x'/Fx + v y'/Fy)}
+//                    (x' = x + (Fx-Lx)/2 - Fx/2), imaging_fold.cu.  HBM: one read of
+//                    the mask.
 //   socs_kernel    : per kernel k, embed K_k*W in an N x N grid, 2-D inverse FFT
 //                    (warp-shuffle radix-2, fft_warp.cuh), accumulate s_k|E|^2 in
 //                    registers; then a forward FFT of the intensity and the
 //                    |f| <= 2N band S[fy][fx] / N^2 is written out.
 //   fi_rows_kernel : T[fy][X] = sum_fx S[fy][fx] e^{+2 pi i fx x'/Fx}   (fy >= 0)
-//   fi_out_kernel  : image[Y][X] = T0 + 2 sum_{fy>0} Re(e^{2 pi i fy y'/Fy} T[fy][X]),
-//                    a rank-(4Ny+1) FP32 contraction whose cos and sin halves give
-//                    rows +y' and -y' from one set of sums, written once with
-//                    16-byte streaming stores.  HBM: one write of the image.
+//   fi_fold_kernel : image[Y][X] = T0 + 2 sum_{fy>0} Re(e^{2 pi i fy y'/Fy} T[fy][X]),
+//                    imaging_fold.cu.  HBM: one write of the image.
 // With C2R's Hermitian completion and the two rolls of litho.cpp:934 and
 // litho.cpp:700, that is exactly FI's zero-padded interpolation followed by
 // crop2DCentered (litho.cpp:164-177, 997-1001).
 #include "litho_internal.cuh"
 #include "fft_warp.cuh"
 #include "fft_lane8.cuh"
-#include "fi_mirror.hpp"
 #include "tc_common.cuh"
 
 #include <algorithm>
 
 namespace litho {
-
-// ---------------------------------------------------------------------------
-// helpers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int pmod(long long a, int m) {
-  long long r = a % m;
-  return (int)(r < 0 ? r + m : r);
-}
-
-// exp(sign * 2 pi i * m / F) for an exact integer phase m (the argument of
-// sincospif is exact because F is a power of two).
-__device__ __forceinline__ float2 cis_exact(long long m, int F, float sign) {
-  const int r = (int)(m & (long long)(F - 1));  // F (an FFT size) is a power of two
-  float s, c;
-  sincospif(2.0f * (float)r / (float)F, &s, &c);
-  return make_float2(c, sign * s);
-}
-
-// ---------------------------------------------------------------------------
-// window DFT column twiddles: twx[x][j], j in [0, NJT):
-//   j <= Nx          : cos(2 pi j x'/Fx)
-//   Nx < j <= 2Nx    : -sin(2 pi (j-Nx) x'/Fx)
-//   otherwise 0 (padding to a multiple of 4)
-// ---------------------------------------------------------------------------
-__global__ void twx_init_kernel(float* __restrict__ twx, int Lx, int Fx, int Nx, int NJT) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= Lx) return;
-  const long long xp = (long long)x + (Fx - Lx) / 2 - Fx / 2;
-  for (int j = 0; j < NJT; ++j) {
-    float v = 0.f;
-    if (j <= 2 * Nx) {
-      const int u = j <= Nx ? j : j - Nx;
-      long long m = ((long long)u * xp) % Fx;
-      if (m < 0) m += Fx;
-      double s, c;
-      sincospi(2.0 * (double)m / (double)Fx, &s, &c);
-      v = j <= Nx ? (float)c : (float)(-s);
-    }
-    twx[(size_t)x * NJT + j] = v;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// window DFT
-// ---------------------------------------------------------------------------
-constexpr int WD_BM = 128;          // mask rows per CTA
-constexpr int WD_BK = 32;           // mask columns per ring stage
-constexpr int WD_SA = WD_BK + 4;    // staged row stride (floats): 16-byte rows, conflict-free 16-byte reads
-constexpr int WD_THREADS = 256;
-
-// ring stages: enough mask bytes in flight per SM (two CTAs of 4 x 16 KB where the
-// accumulators leave room for two, else one CTA of 8)
-template <int NJT>
-struct WinRing {
-  static constexpr int CTAS = NJT <= 20 ? 2 : 1;
-  static constexpr int ST = NJT <= 20 ? 4 : 8;
-  static constexpr int A_F = WD_BM * WD_SA;  // floats of a stage's mask chunk
-  static constexpr int STAGE_F = A_F + WD_BK * NJT;
-};
-
-// shared memory of a window DFT launch: the ring, reused by the k-split reduction and
-// the row transform at the end
-template <int NJT>
-static size_t win_dft_smem(int Ny) {
-  const size_t ring = (size_t)WinRing<NJT>::ST * WinRing<NJT>::STAGE_F * sizeof(float);
-  const size_t tree = (size_t)4 * NJT * WD_BM * sizeof(float);  // the k-split warps' sums
-  const size_t rows = (size_t)NJT * (WD_BM + 4) * sizeof(float) + (size_t)(Ny + 1) * (WD_BM + 2) * sizeof(float2);
-  return std::max(ring, std::max(tree, rows));
-}
-
-__device__ __forceinline__ void wd_cp16(float* dst, const float* src, bool ok) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void wd_cp4(float* dst, const float* src, bool ok) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(ok ? 4 : 0) : "memory");
-}
-
-// One CTA per (row block of WD_BM rows, column split, image): the mask chunks of its
-// columns stream through a ring of cp.async stages (row-major, zero-filled past the
-// mask) with the chunk's column twiddles beside them; warp w multiplies columns
-// 4w..4w+3 of every chunk into its 4 rows x NJT accumulators (rows lane + 32i), in
-// packed f32x2 FMAs.  The eight warps' sums are then added in a fixed tree and each
-// row block's row transforms summed over its rows with the row twiddles.
-template <int NJT, bool VEC>
-__global__ void __launch_bounds__(WD_THREADS, WinRing<NJT>::CTAS) win_dft_kernel(
-    const float* __restrict__ masks, int Lx, int Ly, int Fx, int Fy, int Nx, int Ny, const float* __restrict__ twx,
-    float2* __restrict__ win_part, int part_stride) {
-  using RG = WinRing<NJT>;
-  constexpr int ST = RG::ST;
-  extern __shared__ __align__(16) float sm[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rb = blockIdx.x, cs = blockIdx.y, img = blockIdx.z;
-  const int colSplits = gridDim.y;
-  const int nparts = gridDim.x * gridDim.y;
-  const int part = rb * colSplits + cs;
-  const int y0 = rb * WD_BM;
-  const int nch = (Lx + WD_BK - 1) / WD_BK;
-  const int ch0 = (int)((long long)nch * cs / colSplits);
-  const int ch1 = (int)((long long)nch * (cs + 1) / colSplits);
-  const float* M = masks + (size_t)img * Lx * Ly;
-  auto sA = [&](int st) { return sm + (size_t)st * RG::STAGE_F; };        // [WD_BM][WD_SA]
-  auto sB = [&](int st) { return sm + (size_t)st * RG::STAGE_F + RG::A_F; };  // [WD_BK][NJT]
-
-  // chunk ch into ring slot st: 128 rows x 32 columns (four 16-byte pieces a thread) and
-  // the chunk's twiddle rows (NJT / 4 pieces per column)
-  auto issue = [&](int ch, int st) {
-    const int x0 = ch * WD_BK;
-    float* a = sA(st);
-#pragma unroll
-    for (int i = 0; i < WD_BM * WD_BK / 4 / WD_THREADS; ++i) {
-      const int idx = tid + WD_THREADS * i, row = idx >> 3, c4 = (idx & 7) * 4;
-      const int y = y0 + row, x = x0 + c4;
-      const bool rok = y < Ly;
-      const float* src = M + (size_t)(rok ? y : 0) * Lx;
-      float* dst = a + row * WD_SA + c4;
-      if (VEC) {
-        wd_cp16(dst, src + (rok && x < Lx ? x : 0), rok && x < Lx);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) wd_cp4(dst + e, src + (rok && x + e < Lx ? x + e : 0), rok && x + e < Lx);
-      }
-    }
-    constexpr int Q = NJT / 4;
-    float* b = sB(st);
-    for (int idx = tid; idx < WD_BK * Q; idx += WD_THREADS) {
-      const int kr = idx / Q, c = idx - kr * Q, x = x0 + kr;
-      wd_cp16(b + 4 * idx, twx + (size_t)(x < Lx ? x : 0) * NJT + 4 * c, x < Lx);
-    }
-  };
-
-  // accumulators in column pairs: one packed (f32x2) FMA updates two twiddle columns, each
-  // lane rounding as fmaf does
-  float2 acc2[4][NJT / 2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < NJT / 2; ++j) acc2[i][j] = make_float2(0.f, 0.f);
-  auto acc = [&](int i, int j) -> float& { return (j & 1) ? acc2[i][j >> 1].y : acc2[i][j >> 1].x; };
-
-  // one commit group per ring step (empty past the last chunk), so that waiting for all
-  // but the newest ST - 2 groups means the current stage has landed
-#pragma unroll
-  for (int k = 0; k < ST - 1; ++k) {
-    if (ch0 + k < ch1) issue(ch0 + k, k);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  for (int ch = ch0; ch < ch1; ++ch) {
-    const int it = ch - ch0, st = it % ST;
-    asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
-    __syncthreads();  // the stage is visible to all; every warp is done with the previous one
-    if (ch + ST - 1 < ch1) issue(ch + ST - 1, (it + ST - 1) % ST);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* a = sA(st) + lane * WD_SA + 4 * warp;
-    float4 av[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) av[i] = *reinterpret_cast<const float4*>(a + 32 * i * WD_SA);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      const float4* b4 = reinterpret_cast<const float4*>(sB(st) + (4 * warp + kk) * NJT);
-      float2 ai[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float v = kk == 0 ? av[i].x : kk == 1 ? av[i].y : kk == 2 ? av[i].z : av[i].w;
-        ai[i] = make_float2(v, v);
-      }
-#pragma unroll
-      for (int c = 0; c < NJT / 4; ++c) {
-        const float4 b = b4[c];
-        const float2 blo = make_float2(b.x, b.y), bhi = make_float2(b.z, b.w);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          acc2[i][2 * c] = __ffma2_rn(ai[i], blo, acc2[i][2 * c]);
-          acc2[i][2 * c + 1] = __ffma2_rn(ai[i], bhi, acc2[i][2 * c + 1]);
-        }
-      }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-
-  // tree reduction of the 8 k-split warps: red[w][j][r], r fastest (conflict free)
-  float* red = sm;
-  for (int s = 4; s >= 1; s >>= 1) {
-    if (warp >= s && warp < 2 * s) {
-      float* dst = red + (size_t)(warp - s) * NJT * WD_BM;
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < NJT; ++j) dst[j * WD_BM + lane + 32 * i] = acc(i, j);
-    }
-    __syncthreads();
-    if (warp < s) {
-      const float* src = red + (size_t)warp * NJT * WD_BM;
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < NJT; ++j) acc(i, j) += src[j * WD_BM + lane + 32 * i];
-    }
-    __syncthreads();
-  }
-  // row transforms of this block and the row twiddles, rows padded (132 floats, 130 float2)
-  // so that the threads of a warp (different u, |v|) read different banks
-  constexpr int RS = WD_BM + 4, RT = WD_BM + 2;
-  float* sR = red;  // [NJT][RS]
-  if (warp == 0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < NJT; ++j) sR[j * RS + lane + 32 * i] = acc(i, j);
-  }
-  // row twiddles e^{-2 pi i v y'/Fy}, v = 0..Ny
-  float2* sRT = reinterpret_cast<float2*>(sm + (size_t)NJT * RS);  // [Ny+1][RT]
-  const int oyc = (Fy - Ly) / 2 - Fy / 2;
-  for (int idx = tid; idx < (Ny + 1) * WD_BM; idx += WD_THREADS) {
-    const int v = idx / WD_BM, r = idx - v * WD_BM;
-    sRT[v * RT + r] = cis_exact((long long)v * (y0 + r + oyc), Fy, -1.f);
-  }
-  __syncthreads();
-
-  const int KY = 2 * Ny + 1, NU = Nx + 1;
-  const float scale = 1.0f / ((float)Fx * (float)Fy);
-  // part_stride > 0: images of this launch sit in a larger per-class array with
-  // that many parts per image (the unused parts are zero)
-  const int nps = part_stride > 0 ? part_stride : nparts;
-  float2* out = win_part + ((size_t)img * nps + part) * KY * NU;
-  for (int o = tid; o < KY * NU; o += WD_THREADS) {
-    const int vi = o / NU, u = o - vi * NU;
-    const int v = vi - Ny;
-    const int av = v < 0 ? -v : v;
-    const float ts = v < 0 ? -1.f : 1.f;
-    const float* rc = sR + u * RS;
-    const float* rs = sR + (Nx + u) * RS;
-    const float2* rt = sRT + av * RT;
-    float re = 0.f, im = 0.f;
-    if (u == 0) {
-#pragma unroll 4
-      for (int r = 0; r < WD_BM; ++r) {
-        const float2 t = rt[r];
-        re = fmaf(rc[r], t.x, re);
-        im = fmaf(rc[r], ts * t.y, im);
-      }
-    } else {
-#pragma unroll 4
-      for (int r = 0; r < WD_BM; ++r) {
-        const float2 t = rt[r];
-        const float ty = ts * t.y;
-        re = fmaf(rc[r], t.x, fmaf(-rs[r], ty, re));
-        im = fmaf(rc[r], ty, fmaf(rs[r], t.x, im));
-      }
-    }
-    out[o] = make_float2(re * scale, im * scale);
-  }
-}
 
 // ---------------------------------------------------------------------------
 // SOCS: K inverse FFTs on the N x N conv grid, intensity accumulation in
@@ -756,7 +495,7 @@ __global__ void __launch_bounds__(S128_THREADS) socs128_kernel(
 // is summed by one warp of the first column block.  A CTA keeps its columns'
 // twiddles in registers and walks the images blockIdx.y, blockIdx.y + gridDim.y, ...
 // Two output layouts:
-//   plain  tm[img][r][X]: r = 0 Re T0, 1..2Ny Re T, 2Ny+1..4Ny Im T (fi_out_kernel)
+//   plain  tm[img][r][X]: r = 0 Re T0, 1..2Ny Re T, 2Ny+1..4Ny Im T (fi_fold_kernel)
 //   K-major (tensor-core FI) t0[img][X] = Re T0 and hi/lo TF32 splits of
 //          tm[img][X][KP]: r = fy-1 Re T, 2Ny+fy-1 Im T, zero to KP
 // ---------------------------------------------------------------------------
@@ -781,8 +520,7 @@ __global__ void __launch_bounds__(FR_THREADS) fi_rows_kernel(const float2* __res
   float2 tw[MAXD];
 #pragma unroll
   for (int d = 1; d < MAXD; ++d)
-    tw[d] = (d < ND && live) ? (twF != nullptr ? twF[(size_t)d * Lx + X] : cis_exact((long long)d * (X - nb), Fx, 1.f))
-                             : make_float2(0.f, 0.f);
+    tw[d] = (d < ND && live) ? twF[(size_t)d * Lx + X] : make_float2(0.f, 0.f);
   if (KMAJ)  // the K padding columns stay zero for every image
     for (int idx = tid; idx < FR_ROWS * (KP - 4 * Ny); idx += FR_THREADS) {
       const int c = idx / (KP - 4 * Ny), r = 4 * Ny + idx % (KP - 4 * Ny);
@@ -993,7 +731,9 @@ __global__ void twF_init_kernel(float2* __restrict__ tw, int Lx, int Fx, int ND)
   const int x = blockIdx.x * blockDim.x + threadIdx.x, d = blockIdx.y;
   if (x >= Lx || d >= ND) return;
   const long long xp = (long long)x + (Fx - Lx) / 2 - Fx / 2;
-  tw[(size_t)d * Lx + x] = cis_exact((long long)d * xp, Fx, 1.f);
+  float2 t;
+  cis_round((long long)d * xp, Fx, &t.x, &t.y);
+  tw[(size_t)d * Lx + x] = t;
 }
 
 // cached per (Lx, Fx, Nx) on the context
@@ -1011,144 +751,6 @@ int fi_twiddles(litho_ctx* ctx, const ImgGeom& g, const float2** out) {
   }
   *out = it->second.as<float2>();
   return LITHO_OK;
-}
-
-// ---------------------------------------------------------------------------
-// FI, step 2: image = Cy (Ly x KB) * Tm (KB x Lx), KB = 4Ny+1.
-// ---------------------------------------------------------------------------
-constexpr int FO_BM = 32, FO_BN = 128, FO_THREADS = 256;
-
-// The rows pair up around the centre: with y' = Y + oy (oy = (Fy-Ly)/2 - Fy/2) the image is
-//   image(+b) = A(b) + B(b),  image(-b) = A(b) - B(b),
-//   A(b) = T0 + sum_{r=1..2Ny} 2cos(2 pi r b/Fy) Re T_r,  B(b) = sum_r -2sin(2 pi r b/Fy) Im T_r,
-// so one set of sums over the 4Ny+1 rows of Tm serves rows +b and -b.  Cm[r][b] holds the
-// coefficients of base row b (r = 0: 1; 1..2Ny: 2cos; 2Ny+1..4Ny: -2sin), b < nbp (the
-// base rows |y'| rounded up to FO_BM).  The FI kernel evaluates the same values when it
-// has no table (the allocation-free entry point).
-__device__ __forceinline__ float fo_cm(int r, int b, int Fy, int Ny) {
-  if (r == 0) return 1.f;
-  const int dy = r <= 2 * Ny ? r : r - 2 * Ny;
-  const float2 e = cis_exact((long long)dy * b, Fy, 1.f);
-  return r <= 2 * Ny ? 2.f * e.x : -2.f * e.y;
-}
-
-__global__ void fo_cm_init_kernel(float* __restrict__ cm, int nbp, int Fy, int Ny) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
-  if (b < nbp) cm[(size_t)r * nbp + b] = fo_cm(r, b, Fy, Ny);
-}
-
-// the Cm table of a geometry, cached per (Ly, Fy, Ny) on the context
-static int fo_cm_table(litho_ctx* ctx, const ImgGeom& g, const float** out, int* nbp) {
-  *nbp = (fo_nbase(g.Ly, g.Fy) + FO_BM - 1) / FO_BM * FO_BM;
-  auto key = std::make_tuple(g.Ly, g.Fy, g.Ny, -5001);
-  auto it = ctx->twx_tables.find(key);
-  if (it == ctx->twx_tables.end()) {
-    const int KB = 4 * g.Ny + 1;
-    DevBuf b;
-    LITHO_RET(b.ensure(ctx, (size_t)KB * *nbp * sizeof(float)));
-    StageScope sc(ctx, LITHO_STAGE_UPLOAD);
-    fo_cm_init_kernel<<<dim3(*nbp / FO_BM, KB), FO_BM, 0, ctx->stream>>>(b.as<float>(), *nbp, g.Fy, g.Ny);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
-    it = ctx->twx_tables.emplace(key, b).first;
-  }
-  *out = it->second.as<float>();
-  return LITHO_OK;
-}
-
-// One CTA per (FO_BM base rows, FO_BN columns, image): thread (warp w, lane l) sums base
-// rows 4w..4w+3 over columns 4l..4l+3, the cos rows of Tm into A and the sin rows into B
-// (packed f32x2 FMAs), and writes A + B to row +b and A - B to row -b where they lie in
-// the image.
-template <bool VEC>
-__global__ void __launch_bounds__(FO_THREADS) fi_out_kernel(const float* __restrict__ tm, int Lx, int Ly, int Fy,
-                                                            int Ny, const float* __restrict__ cmt, int nbp,
-                                                            float* __restrict__ images) {
-  extern __shared__ __align__(16) float fo[];
-  const int KB = 4 * Ny + 1;
-  float* sC = fo;                // [KB][FO_BM]
-  float* sT = fo + KB * FO_BM;   // [KB][FO_BN]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int X0 = blockIdx.x * FO_BN, B0 = blockIdx.y * FO_BM, img = blockIdx.z;
-  const float* T = tm + (size_t)img * KB * Lx;
-  if (VEC) {
-    for (int idx = tid; idx < KB * (FO_BN / 4); idx += FO_THREADS) {
-      const int r = idx / (FO_BN / 4), c4 = 4 * (idx - r * (FO_BN / 4));
-      const int X = X0 + c4;
-      reinterpret_cast<float4*>(sT)[idx] =
-          X < Lx ? __ldg(reinterpret_cast<const float4*>(T + (size_t)r * Lx + X)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  } else {
-    for (int idx = tid; idx < KB * FO_BN; idx += FO_THREADS) {
-      const int r = idx / FO_BN, c = idx - r * FO_BN;
-      const int X = X0 + c;
-      sT[idx] = X < Lx ? T[(size_t)r * Lx + X] : 0.f;
-    }
-  }
-  if (cmt != nullptr) {  // the cached table: whole 16-byte pieces of the tile's base rows
-    for (int idx = tid; idx < KB * (FO_BM / 4); idx += FO_THREADS) {
-      const int r = idx / (FO_BM / 4), q = idx - r * (FO_BM / 4);
-      reinterpret_cast<float4*>(sC)[idx] = __ldg(reinterpret_cast<const float4*>(cmt + (size_t)r * nbp + B0) + q);
-    }
-  } else {
-    for (int idx = tid; idx < KB * FO_BM; idx += FO_THREADS) {
-      const int r = idx / FO_BM, bb = idx - r * FO_BM;
-      sC[idx] = fo_cm(r, B0 + bb, Fy, Ny);
-    }
-  }
-  __syncthreads();
-  // A and B of 4 base rows x 4 columns, in column pairs
-  float2 A[4][2], Bs[4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) A[i][j] = Bs[i][j] = make_float2(0.f, 0.f);
-  auto step = [&](int r, float2(&acc)[4][2]) {
-    const float4 c = *reinterpret_cast<const float4*>(sC + r * FO_BM + 4 * warp);  // one address per warp
-    const float4 t = *reinterpret_cast<const float4*>(sT + r * FO_BN + 4 * lane);
-    const float cc[4] = {c.x, c.y, c.z, c.w};
-    const float2 tlo = make_float2(t.x, t.y), thi = make_float2(t.z, t.w);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 ci = make_float2(cc[i], cc[i]);
-      acc[i][0] = __ffma2_rn(ci, tlo, acc[i][0]);
-      acc[i][1] = __ffma2_rn(ci, thi, acc[i][1]);
-    }
-  };
-#pragma unroll 4
-  for (int r = 0; r <= 2 * Ny; ++r) step(r, A);
-#pragma unroll 4
-  for (int r = 2 * Ny + 1; r < KB; ++r) step(r, Bs);
-  const int nbase = fo_nbase(Ly, Fy);
-  float* O = images + (size_t)img * Lx * Ly;
-  const int X = X0 + 4 * lane;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int b = B0 + 4 * warp + i;
-    if (b >= nbase) continue;
-#pragma unroll
-    for (int sgn = 0; sgn < 2; ++sgn) {
-      const int Y = fo_row(b, sgn, Ly, Fy);  // y' = +b, -b (y' = 0 once)
-      if (Y < 0) continue;
-      const float o[4] = {sgn == 0 ? A[i][0].x + Bs[i][0].x : A[i][0].x - Bs[i][0].x,
-                          sgn == 0 ? A[i][0].y + Bs[i][0].y : A[i][0].y - Bs[i][0].y,
-                          sgn == 0 ? A[i][1].x + Bs[i][1].x : A[i][1].x - Bs[i][1].x,
-                          sgn == 0 ? A[i][1].y + Bs[i][1].y : A[i][1].y - Bs[i][1].y};
-      float* row = O + (size_t)Y * Lx;
-      if (VEC && X + 3 < Lx) {
-        __stcs(reinterpret_cast<float4*>(row + X), make_float4(o[0], o[1], o[2], o[3]));
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (X + e < Lx) row[X + e] = o[e];
-      }
-    }
-  }
-}
-
-// launch geometry of the FI output kernel
-static inline dim3 fo_grid(const ImgGeom& g, int batch) {
-  const int nb = fo_nbase(g.Ly, g.Fy);
-  return dim3((g.Lx + FO_BN - 1) / FO_BN, (nb + FO_BM - 1) / FO_BM, batch);
 }
 
 // ---------------------------------------------------------------------------
@@ -1229,25 +831,11 @@ __global__ void __launch_bounds__(FM_THREADS) fft_rows_centred_kernel(
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static int njt_for(int Nx) {
-  const int nj = 2 * Nx + 1;
-  if (nj <= 8) return 8;
-  if (nj <= 12) return 12;
-  if (nj <= 20) return 20;
-  if (nj <= 36) return 36;
-  return -1;
-}
-
 ImgPlan make_plan(const ImgGeom& g, int batch, int sm_count) {
   ImgPlan p;
   p.g = g;
   p.batch = batch;
-  p.rowBlocks = (g.Ly + WD_BM - 1) / WD_BM;
-  const int nch = (g.Lx + WD_BK - 1) / WD_BK;
-  const int want = 2 * sm_count;
-  int cs = (want + p.rowBlocks * batch - 1) / (p.rowBlocks * batch);
-  cs = std::max(1, std::min(cs, std::max(1, nch / 2)));
-  p.colSplits = cs;
+  p.rowBlocks = (g.Ly + 127) / 128;  // of the tensor-core window DFT (win_fold_plan sets the plain one's)
   // SOCS is latency-bound (warp-shuffle FFT chains), but every kernel group also
   // transforms its own partial intensity: ~2.5 CTAs (20 warps) per SM measured best
   // at 1024^2, K=24, 64 masks (4 kernels per CTA: 36.9 us; 3: 38.9; 8: 45.0)
@@ -1259,64 +847,47 @@ ImgPlan make_plan(const ImgGeom& g, int batch, int sm_count) {
   return p;
 }
 
-static int twx_table(litho_ctx* ctx, int Lx, int Fx, int Nx, int NJT, const float** out) {
-  auto key = std::make_tuple(Lx, Fx, Nx, NJT);
+// coefficient tables of the folded transforms, cached per (Ly, Fy, Ny) on the context
+static int fold_table(litho_ctx* ctx, const ImgGeom& g, int kind, size_t floats,
+                      cudaError_t (*init)(cudaStream_t, const ImgGeom&, float*), const float** out) {
+  auto key = std::make_tuple(g.Ly, g.Fy, g.Ny, kind);
   auto it = ctx->twx_tables.find(key);
   if (it == ctx->twx_tables.end()) {
     DevBuf b;
-    LITHO_RET(b.ensure(ctx, (size_t)Lx * NJT * sizeof(float)));
+    LITHO_RET(b.ensure(ctx, floats * sizeof(float)));
     StageScope sc(ctx, LITHO_STAGE_UPLOAD);
-    twx_init_kernel<<<(Lx + 127) / 128, 128, 0, ctx->stream>>>(b.as<float>(), Lx, Fx, Nx, NJT);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
+    LITHO_CUDA_TRY(ctx, init(ctx->stream, g, b.as<float>()));
     it = ctx->twx_tables.emplace(key, b).first;
   }
   *out = it->second.as<float>();
   return LITHO_OK;
 }
 
-template <int NJT>
-static int launch_win_dft_t(litho_ctx* ctx, const ImgPlan& p, const float* masks, const float* twx,
-                            float2* win_part) {
-  const ImgGeom& g = p.g;
-  const size_t smem = win_dft_smem<NJT>(g.Ny);
-  dim3 grid(p.rowBlocks, p.colSplits, p.batch);
-  StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
-  if ((g.Lx & 3) == 0) {
-    auto k = win_dft_kernel<NJT, true>;
-    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, WD_THREADS, smem, ctx->stream>>>(masks, g.Lx, g.Ly, g.Fx, g.Fy, g.Nx, g.Ny, twx, win_part, p.part_stride);
-  } else {
-    auto k = win_dft_kernel<NJT, false>;
-    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, WD_THREADS, smem, ctx->stream>>>(masks, g.Lx, g.Ly, g.Fx, g.Fy, g.Nx, g.Ny, twx, win_part, p.part_stride);
-  }
-  LITHO_CUDA_TRY(ctx, cudaGetLastError());
-  return LITHO_OK;
+// Build the cached tables a plain window DFT of this geometry reads, on the context's
+// stream (so that launches on other streams find them ready).
+static int win_dft_tables(litho_ctx* ctx, const ImgGeom& g, const float** coef, const float2** twF) {
+  LITHO_RET(fold_table(ctx, g, -6001, win_fold_coef_floats(g), win_fold_coefs, coef));
+  return fi_twiddles(ctx, g, twF);
 }
-
-// Build the cached column-twiddle table a plain window DFT of this geometry reads, on the
-// context's stream (so that launches on other streams find it ready).
 int prepare_win_dft(litho_ctx* ctx, const ImgPlan& p) {
-  const int NJT = njt_for(p.g.Nx);
-  if (NJT < 0) return LITHO_OK;  // the launch reports the unsupported size
-  const float* twx = nullptr;
-  return twx_table(ctx, p.g.Lx, p.g.Fx, p.g.Nx, NJT, &twx);
+  const float* coef = nullptr;
+  const float2* twF = nullptr;
+  return win_dft_tables(ctx, p.g, &coef, &twF);
 }
 
 int run_win_dft(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part) {
-  const int NJT = njt_for(p.g.Nx);
-  if (NJT < 0) {
-    set_error(ctx, LITHO_ERR_UNSUPPORTED, "window DFT supports Nx <= 16 (got %d)", p.g.Nx);
+  if (p.g.Nx > 16 || p.g.Ny > 16) {
+    set_error(ctx, LITHO_ERR_UNSUPPORTED, "window DFT supports Nx, Ny <= 16 (got %d, %d)", p.g.Nx, p.g.Ny);
     return LITHO_ERR_UNSUPPORTED;
   }
-  const float* twx = nullptr;
-  LITHO_RET(twx_table(ctx, p.g.Lx, p.g.Fx, p.g.Nx, NJT, &twx));
-  switch (NJT) {
-    case 8: return launch_win_dft_t<8>(ctx, p, masks, twx, win_part);
-    case 12: return launch_win_dft_t<12>(ctx, p, masks, twx, win_part);
-    case 20: return launch_win_dft_t<20>(ctx, p, masks, twx, win_part);
-    default: return launch_win_dft_t<36>(ctx, p, masks, twx, win_part);
-  }
+  const float* coef = nullptr;
+  const float2* twF = nullptr;
+  LITHO_RET(win_dft_tables(ctx, p.g, &coef, &twF));
+  int* err = nullptr;
+  LITHO_RET(tc_err_flag_public(ctx, &err));
+  StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
+  LITHO_CUDA_TRY(ctx, launch_win_fold(ctx->stream, p, masks, coef, twF, win_part, err));
+  return LITHO_OK;
 }
 
 template <int N>
@@ -1370,18 +941,10 @@ int run_fi(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tm,
     StageScope sc(ctx, LITHO_STAGE_FI_PREP);
     LITHO_CUDA_TRY(ctx, launch_fi_rows(ctx->stream, p, band_part, twF, 0, tm, nullptr, nullptr, nullptr));
   }
-  {
-    const int KB = 4 * g.Ny + 1;
-    int nbp = 0;
-    const float* cmt = nullptr;
-    LITHO_RET(fo_cm_table(ctx, g, &cmt, &nbp));
-    const size_t smem = (size_t)KB * (FO_BM + FO_BN) * sizeof(float);
-    StageScope sc(ctx, LITHO_STAGE_FI_OUT);
-    auto k = (g.Lx & 3) == 0 ? fi_out_kernel<true> : fi_out_kernel<false>;
-    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<fo_grid(g, p.batch), FO_THREADS, smem, ctx->stream>>>(tm, g.Lx, g.Ly, g.Fy, g.Ny, cmt, nbp, images);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
-  }
+  const float* coef = nullptr;
+  LITHO_RET(fold_table(ctx, g, -5001, fi_fold_coef_floats(g), fi_fold_coefs, &coef));
+  StageScope sc(ctx, LITHO_STAGE_FI_OUT);
+  LITHO_CUDA_TRY(ctx, launch_fi_fold(ctx->stream, p, tm, coef, images));
   return LITHO_OK;
 }
 
@@ -1425,34 +988,25 @@ __global__ void pack_planes_kernel(const float* __restrict__ kr, const float* __
   if (i < n) out[i] = make_float2(kr[i], ki[i]);
 }
 
-size_t noctx_scratch_layout(const ImgPlan& p, size_t off[6]) {
+// the flag of the kernels' bounded waits; then kernels, scales, window partials, band partials,
+// interpolation rows, and the three tables
+size_t noctx_scratch_layout(const ImgPlan& p, size_t off[8]) {
   const ImgGeom& g = p.g;
   const int KD = (2 * g.Nx + 1) * (2 * g.Ny + 1), KY = 2 * g.Ny + 1;
-  const size_t sz[6] = {(size_t)g.nk * KD * sizeof(float2),
+  const size_t sz[8] = {(size_t)g.nk * KD * sizeof(float2),
                         (size_t)g.nk * sizeof(float),
-                        (size_t)g.Lx * njt_for(g.Nx) * sizeof(float),
                         (size_t)p.nparts() * KY * (g.Nx + 1) * sizeof(float2),
                         (size_t)p.ngroups * KY * (4 * g.Nx + 1) * sizeof(float2),
-                        (size_t)(4 * g.Ny + 1) * g.Lx * sizeof(float)};
-  size_t o = 0;
-  for (int i = 0; i < 6; ++i) {
+                        (size_t)(4 * g.Ny + 1) * g.Lx * sizeof(float),
+                        (size_t)(2 * g.Nx + 1) * g.Lx * sizeof(float2),
+                        win_fold_coef_floats(g) * sizeof(float),
+                        fi_fold_coef_floats(g) * sizeof(float)};
+  size_t o = 256;
+  for (int i = 0; i < 8; ++i) {
     off[i] = o;
     o += (sz[i] + 255) & ~size_t(255);
   }
   return o;
-}
-
-template <int NJT>
-static cudaError_t noctx_win_dft_t(cudaStream_t s, const ImgPlan& p, const float* masks, const float* twx,
-                                   float2* win_part) {
-  const ImgGeom& g = p.g;
-  const size_t smem = win_dft_smem<NJT>(g.Ny);
-  dim3 grid(p.rowBlocks, p.colSplits, p.batch);
-  auto k = (g.Lx & 3) == 0 ? win_dft_kernel<NJT, true> : win_dft_kernel<NJT, false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k<<<grid, WD_THREADS, smem, s>>>(masks, g.Lx, g.Ly, g.Fx, g.Fy, g.Nx, g.Ny, twx, win_part, 0);
-  return cudaGetLastError();
 }
 
 template <int N>
@@ -1483,48 +1037,35 @@ static cudaError_t noctx_socs_t(cudaStream_t s, const ImgPlan& p, const float2* 
 cudaError_t image_pipeline_noctx(cudaStream_t s, const ImgPlan& p, const float* mask, const float* krn_r,
                                  const float* krn_i, const float* scales, char* scratch, float* image) {
   const ImgGeom& g = p.g;
-  size_t off[6];
+  size_t off[8];
   noctx_scratch_layout(p, off);
+  int* err = reinterpret_cast<int*>(scratch);
   float2* krn = reinterpret_cast<float2*>(scratch + off[0]);
   float* sc = reinterpret_cast<float*>(scratch + off[1]);
-  float* twx = reinterpret_cast<float*>(scratch + off[2]);
-  float2* win_part = reinterpret_cast<float2*>(scratch + off[3]);
-  float2* band_part = reinterpret_cast<float2*>(scratch + off[4]);
-  float* tm = reinterpret_cast<float*>(scratch + off[5]);
-  const int KD = (2 * g.Nx + 1) * (2 * g.Ny + 1);
-  const int NJT = njt_for(g.Nx);
+  float2* win_part = reinterpret_cast<float2*>(scratch + off[2]);
+  float2* band_part = reinterpret_cast<float2*>(scratch + off[3]);
+  float* tm = reinterpret_cast<float*>(scratch + off[4]);
+  float2* twF = reinterpret_cast<float2*>(scratch + off[5]);
+  float* wcoef = reinterpret_cast<float*>(scratch + off[6]);
+  float* fcoef = reinterpret_cast<float*>(scratch + off[7]);
+  const int KD = (2 * g.Nx + 1) * (2 * g.Ny + 1), ND = 2 * g.Nx + 1;
   cudaError_t e;
   pack_planes_kernel<<<(g.nk * KD + 255) / 256, 256, 0, s>>>(krn_r, krn_i, g.nk * KD, krn);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(sc, scales, g.nk * sizeof(float), cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-  twx_init_kernel<<<(g.Lx + 127) / 128, 128, 0, s>>>(twx, g.Lx, g.Fx, g.Nx, NJT);
+  twF_init_kernel<<<dim3((g.Lx + 127) / 128, ND), 128, 0, s>>>(twF, g.Lx, g.Fx, ND);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  switch (NJT) {
-    case 8: e = noctx_win_dft_t<8>(s, p, mask, twx, win_part); break;
-    case 12: e = noctx_win_dft_t<12>(s, p, mask, twx, win_part); break;
-    case 20: e = noctx_win_dft_t<20>(s, p, mask, twx, win_part); break;
-    default: e = noctx_win_dft_t<36>(s, p, mask, twx, win_part); break;
-  }
-  if (e != cudaSuccess) return e;
+  if ((e = win_fold_coefs(s, g, wcoef)) != cudaSuccess) return e;
+  if ((e = fi_fold_coefs(s, g, fcoef)) != cudaSuccess) return e;
+  if ((e = launch_win_fold(s, p, mask, wcoef, twF, win_part, err)) != cudaSuccess) return e;
   switch (g.convN) {
     case 32: e = noctx_socs_t<32>(s, p, win_part, krn, sc, band_part); break;
     case 64: e = noctx_socs_t<64>(s, p, win_part, krn, sc, band_part); break;
     default: e = noctx_socs_t<128>(s, p, win_part, krn, sc, band_part); break;
   }
   if (e != cudaSuccess) return e;
-  // no twiddle table here (nothing may be allocated): the kernel evaluates them
-  if ((e = launch_fi_rows(s, p, band_part, nullptr, 0, tm, nullptr, nullptr, nullptr)) != cudaSuccess) return e;
-  {
-    const int KB = 4 * g.Ny + 1;
-    const size_t smem = (size_t)KB * (FO_BM + FO_BN) * sizeof(float);
-    const dim3 grid = fo_grid(g, 1);
-    auto k = (g.Lx & 3) == 0 ? fi_out_kernel<true> : fi_out_kernel<false>;
-    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-      return e;
-    k<<<grid, FO_THREADS, smem, s>>>(tm, g.Lx, g.Ly, g.Fy, g.Ny, nullptr, 0, image);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  if ((e = launch_fi_rows(s, p, band_part, twF, 0, tm, nullptr, nullptr, nullptr)) != cudaSuccess) return e;
+  return launch_fi_fold(s, p, tm, fcoef, image);
 }
 
 // plan of one launch of the mixed form: the persistent tensor-core window kernel splits
@@ -1546,6 +1087,7 @@ int image_pipeline(litho_ctx* ctx, const ImgGeom& g, int batch, const float* mas
   const bool tc = precision == LITHO_PREC_MIXED && tc_supported(g);
   const bool band = use_band_tcc(ctx, ks, batch);
   ImgPlan p = tc ? mixed_plan(g, batch, ctx->sm_count) : make_plan(g, batch, ctx->sm_count);
+  if (!tc) win_fold_plan(p, ctx->sm_count);
   if (band) {
     p.ngroups = ks->band_nc;
     p.kpg = g.nk;

@@ -1,0 +1,576 @@
+// The two FP32 transforms of the plain imaging form, folded four rows at a time (fold.hpp).
+//
+//   win_fold_kernel  W[v][u] = 1/(FxFy) sum_{y,x} m[y][x] e^{-2 pi i (u x'/Fx + v y'/Fy)}:
+//                    the row sums first (over y, per mask column), each base row's four mask
+//                    rows folded by eight additions into the operands of the even/odd cos and
+//                    sin sums; then the short column sums of a CTA's columns.
+//   fi_fold_kernel   image[Y][X] = T0 + sum_r 2 Re(e^{2 pi i r y'/Fy} T_r[X]): the even/odd cos
+//                    and sin sums of a base row give four image rows by eight additions.
+//
+// Every sum stays in FP32 on the CUDA cores.  Per pixel the window takes (2Ny+1)/4 FMAs and two
+// additions and the image (4Ny+1)/4 and two, a quarter of the unfolded contractions (which were
+// bound by the FP32 pipe and by shared-memory reads), so up to Ny = 8 the 4 bytes per pixel of
+// HBM bound both: 1024 masks of 1024^2 (4 GiB each way) measured 1172 -> 639 us (6.7 TB/s) for the
+// window and 1299 -> 639 us for the image, 40 grey masks of 777 x 913 (rows at any alignment)
+// 90 -> 44 and 51 -> 35 us.  At Ny = 16 the FMAs bound the image (44 of 2048^2: 195 us, 3.8 TB/s).
+// Scalar FMAs: packed (f32x2) ones gave no higher rate here and cost register moves.
+#include "litho_internal.cuh"
+#include "fold.hpp"
+#include "tc_common.cuh"
+
+#include <algorithm>
+
+namespace litho {
+
+// element offsets of a base row's four rows, -1 where a row is outside
+__device__ __forceinline__ int4 fold_offsets(int b, int Lx, int Ly, int Fy) {
+  int o[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const FoldRange fr = fold_range(k, Ly, Fy);
+    o[k] = (unsigned)(b - fr.lo) < (unsigned)fr.n ? fold_y(b, k, Ly, Fy) * Lx : -1;
+  }
+  return make_int4(o[0], o[1], o[2], o[3]);
+}
+
+// ---------------------------------------------------------------------------
+// window DFT
+// ---------------------------------------------------------------------------
+// Template support: 2NY+1 sums per column.  Four columns per lane up to NY = 8 (68 accumulator
+// registers); two above (NY = 16: 66).
+constexpr int wf_cpl(int NY) { return NY <= 8 ? 4 : 2; }
+constexpr int wf_stride(int NY) { return 2 * NY; }
+constexpr int WF_WARPS = 8, WF_THREADS = 32 * WF_WARPS;
+constexpr int WF_ST = 4;  // ring stages: three base rows (6 KB) of every warp in flight
+constexpr int WF_AHEAD = (WF_ST - 1) * WF_WARPS;
+// base rows whose coefficients and row offsets are staged at a time
+constexpr int wf_stage(int NY) { return 40 * 1024 / (wf_stride(NY) * 4 + 16) / WF_WARPS * WF_WARPS; }
+
+static int wf_ny(int Ny) { return Ny <= 2 ? 2 : Ny <= 4 ? 4 : Ny <= 8 ? 8 : Ny <= 12 ? 12 : Ny <= 16 ? 16 : -1; }
+
+// coef[b][.]: cos(n t) for n = 1..NY, then sin(n t), t = 2 pi b/Fy; zero past Ny
+__global__ void wf_coef_kernel(float* __restrict__ coef, int nb, int NY, int Ny, int Fy) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x, e = blockIdx.y, n = e % NY + 1;
+  if (b >= nb) return;
+  float c = 0.f, s = 0.f;
+  if (n <= Ny) cis_round((long long)n * b, Fy, &c, &s);
+  coef[(size_t)b * wf_stride(NY) + e] = e < NY ? c : s;
+}
+
+template <int NY>
+struct WinFold {
+  static constexpr int CPL = wf_cpl(NY), COLS = 32 * CPL, KS = wf_stride(NY), NR = 2 * NY + 1;
+  static constexpr int RB = COLS + 4;       // ring row (floats): the columns and one granule of misalignment
+  static constexpr int RING = WF_WARPS * WF_ST * 4 * RB;
+  static constexpr int RS = COLS + 4;       // row stride of the summed row sums (floats)
+  static constexpr int TS = COLS + 2;       // row stride of the column twiddles (float2)
+  static constexpr int ZERO = RB + 4;       // a row of zeros, padded to 16 bytes
+  static constexpr int RED = WF_WARPS * NR * COLS;  // floats of the warps' sums
+  static constexpr int BARS = WF_WARPS * WF_ST * 2;  // floats of the ring's barriers
+};
+
+template <int NY>
+static size_t win_fold_smem(int Nx, int rows) {
+  using P = WinFold<NY>;
+  const size_t tw = (size_t)(Nx + 1) * P::TS * 2;
+  const int st = std::min(rows, wf_stage(NY));
+  const size_t loop = (size_t)P::RING + (size_t)(st + WF_AHEAD) * 4 + (size_t)st * P::KS;
+  const size_t sums = (size_t)P::RED + (size_t)P::NR * P::RS;
+  return (P::BARS + P::ZERO + tw + std::max(loop, sums)) * sizeof(float);
+}
+
+template <int BYTES>
+__device__ __forceinline__ void wf_copy_lane(float* dst, const void* src, bool ok) {  // zeros where !ok
+  const unsigned d = tc::smem_u32(dst);
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+}
+// bulk copy global -> shared (16-byte aligned, whole 16 bytes), counted on an mbarrier
+__device__ __forceinline__ void wf_copy(float* dst, const void* src, int bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   tc::smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
+               : "memory");
+}
+
+// One CTA per (column block of 32 CPL columns, share of the base rows, image).  Row sums
+// C_n = sum_y m cos(2 pi n y'/Fy), S_n = sum_y m sin of every column: warp w takes the base rows
+// b0 + w, b0 + w + 8, ..; their four mask rows stream through the warp's own ring (rows and columns
+// outside the mask as zeros), a lane folds its CPL columns and adds them into its 2NY+1 sums with
+// one broadcast load per four coefficients.  The warps' sums are then added in order and summed
+// over the columns with the column twiddles.
+// VEC (rows 16-byte aligned): every lane copies its own neighbouring columns with cp.async and
+// reads them back.  Otherwise lanes 0-3 issue a bulk copy of one row each, the ring holds whole
+// 16-byte granules and the lanes read their columns (lane + 32 i) past each row's misalignment;
+// every wait is bounded: a warp whose copies do not land in a second sets *err, waits for what it
+// has in flight and goes on without them.  (Measured, window stage: 256 aligned masks of 1024^2
+// 198 us with cp.async, 206 with bulk copies; 44 of 2048^2 184 and 231; 40 ragged 913 x 777 masks
+// 54 and 49, and 138 with plain loads.)
+template <int NY, bool VEC>
+__global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
+    const float* __restrict__ masks, int Lx, int Ly, int Fx, int Fy, int Nx, int Ny, const float* __restrict__ coef,
+    int nb, const float2* __restrict__ twF, float2* __restrict__ win_part, int part_stride, int* err) {
+  using P = WinFold<NY>;
+  constexpr int CPL = P::CPL, COLS = P::COLS, KS = P::KS;
+  extern __shared__ __align__(16) float sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm) + warp * WF_ST;
+  float* zero = sm + P::BARS;
+  float2* sTw = reinterpret_cast<float2*>(zero + P::ZERO);    // [Nx+1][TS]
+  float* sK = zero + P::ZERO + 2 * (Nx + 1) * P::TS;          // ring, row offsets, coefficients; then the warps' sums
+  int4* sOff = reinterpret_cast<int4*>(sK + P::RING);         // [rows + WF_AHEAD]
+  const int srows = min((nb + (int)gridDim.y - 1) / (int)gridDim.y, wf_stage(NY));
+  float* sCoef = sK + P::RING + 4 * (srows + WF_AHEAD);       // [rows][KS]
+  float* ring = sK + warp * (WF_ST * 4 * P::RB);
+  const int cb = blockIdx.x, rs = blockIdx.y, img = blockIdx.z;
+  const int X0 = cb * COLS, ncol = min(COLS, Lx - X0);
+  const int b0 = (int)((long long)nb * rs / gridDim.y), b1 = (int)((long long)nb * (rs + 1) / gridDim.y);
+  const float* M = masks + (size_t)img * Lx * Ly + X0;
+  const int base4 = (int)((reinterpret_cast<uintptr_t>(M) >> 2) & 3);  // misalignment of row 0 (floats)
+
+  auto issue_vec = [&](int4 o4, int st) {  // the rows at offsets o4 (-1: none) into ring stage st
+    const int off[4] = {o4.x, o4.y, o4.z, o4.w};
+    float* dst = ring + st * (4 * P::RB) + CPL * lane;
+    const bool in = CPL * lane < ncol;
+    const float* base = M + (in ? CPL * lane : 0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      wf_copy_lane<4 * CPL>(dst + k * P::RB, base + (off[k] >= 0 ? off[k] : 0), off[k] >= 0 && in);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto issue = [&](int off, int st) {  // lanes 0-3: the row at offset off (-1: none) into ring stage st
+    if (lane >= 4) return;
+    int bytes = off >= 0 ? 4 * ncol : 0;
+    const float* row = M + off;
+    if (bytes) {  // the granules the row touches
+      const uintptr_t g = reinterpret_cast<uintptr_t>(row) & ~uintptr_t(15);
+      bytes = (int)(((reinterpret_cast<uintptr_t>(row + ncol) + 15) & ~uintptr_t(15)) - g);
+      row = reinterpret_cast<const float*>(g);
+    }
+    tc::mbar_arrive_expect_tx(&bar[st], bytes);
+    if (bytes) wf_copy(ring + (st * 4 + lane) * P::RB, row, bytes, &bar[st]);
+  };
+  auto offset_of = [&](int b) {  // this lane's row of base row b
+    int off = -1;
+    if (lane < 4 && b < b1) {
+      const FoldRange fr = fold_range(lane, Ly, Fy);
+      if ((unsigned)(b - fr.lo) < (unsigned)fr.n) off = fold_y(b, lane, Ly, Fy) * Lx;
+    }
+    return off;
+  };
+
+  float c[NY + 1][CPL], s[NY][CPL];  // cos sums n = 0..NY, sin sums n = 1..NY
+#pragma unroll
+  for (int i = 0; i < CPL; ++i) {
+#pragma unroll
+    for (int n = 0; n <= NY; ++n) c[n][i] = 0.f;
+#pragma unroll
+    for (int n = 0; n < NY; ++n) s[n][i] = 0.f;
+  }
+  int b = b0 + warp;
+  if constexpr (VEC) {
+#pragma unroll
+    for (int k = 0; k < WF_ST - 1; ++k) {
+      const int bk = b + k * WF_WARPS;
+      issue_vec(bk < b1 ? fold_offsets(bk, Lx, Ly, Fy) : make_int4(-1, -1, -1, -1), k);
+    }
+  } else {
+    if (lane == 0) {
+      for (int i = 0; i < WF_ST; ++i) tc::mbar_init(&bar[i], 4);  // one arrival per row
+      tc::fence_mbar_init();
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < WF_ST - 1; ++k) issue(offset_of(b + k * WF_WARPS), k);
+    for (int e = tid; e < P::ZERO; e += WF_THREADS) zero[e] = 0.f;
+  }
+  for (int e = tid; e < (Nx + 1) * COLS; e += WF_THREADS) {
+    const int u = e / COLS, x = e - u * COLS;
+    sTw[u * P::TS + x] = x < ncol ? __ldg(twF + (size_t)u * Lx + X0 + x) : make_float2(0.f, 0.f);
+  }
+  int st = 0;
+  uint32_t ph = 0;
+  bool ok = true;
+  for (int t0 = b0; t0 < b1; t0 += wf_stage(NY)) {  // one stage up to 2,000 rows at NY = 8
+    const int t1 = min(b1, t0 + wf_stage(NY));
+    if (t0 > b0) __syncthreads();
+    const float4* src = reinterpret_cast<const float4*>(coef + (size_t)t0 * KS);
+    for (int e = tid; e < (t1 - t0) * (KS / 4); e += WF_THREADS) reinterpret_cast<float4*>(sCoef)[e] = __ldg(src + e);
+    for (int e = tid; e < t1 - t0 + WF_AHEAD; e += WF_THREADS)
+      sOff[e] = t0 + e < b1 ? fold_offsets(t0 + e, Lx, Ly, Fy) : make_int4(-1, -1, -1, -1);
+    __syncthreads();
+    for (; b < t1; b += WF_WARPS) {
+      float p[4][CPL];
+      const float* src = ring + st * (4 * P::RB);
+      if constexpr (VEC) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(WF_ST - 2) : "memory");
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if constexpr (CPL == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(src + k * P::RB + 4 * lane);
+            p[k][0] = v.x;
+            p[k][1] = v.y;
+            p[k][2] = v.z;
+            p[k][3] = v.w;
+          } else {
+            const float2 v = *reinterpret_cast<const float2*>(src + k * P::RB + 2 * lane);
+            p[k][0] = v.x;
+            p[k][1] = v.y;
+          }
+        }
+        issue_vec(sOff[b - t0 + WF_AHEAD], st == 0 ? WF_ST - 1 : st - 1);  // the previous row's slot
+      } else {
+        const int4 o4 = sOff[b - t0];
+        const int off[4] = {o4.x, o4.y, o4.z, o4.w};
+        if (!tc::mbar_wait(&bar[st], ph, ok ? 1000u : 0u)) ok = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float* q = off[k] >= 0 ? src + k * P::RB + ((base4 + off[k]) & 3) : zero;
+#pragma unroll
+          for (int i = 0; i < CPL; ++i) p[k][i] = lane + 32 * i < ncol ? q[lane + 32 * i] : 0.f;
+        }
+        __syncwarp();  // the slot refilled below (the previous row's) has been read by every lane
+        issue(lane < 4 ? reinterpret_cast<const int*>(sOff + (b - t0 + WF_AHEAD))[lane] : -1,
+              st == 0 ? WF_ST - 1 : st - 1);
+      }
+      if (++st == WF_ST) {
+        st = 0;
+        ph ^= 1;
+      }
+      float ce[CPL], co[CPL], se[CPL], so[CPL];  // operands of the even and odd cos sums and sin sums
+#pragma unroll
+      for (int i = 0; i < CPL; ++i) {
+        const float a = p[0][i] + p[1][i], e = p[2][i] + p[3][i], d = p[0][i] - p[1][i], f = p[2][i] - p[3][i];
+        ce[i] = a + e;
+        co[i] = a - e;
+        se[i] = d - f;
+        so[i] = d + f;
+        c[0][i] += ce[i];
+      }
+      const float4* k4 = reinterpret_cast<const float4*>(sCoef + (size_t)(b - t0) * KS);
+#pragma unroll
+      for (int q = 0; q < KS / 4; ++q) {
+        const float4 kv = k4[q];
+        const float kk[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const int e = 4 * q + h;  // cos 1..NY, sin 1..NY
+#pragma unroll
+          for (int i = 0; i < CPL; ++i) {
+            if (e < NY) c[e < NY ? e + 1 : 0][i] = fmaf(kk[h], (e & 1) ? ce[i] : co[i], c[e < NY ? e + 1 : 0][i]);
+            else s[e < NY ? 0 : e - NY][i] = fmaf(kk[h], ((e - NY) & 1) ? se[i] : so[i], s[e < NY ? 0 : e - NY][i]);
+          }
+        }
+      }
+    }
+  }
+  // the ring's memory is reused: what was issued past the last row (nothing copied) completes too
+  if constexpr (VEC) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  } else {
+    for (int k = 0; k < WF_ST - 1; ++k) {
+      if (!tc::mbar_wait(&bar[st], ph, ok ? 1000u : 200u)) ok = false;
+      if (++st == WF_ST) {
+        st = 0;
+        ph ^= 1;
+      }
+    }
+    if (!ok && lane == 0) atomicExch(err, 1);
+  }
+  __syncthreads();  // ring, offsets and coefficients are read: their memory takes the warps' sums
+  float* red = sK;                 // [warps][NR][COLS]
+  float* sC = sK + P::RED;         // [NR][RS]: cos 0..NY, sin 1..NY
+  {
+    float* r = red + (size_t)warp * P::NR * COLS;
+    auto put = [&](int n, const float(&v)[CPL]) {
+      if constexpr (VEC && CPL == 4) {
+        reinterpret_cast<float4*>(r + n * COLS)[lane] = make_float4(v[0], v[1], v[2], v[3]);
+      } else if constexpr (VEC) {
+        reinterpret_cast<float2*>(r + n * COLS)[lane] = make_float2(v[0], v[1]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < CPL; ++i) r[n * COLS + lane + 32 * i] = v[i];
+      }
+    };
+#pragma unroll
+    for (int n = 0; n <= NY; ++n) put(n, c[n]);
+#pragma unroll
+    for (int n = 1; n <= NY; ++n) put(NY + n, s[n - 1]);
+  }
+  __syncthreads();
+  for (int e = tid; e < P::NR * (COLS / 4); e += WF_THREADS) {  // the warps' sums in order
+    const int j = e / (COLS / 4), x = 4 * (e - j * (COLS / 4));
+    float4 t = *reinterpret_cast<const float4*>(red + j * COLS + x);
+#pragma unroll
+    for (int w = 1; w < WF_WARPS; ++w) {
+      const float4 a = *reinterpret_cast<const float4*>(red + (size_t)w * P::NR * COLS + j * COLS + x);
+      t.x += a.x;
+      t.y += a.y;
+      t.z += a.z;
+      t.w += a.w;
+    }
+    *reinterpret_cast<float4*>(sC + j * P::RS + x) = t;
+  }
+  __syncthreads();
+  // Column sums, with C, S the cos and sin row sums of v:
+  //   W[v][u] = sum_x (C - iS)(cos - i sin),  W[-v][u] = sum_x (C + iS)(cos - i sin).
+  // A thread takes v, three u and every Q-th four columns (neighbouring threads neighbouring
+  // columns), so that a loaded C and S serve three u.
+  constexpr int UT = 3;
+  const int KY = 2 * Ny + 1, NU = Nx + 1, UG = (NU + UT - 1) / UT, NP = (Ny + 1) * UG;
+  int Q = 8;
+  while (Q > 1 && NP * Q > WF_THREADS) Q >>= 1;
+  const float scale = 1.0f / ((float)Fx * (float)Fy);
+  const int nps = part_stride > 0 ? part_stride : gridDim.x * gridDim.y;
+  float2* out = win_part + ((size_t)img * nps + (size_t)rs * gridDim.x + cb) * KY * NU;
+  for (int base = 0; base < NP * Q; base += WF_THREADS) {  // uniform bound: whole warps shuffle
+    const int t = base + tid, q = t % Q, pr = min(t / Q, NP - 1), v = pr / UG, u0 = (pr - v * UG) * UT;
+    const float* C = sC + v * P::RS;
+    const float* S = sC + (NY + v) * P::RS;  // v = 0: any row, times zero
+    float A[UT], B[UT], D[UT], E[UT];
+#pragma unroll
+    for (int i = 0; i < UT; ++i) A[i] = B[i] = D[i] = E[i] = 0.f;
+    for (int x = 4 * q; x < COLS; x += 4 * Q) {
+      const float4 c4 = *reinterpret_cast<const float4*>(C + x);
+      float4 s4 = *reinterpret_cast<const float4*>(S + x);
+      if (v == 0) s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < UT; ++i) {
+        const float4* T = reinterpret_cast<const float4*>(sTw + min(u0 + i, Nx) * P::TS + x);
+        const float4 ta = T[0], tb = T[1];
+        A[i] = fmaf(c4.w, tb.z, fmaf(c4.z, tb.x, fmaf(c4.y, ta.z, fmaf(c4.x, ta.x, A[i]))));
+        B[i] = fmaf(c4.w, tb.w, fmaf(c4.z, tb.y, fmaf(c4.y, ta.w, fmaf(c4.x, ta.y, B[i]))));
+        D[i] = fmaf(s4.w, tb.z, fmaf(s4.z, tb.x, fmaf(s4.y, ta.z, fmaf(s4.x, ta.x, D[i]))));
+        E[i] = fmaf(s4.w, tb.w, fmaf(s4.z, tb.y, fmaf(s4.y, ta.w, fmaf(s4.x, ta.y, E[i]))));
+      }
+    }
+    for (int o = Q / 2; o > 0; o >>= 1) {
+#pragma unroll
+      for (int i = 0; i < UT; ++i) {
+        A[i] += __shfl_xor_sync(0xffffffffu, A[i], o);
+        B[i] += __shfl_xor_sync(0xffffffffu, B[i], o);
+        D[i] += __shfl_xor_sync(0xffffffffu, D[i], o);
+        E[i] += __shfl_xor_sync(0xffffffffu, E[i], o);
+      }
+    }
+    if (q == 0 && t < NP * Q) {
+#pragma unroll
+      for (int i = 0; i < UT; ++i) {
+        if (u0 + i > Nx) continue;
+        out[(Ny + v) * NU + u0 + i] = make_float2((A[i] - E[i]) * scale, -(B[i] + D[i]) * scale);
+        if (v > 0) out[(Ny - v) * NU + u0 + i] = make_float2((A[i] + E[i]) * scale, (D[i] - B[i]) * scale);
+      }
+    }
+  }
+}
+
+// column blocks and row splits of a plain window DFT: every split is one more partial per column
+// block and one more start and end of a CTA, so only as many as give each SM two waves of its two
+// CTAs (64 masks of 1024^2: 76 us, and 96 / 135 us with 16 / 28 CTAs per SM asked for)
+void win_fold_plan(ImgPlan& p, int sm_count) {
+  const int cols = 32 * wf_cpl(wf_ny(p.g.Ny));
+  p.rowBlocks = (p.g.Lx + cols - 1) / cols;
+  const long long want = 4LL * sm_count, units = (long long)p.rowBlocks * p.batch;
+  const int most = win_fold_max_splits(p.g);
+  p.colSplits = (int)std::max(1LL, std::min<long long>(most, (want + units - 1) / units));
+}
+// every warp of a CTA keeps at least one base row
+int win_fold_max_splits(const ImgGeom& g) { return std::max(1, fold_nbase(g.Ly, g.Fy) / WF_WARPS); }
+
+size_t win_fold_coef_floats(const ImgGeom& g) { return (size_t)fold_nbase(g.Ly, g.Fy) * wf_stride(wf_ny(g.Ny)); }
+
+cudaError_t win_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef) {
+  const int nb = fold_nbase(g.Ly, g.Fy), NY = wf_ny(g.Ny);
+  wf_coef_kernel<<<dim3((nb + 127) / 128, wf_stride(NY)), 128, 0, s>>>(coef, nb, NY, g.Ny, g.Fy);
+  return cudaGetLastError();
+}
+
+template <int NY>
+static cudaError_t launch_win_fold_t(cudaStream_t s, const ImgPlan& p, const float* masks, const float* coef,
+                                     const float2* twF, float2* win_part, int* err) {
+  const ImgGeom& g = p.g;
+  const int nb = fold_nbase(g.Ly, g.Fy), rows = (nb + p.colSplits - 1) / p.colSplits;
+  const size_t smem = win_fold_smem<NY>(g.Nx, rows);
+  const bool vec = (g.Lx & 3) == 0 && (reinterpret_cast<uintptr_t>(masks) & 15) == 0;
+  auto k = vec ? win_fold_kernel<NY, true> : win_fold_kernel<NY, false>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k<<<dim3(p.rowBlocks, p.colSplits, p.batch), WF_THREADS, smem, s>>>(masks, g.Lx, g.Ly, g.Fx, g.Fy, g.Nx, g.Ny, coef,
+                                                                     nb, twF, win_part, p.part_stride, err);
+  return cudaGetLastError();
+}
+
+// coef from win_fold_coefs, twF the column twiddles of fi_twiddles, err the timeout flag
+cudaError_t launch_win_fold(cudaStream_t s, const ImgPlan& p, const float* masks, const float* coef,
+                            const float2* twF, float2* win_part, int* err) {
+  switch (wf_ny(p.g.Ny)) {
+    case 2: return launch_win_fold_t<2>(s, p, masks, coef, twF, win_part, err);
+    case 4: return launch_win_fold_t<4>(s, p, masks, coef, twF, win_part, err);
+    case 8: return launch_win_fold_t<8>(s, p, masks, coef, twF, win_part, err);
+    case 12: return launch_win_fold_t<12>(s, p, masks, coef, twF, win_part, err);
+    default: return launch_win_fold_t<16>(s, p, masks, coef, twF, win_part, err);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// interpolation output
+// ---------------------------------------------------------------------------
+constexpr int FF_WARPS = 4, FF_THREADS = 32 * FF_WARPS;
+constexpr int ff_cpl(int NY) { return NY <= 8 ? 4 : 2; }
+constexpr int ff_stride(int NY) { return 4 * NY; }
+constexpr int ff_stage(int NY) { return 44 * 1024 / (ff_stride(NY) * 4 + 16) / FF_WARPS * FF_WARPS; }
+
+// coef[b][.]: 2cos(r t) for r = 1..2NY, then -2sin(r t), t = 2 pi b/Fy; zero past 2Ny
+__global__ void ff_coef_kernel(float* __restrict__ coef, int nb, int NY, int Ny, int Fy) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x, e = blockIdx.y, r = e % (2 * NY) + 1;
+  if (b >= nb) return;
+  float c = 0.f, s = 0.f;
+  if (r <= 2 * Ny) cis_round((long long)r * b, Fy, &c, &s);
+  coef[(size_t)b * ff_stride(NY) + e] = e < 2 * NY ? 2.f * c : -2.f * s;
+}
+
+// One CTA per (column block, share of the base rows, image): its four warps take turns at the base
+// rows, each lane with its columns of Tm in registers for all of them (CPL columns: 132 registers
+// at NY = 8, so three CTAs of four warps per SM), so that a base row costs one broadcast load per
+// four coefficients and the stores.  A tile of Tm in shared memory instead (4 x 4 outputs per
+// thread) was bound by its reads.
+template <int NY, bool VEC>
+__global__ void __launch_bounds__(FF_THREADS, 3) fi_fold_kernel(const float* __restrict__ tm, int Lx, int Ly, int Fy,
+                                                                int Ny, const float* __restrict__ coef, int nb,
+                                                                float* __restrict__ images) {
+  constexpr int CPL = ff_cpl(NY), COLS = 32 * CPL, KS = ff_stride(NY);
+  extern __shared__ __align__(16) float sK[];  // [rows][KS] coefficients, then [rows] row offsets
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int X0 = blockIdx.x * COLS, img = blockIdx.z;
+  const int b0 = (int)((long long)nb * blockIdx.y / gridDim.y), b1 = (int)((long long)nb * (blockIdx.y + 1) / gridDim.y);
+  const int xl = VEC ? X0 + CPL * lane : X0 + lane;
+  const float* T = tm + (size_t)img * (4 * Ny + 1) * Lx + xl;
+  float tc[2 * NY + 1][CPL], ts[2 * NY][CPL];  // the lane's columns of Tm: cos rows 0..2NY, sin rows 1..2NY
+  auto row = [&](int r, bool ok, float(&v)[CPL]) {
+    const float* p = T + (size_t)(ok ? r : 0) * Lx;
+    if constexpr (VEC && CPL == 4) {
+      float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (ok && xl < Lx) q = __ldg(reinterpret_cast<const float4*>(p));
+      v[0] = q.x;
+      v[1] = q.y;
+      v[2] = q.z;
+      v[3] = q.w;
+    } else if constexpr (VEC) {
+      float2 q = make_float2(0.f, 0.f);
+      if (ok && xl < Lx) q = __ldg(reinterpret_cast<const float2*>(p));
+      v[0] = q.x;
+      v[1] = q.y;
+    } else {
+#pragma unroll
+      for (int i = 0; i < CPL; ++i) v[i] = ok && xl + 32 * i < Lx ? __ldg(p + 32 * i) : 0.f;
+    }
+  };
+#pragma unroll
+  for (int r = 0; r <= 2 * NY; ++r) row(r, r <= 2 * Ny, tc[r]);
+#pragma unroll
+  for (int r = 1; r <= 2 * NY; ++r) row(2 * Ny + r, r <= 2 * Ny, ts[r - 1]);
+  const int srows = min((nb + (int)gridDim.y - 1) / (int)gridDim.y, ff_stage(NY));
+  int4* sOff = reinterpret_cast<int4*>(sK + srows * KS);
+  float* O = images + (size_t)img * Lx * Ly + xl;
+  for (int t0 = b0; t0 < b1; t0 += ff_stage(NY)) {  // one stage up to 1,200 rows at NY = 8
+    const int t1 = min(b1, t0 + ff_stage(NY));
+    if (t0 > b0) __syncthreads();
+    const float4* src = reinterpret_cast<const float4*>(coef + (size_t)t0 * KS);
+    for (int e = tid; e < (t1 - t0) * (KS / 4); e += FF_THREADS) reinterpret_cast<float4*>(sK)[e] = __ldg(src + e);
+    for (int e = tid; e < t1 - t0; e += FF_THREADS) sOff[e] = fold_offsets(t0 + e, Lx, Ly, Fy);
+    __syncthreads();
+    for (int b = t0 + warp; b < t1; b += FF_WARPS) {
+      const float4* k4 = reinterpret_cast<const float4*>(sK + (size_t)(b - t0) * KS);
+      float ae[CPL], ao[CPL], be[CPL], bo[CPL];  // even and odd cos sums and sin sums
+#pragma unroll
+      for (int i = 0; i < CPL; ++i) {
+        ae[i] = tc[0][i];
+        ao[i] = be[i] = bo[i] = 0.f;
+      }
+#pragma unroll
+      for (int q = 0; q < KS / 4; ++q) {
+        const float4 kv = k4[q];
+        const float kk[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const int e = 4 * q + h;  // cos 1..2NY, sin 1..2NY
+#pragma unroll
+          for (int i = 0; i < CPL; ++i) {
+            if (e < 2 * NY) {
+              if (e & 1) ae[i] = fmaf(kk[h], tc[e < 2 * NY ? e + 1 : 0][i], ae[i]);
+              else ao[i] = fmaf(kk[h], tc[e < 2 * NY ? e + 1 : 0][i], ao[i]);
+            } else {
+              if (e & 1) be[i] = fmaf(kk[h], ts[e < 2 * NY ? 0 : e - 2 * NY][i], be[i]);
+              else bo[i] = fmaf(kk[h], ts[e < 2 * NY ? 0 : e - 2 * NY][i], bo[i]);
+            }
+          }
+        }
+      }
+      float o[4][CPL];
+#pragma unroll
+      for (int i = 0; i < CPL; ++i) {
+        const float u = ae[i] + ao[i], w = ae[i] - ao[i], s = be[i] + bo[i], t = be[i] - bo[i];
+        o[0][i] = u + s;
+        o[1][i] = u - s;
+        o[2][i] = w - t;
+        o[3][i] = w + t;
+      }
+      const int4 o4 = sOff[b - t0];
+      const int off[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float* dst = O + off[k];
+        if constexpr (VEC && CPL == 4) {
+          if (off[k] >= 0 && xl < Lx) __stcs(reinterpret_cast<float4*>(dst), make_float4(o[k][0], o[k][1], o[k][2], o[k][3]));
+        } else if constexpr (VEC) {
+          if (off[k] >= 0 && xl < Lx) __stcs(reinterpret_cast<float2*>(dst), make_float2(o[k][0], o[k][1]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < CPL; ++i)
+            if (off[k] >= 0 && xl + 32 * i < Lx) __stcs(dst + 32 * i, o[k][i]);
+        }
+      }
+    }
+  }
+}
+
+size_t fi_fold_coef_floats(const ImgGeom& g) { return (size_t)fold_nbase(g.Ly, g.Fy) * ff_stride(wf_ny(g.Ny)); }
+
+cudaError_t fi_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef) {
+  const int nb = fold_nbase(g.Ly, g.Fy), NY = wf_ny(g.Ny);
+  ff_coef_kernel<<<dim3((nb + 127) / 128, ff_stride(NY)), 128, 0, s>>>(coef, nb, NY, g.Ny, g.Fy);
+  return cudaGetLastError();
+}
+
+template <int NY>
+static cudaError_t launch_fi_fold_t(cudaStream_t s, const ImgPlan& p, const float* tm, const float* coef,
+                                    float* images) {
+  const ImgGeom& g = p.g;
+  const int nb = fold_nbase(g.Ly, g.Fy), cols = 32 * ff_cpl(NY), ncb = (g.Lx + cols - 1) / cols;
+  // every CTA loads its columns of Tm once: row splits only until there are
+  // four waves of three CTAs per SM (64 masks of 1024^2: 47.5 us; 53 / 68 / 94 us with twice, four and eight times as many)
+  const int sms = p.sms > 0 ? p.sms : 148;
+  const long long want = 12LL * sms, units = (long long)ncb * p.batch;
+  const int R = (int)std::max(1LL, std::min<long long>(std::max(1, nb / FF_WARPS), (want + units - 1) / units));
+  const size_t smem = (size_t)std::min((nb + R - 1) / R, ff_stage(NY)) * (ff_stride(NY) * sizeof(float) + sizeof(int4));
+  const bool vec = (g.Lx & 3) == 0 && ((reinterpret_cast<uintptr_t>(tm) | reinterpret_cast<uintptr_t>(images)) & 15) == 0;
+  auto k = vec ? fi_fold_kernel<NY, true> : fi_fold_kernel<NY, false>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k<<<dim3(ncb, R, p.batch), FF_THREADS, smem, s>>>(tm, g.Lx, g.Ly, g.Fy, g.Ny, coef, nb, images);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fi_fold(cudaStream_t s, const ImgPlan& p, const float* tm, const float* coef, float* images) {
+  switch (wf_ny(p.g.Ny)) {
+    case 2: return launch_fi_fold_t<2>(s, p, tm, coef, images);
+    case 4: return launch_fi_fold_t<4>(s, p, tm, coef, images);
+    case 8: return launch_fi_fold_t<8>(s, p, tm, coef, images);
+    case 12: return launch_fi_fold_t<12>(s, p, tm, coef, images);
+    default: return launch_fi_fold_t<16>(s, p, tm, coef, images);
+  }
+}
+
+}  // namespace litho

@@ -88,6 +88,14 @@ __device__ __forceinline__ float2 sum_strided(const float2* __restrict__ p, size
                      ((a[0].y + a[1].y) + (a[2].y + a[3].y)) + ((a[4].y + a[5].y) + (a[6].y + a[7].y)));
 }
 
+// cos and sin of 2 pi m / F (F a power of two) for an exact integer m, rounded once
+__device__ __forceinline__ void cis_round(long long m, int F, float* c, float* s) {
+  double sd, cd;
+  sincospi(2.0 * (double)(m & (long long)(F - 1)) / (double)F, &sd, &cd);
+  *c = (float)cd;
+  *s = (float)sd;
+}
+
 // Autotuned shape of the split-BF16 TCC GEMM for one (n, Kp): column tile width, K
 // slice, schedule (gemm_schedule's sched) and every candidate's measured time.
 struct TccTune {
@@ -126,7 +134,7 @@ struct litho_ctx {
   int band_method = 0;
   // mask bytes per chunk of the host-buffer path (litho_ctx_set_host_chunk); 0: default
   size_t host_chunk_bytes = 0;
-  // window-DFT column twiddle tables keyed by (Lx, Fx, Nx, NJT)
+  // twiddle and coefficient tables keyed by (L, F, N, kind)
   std::map<std::tuple<int, int, int, int>, litho::DevBuf> twx_tables;
   // TCC / eigensolver workspaces
   litho::DevBuf tcc_a, tcc_b, tcc_c, tcc_pq, eig_w, eig_v, eig_work, eig_info;
@@ -190,7 +198,7 @@ struct ImgGeom {
 struct ImgPlan {
   ImgGeom g;
   int batch = 1;
-  int rowBlocks = 1, colSplits = 1;  // window-DFT partition -> nparts
+  int rowBlocks = 1, colSplits = 1;  // window-DFT partition -> nparts (plain: column blocks, row splits)
   int kpg = 1, ngroups = 1;          // SOCS kernels per CTA -> ngroups
   int part_stride = 0;               // >0: window partials per image in a shared per-class array
   int sms = 0;                       // SMs of the device (launch sizing)
@@ -217,13 +225,24 @@ struct WindowSrc {
   const float* mskf_i = nullptr;
 };
 
+// the folded FP32 transforms (imaging_fold.cu): plan fields of a plain window DFT, coefficient
+// tables and launches
+void win_fold_plan(ImgPlan& p, int sm_count);
+int win_fold_max_splits(const ImgGeom& g);
+size_t win_fold_coef_floats(const ImgGeom& g);
+cudaError_t win_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef);
+cudaError_t launch_win_fold(cudaStream_t s, const ImgPlan& p, const float* masks, const float* coef,
+                            const float2* twF, float2* win_part, int* err);
+size_t fi_fold_coef_floats(const ImgGeom& g);
+cudaError_t fi_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef);
+cudaError_t launch_fi_fold(cudaStream_t s, const ImgPlan& p, const float* tm, const float* coef, float* images);
+
 int run_win_dft(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part);
 int prepare_win_dft(litho_ctx* ctx, const ImgPlan& p);  // cached tables, on ctx->stream
 int run_socs(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const float2* krn,
              const float* scales, float2* band_part, float* tmpImgp);
 int run_fi(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tm, float* images);
-// FI step 1 for both layouts (tmh == nullptr: plain tm; else K-major hi/lo + t0);
-// twF == nullptr evaluates the column twiddles in the kernel
+// FI step 1 for both layouts (tmh == nullptr: plain tm; else K-major hi/lo + t0)
 cudaError_t launch_fi_rows(cudaStream_t s, const ImgPlan& p, const float2* band_part, const float2* twF, int KP,
                            float* tm, float* tmh, float* tml, float* t0);
 int fi_twiddles(litho_ctx* ctx, const ImgGeom& g, const float2** out);
@@ -270,5 +289,6 @@ int run_fi_out_tc(litho_ctx* ctx, const ImgPlan& p, const FiTcBufs& b, float* im
 size_t fi_tc_workspace_bytes(const ImgGeom& g, int batch);
 bool tc_supported(const ImgGeom& g);
 int tc_check_flag(litho_ctx* ctx);
+int tc_err_flag_public(litho_ctx* ctx, int** flag);  // the flag of the kernels' bounded waits, made on first use
 
 }  // namespace litho

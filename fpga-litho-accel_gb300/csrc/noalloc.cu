@@ -31,7 +31,7 @@
 
 namespace litho {
 
-size_t noctx_scratch_layout(const ImgPlan& p, size_t off[6]);
+size_t noctx_scratch_layout(const ImgPlan& p, size_t off[8]);
 cudaError_t image_pipeline_noctx(cudaStream_t s, const ImgPlan& p, const float* mask, const float* krn_r,
                                  const float* krn_i, const float* scales, char* scratch, float* image);
 
@@ -79,9 +79,10 @@ extern "C" int litho_image_noalloc(const float* mask, int Lx, int Ly, const floa
   if (cn < 32) cn = 32;
   ImgGeom g{Lx, Ly, Fx, Fy, Nx, Ny, nk, cn};
   ImgPlan p = make_plan(g, 1, sms);
+  win_fold_plan(p, sms);
   while (p.nparts() > NOALLOC_MAX_PARTS && p.colSplits > 1) --p.colSplits;
   if (p.nparts() > NOALLOC_MAX_PARTS) return LITHO_ERR_ARG;
-  size_t off[6];
+  size_t off[8];
   if (noctx_scratch_layout(p, off) > LITHO_NOALLOC_SCRATCH_BYTES) return LITHO_ERR_ARG;
   void* scratch = nullptr;
   if (noalloc_scratch(dev, &scratch) != cudaSuccess) return LITHO_ERR_CUDA;

@@ -217,7 +217,6 @@ int build_pupil(litho_ctx* ctx, const std::vector<SrcPt>& pts, const PupilParams
 
 int tcc_split_bf16(litho_ctx* ctx, const float2* P, const float* J, int n, int ns, int ldp, double2* tcc);
 cudaError_t launch_nonfinite(cudaStream_t s, const double* x, size_t n, int* flag, int sms);
-int tc_err_flag_public(litho_ctx* ctx, int** flag);
 
 }  // namespace litho
 
