@@ -7,15 +7,15 @@
 // createMask convention of common/mask.cpp:31-60: the window DFT only needs the
 // mask's own pixels and its offset in the period); the SOCS and interpolation
 // stages then run once per class over all its images.  Window partials of a
-// class share one array with a common parts stride (unused parts are zeroed at
-// the start of every run).
+// class share one array with a common number of parts per image (the kernel zeroes
+// the parts an image's size does not use).
 //
 // Autotuning (LITHO_BATCH_AUTOTUNE) times, per class, every candidate of
 //   conv grid N in {nextPow2(4N+1), 2x that} (the FFT plan of the SOCS stage),
 //   kernels per CTA in {2, 3, 4, 6, 8, 12} (the SOCS tile), and
-//   window splits (of columns, plain form: of rows) in {1, 2}
+//   window row splits in {r, 2r}, r what the class's tiles take by themselves
 // with CUDA events on the context's stream and keeps the fastest; results are
-// cached on the context by (L, Nx, nk, images, precision).  The plan then
+// cached by (L, Nx, nk, images, precision, band form, r).  The plan then
 // captures the whole sequence in a CUDA graph (LITHO_BATCH_GRAPH).
 #include "litho_internal.cuh"
 
@@ -34,18 +34,19 @@ struct SubBatch {
 struct ClassRun {
   int L = 0;
   const litho_kernel_set* ks = nullptr;
-  int count = 0, maxBlocks = 0;
+  int count = 0, maxBlocks = 0, tiles = 0;  // tiles: of one row split
   float* images = nullptr;
   DevBuf win, band, tmbuf, wsum;
-  int convN = 0, kpg = 1, colSplits = 1, part_stride = 1;  // convN == 0: the TCC band (band_tcc.cu)
+  int convN = 0, kpg = 1, colSplits = 1, splits0 = 1;  // convN == 0: the TCC band (band_tcc.cu)
   double tuned_ms = -1.0;
   int candidates = 0;
 };
 
 struct TuneKey {
-  int L, Nx, nk, count, prec, band;
+  int L, Nx, nk, count, prec, band, splits0;
   bool operator<(const TuneKey& o) const {
-    return std::tie(L, Nx, nk, count, prec, band) < std::tie(o.L, o.Nx, o.nk, o.count, o.prec, o.band);
+    return std::tie(L, Nx, nk, count, prec, band, splits0) <
+           std::tie(o.L, o.Nx, o.nk, o.count, o.prec, o.band, o.splits0);
   }
 };
 struct TuneVal {
@@ -63,10 +64,6 @@ struct litho_batch_plan {
   std::vector<litho::ClassRun> classes;
   std::vector<float*> item_mask, item_image;
   litho::DevBuf mask_pool, image_pool;
-  // the window DFTs of a class's sub-batches run as parallel branches: streams for all
-  // but the largest, a fork event and one join event per branch
-  std::vector<cudaStream_t> wstreams;
-  std::vector<cudaEvent_t> wevents;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -82,75 +79,42 @@ static int default_conv(int Nx, int Ny) {
   return n < 32 ? 32 : n;
 }
 
-// Switch the context's launch stream for a scope (the stage timers follow it).
-struct StreamScope {
-  litho_ctx* ctx;
-  cudaStream_t saved;
-  StreamScope(litho_ctx* c, cudaStream_t s) : ctx(c), saved(c->stream) { c->stream = s; }
-  ~StreamScope() { ctx->stream = saved; }
-};
-
 // enqueue one class on the context's stream: windows of its sub-batches, SOCS,
 // interpolation
 static int run_class(litho_batch_plan* bp, int ci) {
   litho_ctx* ctx = bp->ctx;
   ClassRun& c = bp->classes[ci];
-  const bool tc = bp->precision == LITHO_PREC_MIXED;
-  const int Nx = c.ks->Nx, Ny = c.ks->Ny, KY = 2 * Ny + 1;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(c.win.p, 0, (size_t)c.count * c.part_stride * KY * (Nx + 1) * sizeof(float2),
-                                      ctx->stream));
-  // The sub-batches' window DFTs (one per mask size; each writes its own images'
-  // partials).  Mixed form: one persistent launch over up to WIN_MAX_SIZES mask sizes, so
-  // that the small sizes' few tiles share the SMs with the large ones'.  Plain form:
-  // parallel branches, the largest on the context's stream: all of them stream masks from
-  // HBM, so each fills the others' ramps and tails.
+  const int Nx = c.ks->Nx, Ny = c.ks->Ny;
+  // the sub-batches' window DFTs, up to WIN_MAX_SIZES mask sizes to a launch so that the small
+  // sizes' few tiles share the SMs with the large ones', the largest first
   std::vector<const SubBatch*> sb;
   for (const SubBatch& s : bp->subs)
     if (s.cls == ci) sb.push_back(&s);
   std::stable_sort(sb.begin(), sb.end(), [](const SubBatch* a, const SubBatch* b) {
     return (size_t)a->count * a->mLx * a->mLy > (size_t)b->count * b->mLx * b->mLy;
   });
-  auto win_plan = [&](const SubBatch& s) {
-    ImgGeom gw{s.mLx, s.mLy, c.L, c.L, Nx, Ny, c.ks->nk, c.convN};
-    ImgPlan pw = make_plan(gw, s.count, ctx->sm_count);
-    if (!tc) win_fold_plan(pw, ctx->sm_count);
-    pw.colSplits = std::min(c.colSplits, std::max(1, tc ? (s.mLx + 63) / 64 / 2 : win_fold_max_splits(gw)));
-    pw.part_stride = c.part_stride;
-    return pw;
-  };
-  if (tc) {
-    std::vector<WinPart> parts;
-    for (const SubBatch* s : sb) parts.push_back(WinPart{win_plan(*s), s->masks, s->first_in_class});
-    for (size_t i = 0; i < parts.size(); i += WIN_MAX_SIZES)
-      LITHO_RET(run_win_dft_tc_multi(ctx, parts.data() + i, (int)std::min<size_t>(WIN_MAX_SIZES, parts.size() - i),
-                                     c.win.as<float2>()));
-  } else {
-    if (sb.size() > 1) {
-      // tables shared between sub-batches are built here, before the fork
-      for (const SubBatch* s : sb) LITHO_RET(prepare_win_dft(ctx, win_plan(*s)));
-      LITHO_CUDA_TRY(ctx, cudaEventRecord(bp->wevents[0], ctx->stream));
-      for (size_t k = 1; k < sb.size(); ++k)
-        LITHO_CUDA_TRY(ctx, cudaStreamWaitEvent(bp->wstreams[k - 1], bp->wevents[0], 0));
-    }
-    for (size_t k = 0; k < sb.size(); ++k) {
-      const SubBatch& s = *sb[k];
-      StreamScope scope(ctx, k == 0 ? ctx->stream : bp->wstreams[k - 1]);
-      float2* wp = c.win.as<float2>() + (size_t)s.first_in_class * c.part_stride * KY * (Nx + 1);
-      LITHO_RET(run_win_dft(ctx, win_plan(s), s.masks, wp));
-      if (k > 0) LITHO_CUDA_TRY(ctx, cudaEventRecord(bp->wevents[k], ctx->stream));
-    }
-    for (size_t k = 1; k < sb.size(); ++k) LITHO_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, bp->wevents[k], 0));
+  std::vector<WinPart> parts;
+  int nparts = 1;
+  for (const SubBatch* s : sb) {
+    const ImgGeom gw{s->mLx, s->mLy, c.L, c.L, Nx, Ny, c.ks->nk, c.convN};
+    ImgPlan pw = make_plan(gw, s->count, ctx->sm_count);
+    pw.colSplits = c.colSplits;
+    nparts = std::max(nparts, pw.nparts());
+    parts.push_back(WinPart{pw, s->masks, s->first_in_class});
   }
+  for (size_t i = 0; i < parts.size(); i += WIN_MAX_SIZES)
+    LITHO_RET(run_win_dft(ctx, parts.data() + i, (int)std::min<size_t>(WIN_MAX_SIZES, parts.size() - i),
+                          c.win.as<float2>(), nparts, bp->precision));
   const bool band = c.convN == 0;
   ImgPlan p = make_plan(class_geom(c, band ? default_conv(Nx, Ny) : c.convN), c.count, ctx->sm_count);
   p.kpg = band ? c.ks->nk : std::min(c.kpg, c.ks->nk);
   p.ngroups = band ? c.ks->band_nc : (c.ks->nk + p.kpg - 1) / p.kpg;
   WindowSrc w;
   w.part = c.win.as<float2>();
-  w.nparts = c.part_stride;
+  w.nparts = nparts;
   if (band) LITHO_RET(run_band_tcc(ctx, p, w, c.ks, c.wsum.as<float2>(), c.band.as<float2>()));
   else LITHO_RET(run_socs(ctx, p, w, c.ks->krn, c.ks->scales, c.band.as<float2>(), nullptr));
-  if (tc) return run_fi_tc(ctx, p, c.band.as<float2>(), c.tmbuf.as<float>(), c.images);
+  if (bp->precision == LITHO_PREC_MIXED && fi_tc_serves(p.g)) return run_fi_tc(ctx, p, c.band.as<float2>(), c.tmbuf.as<float>(), c.images);
   return run_fi(ctx, p, c.band.as<float2>(), c.tmbuf.as<float>(), c.images);
 }
 
@@ -192,7 +156,7 @@ static int tune_class(litho_batch_plan* bp, int ci) {
   ClassRun& c = bp->classes[ci];
   const bool band_ok = band_tcc_available(bp->ctx, c.ks);
   const int method = band_ok ? (bp->ctx->band_method == LITHO_BAND_TCC ? 2 : 1) : 0;
-  const TuneKey key{c.L, c.ks->Nx, c.ks->nk, c.count, bp->precision, method};
+  const TuneKey key{c.L, c.ks->Nx, c.ks->nk, c.count, bp->precision, method, c.splits0};
   auto it = g_tune_cache.find(key);
   if (it != g_tune_cache.end()) {
     c.convN = it->second.convN;
@@ -214,7 +178,7 @@ static int tune_class(litho_batch_plan* bp, int ci) {
   for (int k : {2, 3, 4, 6, 8, 12})
     if (k <= c.ks->nk) kpgs.push_back(k);
   if (kpgs.empty()) kpgs.push_back(1);
-  std::vector<int> splits{1, 2};
+  const std::vector<int> splits{c.splits0, 2 * c.splits0};
   // the best candidate of each band form (FFT grids, TCC band) ...
   TuneVal best_fft{convs[0], kpgs[0], 1, 1e30}, best_tcc{0, kpgs[0], 1, 1e30};
   for (int cn : convs)
@@ -321,11 +285,10 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
     ClassRun& c = bp->classes[s.cls];
     s.first_in_class = c.count;
     c.count += s.count;
-    // partials of one split: 128-row blocks (tensor cores) or column blocks (plain)
     const ImgGeom gw{s.mLx, s.mLy, c.L, c.L, c.ks->Nx, c.ks->Ny, c.ks->nk, c.convN};
-    ImgPlan pw = make_plan(gw, s.count, ctx->sm_count);
-    if (precision != LITHO_PREC_MIXED) win_fold_plan(pw, ctx->sm_count);
-    c.maxBlocks = std::max(c.maxBlocks, pw.rowBlocks);
+    const int blocks = make_plan(gw, s.count, ctx->sm_count).rowBlocks;
+    c.maxBlocks = std::max(c.maxBlocks, blocks);
+    c.tiles += blocks * s.count;
   }
   for (auto& c : bp->classes) image_floats += (size_t)c.count * c.L * c.L;
   int rc = bp->mask_pool.ensure(ctx, mask_floats * sizeof(float));
@@ -362,36 +325,17 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
   for (auto& c : bp->classes) {
     if (c.count == 0) continue;
     const int Nx = c.ks->Nx, Ny = c.ks->Ny, KY = 2 * Ny + 1;
-    c.part_stride = c.maxBlocks * 2;  // up to two splits
-    rc = c.win.ensure(ctx, (size_t)c.count * c.part_stride * KY * (Nx + 1) * sizeof(float2));
+    // row splits of the window DFTs: as one launch of the class's tiles would take, or twice as many
+    c.splits0 = win_fold_splits(class_geom(c, c.convN), c.maxBlocks, c.tiles, ctx->sm_count);
+    c.colSplits = c.splits0;
+    rc = c.win.ensure(ctx, (size_t)c.count * c.maxBlocks * 2 * c.splits0 * KY * (Nx + 1) * sizeof(float2));
     const int groups = std::max(c.ks->nk, c.ks->band_nc);  // the FFT form's kernel groups or the band chunks
     if (rc == LITHO_OK) rc = c.band.ensure(ctx, (size_t)c.count * groups * KY * (4 * Nx + 1) * sizeof(float2));
     const ImgGeom g = class_geom(c, c.convN);
     if (rc == LITHO_OK && c.ks->band_nc > 0) rc = c.wsum.ensure(ctx, band_wsum_bytes(g, c.count));
-    const size_t tmb = precision == LITHO_PREC_MIXED ? fi_tc_workspace_bytes(g, c.count)
+    const size_t tmb = precision == LITHO_PREC_MIXED && fi_tc_serves(g) ? fi_tc_workspace_bytes(g, c.count)
                                                      : (size_t)c.count * (4 * Ny + 1) * c.L * sizeof(float);
     if (rc == LITHO_OK) rc = c.tmbuf.ensure(ctx, tmb);
-    if (rc != LITHO_OK) {
-      litho_batch_plan_destroy(bp);
-      return rc;
-    }
-  }
-  // branch streams and events for the sub-batches' window DFTs (as many as the largest
-  // class has sub-batches)
-  {
-    std::vector<int> per(nsets, 0);
-    int most = 0;
-    for (const auto& sbt : bp->subs) most = std::max(most, ++per[sbt.cls]);
-    for (int k = 0; k < most && rc == LITHO_OK; ++k) {
-      cudaEvent_t e = nullptr;
-      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) rc = LITHO_ERR_CUDA;
-      else bp->wevents.push_back(e);
-      if (rc == LITHO_OK && k > 0) {
-        cudaStream_t st = nullptr;
-        if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) rc = LITHO_ERR_CUDA;
-        else bp->wstreams.push_back(st);
-      }
-    }
     if (rc != LITHO_OK) {
       litho_batch_plan_destroy(bp);
       return rc;
@@ -501,11 +445,6 @@ int litho_batch_plan_destroy(litho_batch_plan* bp) {
     c.tmbuf.release();
     c.wsum.release();
   }
-  for (cudaStream_t st : bp->wstreams) {
-    cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
-  }
-  for (cudaEvent_t e : bp->wevents) cudaEventDestroy(e);
   bp->mask_pool.release();
   bp->image_pool.release();
   delete bp;

@@ -478,8 +478,8 @@ int litho_image_batch(litho_ctx* ctx, const litho_kernel_set* ks, const float* m
   LITHO_RET(check_geom(ctx, Lx, Ly, ks->Nx, ks->Ny, ks->nk));
   LITHO_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   ImgGeom g{Lx, Ly, next_pow2(Lx), next_pow2(Ly), ks->Nx, ks->Ny, ks->nk, default_conv_n(ks->Nx, ks->Ny)};
-  if (precision == LITHO_PREC_MIXED && !tc_supported(g)) {
-    set_error(ctx, LITHO_ERR_UNSUPPORTED, "mixed precision needs Lx %% 32 == 0 and Nx <= 16 (Lx=%d)", Lx);
+  if (precision == LITHO_PREC_MIXED && (Lx % 4) != 0) {  // rows the tensor maps of the larger supports take
+    set_error(ctx, LITHO_ERR_UNSUPPORTED, "mixed precision needs Lx %% 4 == 0 (Lx=%d)", Lx);
     return LITHO_ERR_UNSUPPORTED;
   }
   const size_t img = (size_t)Lx * Ly * sizeof(float);

@@ -710,20 +710,16 @@ cudaError_t launch_fi_rows(cudaStream_t s, const ImgPlan& p, const float2* band_
                            float* tm, float* tmh, float* tml, float* t0) {
   const int ND = 2 * p.g.Nx + 1;
   const bool km = tmh != nullptr;
-  if (km && KP == 32) {  // the K-major width of Ny <= 8 at compile time
-    if (ND <= 5) return launch_fi_rows_t<5, true, 32>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
-    if (ND <= 9) return launch_fi_rows_t<9, true, 32>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
-    if (ND <= 17) return launch_fi_rows_t<17, true, 32>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
-    return launch_fi_rows_t<33, true, 32>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+  if (km) {  // Ny > 8: the K-major rows are 64 wide
+    if (ND <= 5) return launch_fi_rows_t<5, true, 64>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+    if (ND <= 9) return launch_fi_rows_t<9, true, 64>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+    if (ND <= 17) return launch_fi_rows_t<17, true, 64>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+    return launch_fi_rows_t<33, true, 64>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
   }
-  if (ND <= 5) return km ? launch_fi_rows_t<5, true>(s, p, band_part, twF, KP, tm, tmh, tml, t0)
-                         : launch_fi_rows_t<5, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
-  if (ND <= 9) return km ? launch_fi_rows_t<9, true>(s, p, band_part, twF, KP, tm, tmh, tml, t0)
-                         : launch_fi_rows_t<9, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
-  if (ND <= 17) return km ? launch_fi_rows_t<17, true>(s, p, band_part, twF, KP, tm, tmh, tml, t0)
-                          : launch_fi_rows_t<17, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
-  return km ? launch_fi_rows_t<33, true>(s, p, band_part, twF, KP, tm, tmh, tml, t0)
-            : launch_fi_rows_t<33, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+  if (ND <= 5) return launch_fi_rows_t<5, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+  if (ND <= 9) return launch_fi_rows_t<9, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+  if (ND <= 17) return launch_fi_rows_t<17, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
+  return launch_fi_rows_t<33, false>(s, p, band_part, twF, KP, tm, tmh, tml, t0);
 }
 
 // twF[d][X] = e^{+2 pi i d x'/Fx}, d = 0..2Nx: the FI column twiddles
@@ -835,7 +831,7 @@ ImgPlan make_plan(const ImgGeom& g, int batch, int sm_count) {
   ImgPlan p;
   p.g = g;
   p.batch = batch;
-  p.rowBlocks = (g.Ly + 127) / 128;  // of the tensor-core window DFT (win_fold_plan sets the plain one's)
+  win_fold_plan(p, sm_count);
   // SOCS is latency-bound (warp-shuffle FFT chains), but every kernel group also
   // transforms its own partial intensity: ~2.5 CTAs (20 warps) per SM measured best
   // at 1024^2, K=24, 64 masks (4 kernels per CTA: 36.9 us; 3: 38.9; 8: 45.0)
@@ -863,30 +859,32 @@ static int fold_table(litho_ctx* ctx, const ImgGeom& g, int kind, size_t floats,
   return LITHO_OK;
 }
 
-// Build the cached tables a plain window DFT of this geometry reads, on the context's
-// stream (so that launches on other streams find them ready).
-static int win_dft_tables(litho_ctx* ctx, const ImgGeom& g, const float** coef, const float2** twF) {
-  LITHO_RET(fold_table(ctx, g, -6001, win_fold_coef_floats(g), win_fold_coefs, coef));
-  return fi_twiddles(ctx, g, twF);
-}
-int prepare_win_dft(litho_ctx* ctx, const ImgPlan& p) {
-  const float* coef = nullptr;
-  const float2* twF = nullptr;
-  return win_dft_tables(ctx, p.g, &coef, &twF);
-}
-
-int run_win_dft(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part) {
-  if (p.g.Nx > 16 || p.g.Ny > 16) {
-    set_error(ctx, LITHO_ERR_UNSUPPORTED, "window DFT supports Nx, Ny <= 16 (got %d, %d)", p.g.Nx, p.g.Ny);
+int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int precision) {
+  const ImgGeom& g0 = parts[0].plan.g;
+  if (g0.Nx > 16 || g0.Ny > 16) {
+    set_error(ctx, LITHO_ERR_UNSUPPORTED, "window DFT supports Nx, Ny <= 16 (got %d, %d)", g0.Nx, g0.Ny);
     return LITHO_ERR_UNSUPPORTED;
   }
-  const float* coef = nullptr;
-  const float2* twF = nullptr;
-  LITHO_RET(win_dft_tables(ctx, p.g, &coef, &twF));
+  if (n < 1 || n > WIN_MAX_SIZES) {
+    set_error(ctx, LITHO_ERR_ARG, "window DFT over %d mask sizes (1..%d)", n, WIN_MAX_SIZES);
+    return LITHO_ERR_ARG;
+  }
+  const float* coef[WIN_MAX_SIZES];
+  const float2* twF[WIN_MAX_SIZES];
+  for (int i = 0; i < n; ++i) {
+    const ImgGeom& g = parts[i].plan.g;
+    if (g.Fx != g0.Fx || g.Fy != g0.Fy || g.Nx != g0.Nx || g.Ny != g0.Ny || parts[i].plan.nparts() > nparts) {
+      set_error(ctx, LITHO_ERR_ARG, "window DFT mask sizes of one launch must share the period and the kernels");
+      return LITHO_ERR_ARG;
+    }
+    LITHO_RET(fold_table(ctx, g, -6001, win_fold_coef_floats(g), win_fold_coefs, &coef[i]));
+    LITHO_RET(fi_twiddles(ctx, g, &twF[i]));
+  }
   int* err = nullptr;
   LITHO_RET(tc_err_flag_public(ctx, &err));
   StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
-  LITHO_CUDA_TRY(ctx, launch_win_fold(ctx->stream, p, masks, coef, twF, win_part, err));
+  LITHO_CUDA_TRY(ctx, launch_win_fold(ctx->stream, parts, n, coef, twF, win_part, nparts,
+                                      precision == LITHO_PREC_MIXED ? ctx->test_stall_chunk : -1, err));
   return LITHO_OK;
 }
 
@@ -1057,7 +1055,10 @@ cudaError_t image_pipeline_noctx(cudaStream_t s, const ImgPlan& p, const float* 
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = win_fold_coefs(s, g, wcoef)) != cudaSuccess) return e;
   if ((e = fi_fold_coefs(s, g, fcoef)) != cudaSuccess) return e;
-  if ((e = launch_win_fold(s, p, mask, wcoef, twF, win_part, err)) != cudaSuccess) return e;
+  const WinPart part{p, mask, 0};
+  const float* wc = wcoef;
+  const float2* wt = twF;
+  if ((e = launch_win_fold(s, &part, 1, &wc, &wt, win_part, p.nparts(), -1, err)) != cudaSuccess) return e;
   switch (g.convN) {
     case 32: e = noctx_socs_t<32>(s, p, win_part, krn, sc, band_part); break;
     case 64: e = noctx_socs_t<64>(s, p, win_part, krn, sc, band_part); break;
@@ -1068,26 +1069,12 @@ cudaError_t image_pipeline_noctx(cudaStream_t s, const ImgPlan& p, const float* 
   return launch_fi_fold(s, p, tm, fcoef, image);
 }
 
-// plan of one launch of the mixed form: the persistent tensor-core window kernel splits
-// the 64-column chunks of a row block into tiles until there are ~6 tiles per SM, so the
-// last round of tiles is short (each split adds an epilogue and a partial)
-static ImgPlan mixed_plan(const ImgGeom& g, int batch, int sm_count) {
-  ImgPlan p = make_plan(g, batch, sm_count);
-  const int nch = (g.Lx + 63) / 64;
-  const int units = p.rowBlocks * batch;
-  const int want = 6 * sm_count;
-  const int cs = units < want ? (want + units - 1) / units : 1;
-  p.colSplits = std::max(1, std::min(cs, std::min(4, nch / 2)));
-  return p;
-}
-
 int image_pipeline(litho_ctx* ctx, const ImgGeom& g, int batch, const float* masks, const litho_kernel_set* ks,
                    float* images, int precision) {
   const int KY = 2 * g.Ny + 1;
-  const bool tc = precision == LITHO_PREC_MIXED && tc_supported(g);
+  const bool tc = precision == LITHO_PREC_MIXED && fi_tc_serves(g);
   const bool band = use_band_tcc(ctx, ks, batch);
-  ImgPlan p = tc ? mixed_plan(g, batch, ctx->sm_count) : make_plan(g, batch, ctx->sm_count);
-  if (!tc) win_fold_plan(p, ctx->sm_count);
+  ImgPlan p = make_plan(g, batch, ctx->sm_count);
   if (band) {
     p.ngroups = ks->band_nc;
     p.kpg = g.nk;
@@ -1095,12 +1082,9 @@ int image_pipeline(litho_ctx* ctx, const ImgGeom& g, int batch, const float* mas
   LITHO_RET(ctx->win_part.ensure(ctx, (size_t)batch * p.nparts() * KY * (g.Nx + 1) * sizeof(float2)));
   LITHO_RET(ctx->band_part.ensure(ctx, (size_t)batch * p.ngroups * KY * (4 * g.Nx + 1) * sizeof(float2)));
   if (band) LITHO_RET(ctx->band_w.ensure(ctx, band_wsum_bytes(g, batch)));
-  if (tc) {
-    LITHO_RET(run_win_dft_tc(ctx, p, masks, ctx->win_part.as<float2>()));
-  } else {
-    LITHO_RET(ctx->tm.ensure(ctx, (size_t)batch * (4 * g.Ny + 1) * g.Lx * sizeof(float)));
-    LITHO_RET(run_win_dft(ctx, p, masks, ctx->win_part.as<float2>()));
-  }
+  if (!tc) LITHO_RET(ctx->tm.ensure(ctx, (size_t)batch * (4 * g.Ny + 1) * g.Lx * sizeof(float)));
+  const WinPart part{p, masks, 0};
+  LITHO_RET(run_win_dft(ctx, &part, 1, ctx->win_part.as<float2>(), p.nparts(), precision));
   WindowSrc w;
   w.part = ctx->win_part.as<float2>();
   w.nparts = p.nparts();

@@ -104,14 +104,26 @@ __device__ __forceinline__ void wf_copy(float* dst, const void* src, int bytes, 
 // VEC (rows 16-byte aligned): every lane copies its own neighbouring columns with cp.async and
 // reads them back.  Otherwise lanes 0-3 issue a bulk copy of one row each, the ring holds whole
 // 16-byte granules and the lanes read their columns (lane + 32 i) past each row's misalignment;
-// every wait is bounded: a warp whose copies do not land in a second sets *err, waits for what it
-// has in flight and goes on without them.  (Measured, window stage: 256 aligned masks of 1024^2
+// every wait is bounded: a warp whose copies do not land in a second issues no more, waits for what
+// it has in flight and sets *err.  (Measured, window stage: 256 aligned masks of 1024^2
 // 198 us with cp.async, 206 with bulk copies; 44 of 2048^2 184 and 231; 40 ragged 913 x 777 masks
 // 54 and 49, and 138 with plain loads.)
+// The masks of up to WIN_MAX_SIZES sizes that share the period and the kernel support are one
+// launch: its CTAs are the tiles of win_tiles.hpp (per size: image, column block, share of the
+// base rows).  An image has nparts partials; those its size does not use are left zero.
+struct WinSet {
+  WinTiles T;
+  int Lx[WIN_MAX_SIZES], Ly[WIN_MAX_SIZES];
+  const float* masks[WIN_MAX_SIZES];
+  const float* coef[WIN_MAX_SIZES];   // win_fold_coefs
+  const float2* twF[WIN_MAX_SIZES];   // column twiddles (fi_twiddles)
+  int rows;                           // most base rows of a tile
+};
+
 template <int NY, bool VEC>
-__global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
-    const float* __restrict__ masks, int Lx, int Ly, int Fx, int Fy, int Nx, int Ny, const float* __restrict__ coef,
-    int nb, const float2* __restrict__ twF, float2* __restrict__ win_part, int part_stride, int* err) {
+__global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_constant__ WinSet G, int Fx, int Fy, int Nx,
+                                                                 int Ny, float2* __restrict__ win_part, int nparts,
+                                                                 int stall, int* err) {
   using P = WinFold<NY>;
   constexpr int CPL = P::CPL, COLS = P::COLS, KS = P::KS;
   extern __shared__ __align__(16) float sm[];
@@ -121,13 +133,16 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
   float2* sTw = reinterpret_cast<float2*>(zero + P::ZERO);    // [Nx+1][TS]
   float* sK = zero + P::ZERO + 2 * (Nx + 1) * P::TS;          // ring, row offsets, coefficients; then the warps' sums
   int4* sOff = reinterpret_cast<int4*>(sK + P::RING);         // [rows + WF_AHEAD]
-  const int srows = min((nb + (int)gridDim.y - 1) / (int)gridDim.y, wf_stage(NY));
+  const int srows = min(G.rows, wf_stage(NY));
   float* sCoef = sK + P::RING + 4 * (srows + WF_AHEAD);       // [rows][KS]
   float* ring = sK + warp * (WF_ST * 4 * P::RB);
-  const int cb = blockIdx.x, rs = blockIdx.y, img = blockIdx.z;
+  int sz, img, cb, rs, b0, b1;
+  win_tile(G.T, blockIdx.x, 1, sz, img, cb, rs, b0, b1);
+  const int Lx = G.Lx[sz], Ly = G.Ly[sz];
+  const float* coef = G.coef[sz];
+  const float2* twF = G.twF[sz];
   const int X0 = cb * COLS, ncol = min(COLS, Lx - X0);
-  const int b0 = (int)((long long)nb * rs / gridDim.y), b1 = (int)((long long)nb * (rs + 1) / gridDim.y);
-  const float* M = masks + (size_t)img * Lx * Ly + X0;
+  const float* M = G.masks[sz] + (size_t)img * Lx * Ly + X0;
   const int base4 = (int)((reinterpret_cast<uintptr_t>(M) >> 2) & 3);  // misalignment of row 0 (floats)
 
   auto issue_vec = [&](int4 o4, int st) {  // the rows at offsets o4 (-1: none) into ring stage st
@@ -140,7 +155,12 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
       wf_copy_lane<4 * CPL>(dst + k * P::RB, base + (off[k] >= 0 ? off[k] : 0), off[k] >= 0 && in);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  bool ok = VEC || __all_sync(0xffffffffu, *reinterpret_cast<volatile int*>(err) == 0);  // after a timeout, end quickly
+  int flight = 0, unit = 0;  // stages issued and not waited for; stages issued
   auto issue = [&](int off, int st) {  // lanes 0-3: the row at offset off (-1: none) into ring stage st
+    if (!ok || (stall >= 0 && unit >= stall)) return;  // (stall: the error-path test hook)
+    ++flight;
+    ++unit;
     if (lane >= 4) return;
     int bytes = off >= 0 ? 4 * ncol : 0;
     const float* row = M + off;
@@ -192,7 +212,6 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
   }
   int st = 0;
   uint32_t ph = 0;
-  bool ok = true;
   for (int t0 = b0; t0 < b1; t0 += wf_stage(NY)) {  // one stage up to 2,000 rows at NY = 8
     const int t1 = min(b1, t0 + wf_stage(NY));
     if (t0 > b0) __syncthreads();
@@ -224,7 +243,9 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
       } else {
         const int4 o4 = sOff[b - t0];
         const int off[4] = {o4.x, o4.y, o4.z, o4.w};
-        if (!tc::mbar_wait(&bar[st], ph, ok ? 1000u : 0u)) ok = false;
+        if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&bar[st], ph));
+        if (!ok) continue;
+        --flight;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const float* q = off[k] >= 0 ? src + k * P::RB + ((base4 + off[k]) & 3) : zero;
@@ -270,8 +291,8 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
   if constexpr (VEC) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else {
-    for (int k = 0; k < WF_ST - 1; ++k) {
-      if (!tc::mbar_wait(&bar[st], ph, ok ? 1000u : 200u)) ok = false;
+    for (; flight > 0; --flight) {
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&bar[st], ph, ok ? 1000u : 200u))) ok = false;
       if (++st == WF_ST) {
         st = 0;
         ph ^= 1;
@@ -323,8 +344,11 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
   int Q = 8;
   while (Q > 1 && NP * Q > WF_THREADS) Q >>= 1;
   const float scale = 1.0f / ((float)Fx * (float)Fy);
-  const int nps = part_stride > 0 ? part_stride : gridDim.x * gridDim.y;
-  float2* out = win_part + ((size_t)img * nps + (size_t)rs * gridDim.x + cb) * KY * NU;
+  float2* parts = win_part + (size_t)(G.T.img0[sz] + img) * nparts * KY * NU;
+  const int used = G.T.rows[sz] * G.T.ncs[sz];
+  if (cb == 0 && rs == 0)
+    for (int e = tid; e < (nparts - used) * KY * NU; e += WF_THREADS) parts[(size_t)used * KY * NU + e] = make_float2(0.f, 0.f);
+  float2* out = parts + (size_t)(cb * G.T.ncs[sz] + rs) * KY * NU;
   for (int base = 0; base < NP * Q; base += WF_THREADS) {  // uniform bound: whole warps shuffle
     const int t = base + tid, q = t % Q, pr = min(t / Q, NP - 1), v = pr / UG, u0 = (pr - v * UG) * UT;
     const float* C = sC + v * P::RS;
@@ -366,18 +390,39 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(
   }
 }
 
-// column blocks and row splits of a plain window DFT: every split is one more partial per column
-// block and one more start and end of a CTA, so only as many as give each SM two waves of its two
-// CTAs (64 masks of 1024^2: 76 us, and 96 / 135 us with 16 / 28 CTAs per SM asked for)
+// Row splits of a launch of `units` x splits CTAs of `warps` warps, `slots` of them resident at
+// once: the fewest row steps over all waves, a CTA costing its start and end in row steps besides
+// its own.  A part-filled last wave costs as much as a full one, so small batches take what fits
+// one wave (window of 16 masks of 1024^2: 21 us with the 256 CTAs of two splits, 31 us with 640).
+static int fold_splits(long long units, int nb, int warps, int most, long long slots, int ends) {
+  int best = 1;
+  long long least = -1;
+  for (int r : {1, 2, 3, 4, 5, 6, 8, 12, 16, 24, 32}) {
+    if (r > most) break;
+    const long long cost = (units * r + slots - 1) / slots * ((nb + warps * r - 1) / (warps * r) + ends);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = r;
+    }
+  }
+  return best;
+}
+
+// Row splits of the window DFTs of `tiles` column blocks in all, ncb to an image.  Each split is
+// one more partial per column block for the next stage to add up, so at most 32 partials an image
+// (or two splits): one mask of 1024^2 takes 22 us in the two stages with 32, 44 us with 256.
+int win_fold_splits(const ImgGeom& g, int ncb, long long tiles, int sm_count) {
+  const int nb = fold_nbase(g.Ly, g.Fy);
+  const int most = std::max(1, std::min(nb / WF_WARPS, std::max(2, 32 / ncb)));  // a base row per warp at least
+  return fold_splits(tiles, nb, WF_WARPS, most, 2LL * sm_count, 8);
+}
+
+// column blocks and row splits of a window DFT
 void win_fold_plan(ImgPlan& p, int sm_count) {
   const int cols = 32 * wf_cpl(wf_ny(p.g.Ny));
   p.rowBlocks = (p.g.Lx + cols - 1) / cols;
-  const long long want = 4LL * sm_count, units = (long long)p.rowBlocks * p.batch;
-  const int most = win_fold_max_splits(p.g);
-  p.colSplits = (int)std::max(1LL, std::min<long long>(most, (want + units - 1) / units));
+  p.colSplits = win_fold_splits(p.g, p.rowBlocks, (long long)p.rowBlocks * p.batch, sm_count);
 }
-// every warp of a CTA keeps at least one base row
-int win_fold_max_splits(const ImgGeom& g) { return std::max(1, fold_nbase(g.Ly, g.Fy) / WF_WARPS); }
 
 size_t win_fold_coef_floats(const ImgGeom& g) { return (size_t)fold_nbase(g.Ly, g.Fy) * wf_stride(wf_ny(g.Ny)); }
 
@@ -388,29 +433,46 @@ cudaError_t win_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef) {
 }
 
 template <int NY>
-static cudaError_t launch_win_fold_t(cudaStream_t s, const ImgPlan& p, const float* masks, const float* coef,
-                                     const float2* twF, float2* win_part, int* err) {
-  const ImgGeom& g = p.g;
-  const int nb = fold_nbase(g.Ly, g.Fy), rows = (nb + p.colSplits - 1) / p.colSplits;
-  const size_t smem = win_fold_smem<NY>(g.Nx, rows);
-  const bool vec = (g.Lx & 3) == 0 && (reinterpret_cast<uintptr_t>(masks) & 15) == 0;
+static cudaError_t launch_win_fold_t(cudaStream_t s, const WinSet& G, const ImgGeom& g, bool vec, float2* win_part,
+                                     int nparts, int stall, int* err) {
+  const size_t smem = win_fold_smem<NY>(g.Nx, G.rows);
   auto k = vec ? win_fold_kernel<NY, true> : win_fold_kernel<NY, false>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k<<<dim3(p.rowBlocks, p.colSplits, p.batch), WF_THREADS, smem, s>>>(masks, g.Lx, g.Ly, g.Fx, g.Fy, g.Nx, g.Ny, coef,
-                                                                     nb, twF, win_part, p.part_stride, err);
+  k<<<G.T.tile0[G.T.n], WF_THREADS, smem, s>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, win_part, nparts, stall, err);
   return cudaGetLastError();
 }
 
-// coef from win_fold_coefs, twF the column twiddles of fi_twiddles, err the timeout flag
-cudaError_t launch_win_fold(cudaStream_t s, const ImgPlan& p, const float* masks, const float* coef,
-                            const float2* twF, float2* win_part, int* err) {
-  switch (wf_ny(p.g.Ny)) {
-    case 2: return launch_win_fold_t<2>(s, p, masks, coef, twF, win_part, err);
-    case 4: return launch_win_fold_t<4>(s, p, masks, coef, twF, win_part, err);
-    case 8: return launch_win_fold_t<8>(s, p, masks, coef, twF, win_part, err);
-    case 12: return launch_win_fold_t<12>(s, p, masks, coef, twF, win_part, err);
-    default: return launch_win_fold_t<16>(s, p, masks, coef, twF, win_part, err);
+// n <= WIN_MAX_SIZES mask sizes of one period and support, nparts partials per image; err: the
+// timeout flag; stall >= 0: the error-path test hook
+cudaError_t launch_win_fold(cudaStream_t s, const WinPart* parts, int n, const float* const* coef,
+                            const float2* const* twF, float2* win_part, int nparts, int stall, int* err) {
+  const ImgGeom& g0 = parts[0].plan.g;
+  WinSet G = {};
+  G.T.n = n;
+  bool vec = stall < 0;
+  for (int i = 0; i < n; ++i) {
+    const ImgPlan& p = parts[i].plan;
+    const int nb = fold_nbase(p.g.Ly, p.g.Fy);
+    G.T.Lx[i] = nb;  // the extent that the splits share out: base rows
+    G.T.rows[i] = p.rowBlocks;
+    G.T.ncs[i] = p.colSplits;
+    G.T.img0[i] = parts[i].img0;
+    G.T.tile0[i + 1] = G.T.tile0[i] + p.rowBlocks * p.colSplits * p.batch;
+    G.Lx[i] = p.g.Lx;
+    G.Ly[i] = p.g.Ly;
+    G.masks[i] = parts[i].masks;
+    G.coef[i] = coef[i];
+    G.twF[i] = twF[i];
+    G.rows = std::max(G.rows, (nb + p.colSplits - 1) / p.colSplits);
+    vec = vec && (p.g.Lx & 3) == 0 && (reinterpret_cast<uintptr_t>(parts[i].masks) & 15) == 0;
+  }
+  switch (wf_ny(g0.Ny)) {
+    case 2: return launch_win_fold_t<2>(s, G, g0, vec, win_part, nparts, stall, err);
+    case 4: return launch_win_fold_t<4>(s, G, g0, vec, win_part, nparts, stall, err);
+    case 8: return launch_win_fold_t<8>(s, G, g0, vec, win_part, nparts, stall, err);
+    case 12: return launch_win_fold_t<12>(s, G, g0, vec, win_part, nparts, stall, err);
+    default: return launch_win_fold_t<16>(s, G, g0, vec, win_part, nparts, stall, err);
   }
 }
 
@@ -549,11 +611,8 @@ static cudaError_t launch_fi_fold_t(cudaStream_t s, const ImgPlan& p, const floa
                                     float* images) {
   const ImgGeom& g = p.g;
   const int nb = fold_nbase(g.Ly, g.Fy), cols = 32 * ff_cpl(NY), ncb = (g.Lx + cols - 1) / cols;
-  // every CTA loads its columns of Tm once: row splits only until there are
-  // four waves of three CTAs per SM (64 masks of 1024^2: 47.5 us; 53 / 68 / 94 us with twice, four and eight times as many)
-  const int sms = p.sms > 0 ? p.sms : 148;
-  const long long want = 12LL * sms, units = (long long)ncb * p.batch;
-  const int R = (int)std::max(1LL, std::min<long long>(std::max(1, nb / FF_WARPS), (want + units - 1) / units));
+  const int R = fold_splits((long long)ncb * p.batch, nb, FF_WARPS, std::max(1, std::min(32, nb / FF_WARPS)),
+                            3LL * (p.sms > 0 ? p.sms : 148), 7);
   const size_t smem = (size_t)std::min((nb + R - 1) / R, ff_stage(NY)) * (ff_stride(NY) * sizeof(float) + sizeof(int4));
   const bool vec = (g.Lx & 3) == 0 && ((reinterpret_cast<uintptr_t>(tm) | reinterpret_cast<uintptr_t>(images)) & 15) == 0;
   auto k = vec ? fi_fold_kernel<NY, true> : fi_fold_kernel<NY, false>;

@@ -155,8 +155,8 @@ struct litho_ctx {
   std::map<std::pair<int, int>, litho::TccTune> tcc_tune;
   std::map<std::tuple<int, int, int, int>, std::shared_ptr<void>> gemm_tables;
   int tcc_force_bn = 0, tcc_force_bk = 64, tcc_force_sched = 0;  // litho_tcc_gemm_shape: bn > 0 bypasses the tuner
-  // error-path test hook (litho_ctx_set_test_stall): >= 0 stops the mixed window
-  // DFT's TMA producer at that chunk of every CTA's work; -1 = off
+  // error-path test hook (litho_ctx_set_test_stall): >= 0 stops the copies of a mixed call's
+  // window DFT after that many steps of every warp; -1 = off
   int test_stall_chunk = -1;
 };
 
@@ -198,9 +198,8 @@ struct ImgGeom {
 struct ImgPlan {
   ImgGeom g;
   int batch = 1;
-  int rowBlocks = 1, colSplits = 1;  // window-DFT partition -> nparts (plain: column blocks, row splits)
+  int rowBlocks = 1, colSplits = 1;  // window DFT: column blocks, row splits -> nparts
   int kpg = 1, ngroups = 1;          // SOCS kernels per CTA -> ngroups
-  int part_stride = 0;               // >0: window partials per image in a shared per-class array
   int sms = 0;                       // SMs of the device (launch sizing)
   int nparts() const { return rowBlocks * colSplits; }
 };
@@ -228,17 +227,25 @@ struct WindowSrc {
 // the folded FP32 transforms (imaging_fold.cu): plan fields of a plain window DFT, coefficient
 // tables and launches
 void win_fold_plan(ImgPlan& p, int sm_count);
-int win_fold_max_splits(const ImgGeom& g);
+int win_fold_splits(const ImgGeom& g, int ncb, long long tiles, int sm_count);
 size_t win_fold_coef_floats(const ImgGeom& g);
 cudaError_t win_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef);
-cudaError_t launch_win_fold(cudaStream_t s, const ImgPlan& p, const float* masks, const float* coef,
-                            const float2* twF, float2* win_part, int* err);
+// masks of one size for a window launch over several sizes (at most WIN_MAX_SIZES, win_tiles.hpp):
+// its plan, its masks and its first image in the shared partial array
+struct WinPart {
+  ImgPlan plan;
+  const float* masks;
+  int img0;
+};
+cudaError_t launch_win_fold(cudaStream_t s, const WinPart* parts, int n, const float* const* coef,
+                            const float2* const* twF, float2* win_part, int nparts, int stall, int* err);
 size_t fi_fold_coef_floats(const ImgGeom& g);
 cudaError_t fi_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef);
 cudaError_t launch_fi_fold(cudaStream_t s, const ImgPlan& p, const float* tm, const float* coef, float* images);
 
-int run_win_dft(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part);
-int prepare_win_dft(litho_ctx* ctx, const ImgPlan& p);  // cached tables, on ctx->stream
+// window DFT of up to WIN_MAX_SIZES mask sizes, nparts partials per image; precision: whether the
+// error-path test hook acts
+int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int precision);
 int run_socs(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const float2* krn,
              const float* scales, float2* band_part, float* tmpImgp);
 int run_fi(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tm, float* images);
@@ -268,17 +275,9 @@ inline bool band_tcc_available(const litho_ctx* ctx, const litho_kernel_set* ks)
 // LITHO_BAND_AUTO where the band cost model (band_sched.hpp) expects it to be faster
 bool use_band_tcc(const litho_ctx* ctx, const litho_kernel_set* ks, int batch);
 
-// mixed precision window DFT / interpolation (imaging_tc.cu)
-int run_win_dft_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part);
-// masks of one size for a multi-size window launch (at most WIN_MAX_SIZES, win_tiles.hpp):
-// its plan, its masks and its first image
-// in the shared partial array
-struct WinPart {
-  ImgPlan plan;
-  const float* masks;
-  int img0;
-};
-int run_win_dft_tc_multi(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part);
+// mixed precision interpolation (imaging_tc.cu): whether it serves a geometry of the mixed form
+// (elsewhere the folded FP32 kernel does), and its launches
+bool fi_tc_serves(const ImgGeom& g);
 int run_fi_tc(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tmT, float* images);
 struct FiTcBufs {
   float *tmh, *tml, *t0;
@@ -287,7 +286,6 @@ FiTcBufs fi_tc_bufs(float* base, const ImgGeom& g, int total, int first);
 int run_fi_rows_tc(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, const FiTcBufs& b);
 int run_fi_out_tc(litho_ctx* ctx, const ImgPlan& p, const FiTcBufs& b, float* images);
 size_t fi_tc_workspace_bytes(const ImgGeom& g, int batch);
-bool tc_supported(const ImgGeom& g);
 int tc_check_flag(litho_ctx* ctx);
 int tc_err_flag_public(litho_ctx* ctx, int** flag);  // the flag of the kernels' bounded waits, made on first use
 

@@ -79,7 +79,6 @@ extern "C" int litho_image_noalloc(const float* mask, int Lx, int Ly, const floa
   if (cn < 32) cn = 32;
   ImgGeom g{Lx, Ly, Fx, Fy, Nx, Ny, nk, cn};
   ImgPlan p = make_plan(g, 1, sms);
-  win_fold_plan(p, sms);
   while (p.nparts() > NOALLOC_MAX_PARTS && p.colSplits > 1) --p.colSplits;
   if (p.nparts() > NOALLOC_MAX_PARTS) return LITHO_ERR_ARG;
   size_t off[8];

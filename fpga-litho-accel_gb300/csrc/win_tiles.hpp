@@ -1,8 +1,8 @@
-// Tiles of one mixed window-DFT launch over up to WIN_MAX_SIZES mask sizes (imaging_tc.cu,
-// win_dft_tc_kernel): per size its width, 128-row blocks, column splits, first image in the
-// shared partial array and first tile; tiles are numbered size after size, then image, row
-// block and column split.  Plain C++ (host and device), so the numbering is also checked on
-// the CPU.
+// Tiles of one window DFT launch over up to WIN_MAX_SIZES mask sizes: per size an extent that
+// its splits share out in chunks, the blocks across it, the splits, the first image in the
+// shared partial array and the first tile; tiles are numbered size after size, then image, block
+// and split.  (imaging_fold.cu: the extent is the base rows, a chunk one of them, and the blocks
+// are column blocks.)  Plain C++ (host and device), so the numbering is also checked on the CPU.
 #pragma once
 
 #ifdef __CUDACC__
@@ -17,15 +17,14 @@ constexpr int WIN_MAX_SIZES = 4;  // mask sizes one window launch takes
 
 struct WinTiles {
   int n;                              // mask sizes
-  int Lx[WIN_MAX_SIZES];              // mask width
-  int rows[WIN_MAX_SIZES];            // 128-row blocks
-  int ncs[WIN_MAX_SIZES];             // column splits
+  int Lx[WIN_MAX_SIZES];              // extent
+  int rows[WIN_MAX_SIZES];            // blocks
+  int ncs[WIN_MAX_SIZES];             // splits
   int img0[WIN_MAX_SIZES];            // first image in the partial array
   int tile0[WIN_MAX_SIZES + 1];       // first tile (tile0[n]: all tiles)
 };
 
-// tile t -> (size g, image, row block, column split) and its range [c0, c1) of column chunks
-// of `chunk` columns
+// tile t -> (size g, image, block, split) and its range [c0, c1) of chunks of `chunk`
 LITHO_WT_HD inline void win_tile(const WinTiles& T, int t, int chunk, int& g, int& img, int& rb, int& cs, int& c0,
                                  int& c1) {
   g = 0;

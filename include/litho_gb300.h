@@ -125,12 +125,12 @@ int litho_ctx_stage_times(litho_ctx* ctx, double* ms, long long* launches, int r
 
 /* ---- error-path test hook for the bounded device-side waits ----------------
  * No counterpart in the reference, whose failure handling is assert and exit
- * (common/file_io.cpp:137-150, litho.cpp:246-248).  chunk >= 0 makes the TMA
- * producer of the mixed-precision window DFT (LITHO_PREC_MIXED imaging) stop
- * issuing loads at that 64-column chunk of every CTA's share of the work, as if
- * it had been lost.  The consumers' waits then give up after their limit (about
- * one second), every role of the kernel leaves, the kernel frees its tensor
- * memory, and the call (or the next litho_ctx_synchronize, for device pointers)
+ * (common/file_io.cpp:137-150, litho.cpp:246-248).  chunk >= 0 makes every warp of
+ * the window DFT of a LITHO_PREC_MIXED call stop issuing bulk copies after that
+ * many steps of its share of the work, as if the rest had been lost (the call
+ * takes the kernel's bulk-copy form, the one that waits).  The waits then give up
+ * after their limit (about one second), the kernel waits for what is in flight and
+ * leaves, and the call (or the next litho_ctx_synchronize, for device pointers)
  * returns LITHO_ERR_TIMEOUT; the images of that call are undefined.  -1, the
  * default, turns the hook off.  The value is read when a window DFT is launched
  * (and baked into a batch plan's graph when the plan is created).  For tests of
