@@ -501,10 +501,10 @@ __global__ void __launch_bounds__(S128_THREADS) socs128_kernel(
 // ---------------------------------------------------------------------------
 constexpr int FR_THREADS = 256, FR_COLS = 128, FR_ROWS = 2 * FR_COLS + 1;  // column, mirror, x' = 0
 
-template <int MAXD, bool KMAJ, int KPC>
+template <int MAXD, bool KMAJ, int KPC, int PRE>
 __global__ void __launch_bounds__(FR_THREADS) fi_rows_kernel(const float2* __restrict__ band_part, int ngroups,
                                                              const float2* __restrict__ twF, int Lx, int Fx,
-                                                             int Nx, int Ny, int kp_rt, int batch, int raw_n,
+                                                             int Nx, int Ny, int kp_rt, int batch,
                                                              float* __restrict__ tm, float* __restrict__ tmh,
                                                              float* __restrict__ tml, float* __restrict__ t0) {
   extern __shared__ __align__(16) float4 frs[];
@@ -535,11 +535,11 @@ __global__ void __launch_bounds__(FR_THREADS) fi_rows_kernel(const float2* __res
   const int nmir = max(0, nbase - imin), Mlo = M - X0 - nbase + 1;
   const int nrows = nbase + nmir + (xtra ? 1 : 0);
   // the next image's band partials stream into shared memory (8-byte cp.async) while
-  // this image is computed, when the two buffers fit (raw_n > 0)
+  // this image is computed where two buffers fit (PRE = 2); with one (PRE = 1) this image's all
+  // arrive together, and without (PRE = 0) they are summed from L2, eight loads in flight
   const int RAWN = ngroups * BH * BW;
-  float2* raw = raw_n > 0 ? reinterpret_cast<float2*>(
-                                (reinterpret_cast<uintptr_t>(sO + (KMAJ ? FR_ROWS * (KP + 1) : 0)) + 15) & ~uintptr_t(15))
-                          : nullptr;
+  float2* raw = reinterpret_cast<float2*>(
+      (reinterpret_cast<uintptr_t>(sO + (KMAJ ? FR_ROWS * (KP + 1) : 0)) + 15) & ~uintptr_t(15));
   auto fetch = [&](int im, float2* dst) {
     const float2* src = band_part + (size_t)im * RAWN;
     for (int e = tid; e < RAWN; e += FR_THREADS) {
@@ -547,29 +547,40 @@ __global__ void __launch_bounds__(FR_THREADS) fi_rows_kernel(const float2* __res
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(da), "l"(src + e) : "memory");
     }
   };
-  if (raw != nullptr) {
+  if (PRE == 2) {
     if ((int)blockIdx.y < batch) fetch(blockIdx.y, raw);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   for (int img = blockIdx.y, k = 0; img < batch; img += gridDim.y, ++k) {
-    if (raw != nullptr) {
+    if (PRE == 2) {
       if (img + (int)gridDim.y < batch) fetch(img + gridDim.y, raw + (size_t)((k + 1) & 1) * RAWN);
       asm volatile("cp.async.commit_group;" ::: "memory");
       asm volatile("cp.async.wait_group 1;" ::: "memory");  // this image's partials have landed
     }
+    if (PRE == 1) {  // every thread is past the previous image's combine (the barrier behind it)
+      fetch(img, raw);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    }
     __syncthreads();  // the previous image is out of sC and sO (and this one's partials are visible)
-    const float2* B = raw != nullptr ? raw + (size_t)(k & 1) * RAWN : band_part + (size_t)img * RAWN;
+    const float2* B = PRE ? raw + (size_t)(PRE == 2 ? k & 1 : 0) * RAWN : band_part + (size_t)img * RAWN;
     for (int idx = tid; idx < BH * MAXD; idx += FR_THREADS) {
       const int fy = idx / MAXD, d = idx - fy * MAXD;  // MAXD: a compile-time divisor
       if (d >= ND) continue;
       const float2* S = B + fy * BW + 2 * Nx;
-      float2 pv = S[d], qv = S[-d];
-      for (int gi = 1; gi < ngroups; ++gi) {  // the kernel groups' partials, in order
-        const float2 a = S[gi * pst + d], b = S[gi * pst - d];
-        pv.x += a.x;
-        pv.y += a.y;
-        qv.x += b.x;
-        qv.y += b.y;
+      float2 pv, qv;  // the kernel groups' partials in a fixed order
+      if constexpr (PRE != 0) {
+        pv = S[d];
+        qv = S[-d];
+        for (int gi = 1; gi < ngroups; ++gi) {
+          const float2 a = S[gi * pst + d], b = S[gi * pst - d];
+          pv.x += a.x;
+          pv.y += a.y;
+          qv.x += b.x;
+          qv.y += b.y;
+        }
+      } else {
+        pv = sum_strided(S + d, pst, ngroups);
+        qv = d > 0 ? sum_strided(S - d, pst, ngroups) : pv;
       }
       if (d == 0) {
         sC[fy * MAXD] = make_float4(pv.x, pv.y, 0.f, 0.f);
@@ -682,13 +693,17 @@ template <int MAXD, bool KMAJ, int KPC = 0>
 static cudaError_t launch_fi_rows_t(cudaStream_t s, const ImgPlan& p, const float2* band_part, const float2* twF,
                                     int KP, float* tm, float* tmh, float* tml, float* t0) {
   const ImgGeom& g = p.g;
-  // two shared buffers for the band partials of the next image when they fit in 32 KB
+  // shared memory for the band partials: two buffers where they fit in 32 KB (the next image's
+  // arrive meanwhile), one up to 110 KB (small batches have many kernel groups: one image of
+  // 1024^2 with 24 of them took 23 us when they were summed from L2)
   const int rawn = p.ngroups * (2 * g.Ny + 1) * (4 * g.Nx + 1);
-  const bool pre = (size_t)2 * rawn * sizeof(float2) <= 32 * 1024;
+  const size_t raw = (size_t)rawn * sizeof(float2);
+  const int pre = 2 * raw <= 32 * 1024 ? 2 : raw <= 110 * 1024 ? 1 : 0;
   const size_t smem = (size_t)(2 * g.Ny + 1) * MAXD * sizeof(float4) +
                       (KMAJ ? (size_t)FR_ROWS * (KP + 1) * sizeof(float) : 0) +
-                      (pre ? 2 * (size_t)rawn * sizeof(float2) + 16 : 0);
-  auto k = fi_rows_kernel<MAXD, KMAJ, KPC>;
+                      (pre ? pre * raw + 16 : 0);
+  auto k = pre == 2 ? fi_rows_kernel<MAXD, KMAJ, KPC, 2> : pre == 1 ? fi_rows_kernel<MAXD, KMAJ, KPC, 1>
+                                                                    : fi_rows_kernel<MAXD, KMAJ, KPC, 0>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   // column blocks over the x' < 0 half; as many image groups as keep every CTA resident
@@ -702,7 +717,7 @@ static cudaError_t launch_fi_rows_t(cudaStream_t s, const ImgPlan& p, const floa
   if (e != cudaSuccess) return e;
   const int groups = std::max(1, std::min(p.batch, std::max(1, per_sm) * sms / ncb));
   k<<<dim3(ncb, groups), FR_THREADS, smem, s>>>(band_part, p.ngroups, twF, g.Lx, g.Fx, g.Nx, g.Ny, KP, p.batch,
-                                                pre ? rawn : 0, tm, tmh, tml, t0);
+                                                tm, tmh, tml, t0);
   return cudaGetLastError();
 }
 
