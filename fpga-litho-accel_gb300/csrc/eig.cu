@@ -9,6 +9,8 @@
 //      on the lower-triangle tiles, mirrored.  The off-diagonal comes out real.
 //      Column k below the diagonal is read as the conjugate of row k (A stays
 //      Hermitian in full), and v_k is packed contiguously for the back-transform.
+//      Matrices whose rows fit the SMs' shared memory take one cooperative launch
+//      instead (tridiag_kernel).
 //      Both kernels are bound by the FP64 pipe (GB300: 2 DFMA/clk/SM), so the
 //      arithmetic is written as FMA chains and the update touches each element
 //      pair once.
@@ -30,6 +32,7 @@
 //                           krn[i][j] = y_i[n-1-j] (litho.cpp:626-634 reversal).
 // No kernel waits on another; every step is a separate launch on the stream.
 #include "litho_internal.cuh"
+#include "tc_common.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -270,6 +273,268 @@ __global__ void __launch_bounds__(256) her2_kernel(double2* __restrict__ A, int 
     const int jj = ty + 8 * r, ii = tx;
     const int row = J * 32 + jj, col = I * 32 + ii;
     if (row < m && col < m) A[(size_t)(k + 1 + row) * n + (k + 1 + col)] = zconj_bits(tile[ii][jj]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same reduction in one cooperative launch, for matrices whose rows fit the SMs' shared
+// memory (n <= ~1200): CTA c keeps rows c, c + G, .. there in full for the whole reduction, and a
+// column costs one grid barrier instead of two launches.  Per column k, with r the pivot row right
+// of the diagonal (v = (1, scl conj(r[1:]))):
+//   product   x_i = tau (B_i0 + scl sum_j B_ij conj(r_j)) for the CTA's rows, and its partial of
+//             gamma = 2 Re(-tau/2 x^H v); the owner of row k + 1 has published that row as it is
+//   barrier
+//   update    B_ij -= v_i conj(x_j) + u_i conj(v_j),  u = x + gamma v,
+//             which is v w^H + w v^H with w = x - tau/2 (x^H v) v; conj(v_j) = conj(scl) r_j, so
+//             neither v nor w is formed but for the CTA's own rows.  Every CTA updates the next
+//             pivot row for itself first (v_i = 1 there), so that its norm and scalars, formed by
+//             the ninth warp meanwhile, need no exchange of their own.
+// The FP64 units bound it: each quarter of an SM takes a warp's FP64 instruction every ~66 cycles,
+// dependent or not and whatever its lanes do.  Large matrices spend them on 12 m^2 FMAs per column
+// over all SMs (full rows: half of the update is done twice, which costs less than exchanging the
+// halves would), small ones on the chain from the barrier to the next x; the barrier takes ~3,000
+// cycles.  Measured, reduction: n = 289 6.0 -> 1.8 ms, n = 1089 31 -> 17.2 ms.  Polling values
+// in place of a barrier was slower (n = 289: 9,000 cycles an exchange: 152 CTAs poll every value).
+// ---------------------------------------------------------------------------
+constexpr int TD_WARPS = 8, TD_THREADS = 32 * (TD_WARPS + 1);
+constexpr int TD_MAX_ROWS = 16;
+
+size_t tridiag_smem(int n, int G) {
+  return ((size_t)((n + G - 1) / G) * n + 3 * (size_t)n) * sizeof(double2);
+}
+
+// Waits until *p has reached `target` (bounded: false after a second, with *err set).
+__device__ __forceinline__ bool td_wait(const unsigned* p, unsigned target, int* err) {
+  uint64_t t0 = 0;
+  for (int spin = 0;; ++spin) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    if (v >= target) return true;
+    if ((spin & 255) == 255) {
+      const uint64_t t = tc::global_ns();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > 1000000000ull || *reinterpret_cast<volatile int*>(err) != 0) {
+        atomicExch(err, 1);
+        return false;
+      }
+    }
+  }
+}
+// grid barrier in two halves: arrive() after the CTA's writes, wait() for every CTA's arrival
+__device__ __forceinline__ void td_arrive(unsigned* count) {
+  __syncthreads();
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+}
+__device__ __forceinline__ bool td_arrived(const unsigned* count, unsigned target, int* err, int* s_ok) {
+  if (threadIdx.x == 0) *s_ok = td_wait(count, target, err);
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// (re, im) summed over the warp: re in lanes 0-15, im in lanes 16-31
+__device__ __forceinline__ double pair_sum(double re, double im, int lane) {
+  const bool up = lane & 16;
+  double v = (up ? im : re) + __shfl_xor_sync(0xffffffffu, up ? re : im, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// the reflector of a pivot row with pivot alpha = conj(first) and squared norm xn2 past it: the
+// zlarfg scalars, the two reciprocals side by side in lanes 0 and 1 (whole warp)
+struct TdScalars {
+  double2 tau, scl;  // scl = 1 / (alpha - beta)
+  double beta;
+};
+__device__ __forceinline__ TdScalars td_reflector(double2 first, double xn2, int lane) {
+  const double2 alpha = zconj(first);
+  const bool plain = xn2 == 0.0 && alpha.y == 0.0;
+  const double nr = sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn2)));
+  TdScalars r;
+  r.beta = plain ? alpha.x : alpha.x >= 0.0 ? -nr : nr;
+  const double dr = alpha.x - r.beta;
+  const double inv = 1.0 / (lane == 0 ? r.beta : fma(dr, dr, alpha.y * alpha.y));
+  const double ib = __shfl_sync(0xffffffffu, inv, 0), id = __shfl_sync(0xffffffffu, inv, 1);
+  const double2 z = make_double2(0.0, 0.0);
+  r.tau = plain ? z : make_double2(-dr * ib, -alpha.y * ib);
+  r.scl = plain ? z : make_double2(dr * id, -alpha.y * id);
+  return r;
+}
+
+// How many warps share a row, for rows of `steps` warp-widths: the FP64 unit of a quarter of an SM
+// takes one warp instruction per ~66 cycles whatever else there is, so the load of the fullest
+// quarter decides (per step and 5 for the reduction over the lanes).
+__device__ __forceinline__ int td_split(int nact, int steps) {
+  const int c1 = (nact + 3) / 4 * (12 * steps + 5), c2 = (nact + 1) / 2 * (6 * steps + 11),
+            c4 = nact * (3 * steps + 14);
+  return c1 <= c2 && c1 <= c4 ? 1 : c2 <= c4 ? 2 : 4;
+}
+
+__global__ void __launch_bounds__(TD_THREADS, 1) tridiag_kernel(const double2* __restrict__ A, int n,
+                                                                double2* __restrict__ vpack, double2* __restrict__ tau,
+                                                                double* __restrict__ d, double* __restrict__ e,
+                                                                double* __restrict__ e2, double2* __restrict__ xg,
+                                                                double2* __restrict__ rowbuf, double* __restrict__ part,
+                                                                unsigned* count, int* err) {
+  extern __shared__ __align__(16) double2 tds[];
+  __shared__ double s_dot[TD_MAX_ROWS][4][2];  // per row and warp of the row: (re, im)
+  __shared__ double2 s_x[TD_MAX_ROWS], s_v[TD_MAX_ROWS], s_us[TD_MAX_ROWS], s_us1;
+  __shared__ TdScalars s_sc;
+  __shared__ double2 s_ts;  // tau scl
+  __shared__ int s_ok;
+  const int c = blockIdx.x, G = gridDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int T = (n - c + G - 1) / G;  // rows c + G t, t < T
+  double2* rows = tds;                                // [T][n]
+  double2* xs = tds + (size_t)((n + G - 1) / G) * n;  // [n]
+  double2* rs = xs + n;                               // [n] pivot row
+  double2* rn = rs + n;                               // [n] next pivot row
+  // the ninth warp: norm of pivot row k past its pivot and the reflector's scalars
+  auto scalars = [&](int k, const double2* r) {
+    double q = 0.0;
+    for (int j = k + 2 + lane; j < n; j += 32) q = fma(r[j].x, r[j].x, fma(r[j].y, r[j].y, q));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    const TdScalars t = td_reflector(r[k + 1], q, lane);
+    const double2 ts = zmul(t.tau, t.scl);
+    if (lane == 0) {
+      s_sc = t;
+      s_ts = ts;
+      if (c == 0) {
+        tau[k] = t.tau;
+        e[k] = t.beta;
+        e2[k] = t.beta * t.beta;
+      }
+    }
+  };
+  for (int t = 0; t < T; ++t)
+    for (int j = tid; j < n; j += TD_THREADS) rows[(size_t)t * n + j] = A[(size_t)(c + G * t) * n + j];
+  for (int j = tid; j < n; j += TD_THREADS) rs[j] = A[j];
+  __syncthreads();
+  if (warp == TD_WARPS) scalars(0, rs);
+  if (c == 0 && tid == 0) d[0] = rs[0].x;
+  for (int k = 0; k + 1 < n; ++k) {
+    const int t0 = k < c ? 0 : (k - c) / G + 1, nact = T - t0;  // the CTA's rows past k
+    const int wpr = td_split(nact, (n - k - 2 + 31) / 32), rstep = TD_WARPS / wpr, sub = warp & (wpr - 1);
+    double2* xk = xg + (size_t)(k & 1) * n;
+    double2* rowk = rowbuf + (size_t)(k & 1) * n;  // row k + 1
+    double* pk = part + (size_t)(k & 1) * G;
+    if (warp < TD_WARPS) {
+      if (c == (k + 1) % G)
+        for (int j = k + 1 + tid; j < n; j += 32 * TD_WARPS) __stcg(rowk + j, rows[(size_t)t0 * n + j]);
+      for (int a = warp / wpr; a < nact; a += rstep) {
+        const double2* row = rows + (size_t)(t0 + a) * n;
+        double re = 0.0, im = 0.0;
+        for (int j = k + 2 + 32 * sub + lane; j < n; j += 32 * wpr) {
+          const double2 b = row[j], r = rs[j];  // b * conj(r)
+          re = fma(b.x, r.x, re);
+          re = fma(b.y, r.y, re);
+          im = fma(b.y, r.x, im);
+          im = fma(-b.x, r.y, im);
+        }
+        const double v = pair_sum(re, im, lane);
+        if ((lane & 15) == 0) s_dot[a][sub][lane >> 4] = v;
+      }
+    }
+    __syncthreads();  // products, and the scalars of the ninth warp
+    if (warp == 0) {
+      // lane a < 16: x of row a; lane 16 + a: its v and tau v (an FP64 instruction takes a warp's
+      // time whatever its lanes do, so the two halves do different products at once)
+      const int a = lane & 15, i = c + G * (t0 + a);
+      const bool live = a < nact, hi = lane >= 16;
+      double2 dt = make_double2(0.0, 0.0), p = dt, q = dt;
+      if (live) {
+        dt = make_double2(s_dot[a][0][0], s_dot[a][0][1]);
+        for (int w = 1; w < wpr; ++w) {
+          dt.x += s_dot[a][w][0];
+          dt.y += s_dot[a][w][1];
+        }
+        p = hi ? (i == k + 1 ? make_double2(1.0, 0.0) : zconj(rs[i])) : s_sc.tau;
+        q = hi ? (i == k + 1 ? make_double2(1.0, 0.0) : s_sc.scl) : rows[(size_t)(t0 + a) * n + k + 1];
+      }
+      const double2 z1 = zmul(p, q);                                // tau a0 | v
+      const double2 z2 = zmul(hi ? s_sc.tau : s_ts, hi ? z1 : dt);  // tau scl dot | tau v
+      const double2 x = make_double2(z1.x + z2.x, z1.y + z2.y);
+      const double2 tv = make_double2(__shfl_down_sync(0xffffffffu, z2.x, 16), __shfl_down_sync(0xffffffffu, z2.y, 16));
+      if (live && !hi) {
+        __stcg(xk + i, x);
+        s_x[a] = x;
+      }
+      double g = live && !hi ? -fma(x.x, tv.x, x.y * tv.y) : 0.0;  // -Re(tau conj(x) v)
+      for (int o = nact <= 1 ? 0 : nact <= 2 ? 1 : nact <= 4 ? 2 : 8; o > 0; o >>= 1)
+        g += __shfl_xor_sync(0xffffffffu, g, o);
+      if (lane == 0) __stcg(pk + c, g);
+      if (live && hi) {
+        s_v[a] = z1;
+        vpack[vpack_off(n, k) + i - (k + 1)] = z1;
+      }
+    }
+    td_arrive(count);
+    if (!td_arrived(count, (unsigned)G * (k + 1), err, &s_ok)) return;
+    if (warp < TD_WARPS) {
+      for (int j = k + 1 + tid; j < n; j += 32 * TD_WARPS) {
+        xs[j] = __ldcg(xk + j);
+        rn[j] = __ldcg(rowk + j);
+      }
+    } else {  // gamma, then u conj(scl) of the rows (lanes < 16) and of the next pivot row (lane 16)
+      double g = 0.0;
+      for (int p = lane; p < G; p += 160) {
+        double v[5];
+#pragma unroll
+        for (int u = 0; u < 5; ++u) v[u] = p + 32 * u < G ? __ldcg(pk + p + 32 * u) : 0.0;
+        g += ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+      }
+      const double2 x1 = __ldcg(xk + k + 1);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+      const bool mine = lane < nact, one = lane == 16;
+      const double2 x = mine ? s_x[lane & 15] : x1, v = mine ? s_v[lane & 15] : make_double2(1.0, 0.0);
+      const double2 u = make_double2(fma(g, v.x, x.x), fma(g, v.y, x.y)), us = zmul(u, zconj(s_sc.scl));
+      if (mine) s_us[lane] = us;
+      if (one) {
+        s_us1 = us;
+        if (c == 0) d[k + 1] = __ldcg(rowk + k + 1).x - x1.x - u.x;  // conj(v) = 1 there, and real
+      }
+    }
+    __syncthreads();
+    {  // the next pivot row
+      const double2 us = s_us1;
+      for (int j = k + 2 + tid; j < n; j += TD_THREADS) {
+        const double2 b = rn[j], xj = xs[j], r = rs[j];
+        double re = b.x - xj.x, im = b.y + xj.y;  // b - conj(xj) - us r
+        re = fma(-us.x, r.x, re);
+        re = fma(us.y, r.y, re);
+        im = fma(-us.x, r.y, im);
+        im = fma(-us.y, r.x, im);
+        rn[j] = make_double2(re, im);
+      }
+    }
+    __syncthreads();
+    if (warp == TD_WARPS) {
+      if (k + 2 < n) scalars(k + 1, rn);
+    } else {
+      for (int a = warp / wpr; a < nact; a += rstep) {
+        if (c + G * (t0 + a) == k + 1) continue;
+        double2* row = rows + (size_t)(t0 + a) * n;
+        const double2 v = s_v[a], us = s_us[a];
+        for (int j = k + 2 + 32 * sub + lane; j < n; j += 32 * wpr) {
+          const double2 b = row[j], xj = xs[j], r = rs[j];
+          // b - v conj(xj) - us r
+          double re = fma(-v.x, xj.x, b.x);
+          re = fma(-v.y, xj.y, re);
+          re = fma(-us.x, r.x, re);
+          re = fma(us.y, r.y, re);
+          double im = fma(-v.y, xj.x, b.y);
+          im = fma(v.x, xj.y, im);
+          im = fma(-us.x, r.y, im);
+          im = fma(-us.y, r.x, im);
+          row[j] = make_double2(re, im);
+        }
+      }
+      tc::named_bar(1, 32 * TD_WARPS);  // rows updated, before other warps take them
+    }
+    double2* t = rs;
+    rs = rn;
+    rn = t;
   }
 }
 
@@ -951,9 +1216,11 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
   const size_t iv_scratch = iv_in_smem ? 0 : (size_t)IV_CHUNK * 6 * n * sizeof(double);
   const size_t vpack_bytes = (size_t)n * (n - 1) / 2 * sizeof(double2) + sizeof(double2);
   const size_t part_bytes = (size_t)((n + 7) / 8) * sizeof(double2);
+  const size_t td_part_bytes = (size_t)2 * ctx->sm_count * sizeof(double) + 64;  // partials by parity, barrier count
   const size_t wbytes = 3 * n * sizeof(double2) + vpack_bytes + part_bytes + 3 * n * sizeof(double) + nk * sizeof(double) +
                         (size_t)nk * n * sizeof(double) + iv_scratch + (size_t)nk * n * sizeof(double2) +
-                        (size_t)((n + WY_NB - 1) / WY_NB + 1) * WY_NB * WY_NB * sizeof(double2) + 17 * 64;
+                        (size_t)((n + WY_NB - 1) / WY_NB + 1) * WY_NB * WY_NB * sizeof(double2) +
+                        (size_t)4 * n * sizeof(double2) + td_part_bytes + 19 * 64;
   LITHO_RET(ctx->eig_work.ensure(ctx, wbytes));
   char* w = ctx->eig_work.as<char>();
   auto take = [&](size_t b) {
@@ -975,25 +1242,47 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
   double2* Y = reinterpret_cast<double2*>(take((size_t)nk * n * sizeof(double2)));
   const int wy_blocks = n > 1 ? (n - 1 + WY_NB - 1) / WY_NB : 0;
   double2* Tg = reinterpret_cast<double2*>(take((size_t)(wy_blocks > 0 ? wy_blocks : 1) * WY_NB * WY_NB * sizeof(double2)));
+  double2* td_vec = reinterpret_cast<double2*>(take((size_t)4 * n * sizeof(double2)));  // x and pivot rows, by parity
+  double* td_part = reinterpret_cast<double*>(take(td_part_bytes));
   double2* A = ctx->eig_v.as<double2>();
   {
-    // hermitize, 2 per reflector, last diagonal, e^2, multisection, inverse iteration
-    // (one launch, or one per chunk of IV_CHUNK vectors), cluster Rayleigh-Ritz, WY factors, back-transform
+    // hermitize, reduction (one cooperative launch, or two per reflector, last diagonal and e^2),
+    // multisection, inverse iteration (one launch, or one per chunk of IV_CHUNK vectors), cluster
+    // Rayleigh-Ritz, WY factors, back-transform
     const int iv_launches = iv_in_smem ? 1 : (nk + IV_CHUNK - 1) / IV_CHUNK;
-    StageScope sc(ctx, LITHO_STAGE_EIG, 2 * (n > 1 ? n - 1 : 0) + 6 + (wy_blocks > 0 ? 1 : 0) + iv_launches);
+    const int G = std::min(n, ctx->sm_count);
+    const size_t td_smem = tridiag_smem(n, G);
+    const bool coop = n > 1 && td_smem <= 224 * 1024 && (n + G - 1) / G <= TD_MAX_ROWS;
+    StageScope sc(ctx, LITHO_STAGE_EIG, (coop ? 1 : 2 * n) + 4 + (wy_blocks > 0 ? 1 : 0) + iv_launches);
     hermitize_kernel<<<dim3((n + 127) / 128, n), 128, 0, ctx->stream>>>(static_cast<const double2*>(dtcc), A, n);
     LITHO_CUDA_TRY(ctx, cudaGetLastError());
     LITHO_CUDA_TRY(ctx, cudaMemsetAsync(e, 0, n * sizeof(double), ctx->stream));
-    for (int k = 0; k + 1 < n; ++k) {
-      const int m = n - k - 1;
-      const int nb = (m + 7) / 8;
-      symv_hh_kernel<<<nb, 256, 0, ctx->stream>>>(A, n, k, vbuf, vpack, tau, d, e, xbuf, part);
-      const int nt = (m + 31) / 32;
-      her2_kernel<<<nt * (nt + 1) / 2, 256, 0, ctx->stream>>>(A, n, k, vbuf, xbuf, tau, part, nb);
+    if (coop) {
+      int* err = nullptr;
+      LITHO_RET(tc_err_flag_public(ctx, &err));
+      unsigned* count = reinterpret_cast<unsigned*>(td_part + 2 * G);
+      LITHO_CUDA_TRY(ctx, cudaMemsetAsync(count, 0, sizeof(unsigned), ctx->stream));
+      LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)td_smem));
+      const double2* Ac = A;
+      double2 *xg = td_vec, *rowbuf = td_vec + 2 * (size_t)n;
+      int nn_ = n;
+      void* args[] = {&Ac, &nn_, &vpack, &tau, &d, &e, &e2, &xg, &rowbuf, &td_part, &count, &err};
+      // cooperative: all CTAs are resident at once, as their waits on one another need
+      LITHO_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)tridiag_kernel, dim3(G), dim3(TD_THREADS), args,
+                                                      td_smem, ctx->stream));
+    } else {
+      for (int k = 0; k + 1 < n; ++k) {
+        const int m = n - k - 1;
+        const int nb = (m + 7) / 8;
+        symv_hh_kernel<<<nb, 256, 0, ctx->stream>>>(A, n, k, vbuf, vpack, tau, d, e, xbuf, part);
+        const int nt = (m + 31) / 32;
+        her2_kernel<<<nt * (nt + 1) / 2, 256, 0, ctx->stream>>>(A, n, k, vbuf, xbuf, tau, part, nb);
+      }
+      LITHO_CUDA_TRY(ctx, cudaGetLastError());
+      last_diag_kernel<<<1, 32, 0, ctx->stream>>>(A, n, d);
+      square_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(e, e2, n - 1);
     }
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
-    last_diag_kernel<<<1, 32, 0, ctx->stream>>>(A, n, d);
-    square_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(e, e2, n - 1);
     multisect_kernel<<<nk, MS_THREADS, 0, ctx->stream>>>(d, e, e2, n, nk, ev);
     if (iv_in_smem) {
       LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(invvec_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1039,6 +1328,7 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
     if (scales64)
       LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(scales64, os64, nk * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    LITHO_RET(tc_check_flag(ctx));
     for (int i = 0; i < nk; ++i)
       if (!std::isfinite(scales[i])) {
         set_error(ctx, LITHO_ERR_NAN, "non-finite eigenvalue %d", i);
