@@ -43,12 +43,16 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // T entries of task-chunk blockIdx.x in consumption order, accumulated in FP64 over
-// the kernels in order and rounded once; zero for idle slots.
+// the kernels in order and rounded once; zero for idle slots.  FP64-bound (ten
+// instructions per kernel and entry), so the entries of a chunk are shared out over
+// BT_SLICES CTAs: with one CTA per chunk nine SMs did it all (Nx = Ny = 8, K = 24:
+// 405 -> 40 us; Nx = Ny = 16, where more chunks shared it already: 420 -> 320).
+constexpr int BT_SLICES = 32;
 __global__ void band_tab_kernel(const float2* __restrict__ krn, const float* __restrict__ scales, int nk, int Nx,
                                 int Ny, int nc, float2* __restrict__ tab) {
   const BandTask d = bt_task(blockIdx.x, Nx, Ny, nc);
   const int KX = 2 * Nx + 1, KD = KX * (2 * Ny + 1), NL = 2 * Nx, NS = bt_slots(Nx);
-  for (int e = threadIdx.x; e < d.size; e += blockDim.x) {
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < d.size; e += gridDim.y * blockDim.x) {
     const int j = e % NL, rest = e / NL, sl = rest % NS, rr = rest / NS;
     const int l = rr >= d.npy[0] ? 1 : 0, r = rr - (l ? d.npy[0] : 0);
     const int py0 = l ? d.py0[1] : d.py0[0], fy = l ? d.fy[1] : d.fy[0];
@@ -262,7 +266,7 @@ int build_band_table(litho_ctx* ctx, litho_kernel_set* ks, cudaStream_t stream) 
     set_error(ctx, LITHO_ERR_NOMEM, "band table allocation failed");
     return LITHO_ERR_NOMEM;
   }
-  band_tab_kernel<<<(ks->Ny + 1) * nc, 256, 0, stream>>>(ks->krn, ks->scales, ks->nk, ks->Nx, ks->Ny, nc,
+  band_tab_kernel<<<dim3((ks->Ny + 1) * nc, BT_SLICES), 256, 0, stream>>>(ks->krn, ks->scales, ks->nk, ks->Nx, ks->Ny, nc,
                                                          ks->band_tab);
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   ks->band_nc = nc;
