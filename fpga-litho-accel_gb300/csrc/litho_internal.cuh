@@ -137,7 +137,7 @@ struct litho_ctx {
   // twiddle and coefficient tables keyed by (L, F, N, kind)
   std::map<std::tuple<int, int, int, int>, litho::DevBuf> twx_tables;
   // TCC / eigensolver workspaces
-  litho::DevBuf tcc_a, tcc_b, tcc_c, tcc_pq, eig_w, eig_v, eig_work, eig_info;
+  litho::DevBuf tcc_a, tcc_b, tcc_c, tcc_pq, tcc_part, eig_w, eig_v, eig_work, eig_info;
   // mixed-precision (tensor-core) workspaces
   litho::DevBuf mx_b, mx_c, mx_d;
   // host-buffer batches: copy streams and per-slot events of the staging pipeline

@@ -12,6 +12,7 @@
 // The split-BF16 tensor-core contraction lives in tcc_tc.cu.
 #include "litho_internal.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -68,33 +69,59 @@ __global__ void pupil_kernel(const int2* __restrict__ pq, PupilParams pp, float2
   P[(size_t)id * ldp + s] = v;
 }
 
-// Upper-triangle tiles of TCC in FP64; tile (bi, bj) with bi <= bj.  Each CTA
-// computes a 32 x 32 tile with 256 threads (2 x 2 complex outputs per thread).
+// Upper-triangle tiles of TCC in FP64; tile (bi, bj) with bi <= bj.  Each CTA computes a 32 x 32
+// tile over its share of the sources with 256 threads (2 x 2 complex outputs per thread, one in
+// each 16 x 16 quarter; quarters below the diagonal or past the matrix are skipped).  The FP64
+// units bound it (2 DFMA/clk/SM), so the sources are split over blockIdx.y until every SM has
+// ~ten CTAs (n = 289, ~2,000 sources: 55 tiles on 152 SMs took 2,134 us, the shares take 864; the
+// multiply-adds alone are ~590); the shares' partial tiles
+// are then added in order by tcc_join_kernel.
 constexpr int TT = 32, TK = 16;
 
-__global__ void __launch_bounds__(256) tcc_fp64_kernel(const float2* __restrict__ P, const float* __restrict__ J,
-                                                       int n, int ns, int ldp, double2* __restrict__ tcc) {
-  // map the linear block index onto the upper triangle of the tile grid
-  const int nt = (n + TT - 1) / TT;
-  int b = blockIdx.x, bi = 0;
+__device__ __forceinline__ void tcc_tile(int b, int nt, int& bi, int& bj) {
+  bi = 0;
   while (b >= nt - bi) {
     b -= nt - bi;
     ++bi;
   }
-  const int bj = bi + b;
+  bj = bi + b;
+}
+// entry (i, j) of the upper triangle and its conjugate mirror
+__device__ __forceinline__ void tcc_store(double2* tcc, int n, int i, int j, double2 v) {
+  if (i >= n || j >= n || i > j) return;
+  if (i == j) v.y = 0.0;  // the reference's diagonal sum J|p|^2 is exactly real
+  tcc[(size_t)i * n + j] = v;
+  if (i != j) tcc[(size_t)j * n + i] = make_double2(v.x, -v.y);
+}
+
+// part: [tiles][shares][32][32], or nullptr with one share: straight into tcc
+__global__ void __launch_bounds__(256) tcc_fp64_kernel(const float2* __restrict__ P, const float* __restrict__ J,
+                                                       int n, int ns, int ldp, double2* __restrict__ tcc,
+                                                       double2* __restrict__ part) {
+  // map the linear block index onto the upper triangle of the tile grid
+  int bi, bj;
+  tcc_tile(blockIdx.x, (n + TT - 1) / TT, bi, bj);
   __shared__ double2 sA[TK][TT + 1];
   __shared__ double2 sB[TK][TT + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int i0 = bi * TT, j0 = bj * TT;
+  const int ch = (ns + TK - 1) / TK;
+  const int k0s = (int)((long long)ch * blockIdx.y / gridDim.y) * TK;
+  const int k1s = min(ns, (int)((long long)ch * (blockIdx.y + 1) / gridDim.y) * TK);
+  const bool low = i0 + 16 < n, right = j0 + 16 < n, corner = low && bi != bj;
   double2 acc[2][2];
   for (int a = 0; a < 2; ++a)
     for (int c = 0; c < 2; ++c) acc[a][c] = make_double2(0.0, 0.0);
-  for (int k0 = 0; k0 < ns; k0 += TK) {
+  auto add = [](double2& s, double2 a, double2 b) {  // a * conj(b)
+    s.x = fma(a.x, b.x, fma(a.y, b.y, s.x));
+    s.y = fma(a.y, b.x, fma(-a.x, b.y, s.y));
+  };
+  for (int k0 = k0s; k0 < k1s; k0 += TK) {
     for (int idx = threadIdx.x; idx < TK * TT; idx += 256) {
       const int r = idx / TK, k = idx % TK;
       const int s = k0 + k;
       double2 a = make_double2(0.0, 0.0), bb = make_double2(0.0, 0.0);
-      if (s < ns) {
+      if (s < k1s) {
         const double w = (double)J[s];
         if (i0 + r < n) {
           const float2 t = P[(size_t)(i0 + r) * ldp + s];
@@ -111,27 +138,40 @@ __global__ void __launch_bounds__(256) tcc_fp64_kernel(const float2* __restrict_
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < TK; ++k) {
-      const double2 a0 = sA[k][ty], a1 = sA[k][ty + 16];
-      const double2 b0 = sB[k][tx], b1 = sB[k][tx + 16];
-      const double2 av[2] = {a0, a1}, bv[2] = {b0, b1};
-      for (int a = 0; a < 2; ++a)
-        for (int c = 0; c < 2; ++c) {
-          // a * conj(b)
-          acc[a][c].x = fma(av[a].x, bv[c].x, fma(av[a].y, bv[c].y, acc[a][c].x));
-          acc[a][c].y = fma(av[a].y, bv[c].x, fma(-av[a].x, bv[c].y, acc[a][c].y));
-        }
+      const double2 a0 = sA[k][ty], b0 = sB[k][tx];
+      add(acc[0][0], a0, b0);
+      if (right) add(acc[0][1], a0, sB[k][tx + 16]);
+      if (low) {
+        const double2 a1 = sA[k][ty + 16];
+        if (corner) add(acc[1][0], a1, b0);
+        if (right) add(acc[1][1], a1, sB[k][tx + 16]);
+      }
     }
     __syncthreads();
   }
   for (int a = 0; a < 2; ++a)
     for (int c = 0; c < 2; ++c) {
-      const int i = i0 + ty + 16 * a, j = j0 + tx + 16 * c;
-      if (i >= n || j >= n || i > j) continue;
-      double2 v = acc[a][c];
-      if (i == j) v.y = 0.0;  // the reference's diagonal sum J|p|^2 is exactly real
-      tcc[(size_t)i * n + j] = v;
-      if (i != j) tcc[(size_t)j * n + i] = make_double2(v.x, -v.y);
+      const int r = ty + 16 * a, q = tx + 16 * c;
+      if (part != nullptr) part[((size_t)blockIdx.x * gridDim.y + blockIdx.y) * TT * TT + r * TT + q] = acc[a][c];
+      else tcc_store(tcc, n, i0 + r, j0 + q, acc[a][c]);
     }
+}
+
+// the shares of tile blockIdx.x, added in order; blockIdx.y: a quarter of its entries
+__global__ void __launch_bounds__(256) tcc_join_kernel(const double2* __restrict__ part, int shares, int n,
+                                                       double2* __restrict__ tcc) {
+  int bi, bj;
+  tcc_tile(blockIdx.x, (n + TT - 1) / TT, bi, bj);
+  const int e = blockIdx.y * 256 + threadIdx.x;
+  const double2* p = part + (size_t)blockIdx.x * shares * TT * TT + e;
+  double2 v = make_double2(0.0, 0.0);
+#pragma unroll 8
+  for (int s = 0; s < shares; ++s) {
+    const double2 t = __ldcs(p + (size_t)s * TT * TT);
+    v.x += t.x;
+    v.y += t.y;
+  }
+  tcc_store(tcc, n, bi * TT + e / TT, bj * TT + e % TT, v);
 }
 
 // Host side: enumerate lit source points in the reference's loop order and
@@ -271,9 +311,19 @@ int litho::calc_tcc_impl(litho_ctx* ctx, const float* src, int srcSize, float ou
       if (tccPrecision == LITHO_TCC_SPLIT_BF16) {
         LITHO_RET(tcc_split_bf16(ctx, P, J, n, ns, ldp, out));
       } else {
-        const int nt = (n + TT - 1) / TT;
-        tcc_fp64_kernel<<<nt * (nt + 1) / 2, 256, 0, ctx->stream>>>(P, J, n, ns, ldp, out);
+        const int nt = (n + TT - 1) / TT, tiles = nt * (nt + 1) / 2;
+        const int shares = std::max(1, std::min((ns + 4 * TK - 1) / (4 * TK), (10 * ctx->sm_count + tiles - 1) / tiles));
+        double2* part = nullptr;
+        if (shares > 1) {
+          LITHO_RET(ctx->tcc_part.ensure(ctx, (size_t)tiles * shares * TT * TT * sizeof(double2)));
+          part = ctx->tcc_part.as<double2>();
+        }
+        tcc_fp64_kernel<<<dim3(tiles, shares), 256, 0, ctx->stream>>>(P, J, n, ns, ldp, out, part);
         LITHO_CUDA_TRY(ctx, cudaGetLastError());
+        if (shares > 1) {
+          tcc_join_kernel<<<dim3(tiles, TT * TT / 256), 256, 0, ctx->stream>>>(part, shares, n, out);
+          LITHO_CUDA_TRY(ctx, cudaGetLastError());
+        }
       }
     }
   }
