@@ -15,9 +15,9 @@
 //      arithmetic is written as FMA chains and the update touches each element
 //      pair once.
 //   3. multisect_kernel     the nk largest eigenvalues of the real tridiagonal T
-//                           by Sturm counts, one warp per eigenvalue and one CTA
-//                           per SM: each round evaluates 32 points of the
-//                           bracketing interval at once (33-way multisection);
+//                           by Sturm counts taken from both ends of T, a cluster of
+//                           CTAs per eigenvalue: each round evaluates up to 256
+//                           points of the bracketing interval at once;
 //   4. invvec_kernel        eigenvector j of T by inverse iteration on the
 //                           pivoted tridiagonal LU of T - shift_j I (the dgttrf
 //                           recurrence), one CTA per eigenvector with the LU in
@@ -33,6 +33,8 @@
 // No kernel waits on another; every step is a separate launch on the stream.
 #include "litho_internal.cuh"
 #include "tc_common.cuh"
+
+#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cfloat>
@@ -547,55 +549,88 @@ __global__ void square_kernel(const double* __restrict__ e, double* __restrict__
   if (i < m) e2[i] = e[i] * e[i];
 }
 
-// Number of eigenvalues of T below x: the sign changes of the leading principal
-// minors p_i of T - xI, p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (p_{-1} = 1),
-// i.e. the rows with q_i = p_i / p_{i-1} < 0 of the classical ratio recurrence,
-// without its division per row (a division is some ten FP64 operations, and
-// GB300 issues two FP64 FMAs per clock per SM).  A minor that comes out zero is
-// replaced by -pivmin p_{i-1} (the ratio recurrence's q_i = -pivmin).  p_{i-1},
-// p_i are rescaled together by 2^-256 / 2^256 (exact) when p_i leaves
-// [2^-256, 2^256), so both stay below 2^512 and a step cannot overflow; the
-// test reads the exponent bits on the integer pipe.
-__device__ int sturm_count_lt(const double* d, const double* e2, int n, double x, double pivmin) {
-  int c = 0;
-  double pm = 1.0;       // p_{i-1}
-  double p = d[0] - x;   // p_i
-  if (p == 0.0) p = -pivmin;
-  c += p < 0.0;
-  for (int i = 1; i < n; ++i) {
-    double pn = fma(d[i] - x, p, -e2[i - 1] * pm);
-    if (pn == 0.0) pn = -pivmin * p;
-    c += (__double_as_longlong(pn) ^ __double_as_longlong(p)) < 0;  // sign change
-    pm = p;
-    p = pn;
-    const unsigned ex = (unsigned)(__double_as_longlong(p) >> 52) & 0x7FFu;
-    if (ex - 767u >= 512u) {  // |p| outside [2^-256, 2^256) (or subnormal)
-      const int sh = ex >= 1279u ? -256 : 256;
-      p = ldexp(p, sh);
-      pm = ldexp(pm, sh);
-    }
-  }
-  return c;
+// Number of eigenvalues of T below x (Sylvester's law of inertia on the twisted factorisation
+// of T - xI at row h): the negative pivots of the leading h rows, taken downwards, of the rows
+// past h, taken upwards, and the sign of what both leave at row h.  The two halves are as long and
+// independent, so two lanes share a point: lane l < 16 of a warp goes down, lane l + 16 up, and a
+// count costs half the serial chain of the usual one-way recurrence.
+//
+// A half's pivots are the ratios q_i = p_i / p_{i-1} of its minors, p_i = (d_i - x) p_{i-1} -
+// e_i^2 p_{i-2}, so a negative pivot is a sign change of p.  A row takes three FP64 instructions and
+// nothing else on that pipe: a quarter of an SM issues one warp instruction per ~66 cycles, and a
+// division is ten of them.  Signs, zeros and exponents are read as integers.  A minor that comes out
+// zero is replaced by -pivmin p_{i-1} (the pivot -pivmin).  When a lane's |p_i| leaves
+// [2^-256, 2^256), every lane of the warp brings its p_i towards 1 by a power of two of at most
+// 2^+-256 (exact), p_{i-1} along with it: the lanes of a warp drift alike, so they go rarely together
+// instead of often one by one.  p stays below 2^512, so a step cannot overflow.
+__device__ __noinline__ double2 sturm_rescale(double pn, double p, double m, double pivmin) {
+  if (pn == 0.0) pn = -pivmin * p;
+  const int ex = (int)(((unsigned)__double2hiint(pn) >> 20) & 0x7FFu);
+  const double f = __hiloint2double((1023 + max(-256, min(256, 1023 - ex))) << 20, 0);
+  return make_double2(pn * f, m * f);
 }
 
-// eigenvalue j (0 = largest) of T (diagonal d, off-diagonal e) by multisection:
-// one CTA of MS_THREADS per eigenvalue (blockIdx.x); every round evaluates the Sturm
-// count at MS_THREADS interior points of the bracket [lo, hi], count(lo) <= m <
-// count(hi) with m the ascending index, and keeps the sub-interval holding the
-// crossing.  A Sturm count is a sequential FP64 recurrence with a division per row,
-// so one count is latency-bound; the points of a round run side by side, and a
-// 129-way split needs ~8 rounds where bisection needs ~52.  The rounds stop when the
-// bracket no longer shrinks in floating point.
-constexpr int MS_THREADS = 128;
+__device__ __forceinline__ int sturm_count_lt(const double* __restrict__ d, const double* __restrict__ e2, int n,
+                                              double x, double pivmin, int lane) {
+  const bool up = lane & 16;
+  const int h = (n - 1) / 2, step = up ? -1 : 1;  // rows past h: h, or h + 1 where n is even
+  const double* pd = up ? d + (n - 1) : d;        // the half's row i: pd[step i]
+  const double* pe = up ? e2 + (n - 2) : e2;      // its coupling to the next row (the last one's: to row h)
+  int c = 0;
+  double p = 1.0, m = 0.0, a = *pd - x;  // p_{i-1}, e_{i-1}^2 p_{i-2}, d_i - x
+  // a row ahead of their use: a load takes longer than a row leaves it
+  double d1 = n > 1 ? pd[step] : 0.0, e1 = n > 1 ? *pe : 0.0;
+  for (int i = 0; i < h; ++i) {
+    const double dn = d1, en = e1;
+    d1 = pd[step * (i + 2)];
+    e1 = pe[step * (i + 1)];
+    double pn = fma(a, p, -m);
+    a = dn - x;
+    m = en * p;  // these two don't wait for pn, so the pipe is never idle
+    // outside [2^-256, 2^256), zero or subnormal
+    const bool out = (((unsigned)__double2hiint(pn) >> 20) & 0x7FFu) - 767u >= 512u;
+    if (__any_sync(0xffffffffu, out)) {
+      const double2 r = sturm_rescale(pn, p, m, pivmin);
+      pn = r.x;
+      m = r.y;
+    }
+    c += (unsigned)(__double2hiint(pn) ^ __double2hiint(p)) >> 31;
+    p = pn;
+  }
+  if (up && n - 1 - h > h) {
+    double pn = fma(a, p, -m);
+    m = e1 * p;
+    if (pn == 0.0) pn = -pivmin * p;
+    c += (unsigned)(__double2hiint(pn) ^ __double2hiint(p)) >> 31;
+    p = pn;
+  }
+  // row h: (d_h - x) - e_{h-1}^2 / q_{h-1} - e_h^2 / q_{h+1}
+  const double q = m / p;  // 0 for a half without rows
+  const double qo = __shfl_xor_sync(0xffffffffu, q, 16);
+  c += __shfl_xor_sync(0xffffffffu, c, 16);
+  return c + (((d[h] - x) - (up ? qo : q)) - (up ? q : qo) < 0.0 ? 1 : 0);
+}
+
+// eigenvalue j (0 = largest) of T (diagonal d, off-diagonal e) by multisection: one cluster of C CTAs
+// per eigenvalue; every round evaluates the Sturm count at 64 C interior points of the bracket
+// [lo, hi], count(lo) <= m < count(hi) with m the ascending index, and keeps the sub-interval
+// holding the crossing.  A count is a serial FP64 chain, the points of a round run side by side, one
+// warp on each quarter of an SM (a second one there would wait for the first), so a round over four
+// SMs gains log2(257) bits where bisection gains one.  The rounds stop when the bracket no longer
+// shrinks in floating point.
+// 24 eigenvalues, n = 289: 940 -> 202 us; n = 1089: 3,502 -> 708 us.
+constexpr int MS_THREADS = 128, MS_POINTS = MS_THREADS / 2, MS_CMAX = 4;
 
 __global__ void __launch_bounds__(MS_THREADS) multisect_kernel(const double* __restrict__ d,
                                                                const double* __restrict__ e,
-                                                               const double* __restrict__ e2, int n, int nk,
+                                                               const double* __restrict__ e2, int n,
                                                                double* __restrict__ evals) {
+  namespace cg = cooperative_groups;
   __shared__ double sh[3][MS_THREADS / 32];
-  __shared__ unsigned masks[MS_THREADS / 32];
-  const int j = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (j >= nk) return;
+  __shared__ unsigned masks[2][MS_CMAX][MS_THREADS / 32];  // by parity of the round: 16 points a warp
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int j = blockIdx.x / C, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   double lo = 1e300, hi = -1e300, emax = 0.0;
   for (int i = t; i < n; i += MS_THREADS) {
     const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
@@ -625,26 +660,34 @@ __global__ void __launch_bounds__(MS_THREADS) multisect_kernel(const double* __r
   hi += 2.0 * DBL_EPSILON * span + 1e-300;
   const double pivmin = 1e-290 * fmax(1.0, emax);
   const int m = n - 1 - j;  // ascending index
+  const int points = MS_POINTS * C;
+  const int mine = rank * MS_POINTS + warp * 16 + (lane & 15);
+  cl.sync();  // every CTA of the cluster runs before its shared memory is written
   for (int it = 0; it < 64; ++it) {
     // every thread evaluates the same expressions, so lo, hi stay identical in all
-    const double w = (hi - lo) / (double)(MS_THREADS + 1);
-    const double x = lo + w * (double)(t + 1);
-    const bool above = x > lo && x < hi && sturm_count_lt(d, e2, n, x, pivmin) > m;
-    const unsigned up = __ballot_sync(0xffffffffu, above);
-    __syncthreads();  // the previous round's masks have been read
-    if (lane == 0) masks[warp] = up;
-    __syncthreads();
+    const double mid = 0.5 * (lo + hi);
+    if (!(mid > lo && mid < hi)) break;  // neighbours: no point between them
+    const double w = (hi - lo) / (double)(points + 1);
+    const double x = lo + w * (double)(mine + 1);
+    const bool in = x > lo && x < hi;
+    const bool above = sturm_count_lt(d, e2, n, in ? x : lo, pivmin, lane) > m && in;
+    const unsigned up = __ballot_sync(0xffffffffu, above) & 0xffffu;
+    if (lane < C) *cl.map_shared_rank(&masks[it & 1][rank][warp], lane) = up;
+    cl.sync();  // the masks of every CTA; those of the round before last are no longer read
     // counts grow with the point index: the first point above m
-    int f = MS_THREADS;
-    for (int ww = MS_THREADS / 32 - 1; ww >= 0; --ww)
-      if (masks[ww]) f = 32 * ww + __ffs(masks[ww]) - 1;
+    int f = points;
+    for (int c = C - 1; c >= 0; --c)
+      for (int ww = MS_THREADS / 32 - 1; ww >= 0; --ww) {
+        const unsigned u = masks[it & 1][c][ww];
+        if (u) f = c * MS_POINTS + 16 * ww + __ffs(u) - 1;
+      }
     const double nlo = f == 0 ? lo : lo + w * (double)f;
-    const double nhi = f == MS_THREADS ? hi : lo + w * (double)(f + 1);
+    const double nhi = f == points ? hi : lo + w * (double)(f + 1);
     if (!(nhi - nlo < hi - lo)) break;  // no progress: the bracket is a few ulps wide
     lo = nlo;
     hi = nhi;
   }
-  if (t == 0) evals[j] = 0.5 * (lo + hi);
+  if (rank == 0 && t == 0) evals[j] = 0.5 * (lo + hi);
 }
 
 // Eigenvector j of T by inverse iteration, one CTA per eigenvector.  Inside a
@@ -1190,6 +1233,24 @@ __global__ void output_kernel(const double2* __restrict__ Y, const double* __res
   }
 }
 
+// `groups` clusters of C CTAs each
+template <typename... P, typename... A>
+static cudaError_t launch_clusters(void (*k)(P...), int groups, int C, int threads, size_t smem, cudaStream_t stream,
+                                   A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)C;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(groups * C));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 }  // namespace litho
 
 using namespace litho;
@@ -1283,7 +1344,9 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
       last_diag_kernel<<<1, 32, 0, ctx->stream>>>(A, n, d);
       square_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(e, e2, n - 1);
     }
-    multisect_kernel<<<nk, MS_THREADS, 0, ctx->stream>>>(d, e, e2, n, nk, ev);
+    // four SMs per eigenvalue while there are as many; further eigenvalues take one each
+    LITHO_CUDA_TRY(ctx, launch_clusters(multisect_kernel, nk, nk * MS_CMAX <= ctx->sm_count ? MS_CMAX : 1, MS_THREADS, 0,
+                                        ctx->stream, (const double*)d, (const double*)e, (const double*)e2, n, ev));
     if (iv_in_smem) {
       LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(invvec_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)iv_smem));
