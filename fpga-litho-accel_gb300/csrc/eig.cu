@@ -342,6 +342,15 @@ __device__ __forceinline__ double pair_sum(double re, double im, int lane) {
   return v;
 }
 
+// the same over each half of the warp by itself: re in the half's first eight lanes, im in its last
+__device__ __forceinline__ double half_pair_sum(double re, double im, int lane) {
+  const bool up = lane & 8;
+  double v = (up ? im : re) + __shfl_xor_sync(0xffffffffu, up ? re : im, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // the reflector of a pivot row with pivot alpha = conj(first) and squared norm xn2 past it: the
 // zlarfg scalars, the two reciprocals side by side in lanes 0 and 1 (whole warp)
 struct TdScalars {
@@ -1080,27 +1089,31 @@ __global__ void __launch_bounds__(RR_THREADS) cluster_rr_kernel(const double* __
   }
 }
 
-// y = H_0 H_1 ... H_{n-2} z for eigenvector j = blockIdx.x; H_k = I - tau_k v_k v_k^H
-// acting on rows k+1..n-1, v_k packed contiguously in vpack.
-// y_j = H_0 H_1 ... H_{n-2} z_j for every eigenvector j, with the reflectors taken
-// WY_NB at a time in compact WY form: H_k0 ... H_{k0+nb-1} = I - V T V^H (V the
-// block's reflectors as columns, T upper triangular: T_jj = tau_j,
-// T[0:j, j] = -tau_j T[0:j, 0:j] (V[:, 0:j]^H v_j)), so a block costs three block
-// barriers (w = V^H y reduced over the CTA, u = T w, y -= V u) instead of one per
-// reflector, for the same FP64 work.
-constexpr int WY_NB = 16;
+// y_j = H_0 H_1 ... H_{n-2} z_j for every eigenvector j; H_k = I - tau_k v_k v_k^H acting on rows
+// k+1..n-1, v_k packed contiguously in vpack.  The reflectors are taken WY_NB at a time in compact
+// WY form: H_k0 ... H_{k0+nb-1} = I - V T V^H (V the block's reflectors as columns, T upper
+// triangular: T_jj = tau_j, T[0:j, j] = -tau_j T[0:j, 0:j] (V[:, 0:j]^H v_j)), so a block costs one
+// exchange (w = V^H y summed over the rows, u = T w, y -= V u) instead of one per reflector, for
+// the same FP64 work.
+constexpr int WY_NB = 16, WY_THREADS = 256, WY_CLUSTER = 4;
 
-// T of every block (one CTA per block): the Gram products v_i^H v_j (i < j, over
-// v_j's support) one warp per pair, then the triangular recurrence on one thread
-__global__ void __launch_bounds__(256) wy_t_kernel(const double2* __restrict__ vpack,
-                                                   const double2* __restrict__ tau, int n,
-                                                   double2* __restrict__ Tg) {
-  __shared__ double2 G[WY_NB][WY_NB];
-  __shared__ double2 T[WY_NB][WY_NB];
-  const int b = blockIdx.x, k0 = b * WY_NB, nbb = min(WY_NB, n - 1 - k0);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// T of every block (one cluster per block): the Gram products v_i^H v_j (i < j, over v_j's support)
+// one warp per pair, the pairs shared out over the cluster; then the triangular recurrence, a column
+// at a time over the rows and summands, in the first CTA.  FP64-bound: one CTA per block, with the
+// recurrence on one thread, took 242 us at n = 289 and 340 at n = 1089; this takes 33 and 87.
+__global__ void __launch_bounds__(WY_THREADS) wy_t_kernel(const double2* __restrict__ vpack,
+                                                          const double2* __restrict__ tau, int n,
+                                                          double2* __restrict__ Tg) {
+  namespace cg = cooperative_groups;
+  __shared__ double G[WY_NB][WY_NB][2];
+  __shared__ double2 T[WY_NB][WY_NB + 1];
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int b = blockIdx.x / C, k0 = b * WY_NB, nbb = min(WY_NB, n - 1 - k0);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int np = nbb * (nbb - 1) / 2;
-  for (int p = warp; p < np; p += 8) {
+  cl.sync();  // every CTA of the cluster runs before its shared memory is written
+  for (int p = warp * C + rank; p < np; p += WY_THREADS / 32 * C) {
     int j = 1;
     while ((j + 1) * j / 2 <= p) ++j;  // p = j (j - 1) / 2 + i, i < j
     const int i = p - j * (j - 1) / 2;
@@ -1108,111 +1121,136 @@ __global__ void __launch_bounds__(256) wy_t_kernel(const double2* __restrict__ v
     const double2* vi = vpack + vpack_off(n, ki) - (ki + 1);  // v_i[r], r in [ki+1, n)
     const double2* vj = vpack + vpack_off(n, kj) - (kj + 1);
     double sr = 0.0, si = 0.0;  // conj(v_i) . v_j
+#pragma unroll 4
     for (int r = kj + 1 + lane; r < n; r += 32) {
       const double2 a = vi[r], c = vj[r];
       sr = fma(a.x, c.x, fma(a.y, c.y, sr));
       si = fma(a.x, c.y, fma(-a.y, c.x, si));
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sr += __shfl_xor_sync(0xffffffffu, sr, o);
-      si += __shfl_xor_sync(0xffffffffu, si, o);
-    }
-    if (lane == 0) G[i][j] = make_double2(sr, si);
+    const double v = pair_sum(sr, si, lane);
+    if ((lane & 15) == 0) *cl.map_shared_rank(&G[i][j][lane >> 4], 0) = v;
   }
+  cl.sync();
+  if (rank != 0) return;
+  const int ii = t >> 4, l = t & 15;
+  T[ii][l] = ii == l && ii < nbb ? tau[k0 + ii] : make_double2(0.0, 0.0);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int jj = 0; jj < WY_NB; ++jj)
-      for (int ii = 0; ii < WY_NB; ++ii) T[ii][jj] = make_double2(0.0, 0.0);
-    for (int jj = 0; jj < nbb; ++jj) {
-      const double2 tj = tau[k0 + jj];
-      T[jj][jj] = tj;
-      for (int ii = 0; ii < jj; ++ii) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int l = ii; l < jj; ++l) {
-          const double2 t = T[ii][l], g = G[l][jj];
-          acc.x += t.x * g.x - t.y * g.y;
-          acc.y += t.x * g.y + t.y * g.x;
-        }
-        T[ii][jj] = make_double2(-(tj.x * acc.x - tj.y * acc.y), -(tj.x * acc.y + tj.y * acc.x));
-      }
+  for (int jj = 1; jj < nbb; ++jj) {
+    double2 z = make_double2(0.0, 0.0);
+    if (ii <= l && l < jj) z = zmul(T[ii][l], make_double2(G[l][jj][0], G[l][jj][1]));
+    const double s = half_pair_sum(z.x, z.y, lane);
+    const double im = __shfl_down_sync(0xffffffffu, s, 8);
+    const double2 tj = T[jj][jj];
+    if (l == 0 && ii < jj) {
+      const double2 v = zmul(tj, make_double2(s, im));
+      T[ii][jj] = make_double2(-v.x, -v.y);
     }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < WY_NB * WY_NB; e += 256) Tg[(size_t)b * WY_NB * WY_NB + e] = T[e / WY_NB][e % WY_NB];
+  Tg[(size_t)b * WY_NB * WY_NB + t] = T[ii][l];
 }
 
-// one CTA per vector; thread t owns the elements y[t + 256 s] for the whole loop
-__global__ void __launch_bounds__(256) backtransform_kernel(const double2* __restrict__ vpack, int n,
-                                                            const double2* __restrict__ Tg,
-                                                            const double* __restrict__ Z, double2* __restrict__ Y) {
-  __shared__ double2 red[8][WY_NB];
+// One cluster of CTAs per vector; the rows go to the CTAs 32 at a time in turn, which spreads the
+// shrinking support of the reflectors evenly, and stay in shared memory for the whole loop.  Per
+// block: each warp forms two entries of w over the CTA's rows, the CTAs exchange the partial w
+// through the cluster's shared memory (one cluster barrier; two buffers, by parity), every CTA forms u,
+// and each warp updates 32 rows.  FP64-bound (a quarter of an SM issues one warp instruction per ~66
+// cycles), so a vector takes as many SMs as there are for it; on one SM each, 24 vectors took 467 us
+// at n = 289 and 2,674 at n = 1089, now 144 and 648.
+constexpr int BK_CMAX = 8;
+
+size_t backtransform_smem(int n, int C) {
+  const int chunks = (n + 31) / 32;
+  return (size_t)((chunks + C - 1) / C) * 32 * sizeof(double2);
+}
+
+__global__ void __launch_bounds__(WY_THREADS) backtransform_kernel(const double2* __restrict__ vpack, int n,
+                                                                   const double2* __restrict__ Tg,
+                                                                   const double* __restrict__ Z,
+                                                                   double2* __restrict__ Y) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) double2 s_y[];          // [local chunk][32]
+  __shared__ double s_part[2][BK_CMAX][2 * WY_NB];        // w of every CTA: re, im interleaved
   __shared__ double2 s_w[WY_NB], s_u[WY_NB];
-  __shared__ long long s_base[WY_NB];  // v_i[r] = vpack[s_base[i] + r]
-  const int j = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
-  double2* y = Y + (size_t)j * n;
-  for (int i = t; i < n; i += 256) y[i] = make_double2(Z[(size_t)j * n + i], 0.0);
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int j = blockIdx.x / C, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int chunks = (n + 31) / 32;
+  const int mine = (chunks - rank + C - 1) / C;  // chunks rank, rank + C, ...
+  for (int q = warp; q < mine; q += WY_THREADS / 32) {
+    const int r = (rank + q * C) * 32 + lane;
+    s_y[q * 32 + lane] = make_double2(r < n ? Z[(size_t)j * n + r] : 0.0, 0.0);
+  }
+  cl.sync();  // s_y; also, every CTA of the cluster runs before its shared memory is written
   const int nblk = (n - 1 + WY_NB - 1) / WY_NB;
   for (int b = nblk - 1; b >= 0; --b) {
     const int k0 = b * WY_NB, nbb = min(WY_NB, n - 1 - k0);
-    if (t < WY_NB) s_base[t] = t < nbb ? (long long)vpack_off(n, k0 + t) - (k0 + t + 1) : 0;
-    __syncthreads();  // s_base; also, every thread is past the previous block's reads of s_u
-    int r0 = t;
-    if (r0 < k0 + 1) r0 += ((k0 + 1 - r0 + 255) / 256) * 256;
-    double ar[WY_NB], ai[WY_NB];
-#pragma unroll
-    for (int i = 0; i < WY_NB; ++i) ar[i] = ai[i] = 0.0;
-    for (int r = r0; r < n; r += 256) {
-      const double2 yy = y[r];
-#pragma unroll
-      for (int i = 0; i < WY_NB; ++i)
-        if (i < nbb && r > k0 + i) {
-          const double2 vv = vpack[s_base[i] + r];
-          ar[i] = fma(vv.x, yy.x, fma(vv.y, yy.y, ar[i]));  // conj(v) * y
-          ai[i] = fma(vv.x, yy.y, fma(-vv.y, yy.x, ai[i]));
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < WY_NB; ++i) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        ar[i] += __shfl_xor_sync(0xffffffffu, ar[i], o);
-        ai[i] += __shfl_xor_sync(0xffffffffu, ai[i], o);
+    // the first local chunk that reaches past row k0 (c = rank + q C with 32 c + 31 > k0)
+    const int cf = (k0 + 1) / 32, q0 = max(0, (cf - rank + C - 1) / C);
+    const double2 tv = Tg[(size_t)b * WY_NB * WY_NB + t];
+    {
+      const int i0 = 2 * warp, i1 = i0 + 1;
+      // v_i[r] = vpack[base_i + r] for r in (k0 + i, n)
+      const double2* v0 = vpack + ((long long)vpack_off(n, k0 + (i0 < nbb ? i0 : 0)) - (k0 + (i0 < nbb ? i0 : 0) + 1));
+      const double2* v1 = vpack + ((long long)vpack_off(n, k0 + (i1 < nbb ? i1 : 0)) - (k0 + (i1 < nbb ? i1 : 0) + 1));
+      const int f0 = i0 < nbb ? k0 + i0 : n, f1 = i1 < nbb ? k0 + i1 : n;
+      double a0r = 0.0, a0i = 0.0, a1r = 0.0, a1i = 0.0;
+#pragma unroll 3
+      for (int q = q0; q < mine; ++q) {
+        const int r = (rank + q * C) * 32 + lane;
+        const double2 yy = s_y[q * 32 + lane];
+        double2 p = make_double2(0.0, 0.0), s = p;
+        if (r > f0 && r < n) p = v0[r];
+        if (r > f1 && r < n) s = v1[r];
+        a0r = fma(p.x, yy.x, fma(p.y, yy.y, a0r));  // conj(v) y
+        a0i = fma(p.x, yy.y, fma(-p.y, yy.x, a0i));
+        a1r = fma(s.x, yy.x, fma(s.y, yy.y, a1r));
+        a1i = fma(s.x, yy.y, fma(-s.y, yy.x, a1i));
       }
-      if (lane == 0) red[w][i] = make_double2(ar[i], ai[i]);
+      // reflector i0 in lanes 0-15, i1 in 16-31, then their re and im in halves of those
+      const bool hi = lane & 16;
+      const double kr = (hi ? a1r : a0r) + __shfl_xor_sync(0xffffffffu, hi ? a0r : a1r, 16);
+      const double ki = (hi ? a1i : a0i) + __shfl_xor_sync(0xffffffffu, hi ? a0i : a1i, 16);
+      const double v = half_pair_sum(kr, ki, lane);
+      // every lane of a group of eight holds its sum: lane c of the group writes to CTA c
+      const int c = lane & 7;
+      if (c < C) *cl.map_shared_rank(&s_part[b & 1][rank][4 * warp + (lane >> 3)], c) = v;
+    }
+    cl.sync();  // the parts of this block; nobody still reads those of the block before last
+    if (t < 2 * WY_NB) {
+      double v = s_part[b & 1][0][t];
+      for (int c = 1; c < C; ++c) v += s_part[b & 1][c][t];
+      reinterpret_cast<double*>(s_w)[t] = v;
     }
     __syncthreads();
-    if (t < WY_NB) {
-      double2 sm = red[0][t];
-      for (int q = 1; q < 8; ++q) {
-        sm.x += red[q][t].x;
-        sm.y += red[q][t].y;
-      }
-      s_w[t] = sm;
+    {  // u = T w: row t / 16, summand t % 16 (T is zero below its diagonal and past nbb)
+      const double2 z = zmul(tv, s_w[t & 15]);
+      const double s = half_pair_sum(z.x, z.y, lane);
+      if ((lane & 7) == 0) reinterpret_cast<double*>(s_u)[2 * (t >> 4) + ((lane >> 3) & 1)] = s;
     }
     __syncthreads();
-    if (t < WY_NB) {  // u = T w (T upper triangular)
-      const double2* Tb = Tg + (size_t)b * WY_NB * WY_NB + (size_t)t * WY_NB;
-      double2 u = make_double2(0.0, 0.0);
-      for (int l = t; l < nbb; ++l) {
-        const double2 a = Tb[l], c = s_w[l];
-        u.x += a.x * c.x - a.y * c.y;
-        u.y += a.x * c.y + a.y * c.x;
-      }
-      s_u[t] = u;
-    }
-    __syncthreads();
-    for (int r = r0; r < n; r += 256) {  // y -= V u
-      double2 yy = y[r];
+    for (int q = q0 + warp; q < mine; q += WY_THREADS / 32) {  // y -= V u
+      const int r = (rank + q * C) * 32 + lane;
+      double2 yy = s_y[q * 32 + lane];
+      const double2* v = vpack + ((long long)vpack_off(n, k0) - (k0 + 1)) + r;
 #pragma unroll
-      for (int i = 0; i < WY_NB; ++i)
-        if (i < nbb && r > k0 + i) {
-          const double2 vv = vpack[s_base[i] + r], u = s_u[i];
+      for (int i = 0; i < WY_NB; ++i) {
+        if (i < nbb) {
+          double2 vv = make_double2(0.0, 0.0);
+          if (r > k0 + i && r < n) vv = *v;
+          const double2 u = s_u[i];
           yy.x = fma(-u.x, vv.x, fma(u.y, vv.y, yy.x));
           yy.y = fma(-u.x, vv.y, fma(-u.y, vv.x, yy.y));
+          v += n - 2 - (k0 + i);  // the next reflector starts one row later and is one shorter
         }
-      y[r] = yy;
+      }
+      s_y[q * 32 + lane] = yy;
     }
+    __syncthreads();
+  }
+  for (int q = warp; q < mine; q += WY_THREADS / 32) {
+    const int r = (rank + q * C) * 32 + lane;
+    if (r < n) Y[(size_t)j * n + r] = s_y[q * 32 + lane];
   }
 }
 
@@ -1356,8 +1394,18 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
         invvec_kernel<false><<<std::min(IV_CHUNK, nk - j0), IV_THREADS, 0, ctx->stream>>>(d, e, n, j0, ev, Z, ivs);
     }
     cluster_rr_kernel<<<nk, RR_THREADS, 0, ctx->stream>>>(d, e, n, nk, ev, Z);
-    if (wy_blocks > 0) wy_t_kernel<<<wy_blocks, 256, 0, ctx->stream>>>(vpack, tau, n, Tg);
-    backtransform_kernel<<<nk, 256, 0, ctx->stream>>>(vpack, n, Tg, Z, Y);
+    const double2 *cvpack = vpack, *ctau = tau, *cTg = Tg;
+    if (wy_blocks > 0)
+      LITHO_CUDA_TRY(ctx, launch_clusters(wy_t_kernel, wy_blocks, WY_CLUSTER, WY_THREADS, 0, ctx->stream, cvpack, ctau, n, Tg));
+    // as many SMs per vector as there are, up to the portable cluster size and the row chunks; a fifth
+    // of the SMs is left, as clusters don't fill every GPC (24 vectors, n = 1089: 648 us on clusters
+    // of five, 783 on six and 710 on four)
+    const int bc = std::max(1, std::min({BK_CMAX, ctx->sm_count * 4 / 5 / nk, (n + 31) / 32}));
+    const size_t bt_smem = backtransform_smem(n, bc);
+    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(backtransform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)bt_smem));
+    LITHO_CUDA_TRY(ctx, launch_clusters(backtransform_kernel, nk, bc, WY_THREADS, bt_smem, ctx->stream, cvpack, n, cTg,
+                                        (const double*)Z, Y));
     LITHO_CUDA_TRY(ctx, cudaGetLastError());
   }
   float *okr = krn_r, *oki = krn_i, *osc = scales;
