@@ -705,7 +705,11 @@ __global__ void __launch_bounds__(MS_THREADS) multisect_kernel(const double* __r
 // and rotated afterwards (cluster_rr_kernel).  Thread 0 runs the pivoted
 // tridiagonal LU of T - shift I (the dgttrf recurrence) and the triangular solves,
 // which are sequential by nature, on arrays in shared memory (or in this CTA's
-// slice of global scratch when n is large); the CTA normalises between iterations.
+// slice of global scratch when n is large); the CTA does what is not.
+// Thread 0's chain bounds it: an FP64 instruction takes ~66 cycles and a division ten of them, so
+// the LU's recurrence carries numerators over a common denominator (four instructions a row, the
+// divisions follow side by side), the solves' rows carry one and two, and operands are loaded a
+// row ahead.  24 vectors, n = 289: 477 -> 279 us; n = 1089: 1,757 -> 1,002 us.
 constexpr int IV_THREADS = 128;
 constexpr int IV_ITERS = 4;
 
@@ -737,9 +741,9 @@ __global__ void __launch_bounds__(IV_THREADS) invvec_kernel(const double* __rest
   const int j = j0 + blockIdx.x;
   double* base = SMEM ? ivs : scratch + (size_t)blockIdx.x * 6 * n;
   double* dl = base;           // L multipliers
-  double* dd = base + n;       // U diagonal (its reciprocal after the factorisation)
-  double* du = base + 2 * n;   // U first super-diagonal
-  double* du2 = base + 3 * n;  // U second super-diagonal
+  double* dd = base + n;       // U diagonal, as its reciprocal
+  double* du = base + 2 * n;   // U first super-diagonal, over the diagonal
+  double* du2 = base + 3 * n;  // U second super-diagonal, over the diagonal
   double* z = base + 4 * n;
   unsigned char* pivb = reinterpret_cast<unsigned char*>(base + 5 * n);  // SMEM: bytes
   double* pivd = base + 5 * n;                                           // global: doubles
@@ -770,63 +774,101 @@ __global__ void __launch_bounds__(IV_THREADS) invvec_kernel(const double* __rest
     z[i] = ((double)(h & 0xffffff) / 16777216.0) - 0.5;
   }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < n; ++i) {
-      dd[i] = d[i] - lam;
-      du[i] = i < n - 1 ? e[i] : 0.0;
-      dl[i] = i < n - 1 ? e[i] : 0.0;
-      du2[i] = 0.0;
-    }
+    // row i of U before its elimination: a / s on the diagonal, b / s past it
+    double a = d[0] - lam, b = n > 1 ? e[0] : 0.0, s = 1.0;
+    double l = b, dn = n > 1 ? d[1] : 0.0;  // e[i], d[i + 1]
     for (int i = 0; i < n - 1; ++i) {
-      bool sw = false;
-      if (fabs(dd[i]) >= fabs(dl[i])) {
-        if (dd[i] == 0.0) dd[i] = tiny;
-        const double f = dl[i] / dd[i];
-        dl[i] = f;
-        dd[i + 1] -= f * du[i];
-        du2[i] = 0.0;
-      } else {
-        const double f = dd[i] / dl[i];
-        dd[i] = dl[i];
-        dl[i] = f;
-        const double t = du[i];
-        du[i] = dd[i + 1];
-        dd[i + 1] = t - f * dd[i + 1];
-        if (i < n - 2) {
-          du2[i] = du[i + 1];
-          du[i + 1] = -f * du[i + 1];
-        }
-        sw = true;
-      }
+      const double un = i < n - 2 ? e[i + 1] : 0.0, dnn = i < n - 2 ? d[i + 2] : 0.0;
+      const double g = l * s;
+      const long long ab = __double_as_longlong(a) & 0x7fffffffffffffffll,
+                      gb = __double_as_longlong(g) & 0x7fffffffffffffffll;
+      const bool sw = ab < gb;  // |a / s| < |e[i]|
+      if (!sw && ab == 0) a = tiny * s;
+      dd[i] = a;
+      du[i] = b;
+      dl[i] = s;
       if (SMEM) pivb[i] = sw ? 1 : 0;
       else pivd[i] = sw ? 1.0 : 0.0;
+      // kept: (dn a - l b) / a, un a / a; exchanged: (b l - a dn) / (s l), -a un / (s l)
+      const long long flip = sw ? (long long)0x8000000000000000ull : 0;
+      const double na = fma(dn - lam, a, -(l * b)), nb = un * a;
+      s = sw ? g : a;
+      a = __longlong_as_double(__double_as_longlong(na) ^ flip);
+      b = __longlong_as_double(__double_as_longlong(nb) ^ flip);
+      const unsigned ex = ((unsigned)__double2hiint(s) >> 20) & 0x7FFu;
+      if (ex - 767u >= 512u) {  // s outside [2^-256, 2^256): all three by a power of two (exact)
+        const double f = ex >= 1279u ? 0x1p-256 : 0x1p256;
+        a *= f;
+        b *= f;
+        s *= f;
+      }
+      l = un;
+      dn = dnn;
     }
-    if (dd[n - 1] == 0.0) dd[n - 1] = tiny;
+    dd[n - 1] = a;
+    dl[n - 1] = s;
   }
   __syncthreads();
-  // U's diagonal, clamped away from zero, is kept as its reciprocal: the serial
-  // back substitutions multiply (an FP64 division is a multi-instruction sequence,
-  // and GB300 issues two FP64 operations per clock per SM)
+  // the multipliers; U's rows over their diagonal (clamped away from zero) and its reciprocal
   for (int i = threadIdx.x; i < n; i += IV_THREADS) {
-    double v = dd[i];
+    const double s = dl[i], a = dd[i], b = du[i];
+    const bool sw = i < n - 1 && (SMEM ? pivb[i] != 0 : pivd[i] != 0.0);
+    double v = a / s, f = 0.0, u = 0.0, u2 = 0.0;
+    if (sw) {
+      f = v / e[i];
+      v = e[i];
+      u = d[i + 1] - lam;
+      u2 = i < n - 2 ? e[i + 1] : 0.0;
+    } else {
+      if (v == 0.0) v = tiny;
+      if (i < n - 1) {
+        f = e[i] / v;
+        u = b / s;
+      }
+    }
     if (fabs(v) < tiny) v = v < 0.0 ? -tiny : tiny;
-    dd[i] = 1.0 / v;
+    const double r = 1.0 / v;
+    dl[i] = f;
+    dd[i] = r;
+    du[i] = u * r;
+    du2[i] = u2 * r;
   }
   __syncthreads();
   for (int it = 0; it < IV_ITERS; ++it) {
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0) {  // L
+      double cur = z[0], zn = z[min(1, n - 1)], f = dl[0];
+      bool sw = n > 1 && (SMEM ? pivb[0] != 0 : pivd[0] != 0.0);
       for (int i = 0; i < n - 1; ++i) {
-        const bool sw = SMEM ? pivb[i] != 0 : pivd[i] != 0.0;
-        if (!sw) {
-          z[i + 1] -= dl[i] * z[i];
-        } else {
-          const double t = z[i];
-          z[i] = z[i + 1];
-          z[i + 1] = t - dl[i] * z[i];
-        }
+        const int i1 = min(i + 1, n - 2);
+        const double zn2 = z[min(i + 2, n - 1)], f1 = dl[i1];
+        const bool sw1 = SMEM ? pivb[i1] != 0 : pivd[i1] != 0.0;
+        const double p = sw ? zn : cur, q = sw ? cur : zn;
+        z[i] = p;
+        cur = fma(-f, p, q);
+        zn = zn2;
+        f = f1;
+        sw = sw1;
       }
-      z[n - 1] *= dd[n - 1];
-      if (n > 1) z[n - 2] = (z[n - 2] - du[n - 2] * z[n - 1]) * dd[n - 2];
-      for (int i = n - 3; i >= 0; --i) z[i] = (z[i] - du[i] * z[i + 1] - du2[i] * z[i + 2]) * dd[i];
+      z[n - 1] = cur;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += IV_THREADS) z[i] *= dd[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {  // U, rows over their diagonal
+      double z1 = z[n - 1], z2 = 0.0;
+      int i1 = max(n - 2, 0);
+      double t = z[i1], u = du[i1], u2 = du2[i1];
+      for (int i = n - 2; i >= 0; --i) {
+        i1 = max(i - 1, 0);
+        const double tn = z[i1], un = du[i1], u2n = du2[i1];
+        const double v = fma(-u, z1, fma(-u2, z2, t));
+        z[i] = v;
+        z2 = z1;
+        z1 = v;
+        t = tn;
+        u = un;
+        u2 = u2n;
+      }
     }
     __syncthreads();
     double sq = 0.0;
