@@ -202,130 +202,171 @@ __global__ void __launch_bounds__(THREADS) lift_dft_kernel(int L, int rows, cons
 // tensor cores in TF32 (mma.sync m16n8k8, FP32 accumulate):
 //   DFT_y : [2J x 2L] . [2L x C],  rows 2j+ro, K index 2y+ri
 //   inverse: [2L x 2J] . [2J x C], rows 2y+ro, K index 2j+ri
-// The twiddle operand is generated from a cos/sin table.  The mode weights
-// R[.][kx] are read once per CTA for all G masks (FP32 mixing).
+// The mode weights R[.][kx] are read once per CTA for all G masks (FP32 mixing).
+//
+// What it must move is Xin once and Gout once (67 MB each at 64 masks of 256 x 256); the products
+// themselves are short, so the operands' way to the registers decides.  The twiddles depend on
+// neither kx nor the mask: column_tables_kernel lays them out once as the fragments a lane holds, one
+// 16-byte load each (gathered from a cosine table they took four loads, four selects and four
+// conversions).  A mask has 8 / G warps of its own: its column goes from global memory straight into
+// fragments, a step ahead of its use, each serving two row tiles, and its mixed modes stay in
+// registers for all rows of the inverse.
+// 64 masks: 142 -> 51 us a launch; 32 masks: forward 84 -> 31, backward 75 -> 36.
 // ---------------------------------------------------------------------------
 constexpr int COL_G = 4;
+constexpr int CP = C + 8;  // padded row of the modes in shared memory: fragment loads of two rows miss each other's banks
 
 __device__ __forceinline__ uint32_t tf32r(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ void mma1688(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma1688(float* d, const uint4& a, uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+      : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
 
-template <bool BWD>
-__global__ void __launch_bounds__(THREADS) column_kernel(int L, int B, int G, const float* __restrict__ theta,
-                                                         int layer, const float2* __restrict__ Xin,
-                                                         float2* __restrict__ Gout, float2* __restrict__ modes_out,
-                                                         const float2* __restrict__ twL_g) {
+// A fragments of the two transforms, [row tile][k step][lane]: DFT_y 4 x L/4, inverse L/8 x 8
+__global__ void column_tables_kernel(int L, const float2* __restrict__ twL, uint4* __restrict__ fd,
+                                     uint4* __restrict__ fi) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= L * 32) return;
+  const int lane = i & 31, g = lane >> 2, t = lane & 3, ro = g & 1, ri = t & 1;
+  auto tw = [&](int ky, int y) { return twL[(ky * y) & (L - 1)]; };
+  {
+    const int mt = i / (8 * L), ks = i / 32 % (L / 4);
+    const int j = 8 * mt + (g >> 1);  // rows g and g + 8 -> j and j + 4
+    const int ky0 = j < M ? j : L - J + j, ky1 = (j + 4) < M ? j + 4 : L - J + j + 4;
+    const int y0 = 4 * ks + (t >> 1), y1 = y0 + 2;
+    // ro = 0: (cos, sin); ro = 1: (-sin, cos) over ri = 0, 1
+    auto el = [&](float2 w) { return tf32r(ro == 0 ? (ri == 0 ? w.x : w.y) : (ri == 0 ? -w.y : w.x)); };
+    fd[i] = make_uint4(el(tw(ky0, y0)), el(tw(ky1, y0)), el(tw(ky0, y1)), el(tw(ky1, y1)));
+  }
+  {
+    const int mt = i / 256, ks = i / 32 % 8;
+    const int y = 8 * mt + (g >> 1);  // rows g, g + 8 -> y, y + 4
+    const int j0 = 4 * ks + (t >> 1), j1 = j0 + 2;
+    const int ky0 = j0 < M ? j0 : L - J + j0, ky1 = j1 < M ? j1 : L - J + j1;
+    // ro = 0: (cos, -sin); ro = 1: (sin, cos) over ri = 0, 1
+    auto el = [&](float2 w) { return tf32r(ro == 0 ? (ri == 0 ? w.x : -w.y) : (ri == 0 ? w.y : w.x)); };
+    fi[i] = make_uint4(el(tw(ky0, y)), el(tw(ky0, y + 4)), el(tw(ky1, y)), el(tw(ky1, y + 4)));
+  }
+}
+
+template <bool BWD, int G>
+__global__ void __launch_bounds__(THREADS, 2) column_kernel(int L, int B, const float* __restrict__ theta, int layer,
+                                                            const float2* __restrict__ Xin, float2* __restrict__ Gout,
+                                                            float2* __restrict__ modes_out,
+                                                            const uint4* __restrict__ fd,
+                                                            const uint4* __restrict__ fi) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  float* sX = reinterpret_cast<float*>(smraw);  // [L][C][re,im] tf32; BWD mixing: per-warp transposed R blocks
-  float2* sR = reinterpret_cast<float2*>(smraw);
-  float2* sTw = reinterpret_cast<float2*>(smraw) + std::max((size_t)L * C, (size_t)(THREADS / 32) * C * (C + 1));
-  float2* sV = sTw + L;  // [G][J][C]
+  float2* sV = reinterpret_cast<float2*>(smraw);  // [G][J][CP]
+  float2* sR = sV + G * J * CP;                   // BWD mixing: per-warp transposed R blocks
+  constexpr int WPM = THREADS / 32 / G;           // warps of a mask
+  constexpr int MT = G == 4 ? 2 : 1, NT = G == 1 ? 2 : 4;  // a warp's DFT_y tiles: MT x NT of 4 x 4
   const int kx = blockIdx.x, b0 = blockIdx.y * G, tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, ri = t & 1;
   const int ng = min(G, B - b0);
-  for (int i = tid; i < L; i += THREADS) sTw[i] = twL_g[i];
-  // DFT_y tiles: warp -> m-tile (warp >> 1) of 4, n-tiles 2 (warp & 1) .. +1
-  const int dmt = warp >> 1, dn0 = 2 * (warp & 1);
-  const int jA = 8 * dmt + (g >> 1), roA = g & 1;  // rows g and g + 8 -> j and j + 4
-  const int kyA0 = jA < M ? jA : L - J + jA, kyA1 = (jA + 4) < M ? jA + 4 : L - J + jA + 4;
-  for (int gi = 0; gi < ng; ++gi) {
-    const int b = b0 + gi;
-    __syncthreads();
-    for (int i = tid; i < L * C; i += THREADS) {
-      const int y = i / C, c = i % C;
-      const float2 v = Xin[(((size_t)b * L + y) * M + kx) * C + c];
-      sX[2 * i] = __uint_as_float(tf32r(v.x));
-      sX[2 * i + 1] = __uint_as_float(tf32r(v.y));
-    }
-    __syncthreads();
-    float d[2][4] = {};
-    for (int ks = 0; ks < L / 4; ++ks) {  // 8 K entries = 4 y values
-      const int y0 = 4 * ks + (t >> 1), y1 = y0 + 2, ri = t & 1;
-      // A[m][k]: ro = 0: (cos, sin); ro = 1: (-sin, cos) over ri = 0, 1
-      uint32_t a[4];
-      {
-        const float2 w00 = sTw[(kyA0 * y0) & (L - 1)], w10 = sTw[(kyA1 * y0) & (L - 1)];
-        const float2 w01 = sTw[(kyA0 * y1) & (L - 1)], w11 = sTw[(kyA1 * y1) & (L - 1)];
-        auto el = [&](float2 w) { return roA == 0 ? (ri == 0 ? w.x : w.y) : (ri == 0 ? -w.y : w.x); };
-        a[0] = tf32r(el(w00));
-        a[1] = tf32r(el(w10));
-        a[2] = tf32r(el(w01));
-        a[3] = tf32r(el(w11));
-      }
+  const int gi = warp / WPM, sub = warp % WPM;
+  if (gi < ng) {
+    const int mt0 = G == 1 ? sub >> 1 : sub * MT, n0 = G == 1 ? 2 * (sub & 1) : 0;
+    // X[y][c].ri at y = 4 ks + t / 2 (+ 2), c = 8 n + g: a step of K
+    const float* x = reinterpret_cast<const float*>(Xin + (((size_t)(b0 + gi) * L + (t >> 1)) * M + kx) * C + 8 * n0 + g) + ri;
+    const size_t ys = (size_t)M * C * 2;
+    const uint4* af = fd + ((size_t)mt0 * (L / 4)) * 32 + lane;
+    struct Step {
+      float b[2][NT][2];
+      uint4 a[2][MT];
+    };
+    auto load = [&](Step& q, int k2) {  // K steps 2 k2, 2 k2 + 1
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int c = 8 * (dn0 + q) + g;
-        const uint32_t b0r = __float_as_uint(sX[(y0 * C + c) * 2 + ri]);
-        const uint32_t b1r = __float_as_uint(sX[(y1 * C + c) * 2 + ri]);
-        mma1688(d[q], a, b0r, b1r);
-      }
-    }
-    // D rows m = 16 dmt + g (+8) = 2j + ro, cols c
-    float* sVf = reinterpret_cast<float*>(sV + (size_t)gi * J * C);
+      for (int k = 0; k < 2; ++k) {
+        const float* p = x + (size_t)(8 * k2 + 4 * k) * ys;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int c = 8 * (dn0 + q) + 2 * t;
-      sVf[(jA * C + c) * 2 + roA] = d[q][0];
-      sVf[(jA * C + c + 1) * 2 + roA] = d[q][1];
-      sVf[((jA + 4) * C + c) * 2 + roA] = d[q][2];
-      sVf[((jA + 4) * C + c + 1) * 2 + roA] = d[q][3];
+        for (int n = 0; n < NT; ++n) {
+          q.b[k][n][0] = __ldg(p + 16 * n);
+          q.b[k][n][1] = __ldg(p + 2 * ys + 16 * n);
+        }
+#pragma unroll
+        for (int m = 0; m < MT; ++m) q.a[k][m] = __ldg(af + ((size_t)m * (L / 4) + 2 * k2 + k) * 32);
+      }
+    };
+    float d[MT][NT][4] = {};
+    auto step = [&](const Step& q) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          const uint32_t b0r = tf32r(q.b[k][n][0]), b1r = tf32r(q.b[k][n][1]);
+#pragma unroll
+          for (int m = 0; m < MT; ++m) mma1688(d[m][n], q.a[k][m], b0r, b1r);
+        }
+    };
+    Step q0, q1;
+    load(q0, 0);
+    const int N2 = L / 8;
+    for (int k2 = 0; k2 < N2; k2 += 2) {
+      load(q1, k2 + 1);
+      step(q0);
+      if (k2 + 2 < N2) load(q0, k2 + 2);
+      step(q1);
+    }
+    // D rows m = 16 mt + g (+8) = 2j + ro, cols c
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const int j = 8 * (mt0 + m) + (g >> 1), ro = g & 1;
+      float* v = reinterpret_cast<float*>(sV + ((size_t)gi * J + j) * CP) + ro;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const int c = 8 * (n0 + n) + 2 * t;
+        v[2 * c] = d[m][n][0];
+        v[2 * c + 2] = d[m][n][1];
+        v[4 * CP * 2 + 2 * c] = d[m][n][2];
+        v[4 * CP * 2 + 2 * c + 2] = d[m][n][3];
+      }
     }
   }
   __syncthreads();
   if (modes_out)
     for (int i = tid; i < ng * J * C; i += THREADS) {
-      const int gi = i / (J * C), j = (i / C) % J, c = i % C;
-      modes_out[(((size_t)(b0 + gi) * J + j) * M + kx) * C + c] = sV[i];
+      const int m = i / (J * C), j = (i / C) % J, c = i % C;
+      modes_out[(((size_t)(b0 + m) * J + j) * M + kx) * C + c] = sV[((size_t)m * J + j) * CP + c];
     }
   // mixing: thread (lane = output channel, j = warp + 8 r) for every mask of the group
   const float s = (kx == 0 ? 1.0f : 2.0f) / ((float)L * (float)L);
   const float2* Rl = reinterpret_cast<const float2*>(theta + Off::R + (size_t)layer * Off::RL);
-  float2 u[J / 8][COL_G];
+  float2 u[J / 8][G];
 #pragma unroll
   for (int r = 0; r < J / 8; ++r)
 #pragma unroll
-    for (int gg = 0; gg < COL_G; ++gg) u[r][gg] = make_float2(0.f, 0.f);
+    for (int gg = 0; gg < G; ++gg) u[r][gg] = make_float2(0.f, 0.f);
   float2* sRt = sR + (size_t)warp * C * (C + 1);  // BWD: this warp's block, transposed [o][c] (padded)
 #pragma unroll
   for (int r = 0; r < J / 8; ++r) {
     const int j = warp + 8 * r;
     const float2* Rj = Rl + ((size_t)j * M + kx) * C * C;  // [c][o]
-    if (!BWD) {  // U[o] = s sum_c R[c][o] V[c]
-      for (int c = 0; c < C; ++c) {
-        const float2 rr = Rj[c * C + lane];
-#pragma unroll
-        for (int gg = 0; gg < COL_G; ++gg) {
-          if (gg < ng) {
-            const float2 v = sV[((size_t)gg * J + j) * C + c];
-            u[r][gg].x = fmaf(rr.x, v.x, fmaf(-rr.y, v.y, u[r][gg].x));
-            u[r][gg].y = fmaf(rr.x, v.y, fmaf(rr.y, v.x, u[r][gg].y));
-          }
-        }
-      }
-    } else {  // gV[c] = s sum_o conj(R[c][o]) gU[o]; lane = c
+    if (BWD) {
       __syncwarp();
+#pragma unroll 8
       for (int c = 0; c < C; ++c) sRt[lane * (C + 1) + c] = Rj[c * C + lane];
       __syncwarp();
-      for (int o = 0; o < C; ++o) {
-        const float2 rr = sRt[o * (C + 1) + lane];
+    }
+    // FWD: U[o] = s sum_c R[c][o] V[c]; BWD: gV[c] = s sum_o conj(R[c][o]) gU[o], lane = c
+#pragma unroll 4
+    for (int c = 0; c < C; c += 2) {
+      const float2 ra = BWD ? sRt[c * (C + 1) + lane] : Rj[c * C + lane];
+      const float2 rb = BWD ? sRt[(c + 1) * (C + 1) + lane] : Rj[(c + 1) * C + lane];
+      const float iy = BWD ? -1.f : 1.f;
 #pragma unroll
-        for (int gg = 0; gg < COL_G; ++gg) {
-          if (gg < ng) {
-            const float2 v = sV[((size_t)gg * J + j) * C + o];
-            u[r][gg].x = fmaf(rr.x, v.x, fmaf(rr.y, v.y, u[r][gg].x));
-            u[r][gg].y = fmaf(rr.x, v.y, fmaf(-rr.y, v.x, u[r][gg].y));
-          }
-        }
+      for (int gg = 0; gg < G; ++gg) {
+        const float4 v = *reinterpret_cast<const float4*>(sV + ((size_t)gg * J + j) * CP + c);
+        u[r][gg].x = fmaf(ra.x, v.x, fmaf(-iy * ra.y, v.y, u[r][gg].x));
+        u[r][gg].y = fmaf(ra.x, v.y, fmaf(iy * ra.y, v.x, u[r][gg].y));
+        u[r][gg].x = fmaf(rb.x, v.z, fmaf(-iy * rb.y, v.w, u[r][gg].x));
+        u[r][gg].y = fmaf(rb.x, v.w, fmaf(iy * rb.y, v.z, u[r][gg].y));
       }
     }
   }
@@ -334,52 +375,47 @@ __global__ void __launch_bounds__(THREADS) column_kernel(int L, int B, int G, co
   for (int r = 0; r < J / 8; ++r) {
     const int j = warp + 8 * r;
 #pragma unroll
-    for (int gg = 0; gg < COL_G; ++gg)
-      if (gg < ng)
-        sV[((size_t)gg * J + j) * C + lane] = make_float2(__uint_as_float(tf32r(s * u[r][gg].x)),
-                                                          __uint_as_float(tf32r(s * u[r][gg].y)));
+    for (int gg = 0; gg < G; ++gg)
+      sV[((size_t)gg * J + j) * CP + lane] = make_float2(__uint_as_float(tf32r(s * u[r][gg].x)),
+                                                         __uint_as_float(tf32r(s * u[r][gg].y)));
   }
   __syncthreads();
-  // inverse y as [2L x 2J] . [2J x C]: rows m = 2y + ro, K index 2j + ri
-  //   ro = 0: (cos, -sin); ro = 1: (sin, cos) over ri = 0, 1
-  // warp -> m-tiles warp, warp + 8, ... (2L / 16 = L / 8 of them), all 4 n-tiles
-  for (int gi = 0; gi < ng; ++gi) {
-    const int b = b0 + gi;
-    const float* sUf = reinterpret_cast<const float*>(sV + (size_t)gi * J * C);
-    // B fragments of this mask: k-step ks covers j = 4 ks + t/2 (+2), ri = t & 1
-    for (int mt = warp; mt < L / 8; mt += THREADS / 32) {
-      const int yA = 8 * mt + (g >> 1), ro = g & 1;  // rows g, g + 8 -> y, y + 4
-      float d[4][4] = {};
+  if (gi >= ng) return;
+  // inverse y as [2L x 2J] . [2J x C]: rows m = 2y + ro, K index 2j + ri; the mask's warps share
+  // its L / 8 row tiles, all 4 n-tiles each.  K step ks covers j = 4 ks + t/2 (+2), ri = t & 1
+  uint32_t bf[J / 4][4][2];
 #pragma unroll
-      for (int ks = 0; ks < J / 4; ++ks) {
-        const int j0 = 4 * ks + (t >> 1), j1 = j0 + 2, ri = t & 1;
-        const int ky0 = j0 < M ? j0 : L - J + j0, ky1 = j1 < M ? j1 : L - J + j1;
-        const float2 w00 = sTw[(ky0 * yA) & (L - 1)], w10 = sTw[(ky0 * (yA + 4)) & (L - 1)];
-        const float2 w01 = sTw[(ky1 * yA) & (L - 1)], w11 = sTw[(ky1 * (yA + 4)) & (L - 1)];
-        auto el = [&](float2 w) { return ro == 0 ? (ri == 0 ? w.x : -w.y) : (ri == 0 ? w.y : w.x); };
-        uint32_t a[4] = {tf32r(el(w00)), tf32r(el(w10)), tf32r(el(w01)), tf32r(el(w11))};
+  for (int ks = 0; ks < J / 4; ++ks)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const int c = 8 * n + g;
-          mma1688(d[n], a, __float_as_uint(sUf[(j0 * C + c) * 2 + ri]), __float_as_uint(sUf[(j1 * C + c) * 2 + ri]));
-        }
-      }
-      float* go = reinterpret_cast<float*>(Gout);
+    for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int c = 8 * n + 2 * t;
-        go[((((size_t)b * L + yA) * M + kx) * C + c) * 2 + ro] = d[n][0];
-        go[((((size_t)b * L + yA) * M + kx) * C + c + 1) * 2 + ro] = d[n][1];
-        go[((((size_t)b * L + yA + 4) * M + kx) * C + c) * 2 + ro] = d[n][2];
-        go[((((size_t)b * L + yA + 4) * M + kx) * C + c + 1) * 2 + ro] = d[n][3];
-      }
+      for (int h = 0; h < 2; ++h)
+        bf[ks][n][h] = reinterpret_cast<const uint32_t*>(
+            sV + ((size_t)gi * J + 4 * ks + (t >> 1) + 2 * h) * CP + 8 * n + g)[ri];
+  for (int mt = sub; mt < L / 8; mt += WPM) {
+    const int y = 8 * mt + (g >> 1), ro = g & 1;  // rows g, g + 8 -> y, y + 4
+    const uint4* af = fi + (size_t)mt * 256 + lane;
+    float d[4][4] = {};
+#pragma unroll
+    for (int ks = 0; ks < J / 4; ++ks) {
+      const uint4 a = __ldg(af + 32 * ks);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) mma1688(d[n], a, bf[ks][n][0], bf[ks][n][1]);
+    }
+    // lanes g (re) and g ^ 1 (im) hold channels c, c + 1 of one row: each takes one of the two whole
+    float2* go = Gout + (((size_t)(b0 + gi) * L + y) * M + kx) * C + 2 * t + ro;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const float p = __shfl_xor_sync(0xffffffffu, ro ? d[n][0] : d[n][1], 4);
+      const float q = __shfl_xor_sync(0xffffffffu, ro ? d[n][2] : d[n][3], 4);
+      go[8 * n] = ro ? make_float2(p, d[n][1]) : make_float2(d[n][0], p);
+      go[(size_t)4 * M * C + 8 * n] = ro ? make_float2(q, d[n][3]) : make_float2(d[n][2], q);
     }
   }
 }
 
-size_t column_smem(int L) {
-  const size_t x = std::max((size_t)L * C, (size_t)(THREADS / 32) * C * (C + 1));
-  return (x + L + (size_t)COL_G * J * C) * sizeof(float2);
+size_t column_smem(int G, bool bwd) {
+  return ((size_t)G * J * CP + (bwd ? (THREADS / 32) * C * (C + 1) : 0)) * sizeof(float2);
 }
 
 // ---------------------------------------------------------------------------
@@ -1426,7 +1462,7 @@ struct litho_fno {
   int cap = 0;  // batch capacity of the workspaces
   long long step = 0;
   DevBuf theta, grad, adam_m, adam_v;
-  DevBuf Ttab, TT, twL;
+  DevBuf Ttab, TT, twL, colF, colI;  // tables; the column kernel's as fragments
   DevBuf z[NL];      // z_l (training keeps all; inference ping-pongs z[0], z[1])
   DevBuf Xf, Gy;     // per-row spectral intermediates (also Xg, Gg in backward)
   DevBuf Vs[NL], gU;
@@ -1442,8 +1478,28 @@ namespace {
 
 int fno_grid(litho_fno* f, int rows) { return std::max(1, std::min(rows, 2 * f->ctx->sm_count)); }
 
-// masks per column-kernel CTA: enough CTAs for two per SM, at most COL_G
-int col_group(litho_fno* f, int B) { return std::max(1, std::min(COL_G, B * M / (2 * f->ctx->sm_count))); }
+// The column kernel over B masks, in groups of four, two or one: the more masks share the reading of
+// R the better, while there are three CTAs for every two SMs (32 masks, us
+// forward and backward: four a CTA, 128 CTAs, 47 and 46; two, 256, 31 and 36; one, 512, 46 and 56)
+template <bool BWD>
+int launch_column(litho_fno* f, int B, int layer, const float2* Xin, float2* Gout, float2* modes_out) {
+  litho_ctx* ctx = f->ctx;
+  auto go = [&](auto* k, int G) {
+    const size_t smem = column_smem(G, BWD);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(M, (B + G - 1) / G), THREADS, smem, ctx->stream>>>(f->L, B, f->theta.as<float>(), layer, Xin, Gout, modes_out,
+                                                               f->colF.as<uint4>(), f->colI.as<uint4>());
+    return cudaGetLastError();
+  };
+  const int want = 3 * ctx->sm_count / 2;
+  cudaError_t e;
+  if (M * ((B + 3) / 4) >= want) e = go(column_kernel<BWD, 4>, 4);
+  else if (M * ((B + 1) / 2) >= want) e = go(column_kernel<BWD, 2>, 2);
+  else e = go(column_kernel<BWD, 1>, 1);
+  LITHO_CUDA_TRY(ctx, e);
+  return LITHO_OK;
+}
 
 int ensure_batch(litho_fno* f, int B, bool train) {
   litho_ctx* ctx = f->ctx;
@@ -1477,19 +1533,15 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
   litho_ctx* ctx = f->ctx;
   const int L = f->L, rows = B * L;
   const float* th = f->theta.as<float>();
-  const size_t csm = column_smem(L);
-  LITHO_RET(set_smem(ctx, (const void*)column_kernel<false>, csm));
   LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<false>, row_fwd_smem(L, false)));
   LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<true>, row_fwd_smem(L, true)));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 2 * NL + 1);
   lift_dft_kernel<<<(rows + 7) / 8, THREADS, 0, ctx->stream>>>(L, rows, th, masks, f->twL.as<float2>(),
                                                                f->Xf.as<float2>(), Mrow);
   const int grid = fno_grid(f, rows);
-  const int G = col_group(f, B);
   for (int l = 0; l < NL; ++l) {
-    column_kernel<false><<<dim3(M, (B + G - 1) / G), THREADS, csm, ctx->stream>>>(
-        L, B, G, th, l, f->Xf.as<float2>(), f->Gy.as<float2>(), train ? f->Vs[l].as<float2>() : nullptr,
-        f->twL.as<float2>());
+    LITHO_RET(launch_column<false>(f, B, l, f->Xf.as<float2>(), f->Gy.as<float2>(),
+                                   train ? f->Vs[l].as<float2>() : nullptr));
     RowFwd a;
     a.L = L; a.rows = rows; a.layer = l; a.theta = th; a.masks = masks;
     a.act_in = train ? 1 : 0;   // training keeps z_l, inference keeps GELU(z_l)
@@ -1514,13 +1566,10 @@ int backward(litho_fno* f, const float* masks, const float* targets, int B) {
   litho_ctx* ctx = f->ctx;
   const int L = f->L, rows = B * L, grid = f->bwd_grid;
   const float* th = f->theta.as<float>();
-  const size_t csm = column_smem(L);
-  LITHO_RET(set_smem(ctx, (const void*)column_kernel<true>, csm));
   const BwdSmem sp(L, HEAD_PROJ), ss(L, HEAD_SPEC), sl(L, HEAD_LIFT);
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_PROJ>, sp.total));
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_SPEC>, ss.total));
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_LIFT>, sl.total));
-  const int G = col_group(f, B);
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 3 * NL + 3);
   loss_kernel<<<B, 1024, 0, ctx->stream>>>(L, B, f->out.as<float>(), targets, f->lossb.as<float>(),
                                            f->coef.as<float>());
@@ -1543,9 +1592,7 @@ int backward(litho_fno* f, const float* masks, const float* targets, int B) {
       row_bwd_kernel<HEAD_PROJ><<<grid, THREADS, sp.total, ctx->stream>>>(a);
     else
       row_bwd_kernel<HEAD_SPEC><<<grid, THREADS, ss.total, ctx->stream>>>(a);
-    column_kernel<true><<<dim3(M, (B + G - 1) / G), THREADS, csm, ctx->stream>>>(L, B, G, th, l, Xg, Gg,
-                                                                                  f->gU.as<float2>(),
-                                                                                  f->twL.as<float2>());
+    LITHO_RET(launch_column<true>(f, B, l, Xg, Gg, f->gU.as<float2>()));
     dR_kernel<<<J * M, THREADS, 0, ctx->stream>>>(L, B, l, f->gU.as<float2>(), f->Vs[l].as<float2>(),
                                                   f->grad.as<float>());
     cur ^= 1;
@@ -1640,7 +1687,8 @@ int litho_surrogate_create(litho_ctx* ctx, int L, unsigned long long seed, litho
         (rc = f->adam_v.ensure(ctx, pb)))
       break;
     if ((rc = f->Ttab.ensure(ctx, (size_t)L * J * sizeof(bf16))) || (rc = f->TT.ensure(ctx, (size_t)L * J * sizeof(bf16))) ||
-        (rc = f->twL.ensure(ctx, (size_t)L * sizeof(float2))))
+        (rc = f->twL.ensure(ctx, (size_t)L * sizeof(float2))) || (rc = f->colF.ensure(ctx, (size_t)L * 32 * sizeof(uint4))) ||
+        (rc = f->colI.ensure(ctx, (size_t)L * 32 * sizeof(uint4))))
       break;
     std::vector<float> p;
     init_params(p, seed);
@@ -1654,6 +1702,8 @@ int litho_surrogate_create(litho_ctx* ctx, int L, unsigned long long seed, litho
     }
     tables_kernel<<<(L * M + 255) / 256, 256, 0, ctx->stream>>>(L, f->Ttab.as<bf16>(), f->TT.as<bf16>(),
                                                                f->twL.as<float2>());
+    column_tables_kernel<<<(L * 32 + 255) / 256, 256, 0, ctx->stream>>>(L, f->twL.as<float2>(), f->colF.as<uint4>(),
+                                                                       f->colI.as<uint4>());
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
       set_error(ctx, LITHO_ERR_CUDA, "surrogate table setup failed");
       rc = LITHO_ERR_CUDA;
@@ -1669,7 +1719,7 @@ int litho_surrogate_create(litho_ctx* ctx, int L, unsigned long long seed, litho
 
 void litho_surrogate_destroy(litho_fno* f) {
   if (!f) return;
-  DevBuf* bufs[] = {&f->theta, &f->grad, &f->adam_m, &f->adam_v, &f->Ttab, &f->TT, &f->twL, &f->Xf, &f->Gy,
+  DevBuf* bufs[] = {&f->theta, &f->grad, &f->adam_m, &f->adam_v, &f->Ttab, &f->TT, &f->twL, &f->colF, &f->colI, &f->Xf, &f->Gy,
                     &f->gU, &f->gv[0], &f->gv[1], &f->out, &f->lossb, &f->coef, &f->gpart, &f->Xb, &f->Eres,
                     &f->Enew, &f->Cb, &f->Mrow, &f->Cm, &f->est, &f->stage_m, &f->stage_i};
   for (DevBuf* b : bufs) b->release();
