@@ -164,33 +164,73 @@ __global__ void tables_kernel(int L, bf16* Ttab, bf16* TT, float2* twL) {
 }
 
 // ---------------------------------------------------------------------------
-// lift + x-DFT of layer 0: v0 = Pw m + Pb, so X0[kx][c] = Pw[c] DFT(m)[kx] + Pb[c] L d(kx)
-// One warp per row.
+// x-DFT of four real rows at kx = 0..15 by one warp: lane -> kx = lane & 15, pixels of one parity
+// (lane >> 4), then both parities together; every lane ends with its kx.  The latency of a twiddle
+// gather and a pixel per step bound the form with a row a warp; four rows share the twiddle and take
+// their pixels in one 16-byte read.  sM: the warp's [L] x 4 rows, sTw: e^{+2 pi i k / L}.
+// 16,384 rows of 256: lift_dft 57 -> 28 us, band_rows 52 -> 21.
 // ---------------------------------------------------------------------------
+constexpr int DR = 4;
+__device__ __forceinline__ void rows_dft(int L, const float* __restrict__ src, int nrows, float4* sM,
+                                         const float2* sTw, float (&re)[DR], float (&im)[DR]) {
+  const int lane = threadIdx.x & 31, kx = lane & 15, half = lane >> 4;
+  float* m = reinterpret_cast<float*>(sM);
+#pragma unroll
+  for (int r = 0; r < DR; ++r)
+    for (int px = lane; px < L; px += 32) m[DR * px + r] = r < nrows ? __ldg(src + (size_t)r * L + px) : 0.f;
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < DR; ++r) re[r] = im[r] = 0.f;
+  int ang = kx * half;
+#pragma unroll 4
+  for (int px = half; px < L; px += 2) {
+    const float2 w = sTw[ang];
+    const float4 v = sM[px];
+    ang = (ang + 2 * kx) & (L - 1);
+    re[0] = fmaf(v.x, w.x, re[0]);
+    im[0] = fmaf(-v.x, w.y, im[0]);
+    re[1] = fmaf(v.y, w.x, re[1]);
+    im[1] = fmaf(-v.y, w.y, im[1]);
+    re[2] = fmaf(v.z, w.x, re[2]);
+    im[2] = fmaf(-v.z, w.y, im[2]);
+    re[3] = fmaf(v.w, w.x, re[3]);
+    im[3] = fmaf(-v.w, w.y, im[3]);
+  }
+#pragma unroll
+  for (int r = 0; r < DR; ++r) {
+    re[r] += __shfl_xor_sync(0xffffffffu, re[r], 16);
+    im[r] += __shfl_xor_sync(0xffffffffu, im[r], 16);
+  }
+}
+__host__ __device__ inline size_t rows_dft_smem(int L) {
+  return (size_t)L * sizeof(float2) + (size_t)(THREADS / 32) * L * DR * sizeof(float);
+}
+
+// lift + x-DFT of layer 0: v0 = Pw m + Pb, so X0[kx][c] = Pw[c] DFT(m)[kx] + Pb[c] L d(kx).
 __global__ void __launch_bounds__(THREADS) lift_dft_kernel(int L, int rows, const float* __restrict__ theta,
                                                            const float* __restrict__ masks,
                                                            const float2* __restrict__ twL, float2* __restrict__ Xf,
                                                            float2* __restrict__ Mrow) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float2* sTw = reinterpret_cast<float2*>(smraw);
+  for (int i = threadIdx.x; i < L; i += THREADS) sTw[i] = twL[i];
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * (THREADS / 32) + warp;
-  if (row >= rows) return;
-  const float* m = masks + (size_t)row * L;
-  const int kx = lane & 15, half = lane >> 4;
-  float re = 0.f, im = 0.f;
-  for (int px = half; px < L; px += 2) {
-    const float v = m[px];
-    const float2 w = twL[(kx * px) & (L - 1)];
-    re = fmaf(v, w.x, re);
-    im = fmaf(-v, w.y, im);
-  }
-  re += __shfl_xor_sync(0xffffffffu, re, 16);
-  im += __shfl_xor_sync(0xffffffffu, im, 16);
-  if (Mrow && lane < 16) Mrow[(size_t)row * 16 + lane] = make_float2(re, im);  // mask row DFT, kx < 16
-  float2* out = Xf + (size_t)row * M * C;
-  for (int k = 0; k < M; ++k) {
-    const float mr = __shfl_sync(0xffffffffu, re, k), mi = __shfl_sync(0xffffffffu, im, k);
-    const float pw = theta[Off::Pw + lane], pb = theta[Off::Pb + lane];
-    out[k * C + lane] = make_float2(pw * mr + (k == 0 ? pb * (float)L : 0.f), pw * mi);
+  const int row0 = (blockIdx.x * (THREADS / 32) + warp) * DR, n = min(DR, rows - row0);
+  if (n <= 0) return;
+  float re[DR], im[DR];
+  rows_dft(L, masks + (size_t)row0 * L, n, reinterpret_cast<float4*>(sTw + L) + (size_t)warp * L, sTw, re, im);
+  const float pw = theta[Off::Pw + lane], pb = theta[Off::Pb + lane];
+#pragma unroll
+  for (int r = 0; r < DR; ++r) {
+    if (r >= n) break;
+    if (Mrow && lane < 16) Mrow[(size_t)(row0 + r) * 16 + lane] = make_float2(re[r], im[r]);  // mask row DFT, kx < 16
+    float2* out = Xf + (size_t)(row0 + r) * M * C;
+#pragma unroll
+    for (int k = 0; k < M; ++k) {
+      const float mr = __shfl_sync(0xffffffffu, re[r], k), mi = __shfl_sync(0xffffffffu, im[r], k);
+      out[k * C + lane] = make_float2(pw * mr + (k == 0 ? pb * (float)L : 0.f), pw * mi);
+    }
   }
 }
 
@@ -1257,97 +1297,111 @@ __global__ void rect_masks_kernel(uint64_t seed, long long first, int L, int nmi
 // SOCS image with kernels of half-width Nx = KB/2, Ny = KBy/2) and its
 // out-of-band residual, the surrogate's error estimate.
 // ---------------------------------------------------------------------------
-// x-DFT of each row at kx = 0..KB (KB <= 15); one warp per row
+// x-DFT of each row at kx = 0..KB (KB <= 15)
 __global__ void __launch_bounds__(THREADS) band_rows_kernel(int L, int rows, int KB, const float* __restrict__ img,
                                                             const float2* __restrict__ twL, float2* __restrict__ Xb) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float2* sTw = reinterpret_cast<float2*>(smraw);
+  for (int i = threadIdx.x; i < L; i += THREADS) sTw[i] = twL[i];
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * (THREADS / 32) + warp;
-  if (row >= rows) return;
-  const float* m = img + (size_t)row * L;
-  const int kx = lane & 15, half = lane >> 4;
-  float re = 0.f, im = 0.f;
-  for (int px = half; px < L; px += 2) {
-    const float v = m[px];
-    const float2 w = twL[(kx * px) & (L - 1)];
-    re = fmaf(v, w.x, re);
-    im = fmaf(-v, w.y, im);
-  }
-  re += __shfl_xor_sync(0xffffffffu, re, 16);
-  im += __shfl_xor_sync(0xffffffffu, im, 16);
-  if (half == 0 && kx <= KB) Xb[(size_t)row * 16 + kx] = make_float2(re, im);
+  const int row0 = (blockIdx.x * (THREADS / 32) + warp) * DR, n = min(DR, rows - row0);
+  if (n <= 0) return;
+  float re[DR], im[DR];
+  rows_dft(L, img + (size_t)row0 * L, n, reinterpret_cast<float4*>(sTw + L) + (size_t)warp * L, sTw, re, im);
+#pragma unroll
+  for (int r = 0; r < DR; ++r)
+    if (r < n && lane <= KB && lane < 16) Xb[(size_t)(row0 + r) * 16 + lane] = make_float2(re[r], im[r]);
 }
 
-// per mask: C[ky + KBy][kx] = sum_y X[y][kx] e^{-i ky y} for kx <= KB, |ky| <= KBy (plain 2-D DFT)
+// C[ky + KBy][kx] = sum_y X[y][kx] e^{-i ky y} for kx <= KB, |ky| <= KBy (plain 2-D DFT).  One CTA
+// per mask and ky: 16 kx by 16 shares of the rows, added in order (one thread per coefficient over
+// all rows, one CTA per mask, took 85 us for 64 masks of 256 x 256; now 6).
 __global__ void __launch_bounds__(THREADS) band_coef_kernel(int L, int KB, int KBy, const float2* __restrict__ Xb,
                                                             const float2* __restrict__ twL, float2* __restrict__ Cb) {
-  const int b = blockIdx.x;
-  const int nky = 2 * KBy + 1, ncoef = nky * (KB + 1);
-  for (int q = threadIdx.x; q < ncoef; q += blockDim.x) {
-    const int kyi = q / (KB + 1), kx = q % (KB + 1), ky = kyi - KBy;
-    float re = 0.f, im = 0.f;
-    for (int y = 0; y < L; ++y) {
-      const float2 x = Xb[((size_t)b * L + y) * 16 + kx];
-      const float2 w = twL[((ky + L) * y) & (L - 1)];  // e^{+i ky y}; use conj
+  __shared__ float2 part[THREADS / 16][16];
+  const int b = blockIdx.y, kyi = blockIdx.x, ky = kyi - KBy, kx = threadIdx.x & 15, sh = threadIdx.x >> 4;
+  float re = 0.f, im = 0.f;
+  if (kx <= KB) {
+#pragma unroll 4
+    for (int y = sh; y < L; y += THREADS / 16) {
+      const float2 x = __ldg(Xb + ((size_t)b * L + y) * 16 + kx);
+      const float2 w = __ldg(twL + (((ky + L) * y) & (L - 1)));  // e^{+i ky y}; use conj
       re = fmaf(x.x, w.x, fmaf(x.y, w.y, re));
       im = fmaf(x.y, w.x, fmaf(-x.x, w.y, im));
     }
-    Cb[(size_t)b * nky * 16 + kyi * 16 + kx] = make_float2(re, im);
+  }
+  part[sh][kx] = make_float2(re, im);
+  __syncthreads();
+  if (sh == 0 && kx <= KB) {
+    for (int s = 1; s < THREADS / 16; ++s) {
+      re += part[s][kx].x;
+      im += part[s][kx].y;
+    }
+    Cb[((size_t)b * gridDim.x + kyi) * 16 + kx] = make_float2(re, im);
   }
 }
 
 // in-place synthesis of the band: img[y][x] = 1/L^2 sum_kx w_kx Re(G_y[kx] e^{i kx x}),
 // G_y[kx] = sum_ky Cb[ky][kx] e^{i ky y}; per-row energies of the removed part and of the result.
-// One CTA per row.
-__global__ void __launch_bounds__(THREADS) band_synth_kernel(int L, int KB, int KBy, const float2* __restrict__ Cb,
+// One warp per row, a lane per kx and then per pixel of each 32, so that nothing waits for another
+// warp (a CTA per row, two barriers apart: 75 us for 16,384 rows of 256; now 18).
+__global__ void __launch_bounds__(THREADS) band_synth_kernel(int L, int rows, int KB, int KBy,
+                                                             const float2* __restrict__ Cb,
                                                              const float2* __restrict__ twL, float* __restrict__ img,
                                                              float* __restrict__ Eres, float* __restrict__ Enew) {
-  const int row = blockIdx.x, b = row / L, y = row % L, tid = threadIdx.x;
-  const int nky = 2 * KBy + 1;
-  __shared__ float2 G[16];
-  __shared__ float r0[THREADS / 32], r1[THREADS / 32];
-  if (tid <= KB) {
-    float re = 0.f, im = 0.f;
+  __shared__ float2 sTw[256];
+  constexpr int MAXI = 256 / 32;
+  for (int i = threadIdx.x; i < L; i += THREADS) sTw[i] = twL[i];
+  __syncthreads();
+  const int row = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int b = row / L, y = row % L, nky = 2 * KBy + 1, kx = lane & 15;
+  float* p = img + (size_t)row * L;
+  float old[MAXI];
+#pragma unroll
+  for (int i = 0; i < MAXI; ++i) old[i] = 32 * i < L ? p[lane + 32 * i] : 0.f;
+  float re = 0.f, im = 0.f;
+  if (kx <= KB) {
+    const float2* cb = Cb + (size_t)b * nky * 16 + kx;
+#pragma unroll 4
     for (int kyi = 0; kyi < nky; ++kyi) {
-      const int ky = kyi - KBy;
-      const float2 c = Cb[(size_t)b * nky * 16 + kyi * 16 + tid];
-      const float2 w = twL[((ky + L) * y) & (L - 1)];
+      const float2 c = __ldg(cb + kyi * 16);
+      const float2 w = sTw[((kyi - KBy + L) * y) & (L - 1)];
       re = fmaf(c.x, w.x, fmaf(-c.y, w.y, re));
       im = fmaf(c.x, w.y, fmaf(c.y, w.x, im));
     }
-    const float sc = (tid == 0 ? 1.f : 2.f) / ((float)L * (float)L);
-    G[tid] = make_float2(sc * re, sc * im);
+    const float sc = (kx == 0 ? 1.f : 2.f) / ((float)L * (float)L);
+    re *= sc;
+    im *= sc;
   }
-  __syncthreads();
+  float v[MAXI] = {};
+  for (int k = 0; k <= KB; ++k) {
+    const float gx = __shfl_sync(0xffffffffu, re, k), gy = __shfl_sync(0xffffffffu, im, k);
+#pragma unroll
+    for (int i = 0; i < MAXI; ++i)
+      if (32 * i < L) {
+        const float2 w = sTw[(k * (lane + 32 * i)) & (L - 1)];
+        v[i] = fmaf(gx, w.x, fmaf(-gy, w.y, v[i]));
+      }
+  }
   float er = 0.f, en = 0.f;
-  for (int x = tid; x < L; x += THREADS) {
-    float v = 0.f;
-    for (int kx = 0; kx <= KB; ++kx) {
-      const float2 w = twL[(kx * x) & (L - 1)];
-      v = fmaf(G[kx].x, w.x, fmaf(-G[kx].y, w.y, v));
+#pragma unroll
+  for (int i = 0; i < MAXI; ++i)
+    if (32 * i < L) {
+      const float d = old[i] - v[i];
+      er = fmaf(d, d, er);
+      en = fmaf(v[i], v[i], en);
+      p[lane + 32 * i] = v[i];
     }
-    const size_t i = (size_t)row * L + x;
-    const float d = img[i] - v;
-    er = fmaf(d, d, er);
-    en = fmaf(v, v, en);
-    img[i] = v;
-  }
+#pragma unroll
   for (int k = 16; k > 0; k >>= 1) {
     er += __shfl_xor_sync(0xffffffffu, er, k);
     en += __shfl_xor_sync(0xffffffffu, en, k);
   }
-  if ((tid & 31) == 0) {
-    r0[tid >> 5] = er;
-    r1[tid >> 5] = en;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float a = 0.f, c = 0.f;
-    for (int w = 0; w < THREADS / 32; ++w) {
-      a += r0[w];
-      c += r1[w];
-    }
-    Eres[row] = a;
-    Enew[row] = c;
+  if (lane == 0) {
+    Eres[row] = er;
+    Enew[row] = en;
   }
 }
 
@@ -1369,8 +1423,9 @@ __global__ void oob_est_kernel(int L, int B, const float* __restrict__ Eres, con
 //   I(q) = 1/L^2 sum_k s_k sum_f B_k(f + q) conj(B_k(f)),  B_k(f) = krn_k(f) M(f),
 // M the plain DFT of the mask on the (2Nx+1) x (2Ny+1) window (Cm holds u >= 0).
 // est[b] = alpha * sqrt(sum_q w_q |I_net(q) - I(q)|^2 / L^2) / ||image||, w = 1 at DC, 2 else.
-// One CTA per mask.
-__global__ void __launch_bounds__(128) lowq_est_kernel(int L, int Nx, int Ny, const float2* __restrict__ Cm,
+// One CTA per mask, one thread per q and kernel.
+constexpr int LOWQ_THREADS = 5 * 64;
+__global__ void __launch_bounds__(LOWQ_THREADS) lowq_est_kernel(int L, int Nx, int Ny, const float2* __restrict__ Cm,
                                                        const float2* __restrict__ Cb, const float2* __restrict__ krn,
                                                        const float* __restrict__ scales, int nk,
                                                        const float* __restrict__ Enew, float alpha,
@@ -1391,10 +1446,11 @@ __global__ void __launch_bounds__(128) lowq_est_kernel(int L, int Nx, int Ny, co
     }
     sM[i] = m;
   }
-  if (tid == 0) {
+  if (tid < 32) {
     double a = 0.0;
-    for (int y = 0; y < L; ++y) a += Enew[(size_t)b * L + y];
-    en = a;
+    for (int y = tid; y < L; y += 32) a += Enew[(size_t)b * L + y];
+    for (int k = 16; k > 0; k >>= 1) a += __shfl_xor_sync(0xffffffffu, a, k);
+    if (tid == 0) en = a;
   }
   __syncthreads();
   const int qx[5] = {0, 1, 0, 1, -1}, qy[5] = {0, 0, 1, 1, 1};
@@ -1523,6 +1579,21 @@ int ensure_batch(litho_fno* f, int B, bool train) {
   return LITHO_OK;
 }
 
+// CTAs of the kernels that take DR rows a warp
+int dft_blocks(int rows) { return (rows + DR * THREADS / 32 - 1) / (DR * THREADS / 32); }
+
+// masks in launches of at most 65,535, the limit of the grid's second dimension
+int launch_band_coef(litho_fno* f, int KB, int KBy, int batch, const float2* X, float2* Cb) {
+  litho_ctx* ctx = f->ctx;
+  const int nky = 2 * KBy + 1;
+  for (int b = 0; b < batch; b += 65535) {
+    band_coef_kernel<<<dim3(nky, std::min(65535, batch - b)), THREADS, 0, ctx->stream>>>(
+        f->L, KB, KBy, X + (size_t)b * f->L * 16, f->twL.as<float2>(), Cb + (size_t)b * nky * 16);
+    LITHO_CUDA_TRY(ctx, cudaGetLastError());
+  }
+  return LITHO_OK;
+}
+
 int set_smem(litho_ctx* ctx, const void* fn, size_t bytes) {
   LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return LITHO_OK;
@@ -1536,8 +1607,8 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
   LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<false>, row_fwd_smem(L, false)));
   LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<true>, row_fwd_smem(L, true)));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 2 * NL + 1);
-  lift_dft_kernel<<<(rows + 7) / 8, THREADS, 0, ctx->stream>>>(L, rows, th, masks, f->twL.as<float2>(),
-                                                               f->Xf.as<float2>(), Mrow);
+  lift_dft_kernel<<<dft_blocks(rows), THREADS, rows_dft_smem(L), ctx->stream>>>(L, rows, th, masks, f->twL.as<float2>(),
+                                                                               f->Xf.as<float2>(), Mrow);
   const int grid = fno_grid(f, rows);
   for (int l = 0; l < NL; ++l) {
     LITHO_RET(launch_column<false>(f, B, l, f->Xf.as<float2>(), f->Gy.as<float2>(),
@@ -1615,12 +1686,11 @@ int project(litho_fno* f, int Nx, int Ny, float* images, int batch) {
   LITHO_RET(f->Enew.ensure(ctx, (size_t)rows * sizeof(float)));
   LITHO_RET(f->Cb.ensure(ctx, (size_t)batch * (2 * KBy + 1) * 16 * sizeof(float2)));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 3);
-  band_rows_kernel<<<(rows + 7) / 8, THREADS, 0, ctx->stream>>>(L, rows, KB, images, f->twL.as<float2>(),
-                                                                f->Xb.as<float2>());
-  band_coef_kernel<<<batch, THREADS, 0, ctx->stream>>>(L, KB, KBy, f->Xb.as<float2>(), f->twL.as<float2>(),
-                                                       f->Cb.as<float2>());
-  band_synth_kernel<<<rows, THREADS, 0, ctx->stream>>>(L, KB, KBy, f->Cb.as<float2>(), f->twL.as<float2>(), images,
-                                                       f->Eres.as<float>(), f->Enew.as<float>());
+  band_rows_kernel<<<dft_blocks(rows), THREADS, rows_dft_smem(L), ctx->stream>>>(L, rows, KB, images, f->twL.as<float2>(),
+                                                                                f->Xb.as<float2>());
+  LITHO_RET(launch_band_coef(f, KB, KBy, batch, f->Xb.as<float2>(), f->Cb.as<float2>()));
+  band_synth_kernel<<<(rows + 7) / 8, THREADS, 0, ctx->stream>>>(L, rows, KB, KBy, f->Cb.as<float2>(), f->twL.as<float2>(),
+                                                                 images, f->Eres.as<float>(), f->Enew.as<float>());
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
 }
@@ -1635,9 +1705,8 @@ int predict(litho_fno* f, const litho_kernel_set* ks, const float* masks, int ba
   LITHO_RET(forward(f, masks, batch, false, images, f->Mrow.as<float2>()));
   LITHO_RET(project(f, ks->Nx, ks->Ny, images, batch));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 2);
-  band_coef_kernel<<<batch, THREADS, 0, ctx->stream>>>(L, ks->Nx, ks->Ny, f->Mrow.as<float2>(), f->twL.as<float2>(),
-                                                       f->Cm.as<float2>());
-  lowq_est_kernel<<<batch, 128, 0, ctx->stream>>>(L, ks->Nx, ks->Ny, f->Cm.as<float2>(), f->Cb.as<float2>(), ks->krn,
+  LITHO_RET(launch_band_coef(f, ks->Nx, ks->Ny, batch, f->Mrow.as<float2>(), f->Cm.as<float2>()));
+  lowq_est_kernel<<<batch, LOWQ_THREADS, 0, ctx->stream>>>(L, ks->Nx, ks->Ny, f->Cm.as<float2>(), f->Cb.as<float2>(), ks->krn,
                                                   ks->scales, ks->nk, f->Enew.as<float>(), f->est_alpha, est);
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
