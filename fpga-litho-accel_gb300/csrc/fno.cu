@@ -459,14 +459,117 @@ size_t column_smem(int G, bool bwd) {
 }
 
 // ---------------------------------------------------------------------------
+// shared-memory tiles of the row kernels: [px][32 channels] bf16, rows of 64 bytes whose four 16-byte
+// chunks are permuted by (px / 2) & 3, so that the eight rows of a matrix load touch every bank once.
+// A tile is both a row-major operand (ldmatrix) and a column-major one (ldmatrix.trans), and
+// a row of it is 16 KB of global memory in one piece.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t tile_off(int px, int chunk) {
+  return (uint32_t)(px * 64 + ((chunk ^ ((px >> 1) & 3)) << 4));
+}
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldsm4(uint32_t* r, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t* r, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void stsm4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(r0), "r"(r1),
+               "r"(r2), "r"(r3)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+// A fragment of pixels 16 mt .. + 15, channels 16 ks .. + 15; also the place of a C-layout pair of n tiles
+// 2 ks, 2 ks + 1 (stsm4) with the lane's row and chunk
+__device__ __forceinline__ uint32_t tile_frag(int mt, int ks, int lane) {
+  return tile_off(16 * mt + (lane & 15), 2 * ks + (lane >> 4));
+}
+// the 16 x 32 accumulator of pixels 16 mt .. + 15, rounded to bf16, into the tile
+__device__ __forceinline__ void tile_put(uint32_t tile, int mt, int lane, const float (*v)[4]) {
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks)
+    stsm4(tile + tile_frag(mt, ks, lane), pack2(v[2 * ks][0], v[2 * ks][1]), pack2(v[2 * ks][2], v[2 * ks][3]),
+          pack2(v[2 * ks + 1][0], v[2 * ks + 1][1]), pack2(v[2 * ks + 1][2], v[2 * ks + 1][3]));
+}
+// pixels 16 mt .. + 15 of the tile to their kilobyte of global memory (the warp that wrote them)
+__device__ __forceinline__ void tile_store(const unsigned char* tile, int mt, int lane, bf16* row) {
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int i = 32 * q + lane, px = 16 * mt + (i >> 2);
+    *reinterpret_cast<uint4*>(row + (size_t)(16 * mt) * C + 8 * i) =
+        *reinterpret_cast<const uint4*>(tile + tile_off(px, i & 3));
+  }
+}
+// a row of [L][32] bf16 on its way into a tile
+__device__ __forceinline__ void tile_load(uint32_t tile, const bf16* row, int L, int tid) {
+  for (int i = tid; i < 4 * L; i += THREADS) cp_async16(tile + tile_off(i >> 2, i & 3), row + 8 * i);
+}
+// B fragments of a [n rows][32 k] bf16 table with rows of SP: b[ks][0..1] of the eight rows from n0
+__device__ __forceinline__ void ldsm_b(uint32_t (*b)[2], uint32_t tab, int n0, int lane) {
+  uint32_t r[4];
+  ldsm4(r, tab + (uint32_t)((n0 + (lane & 7)) * SP + 8 * (lane >> 3)) * 2);
+  b[0][0] = r[0];
+  b[0][1] = r[1];
+  b[1][0] = r[2];
+  b[1][1] = r[3];
+}
+// the warp's 16 x 8 tile of X[kxri][c] = sum_px TT[kxri][px] v[px][c] (rows 16 (warp / 4), columns
+// 8 (warp % 4)), to one row of Xf / Xg; T pixel tiles of 16
+__device__ __forceinline__ void row_dft(uint32_t sTT, int LP, uint32_t tile, int T, int warp, int lane, float2* xrow) {
+  const int mt2 = warp >> 2, nt = warp & 3, g = lane >> 2, t = lane & 3;
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  const uint32_t ta = sTT + (uint32_t)((16 * mt2 + (lane & 15)) * LP + 8 * (lane >> 4)) * 2;
+#pragma unroll 2
+  for (int ks = 0; ks < T; ks += 2) {
+    uint32_t b[4], a0[4], a1[4];
+    ldsm4t(b, tile + tile_off(16 * ks + lane, nt));  // pixels 16 ks .. + 31
+    ldsm4(a0, ta + 32 * ks);
+    ldsm4(a1, ta + 32 * ks + 32);
+    mma16816(d, a0, b[0], b[1]);
+    mma16816(d, a1, b[2], b[3]);
+  }
+  // lanes g (re) and g ^ 1 (im) of rows kxri = 2 kx + ri: each takes one of the two channels whole
+  const int ri = g & 1;
+  const float p = __shfl_xor_sync(0xffffffffu, ri ? d[0] : d[1], 4);
+  const float q = __shfl_xor_sync(0xffffffffu, ri ? d[2] : d[3], 4);
+  float2* x = xrow + (8 * mt2 + (g >> 1)) * C + 8 * nt + 2 * t + ri;
+  x[0] = ri ? make_float2(p, d[1]) : make_float2(d[0], p);
+  x[4 * C] = ri ? make_float2(q, d[3]) : make_float2(d[2], q);
+}
+
+// ---------------------------------------------------------------------------
 // forward row kernel (persistent over rows; the next row's inputs are
-// prefetched into registers while the current row is computed)
+// on their way while the current row is computed)
 //   v   = lift(mask) (layer 0) or act_in ? GELU(zin) : zin
 //   z_l = W_l v + Wb_l + E(Gy row)
 //   zout (optional) = act_out ? GELU(z_l) : z_l
 //   !FINAL: Xf = x-DFT(GELU(z_l))        (input of the next column kernel)
 //    FINAL: out = Q2 . GELU(Q1 z_3 + q1b) + q2b
-// The inverse / forward DFT tables live in shared memory.
+// The inverse / forward DFT tables live in shared memory, W_l in registers.
+//
+// !FINAL moves 40 KB a row (16 KB in, 16 KB out, 4 KB of each spectrum) and is to be bound by
+// that.  Activations pass through tiles in shared memory: whole 16-byte pieces on the global side
+// (fragment-sized 4-byte accesses used half of each sector) and matrix loads and stores on the other,
+// where one tile serves the store and, transposed, the x-DFT (it took 16 two-byte stores a lane
+// and tile, and 40 scalar fragment loads).  64 masks of 256 x 256: 220 -> 152 us a launch.
+// FINAL's 128 GELUs a pixel bound it (one MUFU result takes a quarter of an SM 8 cycles a warp: 115 us):
+// a warp takes both its pixel tiles through the projection together, so that they share its operands.
+// 333 -> 294 us.
 // ---------------------------------------------------------------------------
 struct RowFwd {
   int L, rows, layer, act_in, act_out;
@@ -484,18 +587,18 @@ struct RowFwd {
 constexpr int MAXT = 2;  // m-tiles (16 pixels) per warp and row: L <= 256
 
 struct FwdSmem {
-  size_t sW, sG, sT, sTT, sVT, sQ1, sQ, total;
+  size_t sG, sT, sTT, sZ, sV, sQ1, sQ, total;
   __host__ __device__ static size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
   __host__ __device__ FwdSmem(int L, bool fin) {
     const size_t LP = (size_t)L + 8;
     size_t o = 0;
-    sW = o; o += up16(C * SP * 2);
-    sG = o; o += up16(C * SP * 2);
+    sZ = o; o += 2 * (size_t)L * C * 2;  // two rows of zin, by parity
+    sG = o; o += 2 * up16(C * SP * 2);   // two rows, by parity
     sT = o; o += up16((size_t)L * SP * 2);
-    sTT = sVT = sQ1 = sQ = 0;
+    sTT = sV = sQ1 = sQ = 0;
     if (!fin) {
+      sV = o; o += (size_t)L * C * 2;
       sTT = o; o += up16(J * LP * 2);
-      sVT = o; o += up16(C * LP * 2);
     } else {
       sQ1 = o; o += up16(H * SP * 2);
       sQ = o; o += up16(2 * H * sizeof(float));
@@ -509,16 +612,13 @@ __global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int L = a.L, LP = L + 8, l = a.layer, T = L / 16;
   const FwdSmem S(L, FINAL);
-  bf16* sW = reinterpret_cast<bf16*>(smraw + S.sW);    // [C o][SP]
-  bf16* sG = reinterpret_cast<bf16*>(smraw + S.sG);    // [C c][SP]
+  bf16* sG0 = reinterpret_cast<bf16*>(smraw + S.sG);   // [2][C c][SP]
   bf16* sT = reinterpret_cast<bf16*>(smraw + S.sT);    // [L px][SP]: inverse table
   bf16* sTT = reinterpret_cast<bf16*>(smraw + S.sTT);  // [J][LP]: forward table
-  bf16* sVT = reinterpret_cast<bf16*>(smraw + S.sVT);  // [C][LP]
   bf16* sQ1 = reinterpret_cast<bf16*>(smraw + S.sQ1);  // [H][SP]
-  float* sQ = reinterpret_cast<float*>(smraw + S.sQ);  // q1b[H], Q2[H]
+  float* sQ = reinterpret_cast<float*>(smraw + S.sQ);  // q1b[H], Q2[H] / 2
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const float* th = a.theta;
-  for (int i = tid; i < C * C; i += THREADS) sW[(i / C) * SP + i % C] = __float2bfloat16(th[Off::W + l * C * C + i]);
   for (int i = tid; i < L * J / 2; i += THREADS) {
     const int px = i / (J / 2), k = 2 * (i % (J / 2));
     *reinterpret_cast<uint32_t*>(sT + px * SP + k) = *reinterpret_cast<const uint32_t*>(a.Ttab + (size_t)px * J + k);
@@ -532,12 +632,18 @@ __global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
     for (int i = tid; i < H * C; i += THREADS) sQ1[(i / C) * SP + i % C] = __float2bfloat16(th[Off::Q1 + i]);
     for (int i = tid; i < H; i += THREADS) {
       sQ[i] = th[Off::q1b + i];
-      sQ[H + i] = th[Off::Q2 + i];
+      sQ[H + i] = 0.5f * th[Off::Q2 + i];
     }
   }
+  uint32_t bw[4][2][2];  // B fragments of W_l: [n][ks]
   float bias[4][2], pw[2][4], pb[2][4];
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
+    const float* w = th + Off::W + l * C * C + (8 * n + g) * C + 2 * t;
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) bw[n][ks][h] = pack2(w[16 * ks + 8 * h], w[16 * ks + 8 * h + 1]);
     bias[n][0] = th[Off::Wb + l * C + 8 * n + 2 * t];
     bias[n][1] = th[Off::Wb + l * C + 8 * n + 2 * t + 1];
   }
@@ -551,62 +657,54 @@ __global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
   }
   const float q2b = th[Off::q2b];
 
-  // register prefetch of one row's inputs
-  uint32_t zr[MAXT][8];
+  // the next row's inputs: zin into the tile of its parity, the rest into registers
   float mr[MAXT][2];
   float2 gr[2];
-  auto load_row = [&](int row) {
+  auto load_row = [&](int row, int st) {
+    if (l == 0) {
 #pragma unroll
-    for (int i = 0; i < MAXT; ++i) {
-      const int mt = warp + 8 * i;
-      if (mt < T) {
-        const int px0 = 16 * mt;
-        if (l == 0) {
-          mr[i][0] = __ldg(a.masks + (size_t)row * L + px0 + g);
-          mr[i][1] = __ldg(a.masks + (size_t)row * L + px0 + g + 8);
-        } else {
-          const bf16* z0 = a.zin + ((size_t)row * L + px0 + g) * C;
-          const bf16* z1 = z0 + 8 * C;
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            const int c0 = 16 * ks + 2 * t;
-            zr[i][4 * ks + 0] = ldg32(z0 + c0);
-            zr[i][4 * ks + 1] = ldg32(z1 + c0);
-            zr[i][4 * ks + 2] = ldg32(z0 + c0 + 8);
-            zr[i][4 * ks + 3] = ldg32(z1 + c0 + 8);
-          }
+      for (int i = 0; i < MAXT; ++i) {
+        const int mt = warp + 8 * i;
+        if (mt < T) {
+          mr[i][0] = __ldg(a.masks + (size_t)row * L + 16 * mt + g);
+          mr[i][1] = __ldg(a.masks + (size_t)row * L + 16 * mt + g + 8);
         }
       }
+    } else {
+      tile_load(smem_u32(smraw + S.sZ) + st * L * C * 2, a.zin + (size_t)row * L * C, L, tid);
     }
     const float2* gp = a.Gy + (size_t)row * M * C;
     gr[0] = __ldg(gp + tid);
     gr[1] = __ldg(gp + tid + THREADS);
   };
-  if (blockIdx.x < a.rows) load_row(blockIdx.x);
+  if (blockIdx.x < a.rows) load_row(blockIdx.x, 0);
+  cp_async_commit();
 
-  for (int row = blockIdx.x; row < a.rows; row += gridDim.x) {
-    __syncthreads();  // previous row is done with sG / sVT
+  int st = 0;
+  for (int row = blockIdx.x; row < a.rows; row += gridDim.x, st ^= 1) {
+    bf16* sG = sG0 + st * (FwdSmem::up16(C * SP * 2) / 2);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int i = tid + THREADS * q, kx = i / C, c = i % C;
       *reinterpret_cast<uint32_t*>(sG + c * SP + 2 * kx) = pack2(gr[q].x, gr[q].y);
     }
-    uint32_t zc[MAXT][8];
     float mc[MAXT][2];
 #pragma unroll
     for (int i = 0; i < MAXT; ++i) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) zc[i][e] = zr[i][e];
       mc[i][0] = mr[i][0];
       mc[i][1] = mr[i][1];
     }
-    if (row + (int)gridDim.x < a.rows) load_row(row + gridDim.x);
-    __syncthreads();
+    cp_async_wait<0>();
+    __syncthreads();  // this row's inputs; also, the other tile and sV are no longer read
+    if (row + (int)gridDim.x < a.rows) load_row(row + gridDim.x, st ^ 1);
+    cp_async_commit();
+    unsigned char* sZ = smraw + S.sZ + (size_t)st * L * C * 2;
+    const uint32_t tz = smem_u32(sZ), tv = smem_u32(smraw + S.sV);
+    uint32_t bg[4][2][2];
 #pragma unroll
-    for (int i = 0; i < MAXT; ++i) {
-      const int mt = warp + 8 * i;
-      if (mt >= T) break;
-      const int px0 = 16 * mt;
+    for (int n = 0; n < 4; ++n) ldsm_b(bg[n], smem_u32(sG), 8 * n, lane);
+    // z_l of the 16 pixels mt, in C layout
+    auto layer = [&](int i, int mt, float (*acc)[4]) {
       uint32_t A[2][4];
       if (l == 0) {
         const float m0 = mc[i][0], m1 = mc[i][1];
@@ -617,17 +715,17 @@ __global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
           A[ks][2] = pack2(fmaf(pw[ks][2], m0, pb[ks][2]), fmaf(pw[ks][3], m0, pb[ks][3]));
           A[ks][3] = pack2(fmaf(pw[ks][2], m1, pb[ks][2]), fmaf(pw[ks][3], m1, pb[ks][3]));
         }
-      } else if (a.act_in) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float2 f = unpack2(zc[i][e]);
-          A[e >> 2][e & 3] = pack2(gelu(f.x), gelu(f.y));
-        }
       } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) A[e >> 2][e & 3] = zc[i][e];
+        for (int ks = 0; ks < 2; ++ks) ldsm4(A[ks], tz + tile_frag(mt, ks, lane));
+        if (a.act_in) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float2 f = unpack2(A[e >> 2][e & 3]);
+            A[e >> 2][e & 3] = pack2(gelu(f.x), gelu(f.y));
+          }
+        }
       }
-      float acc[4][4];
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         acc[n][0] = bias[n][0]; acc[n][1] = bias[n][1];
@@ -636,102 +734,81 @@ __global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) {
         uint32_t AT[4];
-        const bf16* ta = sT + (px0 + g) * SP + 16 * ks + 2 * t;
-        AT[0] = lds32(ta);
-        AT[1] = lds32(ta + 8 * SP);
-        AT[2] = lds32(ta + 8);
-        AT[3] = lds32(ta + 8 * SP + 8);
+        ldsm4(AT, smem_u32(sT) + (uint32_t)((16 * mt + (lane & 15)) * SP + 16 * ks + 8 * (lane >> 4)) * 2);
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
-          const bf16* bw = sW + (8 * n + g) * SP + 16 * ks + 2 * t;
-          mma16816(acc[n], A[ks], lds32(bw), lds32(bw + 8));
-          const bf16* bg = sG + (8 * n + g) * SP + 16 * ks + 2 * t;
-          mma16816(acc[n], AT, lds32(bg), lds32(bg + 8));
+          mma16816(acc[n], A[ks], bw[n][ks][0], bw[n][ks][1]);
+          mma16816(acc[n], AT, bg[n][ks][0], bg[n][ks][1]);
         }
       }
-      if (!FINAL) {
-        float v[4][4];
+      if (a.zout && (FINAL || !a.act_out)) {  // z_l takes the place of the warp's own input
+        tile_put(tz, mt, lane, acc);
+        tile_store(sZ, mt, lane, a.zout + (size_t)row * L * C);
+      }
+    };
+    if constexpr (!FINAL) {
+#pragma unroll
+      for (int i = 0; i < MAXT; ++i) {
+        const int mt = warp + 8 * i;
+        if (mt >= T) break;
+        float acc[4][4];
+        layer(i, mt, acc);
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) v[n][e] = gelu(acc[n][e]);
-        if (a.zout) {
-          bf16* zo0 = a.zout + ((size_t)row * L + px0 + g) * C;
-          bf16* zo1 = zo0 + 8 * C;
+          for (int e = 0; e < 4; ++e) acc[n][e] = gelu(acc[n][e]);
+        tile_put(tv, mt, lane, acc);
+        if (a.zout && a.act_out) tile_store(smraw + S.sV, mt, lane, a.zout + (size_t)row * L * C);
+      }
+      __syncthreads();
+      row_dft(smem_u32(sTT), LP, tv, T, warp, lane, a.Xf + (size_t)row * M * C);
+    } else if (warp < T) {
+      const bool two = warp + 8 < T;
+      uint32_t Az[MAXT][2][4];
 #pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            const float* src = a.act_out ? v[n] : acc[n];
-            *reinterpret_cast<uint32_t*>(zo0 + 8 * n + 2 * t) = pack2(src[0], src[1]);
-            *reinterpret_cast<uint32_t*>(zo1 + 8 * n + 2 * t) = pack2(src[2], src[3]);
+      for (int i = 0; i < MAXT; ++i) {
+        if (i == 1 && !two) break;
+        float acc[4][4];
+        layer(i, warp + 8 * i, acc);
+        acc_to_a(acc[0], acc[1], Az[i][0]);
+        acc_to_a(acc[2], acc[3], Az[i][1]);
+      }
+      float p[MAXT][2] = {};
+#pragma unroll 2
+      for (int nh = 0; nh < H / 8; ++nh) {
+        uint32_t bq[2][2];
+        ldsm_b(bq, smem_u32(sQ1), 8 * nh, lane);
+        const float2 b = *reinterpret_cast<const float2*>(sQ + 8 * nh + 2 * t);
+        const float2 q = *reinterpret_cast<const float2*>(sQ + H + 8 * nh + 2 * t);
+#pragma unroll
+        for (int i = 0; i < MAXT; ++i) {
+          if (i == 1 && !two) break;
+          float hc[4] = {b.x, b.y, b.x, b.y};
+          mma16816(hc, Az[i][0], bq[0][0], bq[0][1]);
+          mma16816(hc, Az[i][1], bq[1][0], bq[1][1]);
+          // q gelu(x) = (q/2) x + (q/2) x tanh(x (k0 + k0 k1 x^2))
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x = hc[e], hx = (e & 1 ? q.y : q.x) * x;
+            const float th_ = tanh_hw(x * fmaf(GK0 * GK1, x * x, GK0));
+            p[i][e >> 1] = fmaf(hx, th_, p[i][e >> 1] + hx);
           }
         }
+      }
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const int c = 8 * n + 2 * t;
-          sVT[c * LP + px0 + g] = __float2bfloat16(v[n][0]);
-          sVT[(c + 1) * LP + px0 + g] = __float2bfloat16(v[n][1]);
-          sVT[c * LP + px0 + g + 8] = __float2bfloat16(v[n][2]);
-          sVT[(c + 1) * LP + px0 + g + 8] = __float2bfloat16(v[n][3]);
-        }
-      } else {
-        if (a.zout) {
-          bf16* zo0 = a.zout + ((size_t)row * L + px0 + g) * C;
-          bf16* zo1 = zo0 + 8 * C;
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            *reinterpret_cast<uint32_t*>(zo0 + 8 * n + 2 * t) = pack2(acc[n][0], acc[n][1]);
-            *reinterpret_cast<uint32_t*>(zo1 + 8 * n + 2 * t) = pack2(acc[n][2], acc[n][3]);
-          }
-        }
-        uint32_t Az[2][4];
-        acc_to_a(acc[0], acc[1], Az[0]);
-        acc_to_a(acc[2], acc[3], Az[1]);
-        float p0 = 0.f, p1 = 0.f;
-#pragma unroll 4
-        for (int nh = 0; nh < H / 8; ++nh) {
-          const int h0 = 8 * nh + 2 * t;
-          float hc[4] = {sQ[h0], sQ[h0 + 1], sQ[h0], sQ[h0 + 1]};
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            const bf16* bq = sQ1 + (8 * nh + g) * SP + 16 * ks + 2 * t;
-            mma16816(hc, Az[ks], lds32(bq), lds32(bq + 8));
-          }
-          const float q0 = sQ[H + h0], q1 = sQ[H + h0 + 1];
-          p0 = fmaf(q0, gelu(hc[0]), fmaf(q1, gelu(hc[1]), p0));
-          p1 = fmaf(q0, gelu(hc[2]), fmaf(q1, gelu(hc[3]), p1));
-        }
+      for (int i = 0; i < MAXT; ++i) {
+        if (i == 1 && !two) break;
+        float p0 = p[i][0], p1 = p[i][1];
         p0 += __shfl_xor_sync(0xffffffffu, p0, 1);
         p0 += __shfl_xor_sync(0xffffffffu, p0, 2);
         p1 += __shfl_xor_sync(0xffffffffu, p1, 1);
         p1 += __shfl_xor_sync(0xffffffffu, p1, 2);
         if (t == 0) {
-          a.out[(size_t)row * L + px0 + g] = p0 + q2b;
-          a.out[(size_t)row * L + px0 + g + 8] = p1 + q2b;
+          float* o = a.out + (size_t)row * L + 16 * (warp + 8 * i) + g;
+          o[0] = p0 + q2b;
+          o[8] = p1 + q2b;
         }
       }
-    }
-    if (!FINAL) {
-      __syncthreads();
-      // x-DFT of the row: X[kxri][c] = sum_px TT[kxri][px] v[px][c]; warp -> one 16 x 8 tile
-      const int mt2 = warp >> 2, nt = warp & 3;
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-      const bf16* ta = sTT + (16 * mt2 + g) * LP + 2 * t;
-      const bf16* tb = sVT + (8 * nt + g) * LP + 2 * t;
-#pragma unroll 4
-      for (int ks = 0; ks < T; ++ks) {
-        uint32_t AF[4];
-        AF[0] = lds32(ta + 16 * ks);
-        AF[1] = lds32(ta + 8 * LP + 16 * ks);
-        AF[2] = lds32(ta + 16 * ks + 8);
-        AF[3] = lds32(ta + 8 * LP + 16 * ks + 8);
-        mma16816(d, AF, lds32(tb + 16 * ks), lds32(tb + 16 * ks + 8));
-      }
-      float* xf = reinterpret_cast<float*>(a.Xf + (size_t)row * M * C);
-      const int k0 = 16 * mt2 + g, c0 = 8 * nt + 2 * t;  // kxri rows k0, k0 + 8
-      xf[((k0 >> 1) * C + c0) * 2 + (k0 & 1)] = d[0];
-      xf[((k0 >> 1) * C + c0 + 1) * 2 + (k0 & 1)] = d[1];
-      xf[(((k0 + 8) >> 1) * C + c0) * 2 + (k0 & 1)] = d[2];
-      xf[(((k0 + 8) >> 1) * C + c0 + 1) * 2 + (k0 & 1)] = d[3];
     }
   }
 }
