@@ -117,6 +117,60 @@ __device__ __forceinline__ float gelu_grad(float x) {
   const float t = tanh_hw(GK0 * fmaf(GK1 * x, x2, x));
   return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GK0 * fmaf(3.0f * GK1, x2, 1.0f);
 }
+// The same on two values at once with the packed FP32 instructions (each half rounds as the scalar one
+// does): the row kernels run out of issue slots before they run out of arithmetic, and a GELU is seven
+// FP32 instructions and one of the special-function unit.
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ float2 f2_get(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 tanh2(F2 a) {
+  const float2 x = f2_get(a);
+  return f2(tanh_hw(x.x), tanh_hw(x.y));
+}
+__device__ __forceinline__ F2 gelu2(F2 x) {
+  const F2 t = tanh2(f2(GK0) * fma2(f2(GK1) * x, x * x, x));
+  return (f2(0.5f) * x) * (f2(1.0f) + t);
+}
+__device__ __forceinline__ F2 gelu_grad2(F2 x) {
+  const F2 x2 = x * x;
+  const F2 t = tanh2(f2(GK0) * fma2(f2(GK1) * x, x2, x));
+  const F2 h = f2(0.5f) * x, u = fma2(f2(-1.0f) * t, t, f2(1.0f));
+  return fma2(h * u * f2(GK0), fma2(f2(3.0f * GK1), x2, f2(1.0f)), f2(0.5f) * (f2(1.0f) + t));
+}
+__device__ __forceinline__ uint32_t pack2(F2 a) {
+  const float2 x = f2_get(a);
+  return pack2(x.x, x.y);
+}
+__device__ __forceinline__ F2 unpack_f2(uint32_t u) {
+  const float2 x = unpack2(u);
+  return f2(x.x, x.y);
+}
 // GELU and its derivative together
 __device__ __forceinline__ void gelu_both(float x, float& g, float& d) {
   const float x2 = x * x;
@@ -566,10 +620,12 @@ __device__ __forceinline__ void row_dft(uint32_t sTT, int LP, uint32_t tile, int
 // that.  Activations pass through tiles in shared memory: whole 16-byte pieces on the global side
 // (fragment-sized 4-byte accesses used half of each sector) and matrix loads and stores on the other,
 // where one tile serves the store and, transposed, the x-DFT (it took 16 two-byte stores a lane
-// and tile, and 40 scalar fragment loads).  64 masks of 256 x 256: 220 -> 152 us a launch.
+// and tile, and 40 scalar fragment loads).  What is left is the shared memory's bandwidth (70% busy),
+// half of it the x-DFT's operands.  64 masks of 256 x 256: 220 -> 139 us a launch.
+// Two CTAs per SM: a third took the registers of the two pixel tiles (172 us).
 // FINAL's 128 GELUs a pixel bound it (one MUFU result takes a quarter of an SM 8 cycles a warp: 115 us):
 // a warp takes both its pixel tiles through the projection together, so that they share its operands.
-// 333 -> 294 us.
+// 333 -> 267 us.
 // ---------------------------------------------------------------------------
 struct RowFwd {
   int L, rows, layer, act_in, act_out;
@@ -587,14 +643,14 @@ struct RowFwd {
 constexpr int MAXT = 2;  // m-tiles (16 pixels) per warp and row: L <= 256
 
 struct FwdSmem {
-  size_t sG, sT, sTT, sZ, sV, sQ1, sQ, total;
-  __host__ __device__ static size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
+  size_t sG, sW, sTT, sZ, sV, sQ1, sQ, total;
+  __host__ __device__ static constexpr size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
   __host__ __device__ FwdSmem(int L, bool fin) {
     const size_t LP = (size_t)L + 8;
     size_t o = 0;
     sZ = o; o += 2 * (size_t)L * C * 2;  // two rows of zin, by parity
     sG = o; o += 2 * up16(C * SP * 2);   // two rows, by parity
-    sT = o; o += up16((size_t)L * SP * 2);
+    sW = o; o += up16(C * SP * 2);
     sTT = sV = sQ1 = sQ = 0;
     if (!fin) {
       sV = o; o += (size_t)L * C * 2;
@@ -607,22 +663,23 @@ struct FwdSmem {
   }
 };
 
-template <bool FINAL>
-__global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
+enum { FWD_FIRST = 0, FWD_MID = 1, FWD_LAST = 2 };
+constexpr int FWD_CTAS = 2;  // per SM
+
+template <int KIND>
+__global__ void __launch_bounds__(THREADS, FWD_CTAS) row_fwd_kernel(const RowFwd a) {
+  constexpr bool FIRST = KIND == FWD_FIRST, FINAL = KIND == FWD_LAST;
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int L = a.L, LP = L + 8, l = a.layer, T = L / 16;
+  const int L = a.L, LP = L + 8, l = FIRST ? 0 : FINAL ? NL - 1 : a.layer, T = L / 16;
   const FwdSmem S(L, FINAL);
   bf16* sG0 = reinterpret_cast<bf16*>(smraw + S.sG);   // [2][C c][SP]
-  bf16* sT = reinterpret_cast<bf16*>(smraw + S.sT);    // [L px][SP]: inverse table
+  bf16* sW = reinterpret_cast<bf16*>(smraw + S.sW);    // [C o][SP]
   bf16* sTT = reinterpret_cast<bf16*>(smraw + S.sTT);  // [J][LP]: forward table
   bf16* sQ1 = reinterpret_cast<bf16*>(smraw + S.sQ1);  // [H][SP]
   float* sQ = reinterpret_cast<float*>(smraw + S.sQ);  // q1b[H], Q2[H] / 2
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const float* th = a.theta;
-  for (int i = tid; i < L * J / 2; i += THREADS) {
-    const int px = i / (J / 2), k = 2 * (i % (J / 2));
-    *reinterpret_cast<uint32_t*>(sT + px * SP + k) = *reinterpret_cast<const uint32_t*>(a.Ttab + (size_t)px * J + k);
-  }
+  for (int i = tid; i < C * C; i += THREADS) sW[(i / C) * SP + i % C] = __float2bfloat16(th[Off::W + l * C * C + i]);
   if (!FINAL)
     for (int i = tid; i < J * L / 2; i += THREADS) {
       const int k = i / (L / 2), px = 2 * (i % (L / 2));
@@ -635,33 +692,41 @@ __global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
       sQ[H + i] = 0.5f * th[Off::Q2 + i];
     }
   }
-  uint32_t bw[4][2][2];  // B fragments of W_l: [n][ks]
+  // A fragments of the inverse table at the warp's pixels, the same for every row
+  uint32_t AT[MAXT][2][4];
+#pragma unroll
+  for (int i = 0; i < MAXT; ++i)
+    if (warp + 8 * i < T)
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        const bf16* ta = a.Ttab + (size_t)(16 * (warp + 8 * i) + g) * J + 16 * ks + 2 * t;
+        AT[i][ks][0] = ldg32(ta);
+        AT[i][ks][1] = ldg32(ta + 8 * J);
+        AT[i][ks][2] = ldg32(ta + 8);
+        AT[i][ks][3] = ldg32(ta + 8 * J + 8);
+      }
   float bias[4][2], pw[2][4], pb[2][4];
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
-    const float* w = th + Off::W + l * C * C + (8 * n + g) * C + 2 * t;
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) bw[n][ks][h] = pack2(w[16 * ks + 8 * h], w[16 * ks + 8 * h + 1]);
     bias[n][0] = th[Off::Wb + l * C + 8 * n + 2 * t];
     bias[n][1] = th[Off::Wb + l * C + 8 * n + 2 * t + 1];
   }
+  if (FIRST)
 #pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
-    const int c0 = 16 * ks + 2 * t;
-    pw[ks][0] = th[Off::Pw + c0];     pb[ks][0] = th[Off::Pb + c0];
-    pw[ks][1] = th[Off::Pw + c0 + 1]; pb[ks][1] = th[Off::Pb + c0 + 1];
-    pw[ks][2] = th[Off::Pw + c0 + 8]; pb[ks][2] = th[Off::Pb + c0 + 8];
-    pw[ks][3] = th[Off::Pw + c0 + 9]; pb[ks][3] = th[Off::Pb + c0 + 9];
-  }
+    for (int ks = 0; ks < 2; ++ks) {
+      const int c0 = 16 * ks + 2 * t;
+      pw[ks][0] = th[Off::Pw + c0];     pb[ks][0] = th[Off::Pb + c0];
+      pw[ks][1] = th[Off::Pw + c0 + 1]; pb[ks][1] = th[Off::Pb + c0 + 1];
+      pw[ks][2] = th[Off::Pw + c0 + 8]; pb[ks][2] = th[Off::Pb + c0 + 8];
+      pw[ks][3] = th[Off::Pw + c0 + 9]; pb[ks][3] = th[Off::Pb + c0 + 9];
+    }
   const float q2b = th[Off::q2b];
 
   // the next row's inputs: zin into the tile of its parity, the rest into registers
   float mr[MAXT][2];
   float2 gr[2];
   auto load_row = [&](int row, int st) {
-    if (l == 0) {
+    if (FIRST) {
 #pragma unroll
       for (int i = 0; i < MAXT; ++i) {
         const int mt = warp + 8 * i;
@@ -689,126 +754,148 @@ __global__ void __launch_bounds__(THREADS, 2) row_fwd_kernel(const RowFwd a) {
       *reinterpret_cast<uint32_t*>(sG + c * SP + 2 * kx) = pack2(gr[q].x, gr[q].y);
     }
     float mc[MAXT][2];
+    if (FIRST)
 #pragma unroll
-    for (int i = 0; i < MAXT; ++i) {
-      mc[i][0] = mr[i][0];
-      mc[i][1] = mr[i][1];
-    }
+      for (int i = 0; i < MAXT; ++i) {
+        mc[i][0] = mr[i][0];
+        mc[i][1] = mr[i][1];
+      }
     cp_async_wait<0>();
     __syncthreads();  // this row's inputs; also, the other tile and sV are no longer read
     if (row + (int)gridDim.x < a.rows) load_row(row + gridDim.x, st ^ 1);
     cp_async_commit();
     unsigned char* sZ = smraw + S.sZ + (size_t)st * L * C * 2;
     const uint32_t tz = smem_u32(sZ), tv = smem_u32(smraw + S.sV);
-    uint32_t bg[4][2][2];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) ldsm_b(bg[n], smem_u32(sG), 8 * n, lane);
-    // z_l of the 16 pixels mt, in C layout
-    auto layer = [&](int i, int mt, float (*acc)[4]) {
-      uint32_t A[2][4];
-      if (l == 0) {
-        const float m0 = mc[i][0], m1 = mc[i][1];
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-          A[ks][0] = pack2(fmaf(pw[ks][0], m0, pb[ks][0]), fmaf(pw[ks][1], m0, pb[ks][1]));
-          A[ks][1] = pack2(fmaf(pw[ks][0], m1, pb[ks][0]), fmaf(pw[ks][1], m1, pb[ks][1]));
-          A[ks][2] = pack2(fmaf(pw[ks][2], m0, pb[ks][2]), fmaf(pw[ks][3], m0, pb[ks][3]));
-          A[ks][3] = pack2(fmaf(pw[ks][2], m1, pb[ks][2]), fmaf(pw[ks][3], m1, pb[ks][3]));
-        }
-      } else {
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) ldsm4(A[ks], tz + tile_frag(mt, ks, lane));
-        if (a.act_in) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float2 f = unpack2(A[e >> 2][e & 3]);
-            A[e >> 2][e & 3] = pack2(gelu(f.x), gelu(f.y));
-          }
-        }
-      }
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        acc[n][0] = bias[n][0]; acc[n][1] = bias[n][1];
-        acc[n][2] = bias[n][0]; acc[n][3] = bias[n][1];
-      }
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        uint32_t AT[4];
-        ldsm4(AT, smem_u32(sT) + (uint32_t)((16 * mt + (lane & 15)) * SP + 16 * ks + 8 * (lane >> 4)) * 2);
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          mma16816(acc[n], A[ks], bw[n][ks][0], bw[n][ks][1]);
-          mma16816(acc[n], AT, bg[n][ks][0], bg[n][ks][1]);
-        }
-      }
-      if (a.zout && (FINAL || !a.act_out)) {  // z_l takes the place of the warp's own input
-        tile_put(tz, mt, lane, acc);
-        tile_store(sZ, mt, lane, a.zout + (size_t)row * L * C);
-      }
-    };
-    if constexpr (!FINAL) {
-#pragma unroll
-      for (int i = 0; i < MAXT; ++i) {
-        const int mt = warp + 8 * i;
-        if (mt >= T) break;
-        float acc[4][4];
-        layer(i, mt, acc);
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc[n][e] = gelu(acc[n][e]);
-        tile_put(tv, mt, lane, acc);
-        if (a.zout && a.act_out) tile_store(smraw + S.sV, mt, lane, a.zout + (size_t)row * L * C);
-      }
-      __syncthreads();
-      row_dft(smem_u32(sTT), LP, tv, T, warp, lane, a.Xf + (size_t)row * M * C);
-    } else if (warp < T) {
+    // z_l of the warp's pixel tiles in C layout, both at a time: they share the weights' and the
+    // spectrum's fragments and hide each other's latency
+    if (warp < T) {
       const bool two = warp + 8 < T;
-      uint32_t Az[MAXT][2][4];
-#pragma unroll
-      for (int i = 0; i < MAXT; ++i) {
-        if (i == 1 && !two) break;
-        float acc[4][4];
-        layer(i, warp + 8 * i, acc);
-        acc_to_a(acc[0], acc[1], Az[i][0]);
-        acc_to_a(acc[2], acc[3], Az[i][1]);
-      }
-      float p[MAXT][2] = {};
-#pragma unroll 2
-      for (int nh = 0; nh < H / 8; ++nh) {
-        uint32_t bq[2][2];
-        ldsm_b(bq, smem_u32(sQ1), 8 * nh, lane);
-        const float2 b = *reinterpret_cast<const float2*>(sQ + 8 * nh + 2 * t);
-        const float2 q = *reinterpret_cast<const float2*>(sQ + H + 8 * nh + 2 * t);
+      float acc[MAXT][4][4];
+      {
+        uint32_t A[MAXT][2][4];
 #pragma unroll
         for (int i = 0; i < MAXT; ++i) {
           if (i == 1 && !two) break;
-          float hc[4] = {b.x, b.y, b.x, b.y};
-          mma16816(hc, Az[i][0], bq[0][0], bq[0][1]);
-          mma16816(hc, Az[i][1], bq[1][0], bq[1][1]);
-          // q gelu(x) = (q/2) x + (q/2) x tanh(x (k0 + k0 k1 x^2))
+          if (FIRST) {
+            const float m0 = mc[i][0], m1 = mc[i][1];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float x = hc[e], hx = (e & 1 ? q.y : q.x) * x;
-            const float th_ = tanh_hw(x * fmaf(GK0 * GK1, x * x, GK0));
-            p[i][e >> 1] = fmaf(hx, th_, p[i][e >> 1] + hx);
+            for (int ks = 0; ks < 2; ++ks) {
+              A[i][ks][0] = pack2(fmaf(pw[ks][0], m0, pb[ks][0]), fmaf(pw[ks][1], m0, pb[ks][1]));
+              A[i][ks][1] = pack2(fmaf(pw[ks][0], m1, pb[ks][0]), fmaf(pw[ks][1], m1, pb[ks][1]));
+              A[i][ks][2] = pack2(fmaf(pw[ks][2], m0, pb[ks][2]), fmaf(pw[ks][3], m0, pb[ks][3]));
+              A[i][ks][3] = pack2(fmaf(pw[ks][2], m1, pb[ks][2]), fmaf(pw[ks][3], m1, pb[ks][3]));
+            }
+          } else {
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) ldsm4(A[i][ks], tz + tile_frag(warp + 8 * i, ks, lane));
+          }
+        }
+        if (!FIRST && a.act_in)
+#pragma unroll
+          for (int i = 0; i < MAXT; ++i) {
+            if (i == 1 && !two) break;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) A[i][e >> 2][e & 3] = pack2(gelu2(unpack_f2(A[i][e >> 2][e & 3])));
+          }
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          uint32_t bw[2][2], bg[2][2];
+          ldsm_b(bw, smem_u32(sW), 8 * n, lane);
+          ldsm_b(bg, smem_u32(sG), 8 * n, lane);
+#pragma unroll
+          for (int i = 0; i < MAXT; ++i) {
+            acc[i][n][0] = bias[n][0]; acc[i][n][1] = bias[n][1];
+            acc[i][n][2] = bias[n][0]; acc[i][n][3] = bias[n][1];
+          }
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+            for (int i = 0; i < MAXT; ++i) {
+              if (i == 1 && !two) break;
+              mma16816(acc[i][n], A[i][ks], bw[ks][0], bw[ks][1]);
+              mma16816(acc[i][n], AT[i][ks], bg[ks][0], bg[ks][1]);
+            }
+        }
+      }
+      if (a.zout && (FINAL || !a.act_out)) {  // z_l takes the place of the warp's own input
+#pragma unroll
+        for (int i = 0; i < MAXT; ++i) {
+          if (i == 1 && !two) break;
+          tile_put(tz, warp + 8 * i, lane, acc[i]);
+          tile_store(sZ, warp + 8 * i, lane, a.zout + (size_t)row * L * C);
+        }
+      }
+      if constexpr (!FINAL) {
+#pragma unroll
+        for (int i = 0; i < MAXT; ++i) {
+          if (i == 1 && !two) break;
+#pragma unroll
+          for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              const float2 v = f2_get(gelu2(f2(acc[i][n][e], acc[i][n][e + 1])));
+              acc[i][n][e] = v.x;
+              acc[i][n][e + 1] = v.y;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < MAXT; ++i) {
+          if (i == 1 && !two) break;
+          tile_put(tv, warp + 8 * i, lane, acc[i]);
+          if (a.zout && a.act_out) tile_store(smraw + S.sV, warp + 8 * i, lane, a.zout + (size_t)row * L * C);
+        }
+      } else {
+        uint32_t Az[MAXT][2][4];
+#pragma unroll
+        for (int i = 0; i < MAXT; ++i) {
+          acc_to_a(acc[i][0], acc[i][1], Az[i][0]);
+          acc_to_a(acc[i][2], acc[i][3], Az[i][1]);
+        }
+        F2 p[MAXT][2];
+#pragma unroll
+        for (int i = 0; i < MAXT; ++i) p[i][0] = p[i][1] = f2(0.f);
+#pragma unroll 2
+        for (int nh = 0; nh < H / 8; ++nh) {
+          uint32_t bq[2][2];
+          ldsm_b(bq, smem_u32(sQ1), 8 * nh, lane);
+          const float2 b = *reinterpret_cast<const float2*>(sQ + 8 * nh + 2 * t);
+          const float2 qs = *reinterpret_cast<const float2*>(sQ + H + 8 * nh + 2 * t);
+          const F2 q = f2(qs.x, qs.y);
+#pragma unroll
+          for (int i = 0; i < MAXT; ++i) {
+            if (i == 1 && !two) break;
+            float hc[4] = {b.x, b.y, b.x, b.y};
+            mma16816(hc, Az[i][0], bq[0][0], bq[0][1]);
+            mma16816(hc, Az[i][1], bq[1][0], bq[1][1]);
+            // q gelu(x) = (q/2) x + (q/2) x tanh(x (k0 + k0 k1 x^2))
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const F2 x = f2(hc[2 * r], hc[2 * r + 1]), hx = q * x;
+              const F2 th_ = tanh2(x * fma2(f2(GK0 * GK1), x * x, f2(GK0)));
+              p[i][r] = fma2(hx, th_, p[i][r] + hx);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < MAXT; ++i) {
+          if (i == 1 && !two) break;
+          const float2 s0 = f2_get(p[i][0]), s1 = f2_get(p[i][1]);
+          float p0 = s0.x + s0.y, p1 = s1.x + s1.y;
+          p0 += __shfl_xor_sync(0xffffffffu, p0, 1);
+          p0 += __shfl_xor_sync(0xffffffffu, p0, 2);
+          p1 += __shfl_xor_sync(0xffffffffu, p1, 1);
+          p1 += __shfl_xor_sync(0xffffffffu, p1, 2);
+          if (t == 0) {
+            float* o = a.out + (size_t)row * L + 16 * (warp + 8 * i) + g;
+            o[0] = p0 + q2b;
+            o[8] = p1 + q2b;
           }
         }
       }
-#pragma unroll
-      for (int i = 0; i < MAXT; ++i) {
-        if (i == 1 && !two) break;
-        float p0 = p[i][0], p1 = p[i][1];
-        p0 += __shfl_xor_sync(0xffffffffu, p0, 1);
-        p0 += __shfl_xor_sync(0xffffffffu, p0, 2);
-        p1 += __shfl_xor_sync(0xffffffffu, p1, 1);
-        p1 += __shfl_xor_sync(0xffffffffu, p1, 2);
-        if (t == 0) {
-          float* o = a.out + (size_t)row * L + 16 * (warp + 8 * i) + g;
-          o[0] = p0 + q2b;
-          o[8] = p1 + q2b;
-        }
-      }
+    }
+    if constexpr (!FINAL) {
+      __syncthreads();
+      row_dft(smem_u32(sTT), LP, tv, T, warp, lane, a.Xf + (size_t)row * M * C);
     }
   }
 }
@@ -1609,6 +1696,7 @@ struct litho_fno {
 
 namespace {
 
+int fwd_grid(litho_fno* f, int rows) { return std::max(1, std::min(rows, FWD_CTAS * f->ctx->sm_count)); }
 int fno_grid(litho_fno* f, int rows) { return std::max(1, std::min(rows, 2 * f->ctx->sm_count)); }
 
 // The column kernel over B masks, in groups of four, two or one: the more masks share the reading of
@@ -1681,12 +1769,13 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
   litho_ctx* ctx = f->ctx;
   const int L = f->L, rows = B * L;
   const float* th = f->theta.as<float>();
-  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<false>, row_fwd_smem(L, false)));
-  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<true>, row_fwd_smem(L, true)));
+  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<FWD_FIRST>, row_fwd_smem(L, false)));
+  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<FWD_MID>, row_fwd_smem(L, false)));
+  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<FWD_LAST>, row_fwd_smem(L, true)));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 2 * NL + 1);
   lift_dft_kernel<<<dft_blocks(rows), THREADS, rows_dft_smem(L), ctx->stream>>>(L, rows, th, masks, f->twL.as<float2>(),
                                                                                f->Xf.as<float2>(), Mrow);
-  const int grid = fno_grid(f, rows);
+  const int grid = fwd_grid(f, rows);
   for (int l = 0; l < NL; ++l) {
     LITHO_RET(launch_column<false>(f, B, l, f->Xf.as<float2>(), f->Gy.as<float2>(),
                                    train ? f->Vs[l].as<float2>() : nullptr));
@@ -1700,10 +1789,12 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
     a.Xf = f->Xf.as<float2>();
     a.out = images;
     a.Ttab = f->Ttab.as<bf16>(); a.TT = f->TT.as<bf16>();
-    if (l < NL - 1)
-      row_fwd_kernel<false><<<grid, THREADS, row_fwd_smem(L, false), ctx->stream>>>(a);
+    if (l == 0)
+      row_fwd_kernel<FWD_FIRST><<<grid, THREADS, row_fwd_smem(L, false), ctx->stream>>>(a);
+    else if (l < NL - 1)
+      row_fwd_kernel<FWD_MID><<<grid, THREADS, row_fwd_smem(L, false), ctx->stream>>>(a);
     else
-      row_fwd_kernel<true><<<grid, THREADS, row_fwd_smem(L, true), ctx->stream>>>(a);
+      row_fwd_kernel<FWD_LAST><<<grid, THREADS, row_fwd_smem(L, true), ctx->stream>>>(a);
   }
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
