@@ -769,55 +769,103 @@ int fi_twiddles(litho_ctx* ctx, const ImgGeom& g, const float2** out) {
 // shared-memory rows, each pass writing its result transposed.
 //   C[X] = sum_p a[p] e^{-2 pi i (X - F/2)(p - F/2)/F}
 //        = (-1)^(X + F/2) * DFT((-1)^p a[p])[X]
+// Up to three radix-2 stages at a time run in registers (the same butterflies and
+// twiddles as one by one), the first of them straight from global memory, so that
+// a row of 1024 crosses shared memory four times instead of eleven; and a CTA takes
+// four rows instead of sixteen, which gives every SM work (64 CTAs for 1024 rows
+// left most idle).  One 1024 x 1024 mask: 2 x 75 us -> 2 x 14.
 // ---------------------------------------------------------------------------
 constexpr int FM_THREADS = 256;
 
+// place of element i of a row: consecutive ones, and ones F/16 or 8 apart, spread over the banks
+__host__ __device__ __forceinline__ int fm_pad(int i) { return i + (i >> 3) + (i >> 6); }
+__host__ __device__ __forceinline__ int fm_stride(int F) { return ((fm_pad(F - 1) + 16) & ~15) + 4; }
+
+// stages h, 2 h, .. 2^(S-1) h on 2^S elements pos + m h of one group
+template <int S>
+__device__ __forceinline__ void fm_stages(float2 (&x)[8], const float2* tw, int logF, int lh, int pos) {
+#pragma unroll
+  for (int q = 0; q < S; ++q)
+#pragma unroll
+    for (int m = 0; m < (1 << S); ++m)
+      if (!(m & (1 << q))) {
+        const float2 w = tw[(pos + ((m & ((1 << q) - 1)) << lh)) << (logF - lh - q - 1)];
+        const float2 t = cmul(w, x[m | (1 << q)]), a = x[m];
+        x[m] = cadd(a, t);
+        x[m | (1 << q)] = csub(a, t);
+      }
+}
+template <int S>
+__device__ __forceinline__ void fm_pass(float2* s, int SF, const float2* tw, int TR, int logF, int lh) {
+  const int per = 1 << (logF - S);
+  for (int idx = threadIdx.x; idx < TR * per; idx += FM_THREADS) {
+    const int j = idx & (per - 1), pos = j & ((1 << lh) - 1);
+    float2* row = s + (idx >> (logF - S)) * SF;
+    const int base = ((j >> lh) << (lh + S)) + pos;
+    float2 x[8];
+#pragma unroll
+    for (int m = 0; m < (1 << S); ++m) x[m] = row[fm_pad(base + (m << lh))];
+    fm_stages<S>(x, tw, logF, lh, pos);
+#pragma unroll
+    for (int m = 0; m < (1 << S); ++m) row[fm_pad(base + (m << lh))] = x[m];
+  }
+}
+
 // rows: `nrows` input rows of length `len` (real if in_i == nullptr), padded
 // centred into F; output written transposed: out[X][row] (row stride ldo).
+template <int S0>
 __global__ void __launch_bounds__(FM_THREADS) fft_rows_centred_kernel(
     const float* __restrict__ in_r, const float* __restrict__ in_i, const float2* __restrict__ in_c,
-    int nrows, int len, int F, int TR, float scale, float2* __restrict__ out_c, float* __restrict__ out_r,
+    int nrows, int len, int logF, int TR, float scale, float2* __restrict__ out_c, float* __restrict__ out_r,
     float* __restrict__ out_i, int ldo) {
   extern __shared__ __align__(16) float2 fr[];
-  const int SF = F + 1;
+  const int F = 1 << logF, SF = fm_stride(F);
   float2* s = fr;                 // [TR][SF]
   float2* tw = fr + TR * SF;      // [F/2]
   const int tid = threadIdx.x;
   const int r0 = blockIdx.x * TR;
-  const int logF = 31 - __clz(F);
   const int off = (F - len) / 2;
   for (int e = tid; e < F / 2; e += FM_THREADS) {
     float sn, cs;
     sincospif(2.0f * (float)e / (float)F, &sn, &cs);
     tw[e] = make_float2(cs, -sn);
   }
-  // load with bit-reversed placement, pre-multiplied by (-1)^p
-  for (int idx = tid; idx < TR * F; idx += FM_THREADS) {
-    const int r = idx / F, p = idx - r * F;
+  __syncthreads();
+  // the first stages, on elements q + m F / 2^S0 (bit-reversed: adjacent), pre-multiplied by (-1)^p
+  const int per = F >> S0;
+  for (int idx = tid; idx < TR * per; idx += FM_THREADS) {
+    const int r = idx >> (logF - S0), q = idx & (per - 1);
     const int row = r0 + r;
-    float2 v = make_float2(0.f, 0.f);
-    const int q = p - off;
-    if (row < nrows && q >= 0 && q < len) {
-      const size_t o = (size_t)row * len + q;
-      if (in_c) v = in_c[o];
-      else v = make_float2(in_r[o], in_i ? in_i[o] : 0.f);
-      if (p & 1) v = make_float2(-v.x, -v.y);
+    float2 x[8];
+#pragma unroll
+    for (int m = 0; m < (1 << S0); ++m) {
+      const int p = q + (int)(__brev((unsigned)m) >> (32 - S0)) * per, i = p - off;
+      float2 v = make_float2(0.f, 0.f);
+      if (row < nrows && i >= 0 && i < len) {
+        const size_t o = (size_t)row * len + i;
+        if (in_c) v = in_c[o];
+        else v = make_float2(in_r[o], in_i ? in_i[o] : 0.f);
+        if (p & 1) v = make_float2(-v.x, -v.y);
+      }
+      x[m] = v;
     }
-    const int br = (int)(__brev((unsigned)p) >> (32 - logF));
-    s[r * SF + br] = v;
+    fm_stages<S0>(x, tw, logF, 0, 0);
+    const int base = logF == S0 ? 0 : (int)(__brev((unsigned)q) >> (32 - (logF - S0))) << S0;
+#pragma unroll
+    for (int m = 0; m < (1 << S0); ++m) s[r * SF + fm_pad(base + m)] = x[m];
   }
   __syncthreads();
-  for (int h = 1; h < F; h <<= 1) {
-    for (int idx = tid; idx < TR * (F / 2); idx += FM_THREADS) {
-      const int r = idx / (F / 2), b = idx - r * (F / 2);
-      const int grp = b / h, pos = b - grp * h;
-      const int i0 = grp * 2 * h + pos, i1 = i0 + h;
-      const float2 w = tw[pos * (F / (2 * h))];
-      float2* rowp = s + r * SF;
-      const float2 t = cmul(w, rowp[i1]);
-      const float2 a = rowp[i0];
-      rowp[i0] = cadd(a, t);
-      rowp[i1] = csub(a, t);
+  for (int lh = S0; lh < logF;) {
+    const int left = logF - lh;
+    if (left == 3 || left > 4) {
+      fm_pass<3>(s, SF, tw, TR, logF, lh);
+      lh += 3;
+    } else if (left >= 2) {
+      fm_pass<2>(s, SF, tw, TR, logF, lh);
+      lh += 2;
+    } else {
+      fm_pass<1>(s, SF, tw, TR, logF, lh);
+      lh += 1;
     }
     __syncthreads();
   }
@@ -827,7 +875,7 @@ __global__ void __launch_bounds__(FM_THREADS) fft_rows_centred_kernel(
     const int X = idx / TR, r = idx - X * TR;
     const int row = r0 + r;
     if (row >= nrows) continue;
-    float2 v = s[r * SF + X];
+    float2 v = s[r * SF + fm_pad(X)];
     const float sg = ((X & 1) ? -sgnF : sgnF) * scale;
     v = make_float2(v.x * sg, v.y * sg);
     const size_t o = (size_t)X * ldo + row;
@@ -961,33 +1009,30 @@ int run_fi(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tm,
   return LITHO_OK;
 }
 
-static int fm_rows_per_cta(int F) { return std::max(1, 16384 / F) > 16 ? 16 : std::max(1, 16384 / F); }
+// rows per CTA: four (two of 8192, by their shared memory), or enough for every thread
+static int fm_rows_per_cta(int F) { return F >= 8192 ? 16384 / F : std::max(4, std::min(32, 2048 / F)); }
+
+static int run_fft_rows(litho_ctx* ctx, const float* in_r, const float2* in_c, int nrows, int len, int F, float scale,
+                        float2* out_c, float* out_r, float* out_i, int ldo) {
+  const int TR = fm_rows_per_cta(F), logF = 31 - __builtin_clz((unsigned)F);
+  const size_t smem = ((size_t)TR * fm_stride(F) + F / 2) * sizeof(float2);
+  auto k = logF >= 3 ? fft_rows_centred_kernel<3> : logF == 2 ? fft_rows_centred_kernel<2> : fft_rows_centred_kernel<1>;
+  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k<<<(nrows + TR - 1) / TR, FM_THREADS, smem, ctx->stream>>>(in_r, nullptr, in_c, nrows, len, logF, TR, scale, out_c,
+                                                             out_r, out_i, ldo);
+  LITHO_CUDA_TRY(ctx, cudaGetLastError());
+  return LITHO_OK;
+}
 
 int run_fft_mask(litho_ctx* ctx, const float* mask, int Lx, int Ly, float* mskf_r, float* mskf_i) {
   const int Fx = next_pow2(Lx), Fy = next_pow2(Ly);
-  // pass 1: mask rows -> tmp[X][y] (Fx x Ly complex)
   LITHO_RET(ctx->stage_x.ensure(ctx, (size_t)Fx * Ly * sizeof(float2)));
   float2* tmp = ctx->stage_x.as<float2>();
   StageScope sc(ctx, LITHO_STAGE_FFT_MASK, 2);
-  {
-    const int TR = fm_rows_per_cta(Fx);
-    const size_t smem = ((size_t)TR * (Fx + 1) + Fx / 2) * sizeof(float2);
-    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(fft_rows_centred_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    fft_rows_centred_kernel<<<(Ly + TR - 1) / TR, FM_THREADS, smem, ctx->stream>>>(
-        mask, nullptr, nullptr, Ly, Lx, Fx, TR, 1.0f, tmp, nullptr, nullptr, Ly);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
-  }
-  // pass 2: tmp rows (one per X, length Ly) -> mskf[Y][X] / (Fx*Fy)
-  {
-    const int TR = fm_rows_per_cta(Fy);
-    const size_t smem = ((size_t)TR * (Fy + 1) + Fy / 2) * sizeof(float2);
-    const float scale = 1.0f / ((float)Fx * (float)Fy);
-    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(fft_rows_centred_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    fft_rows_centred_kernel<<<(Fx + TR - 1) / TR, FM_THREADS, smem, ctx->stream>>>(
-        nullptr, nullptr, tmp, Fx, Ly, Fy, TR, scale, nullptr, mskf_r, mskf_i, Fx);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
-  }
-  return LITHO_OK;
+  // mask rows -> tmp[X][y] (Fx x Ly complex)
+  LITHO_RET(run_fft_rows(ctx, mask, nullptr, Ly, Lx, Fx, 1.0f, tmp, nullptr, nullptr, Ly));
+  // tmp rows (one per X, length Ly) -> mskf[Y][X] / (Fx*Fy)
+  return run_fft_rows(ctx, nullptr, tmp, Fx, Ly, Fy, 1.0f / ((float)Fx * (float)Fy), nullptr, mskf_r, mskf_i, Fx);
 }
 
 // ---------------------------------------------------------------------------
