@@ -125,7 +125,7 @@ int litho_ctx_destroy(litho_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   DevBuf* bufs[] = {&ctx->win_part, &ctx->band_part, &ctx->tm,     &ctx->stage_in, &ctx->stage_out,
                     &ctx->stage_k,  &ctx->stage_s,   &ctx->stage_x, &ctx->tcc_a,   &ctx->tcc_b,
-                    &ctx->tcc_c,    &ctx->tcc_pq,  &ctx->tcc_part, &ctx->eig_w,     &ctx->eig_v,   &ctx->eig_work, &ctx->eig_info,
+                    &ctx->tcc_c,    &ctx->tcc_pq,  &ctx->tcc_part, &ctx->socs_tmp, &ctx->eig_w,     &ctx->eig_v,   &ctx->eig_work, &ctx->eig_info,
                     &ctx->mx_b,     &ctx->mx_c,      &ctx->mx_d,    &ctx->band_w};
   for (DevBuf* b : bufs) b->release();
   for (auto& kv : ctx->twx_tables) kv.second.release();
@@ -388,8 +388,11 @@ int litho_calc_socs(litho_ctx* ctx, const float* mskf_r, const float* mskf_i, in
   ImgGeom g{physLx, physLy, fftLx, fftLy, Nx, Ny, nk, convN};
   ImgPlan p = make_plan(g, 1, ctx->sm_count);
   if (tmpImgp) {
-    p.kpg = nk;
-    p.ngroups = 1;
+    // each group of kernels writes its own intensity: at most this many of them (a single group, one
+    // CTA of the 128 x 128 form with 10 kernels, took 56 us; ten take 18 and 2 to add them)
+    constexpr int TMP_GROUPS = 32;
+    p.kpg = std::max(p.kpg, (nk + TMP_GROUPS - 1) / TMP_GROUPS);
+    p.ngroups = (nk + p.kpg - 1) / p.kpg;
   }
   const int kdim = (2 * Nx + 1) * (2 * Ny + 1);
   const size_t spec = (size_t)fftLx * fftLy * sizeof(float);
@@ -414,7 +417,13 @@ int litho_calc_socs(litho_ctx* ctx, const float* mskf_r, const float* mskf_i, in
   WindowSrc w;
   w.mskf_r = static_cast<const float*>(dr);
   w.mskf_i = static_cast<const float*>(di);
-  LITHO_RET(run_socs(ctx, p, w, ctx->stage_k.as<float2>(), ctx->stage_s.as<float>(), ctx->band_part.as<float2>(), dtmp));
+  float* parts = dtmp;
+  if (tmpImgp && p.ngroups > 1) {
+    LITHO_RET(ctx->socs_tmp.ensure(ctx, p.ngroups * tmp_bytes));
+    parts = ctx->socs_tmp.as<float>();
+  }
+  LITHO_RET(run_socs(ctx, p, w, ctx->stage_k.as<float2>(), ctx->stage_s.as<float>(), ctx->band_part.as<float2>(), parts));
+  if (parts != dtmp) LITHO_RET(run_tmp_join(ctx, parts, p.ngroups, convN * convN, dtmp));
   LITHO_RET(run_fi(ctx, p, ctx->band_part.as<float2>(), ctx->tm.as<float>(), dimg));
   if (mem == LITHO_MEM_HOST) {
     LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(image, dimg, img_bytes, cudaMemcpyDeviceToHost, ctx->stream));

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(SOCS_THREADS) socs_kernel(
 
   if (tmpImgp != nullptr) {
     // litho.cpp:934 myShift(tmpImg -> tmpImgp, fftshift); positions are bit-reversed
-    float* T = tmpImgp + (size_t)img * N * N;
+    float* T = tmpImgp + ((size_t)img * gridDim.x + g) * N * N;
 #pragma unroll
     for (int m = 0; m < CPW; ++m) {
       const int xs = bitrev<N>(warp + 8 * m);
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(SOCS_THREADS) socs64_kernel(
 
   if (tmpImgp != nullptr) {
     // litho.cpp:934 myShift(tmpImg -> tmpImgp, fftshift)
-    float* T = tmpImgp + (size_t)img * N * N;
+    float* T = tmpImgp + ((size_t)img * gridDim.x + g) * N * N;
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
       const int c = warp + 8 * (q + 4 * m);
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(S128_THREADS) socs128_kernel(
 
   if (tmpImgp != nullptr) {
     // litho.cpp:934 myShift(tmpImg -> tmpImgp, fftshift)
-    float* T = tmpImgp + (size_t)img * N * N;
+    float* T = tmpImgp + ((size_t)img * gridDim.x + g) * N * N;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
       const int c = 32 * m + sl;
@@ -978,12 +978,19 @@ static int launch_socs_t(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, c
   return LITHO_OK;
 }
 
+// tmpImgp of one image: the groups' intensities added in order
+__global__ void tmp_join_kernel(const float* __restrict__ part, int ngroups, int n, float* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float v = part[i];
+#pragma unroll 8
+  for (int g = 1; g < ngroups; ++g) v += part[(size_t)g * n + i];
+  out[i] = v;
+}
+
+// tmpImgp: [image][group][convN][convN]
 int run_socs(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const float2* krn, const float* scales,
              float2* band_part, float* tmpImgp) {
-  if (tmpImgp != nullptr && p.ngroups != 1) {
-    set_error(ctx, LITHO_ERR_ARG, "tmpImgp output needs a single kernel group");
-    return LITHO_ERR_ARG;
-  }
   switch (p.g.convN) {
     case 32: return launch_socs_t<32>(ctx, p, w, krn, scales, band_part, tmpImgp);
     case 64: return launch_socs_t<64>(ctx, p, w, krn, scales, band_part, tmpImgp);
@@ -992,6 +999,13 @@ int run_socs(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const float2*
       set_error(ctx, LITHO_ERR_UNSUPPORTED, "conv grid %d not in {32, 64, 128}", p.g.convN);
       return LITHO_ERR_UNSUPPORTED;
   }
+}
+
+int run_tmp_join(litho_ctx* ctx, const float* part, int ngroups, int n, float* tmpImgp) {
+  StageScope sc(ctx, LITHO_STAGE_SOCS);
+  tmp_join_kernel<<<(n + 127) / 128, 128, 0, ctx->stream>>>(part, ngroups, n, tmpImgp);
+  LITHO_CUDA_TRY(ctx, cudaGetLastError());
+  return LITHO_OK;
 }
 
 int run_fi(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tm, float* images) {

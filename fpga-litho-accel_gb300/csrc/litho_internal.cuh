@@ -137,7 +137,7 @@ struct litho_ctx {
   // twiddle and coefficient tables keyed by (L, F, N, kind)
   std::map<std::tuple<int, int, int, int>, litho::DevBuf> twx_tables;
   // TCC / eigensolver workspaces
-  litho::DevBuf tcc_a, tcc_b, tcc_c, tcc_pq, tcc_part, eig_w, eig_v, eig_work, eig_info;
+  litho::DevBuf socs_tmp, tcc_a, tcc_b, tcc_c, tcc_pq, tcc_part, eig_w, eig_v, eig_work, eig_info;
   // mixed-precision (tensor-core) workspaces
   litho::DevBuf mx_b, mx_c, mx_d;
   // host-buffer batches: copy streams and per-slot events of the staging pipeline
@@ -248,6 +248,7 @@ cudaError_t launch_fi_fold(cudaStream_t s, const ImgPlan& p, const float* tm, co
 int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int precision);
 int run_socs(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const float2* krn,
              const float* scales, float2* band_part, float* tmpImgp);
+int run_tmp_join(litho_ctx* ctx, const float* part, int ngroups, int n, float* tmpImgp);
 int run_fi(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tm, float* images);
 // FI step 1 for both layouts (tmh == nullptr: plain tm; else K-major hi/lo + t0)
 cudaError_t launch_fi_rows(cudaStream_t s, const ImgPlan& p, const float2* band_part, const float2* twF, int KP,
