@@ -395,13 +395,51 @@ int litho_calc_socs(litho_ctx* ctx, const float* mskf_r, const float* mskf_i, in
     p.ngroups = (nk + p.kpg - 1) / p.kpg;
   }
   const int kdim = (2 * Nx + 1) * (2 * Ny + 1);
-  const size_t spec = (size_t)fftLx * fftLy * sizeof(float);
-  const void *dr = nullptr, *di = nullptr;
-  LITHO_RET(stage_in(ctx, ctx->stage_in, mskf_r, spec, mem, &dr));
-  LITHO_RET(stage_in(ctx, ctx->stage_x, mskf_i, spec, mem, &di));
-  LITHO_RET(ctx->stage_k.ensure(ctx, (size_t)nk * kdim * sizeof(float2)));
-  LITHO_RET(ctx->stage_s.ensure(ctx, (size_t)nk * sizeof(float)));
-  LITHO_RET(upload_kernels(ctx, krn_r, krn_i, scales, nk, kdim, mem, ctx->stage_k.as<float2>(), ctx->stage_s.as<float>()));
+  WindowSrc w;
+  w.mskf_r = mskf_r;
+  w.mskf_i = mskf_i;
+  std::vector<float> host;  // kernels (interleaved), spectrum window re, im, scales; outlives its copy
+  struct Drain {
+    litho_ctx* ctx;
+    ~Drain() {
+      if (ctx) cudaStreamSynchronize(ctx->stream);
+    }
+  } drain{nullptr};
+  float2* krn = nullptr;
+  float* scl = nullptr;
+  if (mem == LITHO_MEM_HOST) {
+    // of the spectrum, only the kernels' window is read: it goes up with the kernels in one copy (the
+    // two whole planes were two thirds of what the call moves to the device)
+    const size_t n = (size_t)nk * kdim, total = 2 * n + 2 * (size_t)kdim + nk;
+    host.resize(total);
+    for (size_t i = 0; i < n; ++i) {
+      host[2 * i] = krn_r[i];
+      host[2 * i + 1] = krn_i[i];
+    }
+    float* wr = host.data() + 2 * n;
+    for (int v = 0; v < 2 * Ny + 1; ++v) {
+      const size_t o = (size_t)(fftLy / 2 - Ny + v) * fftLx + (fftLx / 2 - Nx);
+      std::copy(mskf_r + o, mskf_r + o + 2 * Nx + 1, wr + (size_t)v * (2 * Nx + 1));
+      std::copy(mskf_i + o, mskf_i + o + 2 * Nx + 1, wr + kdim + (size_t)v * (2 * Nx + 1));
+    }
+    std::copy(scales, scales + nk, wr + 2 * (size_t)kdim);
+    LITHO_RET(ctx->stage_k.ensure(ctx, total * sizeof(float)));
+    drain.ctx = ctx;
+    LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->stage_k.p, host.data(), total * sizeof(float), cudaMemcpyHostToDevice,
+                                        ctx->stream));
+    krn = ctx->stage_k.as<float2>();
+    w.mskf_r = ctx->stage_k.as<float>() + 2 * n;
+    w.mskf_i = w.mskf_r + kdim;
+    w.Fx = 2 * Nx + 1;
+    w.Fy = 2 * Ny + 1;
+    scl = ctx->stage_k.as<float>() + 2 * n + 2 * (size_t)kdim;
+  } else {
+    LITHO_RET(ctx->stage_k.ensure(ctx, (size_t)nk * kdim * sizeof(float2)));
+    LITHO_RET(ctx->stage_s.ensure(ctx, (size_t)nk * sizeof(float)));
+    krn = ctx->stage_k.as<float2>();
+    scl = ctx->stage_s.as<float>();
+    LITHO_RET(upload_kernels(ctx, krn_r, krn_i, scales, nk, kdim, mem, krn, scl));
+  }
   const size_t img_bytes = (size_t)physLx * physLy * sizeof(float);
   const size_t tmp_bytes = (size_t)convN * convN * sizeof(float);
   float* dimg = image;
@@ -414,15 +452,12 @@ int litho_calc_socs(litho_ctx* ctx, const float* mskf_r, const float* mskf_i, in
   const int KY = 2 * Ny + 1;
   LITHO_RET(ctx->band_part.ensure(ctx, (size_t)p.ngroups * KY * (4 * Nx + 1) * sizeof(float2)));
   LITHO_RET(ctx->tm.ensure(ctx, (size_t)(4 * Ny + 1) * physLx * sizeof(float)));
-  WindowSrc w;
-  w.mskf_r = static_cast<const float*>(dr);
-  w.mskf_i = static_cast<const float*>(di);
   float* parts = dtmp;
   if (tmpImgp && p.ngroups > 1) {
     LITHO_RET(ctx->socs_tmp.ensure(ctx, p.ngroups * tmp_bytes));
     parts = ctx->socs_tmp.as<float>();
   }
-  LITHO_RET(run_socs(ctx, p, w, ctx->stage_k.as<float2>(), ctx->stage_s.as<float>(), ctx->band_part.as<float2>(), parts));
+  LITHO_RET(run_socs(ctx, p, w, krn, scl, ctx->band_part.as<float2>(), parts));
   if (parts != dtmp) LITHO_RET(run_tmp_join(ctx, parts, p.ngroups, convN * convN, dtmp));
   LITHO_RET(run_fi(ctx, p, ctx->band_part.as<float2>(), ctx->tm.as<float>(), dimg));
   if (mem == LITHO_MEM_HOST) {

@@ -971,9 +971,9 @@ static int launch_socs_t(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, c
   LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(p.ngroups, p.batch);
   StageScope sc(ctx, LITHO_STAGE_SOCS);
-  k<<<grid, N == 128 ? S128_THREADS : SOCS_THREADS, smem, ctx->stream>>>(w.part, w.nparts, w.mskf_r, w.mskf_i, g.Fx,
-                                                                       g.Fy, g.Nx, g.Ny, krn,
-                                                scales, g.nk, p.kpg, band_part, tmpImgp);
+  k<<<grid, N == 128 ? S128_THREADS : SOCS_THREADS, smem, ctx->stream>>>(
+      w.part, w.nparts, w.mskf_r, w.mskf_i, w.Fx ? w.Fx : g.Fx, w.Fy ? w.Fy : g.Fy, g.Nx, g.Ny, krn, scales, g.nk, p.kpg,
+      band_part, tmpImgp);
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
 }

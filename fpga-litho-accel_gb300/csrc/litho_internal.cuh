@@ -222,6 +222,7 @@ struct WindowSrc {
   int nparts = 0;
   const float* mskf_r = nullptr;  // or full spectrum planes [batch][Fy][Fx]
   const float* mskf_i = nullptr;
+  int Fx = 0, Fy = 0;             // the planes' size: 0 the image's, or the window's own
 };
 
 // the folded FP32 transforms (imaging_fold.cu): plan fields of a plain window DFT, coefficient
