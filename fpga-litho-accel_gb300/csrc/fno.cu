@@ -903,41 +903,53 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS) row_fwd_kernel(const RowFwd
 size_t row_fwd_smem(int L, bool final_) { return FwdSmem(L, final_).total; }
 
 // ---------------------------------------------------------------------------
-// loss: per mask e = ||out - y||, n = ||y||; loss_b = e / n, coef_b = 1 / (B e n)
+// loss: per mask e = ||out - y||, n = ||y||; loss_b = e / n, coef_b = 1 / (B e n).  The squares are
+// summed in FP64, which bounds it (a quarter of an SM takes one such instruction per ~66 cycles), so a
+// mask is shared by as many CTAs as there are SMs for it, and a second kernel adds their sums in
+// order.  32 masks of 256 x 256: 99 us on a CTA each -> 29 + 4.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) loss_kernel(int L, int B, const float* __restrict__ out,
-                                                    const float* __restrict__ tgt, float* __restrict__ loss_b,
-                                                    float* __restrict__ coef) {
-  const int b = blockIdx.x;
-  const size_t n = (size_t)L * L;
+constexpr int LOSS_SHARES = 16;
+__global__ void __launch_bounds__(THREADS) loss_part_kernel(int L, const float* __restrict__ out,
+                                                            const float* __restrict__ tgt, double2* __restrict__ part) {
+  const size_t b = blockIdx.x / LOSS_SHARES, n = (size_t)L * L;
+  const int sh = blockIdx.x % LOSS_SHARES;
   const float* o = out + b * n;
   const float* y = tgt + b * n;
   double se = 0.0, sy = 0.0;
-  for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const double d = (double)o[i] - (double)y[i];
-    se += d * d;
-    sy += (double)y[i] * (double)y[i];
+#pragma unroll 4
+  for (size_t i = sh * THREADS + threadIdx.x; i < n; i += LOSS_SHARES * THREADS) {
+    const double t = (double)__ldg(y + i), d = (double)__ldg(o + i) - t;
+    se = fma(d, d, se);
+    sy = fma(t, t, sy);
   }
-  __shared__ double r0[32], r1[32];
+  __shared__ double2 r[THREADS / 32];
   for (int k = 16; k > 0; k >>= 1) {
     se += __shfl_xor_sync(0xffffffffu, se, k);
     sy += __shfl_xor_sync(0xffffffffu, sy, k);
   }
-  if ((threadIdx.x & 31) == 0) {
-    r0[threadIdx.x >> 5] = se;
-    r1[threadIdx.x >> 5] = sy;
-  }
+  if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = make_double2(se, sy);
   __syncthreads();
   if (threadIdx.x == 0) {
-    double a = 0.0, c = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      a += r0[w];
-      c += r1[w];
+    for (int w = 1; w < THREADS / 32; ++w) {
+      se += r[w].x;
+      sy += r[w].y;
     }
-    const double e = sqrt(a), nn = sqrt(c);
-    loss_b[b] = nn > 0.0 ? (float)(e / nn) : 0.f;
-    coef[b] = (e > 0.0 && nn > 0.0) ? (float)(1.0 / ((double)B * e * nn)) : 0.f;
+    part[blockIdx.x] = make_double2(se, sy);
   }
+}
+__global__ void loss_kernel(int B, const double2* __restrict__ part, float* __restrict__ loss_b, float* __restrict__ coef) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= B) return;
+  double a = 0.0, c = 0.0;
+#pragma unroll
+  for (int s = 0; s < LOSS_SHARES; ++s) {
+    const double2 v = part[(size_t)b * LOSS_SHARES + s];
+    a += v.x;
+    c += v.y;
+  }
+  const double e = sqrt(a), nn = sqrt(c);
+  loss_b[b] = nn > 0.0 ? (float)(e / nn) : 0.f;
+  coef[b] = (e > 0.0 && nn > 0.0) ? (float)(1.0 / ((double)B * e * nn)) : 0.f;
 }
 
 // ---------------------------------------------------------------------------
@@ -1687,7 +1699,7 @@ struct litho_fno {
   DevBuf Xf, Gy;     // per-row spectral intermediates (also Xg, Gg in backward)
   DevBuf Vs[NL], gU;
   DevBuf gv[2];      // gvpw ping-pong
-  DevBuf out, lossb, coef, gpart;
+  DevBuf out, lossb, lossp, coef, gpart;
   int bwd_grid = 0;
   // error estimate = alpha * ||out-of-band residual|| / ||band part||
   float est_alpha = 1.0f;
@@ -1734,6 +1746,7 @@ int ensure_batch(litho_fno* f, int B, bool train) {
   LITHO_RET(f->lossb.ensure(ctx, (size_t)B * sizeof(float)));
   LITHO_RET(f->coef.ensure(ctx, (size_t)B * sizeof(float)));
   if (train) {
+    LITHO_RET(f->lossp.ensure(ctx, (size_t)B * LOSS_SHARES * sizeof(double2)));
     for (int l = 0; l < NL; ++l) LITHO_RET(f->Vs[l].ensure(ctx, (size_t)B * J * M * C * sizeof(float2)));
     LITHO_RET(f->gU.ensure(ctx, (size_t)B * J * M * C * sizeof(float2)));
     LITHO_RET(f->gv[0].ensure(ctx, act));
@@ -1800,6 +1813,13 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
   return LITHO_OK;
 }
 
+cudaError_t launch_loss(litho_fno* f, const float* targets, int B) {
+  cudaStream_t s = f->ctx->stream;
+  loss_part_kernel<<<(unsigned)B * LOSS_SHARES, THREADS, 0, s>>>(f->L, f->out.as<float>(), targets, f->lossp.as<double2>());
+  loss_kernel<<<(B + 31) / 32, 32, 0, s>>>(B, f->lossp.as<double2>(), f->lossb.as<float>(), f->coef.as<float>());
+  return cudaGetLastError();
+}
+
 // loss (device, per mask) + gradient into f->grad
 int backward(litho_fno* f, const float* masks, const float* targets, int B) {
   litho_ctx* ctx = f->ctx;
@@ -1809,9 +1829,8 @@ int backward(litho_fno* f, const float* masks, const float* targets, int B) {
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_PROJ>, sp.total));
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_SPEC>, ss.total));
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_LIFT>, sl.total));
-  StageScope sc(ctx, LITHO_STAGE_SURROGATE, 3 * NL + 3);
-  loss_kernel<<<B, 1024, 0, ctx->stream>>>(L, B, f->out.as<float>(), targets, f->lossb.as<float>(),
-                                           f->coef.as<float>());
+  StageScope sc(ctx, LITHO_STAGE_SURROGATE, 3 * NL + 4);
+  LITHO_CUDA_TRY(ctx, launch_loss(f, targets, B));
   LITHO_CUDA_TRY(ctx, cudaMemsetAsync(f->gpart.p, 0, (size_t)grid * Dn::N * sizeof(float), ctx->stream));
   float2* Xg = f->Xf.as<float2>();
   float2* Gg = f->Gy.as<float2>();
@@ -1957,7 +1976,7 @@ int litho_surrogate_create(litho_ctx* ctx, int L, unsigned long long seed, litho
 void litho_surrogate_destroy(litho_fno* f) {
   if (!f) return;
   DevBuf* bufs[] = {&f->theta, &f->grad, &f->adam_m, &f->adam_v, &f->Ttab, &f->TT, &f->twL, &f->colF, &f->colI, &f->Xf, &f->Gy,
-                    &f->gU, &f->gv[0], &f->gv[1], &f->out, &f->lossb, &f->coef, &f->gpart, &f->Xb, &f->Eres,
+                    &f->gU, &f->gv[0], &f->gv[1], &f->out, &f->lossb, &f->lossp, &f->coef, &f->gpart, &f->Xb, &f->Eres,
                     &f->Enew, &f->Cb, &f->Mrow, &f->Cm, &f->est, &f->stage_m, &f->stage_i};
   for (DevBuf* b : bufs) b->release();
   for (int l = 0; l < NL; ++l) {
