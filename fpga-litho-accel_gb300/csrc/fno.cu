@@ -108,18 +108,9 @@ __device__ __forceinline__ float tanh_hw(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float gelu(float x) {
-  const float t = tanh_hw(GK0 * fmaf(GK1 * x, x * x, x));
-  return 0.5f * x * (1.0f + t);
-}
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float x2 = x * x;
-  const float t = tanh_hw(GK0 * fmaf(GK1 * x, x2, x));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GK0 * fmaf(3.0f * GK1, x2, 1.0f);
-}
-// The same on two values at once with the packed FP32 instructions (each half rounds as the scalar one
-// does): the row kernels run out of issue slots before they run out of arithmetic, and a GELU is seven
-// FP32 instructions and one of the special-function unit.
+// Two values at once with the packed FP32 instructions (each half rounds as a scalar does): the row
+// kernels run out of issue slots before they run out of arithmetic, and a GELU is seven FP32
+// instructions and one of the special-function unit.
 struct F2 {
   uint64_t v;
 };
@@ -171,29 +162,12 @@ __device__ __forceinline__ F2 unpack_f2(uint32_t u) {
   const float2 x = unpack2(u);
   return f2(x.x, x.y);
 }
-// GELU and its derivative together
-__device__ __forceinline__ void gelu_both(float x, float& g, float& d) {
-  const float x2 = x * x;
-  const float t = tanh_hw(GK0 * fmaf(GK1 * x, x2, x));
-  g = 0.5f * x * (1.0f + t);
-  d = 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GK0 * fmaf(3.0f * GK1, x2, 1.0f);
-}
-
 // A fragment (16 x 16, row major) of a C-layout accumulator pair (n tiles 2ks, 2ks+1)
 __device__ __forceinline__ void acc_to_a(const float* c0, const float* c1, uint32_t* a) {
   a[0] = pack2(c0[0], c0[1]);
   a[1] = pack2(c0[2], c0[3]);
   a[2] = pack2(c1[0], c1[1]);
   a[3] = pack2(c1[2], c1[3]);
-}
-
-// stage one row of Gy/Gg [M][C] complex as bf16 sG[c][2 kx + ri]
-__device__ __forceinline__ void stage_g_row(const float2* __restrict__ gr, bf16* sG, int tid) {
-  for (int i = tid; i < M * C; i += THREADS) {
-    const float2 v = gr[i];
-    const int kx = i / C, c = i % C;
-    *reinterpret_cast<uint32_t*>(sG + c * SP + 2 * kx) = pack2(v.x, v.y);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -961,7 +935,6 @@ __global__ void loss_kernel(int B, const double2* __restrict__ part, float* __re
 //                      gvpw_l = g_z W_l (bf16)
 // ---------------------------------------------------------------------------
 enum { HEAD_PROJ = 0, HEAD_SPEC = 1, HEAD_LIFT = 2 };
-constexpr int NRED = 2 * H + 2 * C + 1;  // per-warp slots of the vector gradient partials
 
 struct RowBwd {
   int L, rows, layer;
@@ -981,400 +954,549 @@ struct RowBwd {
   const bf16* TT;
 };
 
+// the two warps of a pair
+__device__ __forceinline__ void pair_bar(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); }
+// sums over the rows g of a warp's fragments (lanes xor 4, 8, 16)
+__device__ __forceinline__ float red_g(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 8);
+  v += __shfl_xor_sync(0xffffffffu, v, 16);
+  return v;
+}
+// the warp's 16 x 8 tile of dW[o][c] += sum_px gz[px][o] v[px][c] (rows 16 mt2, columns 8 nt)
+__device__ __forceinline__ void row_dw(uint32_t tgz, uint32_t tv, int T, int mt2, int nt, int lane, float* dW) {
+  // the transposed operand's matrices: (o 0-7, px 0-7), (o 8-15, px 0-7), (o 0-7, px 8-15), (o 8-15, px 8-15)
+  const int px = (lane & 7) + 8 * (lane >> 4), ch = 2 * mt2 + ((lane >> 3) & 1);
+#pragma unroll 2
+  for (int ks = 0; ks < T; ks += 2) {
+    uint32_t b[4], a0[4], a1[4];
+    ldsm4t(b, tv + tile_off(16 * ks + lane, nt));
+    ldsm4t(a0, tgz + tile_off(16 * ks + px, ch));
+    ldsm4t(a1, tgz + tile_off(16 * ks + 16 + px, ch));
+    mma16816(dW, a0, b[0], b[1]);
+    mma16816(dW, a1, b[2], b[3]);
+  }
+}
+__device__ __forceinline__ void put_dw(float* w, int mt2, int nt, int lane, const float* dW) {
+  const int o = 16 * mt2 + (lane >> 2), c = 8 * nt + 2 * (lane & 3);
+  w[o * C + c] = dW[0];
+  w[o * C + c + 1] = dW[1];
+  w[(o + 8) * C + c] = dW[2];
+  w[(o + 8) * C + c + 1] = dW[3];
+}
+// v_l = lift(mask) of pixels 16 mt + g, + 8 at fragment ks
+__device__ __forceinline__ void lift_frag(const float* pw, const float* pb, float m0, float m1, uint32_t* A) {
+  A[0] = pack2(fmaf(pw[0], m0, pb[0]), fmaf(pw[1], m0, pb[1]));
+  A[1] = pack2(fmaf(pw[0], m1, pb[0]), fmaf(pw[1], m1, pb[1]));
+  A[2] = pack2(fmaf(pw[2], m0, pb[2]), fmaf(pw[3], m0, pb[3]));
+  A[3] = pack2(fmaf(pw[2], m1, pb[2]), fmaf(pw[3], m1, pb[3]));
+}
+__device__ __forceinline__ void lift_coef(const float* th, int ks, int t, float* pw, float* pb) {
+  const int c0 = 16 * ks + 2 * t;
+  pw[0] = th[Off::Pw + c0];     pb[0] = th[Off::Pb + c0];
+  pw[1] = th[Off::Pw + c0 + 1]; pb[1] = th[Off::Pb + c0 + 1];
+  pw[2] = th[Off::Pw + c0 + 8]; pb[2] = th[Off::Pb + c0 + 8];
+  pw[3] = th[Off::Pw + c0 + 9]; pb[3] = th[Off::Pb + c0 + 9];
+}
+
 struct BwdSmem {
-  size_t sWT, sG, sGZT, sVT, sQ1, sQ1T, sGHT, sV4T, sT, sTT, sRed, total;
-  __host__ __device__ static size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
+  size_t sGv, sV, sZ, sWT, sG, sTT, sRed, total;
+  __host__ __device__ static constexpr size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
   __host__ __device__ BwdSmem(int L, int head) {
-    const size_t LP = (size_t)L + 8;
+    const size_t LP = (size_t)L + 8, tile = (size_t)L * C * 2;
     size_t o = 0;
-    sWT = o; o += up16(C * SP * 2);
-    sG = o; o += up16(C * SP * 2);
-    sGZT = o; o += up16(C * LP * 2);
-    sVT = o; o += up16(C * LP * 2);
-    sQ1 = sQ1T = sGHT = sV4T = 0;
-    if (head == HEAD_PROJ) {
-      sQ1 = o; o += up16(H * SP * 2);
-      sQ1T = o; o += up16(C * (H + 8) * 2);
-      sGHT = o; o += up16(H * LP * 2);
-      sV4T = o; o += up16(C * LP * 2);
+    sGv = o; o += 2 * tile;  // gvin, by parity; g_z takes its place
+    sV = sZ = sTT = sWT = 0;
+    if (head == HEAD_SPEC) {
+      sV = o; o += 2 * tile;  // z_{l-1}, by parity; v_l takes its place
+      sZ = o; o += tile;      // z_l; gvpw_l takes its place
+      sTT = o; o += up16(J * LP * 2);
+      sWT = o; o += up16(C * SP * 2);
     }
-    sT = sTT = 0;
-    if (head != HEAD_PROJ) { sT = o; o += up16((size_t)L * SP * 2); }
-    if (head != HEAD_LIFT) { sTT = o; o += up16(J * LP * 2); }
-    sRed = o; o += up16((size_t)(THREADS / 32) * NRED * sizeof(float));
+    sG = o; o += 2 * up16(C * SP * 2);
+    sRed = o; o += up16((size_t)(THREADS / 32) * 2 * C * sizeof(float));
     total = o;
   }
 };
 
+// HEAD_SPEC and HEAD_LIFT.  SPEC moves 72 KB a row and is to be bound by that: rows arrive by
+// asynchronous copies (z_l, needed for one half of the work, while the other half runs; the rest a row
+// ahead) in the tiles of the forward kernel, results take their operands' places, and the two
+// contractions over the row (dW, Xg) read them transposed.  It took scalar loads of half-used sectors
+// with nothing in flight but the current tile's, and two-byte transposing stores.
+// 32 masks of 256 x 256: 220 -> 143 us a layer; LIFT 78 -> 40.
 template <int HEAD>
-__global__ void __launch_bounds__(THREADS, 1) row_bwd_kernel(const RowBwd a) {
+__global__ void __launch_bounds__(THREADS, 2) row_bwd_kernel(const RowBwd a) {
+  constexpr bool SPEC = HEAD == HEAD_SPEC;
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int L = a.L, LP = L + 8, l = a.layer;
+  const int L = a.L, LP = L + 8, l = a.layer, T = L / 16;
   const BwdSmem S(L, HEAD);
-  bf16* sWT = reinterpret_cast<bf16*>(smraw + S.sWT);    // [C c][SP]: W_l[o][c] at [c][o]
-  bf16* sG = reinterpret_cast<bf16*>(smraw + S.sG);      // [C c][SP]
-  bf16* sGZT = reinterpret_cast<bf16*>(smraw + S.sGZT);  // [C o][LP]
-  bf16* sVT = reinterpret_cast<bf16*>(smraw + S.sVT);    // [C c][LP]
-  bf16* sQ1 = reinterpret_cast<bf16*>(smraw + S.sQ1);    // [H][SP]
-  bf16* sQ1T = reinterpret_cast<bf16*>(smraw + S.sQ1T);  // [C][H + 8]
-  bf16* sGHT = reinterpret_cast<bf16*>(smraw + S.sGHT);  // [H][LP]
-  bf16* sV4T = reinterpret_cast<bf16*>(smraw + S.sV4T);  // [C][LP]
+  const size_t tile = (size_t)L * C * 2;
+  bf16* sWT = reinterpret_cast<bf16*>(smraw + S.sWT);  // [C c][SP]: W_l[o][c] at [c][o]
+  bf16* sG0 = reinterpret_cast<bf16*>(smraw + S.sG);   // [2][C c][SP]
+  bf16* sTT = reinterpret_cast<bf16*>(smraw + S.sTT);  // [J][LP]: forward table
   float* sRed = reinterpret_cast<float*>(smraw + S.sRed);
-  bf16* sT = reinterpret_cast<bf16*>(smraw + S.sT);      // [L px][SP]: inverse table
-  bf16* sTT = reinterpret_cast<bf16*>(smraw + S.sTT);    // [J][LP]: forward table
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const float* th = a.theta;
-  constexpr int HP = H + 8;
-  if (HEAD != HEAD_PROJ)
-    for (int i = tid; i < L * J / 2; i += THREADS) {
-      const int px = i / (J / 2), k = 2 * (i % (J / 2));
-      *reinterpret_cast<uint32_t*>(sT + px * SP + k) = *reinterpret_cast<const uint32_t*>(a.Ttab + (size_t)px * J + k);
-    }
-  if (HEAD != HEAD_LIFT)
+  if (SPEC) {
     for (int i = tid; i < J * L / 2; i += THREADS) {
       const int k = i / (L / 2), px = 2 * (i % (L / 2));
       *reinterpret_cast<uint32_t*>(sTT + k * LP + px) = *reinterpret_cast<const uint32_t*>(a.TT + (size_t)k * L + px);
     }
-
-  if (HEAD != HEAD_LIFT)
     for (int i = tid; i < C * C; i += THREADS) {
       const int o = i / C, c = i % C;
       sWT[c * SP + o] = __float2bfloat16(th[Off::W + l * C * C + i]);
     }
-  if (HEAD == HEAD_PROJ)
-    for (int i = tid; i < H * C; i += THREADS) {
-      const int h = i / C, c = i % C;
-      const bf16 v = __float2bfloat16(th[Off::Q1 + i]);
-      sQ1[h * SP + c] = v;
-      sQ1T[c * HP + h] = v;
-    }
-  for (int i = tid; i < (THREADS / 32) * NRED; i += THREADS) sRed[i] = 0.f;
-  float pw[2][4], pb[2][4];
-#pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
-    const int c0 = 16 * ks + 2 * t;
-    pw[ks][0] = th[Off::Pw + c0];     pb[ks][0] = th[Off::Pb + c0];
-    pw[ks][1] = th[Off::Pw + c0 + 1]; pb[ks][1] = th[Off::Pb + c0 + 1];
-    pw[ks][2] = th[Off::Pw + c0 + 8]; pb[ks][2] = th[Off::Pb + c0 + 8];
-    pw[ks][3] = th[Off::Pw + c0 + 9]; pb[ks][3] = th[Off::Pb + c0 + 9];
   }
-  // per-thread partial sums over rows g, g+8 (columns 8n + 2t, +1)
-  float vb[4][2] = {};       // dWb (tail) or dPb (LIFT)
-  float vw[4][2] = {};       // dPw (LIFT)
-  float dq1b[16][2] = {}, dq2[16][2] = {};
-  float dq2b = 0.f;
-  float dW[4] = {0.f, 0.f, 0.f, 0.f};  // warp's 16 x 8 tile of dW_l
-  float dQ1[4][4] = {};                // warp's four 16 x 8 tiles of dQ1
-
-  for (int row = blockIdx.x; row < a.rows; row += gridDim.x) {
-    const int b = row / L;
-    __syncthreads();
-    if (HEAD != HEAD_PROJ) stage_g_row(a.Gg + (size_t)row * M * C, sG, tid);
-    __syncthreads();
-    for (int mt = warp; mt < L / 16; mt += THREADS / 32) {
-      const int px0 = 16 * mt;
-      const size_t p0 = (size_t)row * L + px0 + g, p1 = p0 + 8;
-      float gz[4][4];
-      if (HEAD == HEAD_PROJ) {
-        // v4 = z_3 as an A fragment, and transposed into sV4T for dQ1
-        uint32_t A[2][4];
-        const bf16* z0 = a.zl + p0 * C;
-        const bf16* z1 = a.zl + p1 * C;
+  uint32_t AT[MAXT][2][4];  // A fragments of the inverse table at the warp's pixels
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-          const int c0 = 16 * ks + 2 * t;
-          A[ks][0] = ldg32(z0 + c0);
-          A[ks][1] = ldg32(z1 + c0);
-          A[ks][2] = ldg32(z0 + c0 + 8);
-          A[ks][3] = ldg32(z1 + c0 + 8);
-          const bf16* e0 = reinterpret_cast<const bf16*>(&A[ks][0]);
-          const bf16* e1 = reinterpret_cast<const bf16*>(&A[ks][1]);
-          const bf16* e2 = reinterpret_cast<const bf16*>(&A[ks][2]);
-          const bf16* e3 = reinterpret_cast<const bf16*>(&A[ks][3]);
-          sV4T[c0 * LP + px0 + g] = e0[0];       sV4T[(c0 + 1) * LP + px0 + g] = e0[1];
-          sV4T[c0 * LP + px0 + g + 8] = e1[0];   sV4T[(c0 + 1) * LP + px0 + g + 8] = e1[1];
-          sV4T[(c0 + 8) * LP + px0 + g] = e2[0]; sV4T[(c0 + 9) * LP + px0 + g] = e2[1];
-          sV4T[(c0 + 8) * LP + px0 + g + 8] = e3[0];
-          sV4T[(c0 + 9) * LP + px0 + g + 8] = e3[1];
-        }
-        const float go0 = (a.out[p0] - a.tgt[p0]) * a.coef[b];
-        const float go1 = (a.out[p1] - a.tgt[p1]) * a.coef[b];
-        if (t == 0) dq2b += go0 + go1;
+  for (int i = 0; i < MAXT; ++i)
+    if (warp + 8 * i < T)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) gz[n][0] = gz[n][1] = gz[n][2] = gz[n][3] = 0.f;
-#pragma unroll
-        for (int kh = 0; kh < H / 16; ++kh) {  // hidden channels 16 kh .. 16 kh + 15
-          float hc[2][4];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int nh = 2 * kh + u, h0 = 8 * nh + 2 * t;
-            const float b0 = th[Off::q1b + h0], b1 = th[Off::q1b + h0 + 1];
-            hc[u][0] = b0; hc[u][1] = b1; hc[u][2] = b0; hc[u][3] = b1;
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-              const bf16* bq = sQ1 + (8 * nh + g) * SP + 16 * ks + 2 * t;
-              mma16816(hc[u], A[ks], lds32(bq), lds32(bq + 8));
-            }
-            const float q0 = th[Off::Q2 + h0], q1 = th[Off::Q2 + h0 + 1];
-            // gh = go * Q2; ghp = gh * GELU'(hpre)
-            float ga[4], gd[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) gelu_both(hc[u][e], ga[e], gd[e]);
-            const float g00 = go0 * q0 * gd[0], g01 = go0 * q1 * gd[1];
-            const float g10 = go1 * q0 * gd[2], g11 = go1 * q1 * gd[3];
-            dq2[nh][0] += go0 * ga[0] + go1 * ga[2];
-            dq2[nh][1] += go0 * ga[1] + go1 * ga[3];
-            dq1b[nh][0] += g00 + g10;
-            dq1b[nh][1] += g01 + g11;
-            hc[u][0] = g00; hc[u][1] = g01; hc[u][2] = g10; hc[u][3] = g11;
-            sGHT[h0 * LP + px0 + g] = __float2bfloat16(g00);
-            sGHT[(h0 + 1) * LP + px0 + g] = __float2bfloat16(g01);
-            sGHT[h0 * LP + px0 + g + 8] = __float2bfloat16(g10);
-            sGHT[(h0 + 1) * LP + px0 + g + 8] = __float2bfloat16(g11);
-          }
-          uint32_t AG[4];
-          acc_to_a(hc[0], hc[1], AG);
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {  // g_v4 += ghp Q1: B[k = h][n = c] = Q1T[c][h]
-            const bf16* bq = sQ1T + (8 * n + g) * HP + 16 * kh + 2 * t;
-            mma16816(gz[n], AG, lds32(bq), lds32(bq + 8));
-          }
-        }
-      } else {
-        // g_v = gvin + E(G row)
-        const bf16* v0 = a.gvin + p0 * C;
-        const bf16* v1 = a.gvin + p1 * C;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const float2 f0 = unpack2(ldg32(v0 + 8 * n + 2 * t)), f1 = unpack2(ldg32(v1 + 8 * n + 2 * t));
-          gz[n][0] = f0.x; gz[n][1] = f0.y; gz[n][2] = f1.x; gz[n][3] = f1.y;
-        }
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-          uint32_t AT[4];
-          const bf16* ta = sT + (px0 + g) * SP + 16 * ks + 2 * t;
-          AT[0] = lds32(ta);
-          AT[1] = lds32(ta + 8 * SP);
-          AT[2] = lds32(ta + 8);
-          AT[3] = lds32(ta + 8 * SP + 8);
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            const bf16* bg = sG + (8 * n + g) * SP + 16 * ks + 2 * t;
-            mma16816(gz[n], AT, lds32(bg), lds32(bg + 8));
-          }
-        }
-        if (HEAD == HEAD_LIFT) {
-          const float m0 = a.masks[p0], m1 = a.masks[p1];
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            vb[n][0] += gz[n][0] + gz[n][2];
-            vb[n][1] += gz[n][1] + gz[n][3];
-            vw[n][0] += gz[n][0] * m0 + gz[n][2] * m1;
-            vw[n][1] += gz[n][1] * m0 + gz[n][3] * m1;
-          }
-          continue;
-        }
-        // g_z_l = g_v * GELU'(z_l)
-        const bf16* z0 = a.zl + p0 * C;
-        const bf16* z1 = a.zl + p1 * C;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const float2 f0 = unpack2(ldg32(z0 + 8 * n + 2 * t)), f1 = unpack2(ldg32(z1 + 8 * n + 2 * t));
-          gz[n][0] *= gelu_grad(f0.x); gz[n][1] *= gelu_grad(f0.y);
-          gz[n][2] *= gelu_grad(f1.x); gz[n][3] *= gelu_grad(f1.y);
-        }
+      for (int ks = 0; ks < 2; ++ks) {
+        const bf16* ta = a.Ttab + (size_t)(16 * (warp + 8 * i) + g) * J + 16 * ks + 2 * t;
+        AT[i][ks][0] = ldg32(ta);
+        AT[i][ks][1] = ldg32(ta + 8 * J);
+        AT[i][ks][2] = ldg32(ta + 8);
+        AT[i][ks][3] = ldg32(ta + 8 * J + 8);
       }
-      // ---- tail: g_z_l in gz (C layout) ----
-      // v_l for dW_l (transposed into sVT)
-      if (l == 0) {
-        const float m0 = a.masks[p0], m1 = a.masks[p1];
+  // per-thread partial sums over rows g, g + 8 (columns 8n + 2t, + 1)
+  float vb[4][2] = {};                 // dWb (SPEC) or dPb (LIFT)
+  float vw[4][2] = {};                 // dPw (LIFT)
+  float dW[4] = {0.f, 0.f, 0.f, 0.f};  // the warp's 16 x 8 tile of dW_l
+
+  float mr[MAXT][2];
+  float2 gr[2];
+  const bool masks = !SPEC || l == 0;
+  auto load_row = [&](int row, int st) {  // all but z_l
+    tile_load(smem_u32(smraw + S.sGv) + st * (uint32_t)tile, a.gvin + (size_t)row * L * C, L, tid);
+    if (SPEC && l > 0) tile_load(smem_u32(smraw + S.sV) + st * (uint32_t)tile, a.zlm1 + (size_t)row * L * C, L, tid);
+    if (masks)
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-          const int c0 = 16 * ks + 2 * t;
-          const int cs[4] = {c0, c0 + 1, c0 + 8, c0 + 9};
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            sVT[cs[q] * LP + px0 + g] = __float2bfloat16(fmaf(pw[ks][q], m0, pb[ks][q]));
-            sVT[cs[q] * LP + px0 + g + 8] = __float2bfloat16(fmaf(pw[ks][q], m1, pb[ks][q]));
-          }
+      for (int i = 0; i < MAXT; ++i)
+        if (warp + 8 * i < T) {
+          mr[i][0] = __ldg(a.masks + (size_t)row * L + 16 * (warp + 8 * i) + g);
+          mr[i][1] = __ldg(a.masks + (size_t)row * L + 16 * (warp + 8 * i) + g + 8);
         }
-      } else {
-        const bf16* z0 = a.zlm1 + p0 * C;
-        const bf16* z1 = a.zlm1 + p1 * C;
+    const float2* gp = a.Gg + (size_t)row * M * C;
+    gr[0] = __ldg(gp + tid);
+    gr[1] = __ldg(gp + tid + THREADS);
+  };
+  auto load_z = [&](int row) {
+    if (SPEC) tile_load(smem_u32(smraw + S.sZ), a.zl + (size_t)row * L * C, L, tid);
+  };
+  if (blockIdx.x < a.rows) {
+    load_row(blockIdx.x, 0);
+    load_z(blockIdx.x);
+  }
+  cp_async_commit();
+
+  int st = 0;
+  for (int row = blockIdx.x; row < a.rows; row += gridDim.x, st ^= 1) {
+    const int next = row + gridDim.x;
+    bf16* sG = sG0 + st * (BwdSmem::up16(C * SP * 2) / 2);
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const int c = 8 * n + 2 * t;
-          const float2 f0 = unpack2(ldg32(z0 + c)), f1 = unpack2(ldg32(z1 + c));
-          sVT[c * LP + px0 + g] = __float2bfloat16(gelu(f0.x));
-          sVT[(c + 1) * LP + px0 + g] = __float2bfloat16(gelu(f0.y));
-          sVT[c * LP + px0 + g + 8] = __float2bfloat16(gelu(f1.x));
-          sVT[(c + 1) * LP + px0 + g + 8] = __float2bfloat16(gelu(f1.y));
-        }
+    for (int q = 0; q < 2; ++q) {
+      const int i = tid + THREADS * q, kx = i / C, c = i % C;
+      *reinterpret_cast<uint32_t*>(sG + c * SP + 2 * kx) = pack2(gr[q].x, gr[q].y);
+    }
+    float mc[MAXT][2];
+#pragma unroll
+    for (int i = 0; i < MAXT; ++i) {
+      mc[i][0] = mr[i][0];
+      mc[i][1] = mr[i][1];
+    }
+    cp_async_wait<0>();
+    __syncthreads();  // this row's inputs; the other parity's tiles are no longer read
+    if (next < a.rows) load_row(next, st ^ 1);
+    cp_async_commit();
+    const uint32_t tgv = smem_u32(smraw + S.sGv) + st * (uint32_t)tile, tv = smem_u32(smraw + S.sV) + st * (uint32_t)tile,
+                   tz = smem_u32(smraw + S.sZ);
+#pragma unroll
+    for (int i = 0; i < MAXT; ++i) {
+      const int mt = warp + 8 * i;
+      if (mt >= T) break;
+      // g_v = gvin + E(G row)
+      float gz[4][4];
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        uint32_t r[4];
+        ldsm4(r, tgv + tile_frag(mt, ks, lane));
+        const float2 f0 = unpack2(r[0]), f1 = unpack2(r[1]), f2_ = unpack2(r[2]), f3 = unpack2(r[3]);
+        gz[2 * ks][0] = f0.x; gz[2 * ks][1] = f0.y; gz[2 * ks][2] = f1.x; gz[2 * ks][3] = f1.y;
+        gz[2 * ks + 1][0] = f2_.x; gz[2 * ks + 1][1] = f2_.y; gz[2 * ks + 1][2] = f3.x; gz[2 * ks + 1][3] = f3.y;
       }
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
-        const int o = 8 * n + 2 * t;
-        vb[n][0] += gz[n][0] + gz[n][2];
-        vb[n][1] += gz[n][1] + gz[n][3];
-        sGZT[o * LP + px0 + g] = __float2bfloat16(gz[n][0]);
-        sGZT[(o + 1) * LP + px0 + g] = __float2bfloat16(gz[n][1]);
-        sGZT[o * LP + px0 + g + 8] = __float2bfloat16(gz[n][2]);
-        sGZT[(o + 1) * LP + px0 + g + 8] = __float2bfloat16(gz[n][3]);
+        uint32_t bg[2][2];
+        ldsm_b(bg, smem_u32(sG), 8 * n, lane);
+        mma16816(gz[n], AT[i][0], bg[0][0], bg[0][1]);
+        mma16816(gz[n], AT[i][1], bg[1][0], bg[1][1]);
       }
-      // gvpw_l = g_z W_l: B[k = o][n = c] = W[o][c] = sWT[c][o]
-      {
-        uint32_t AZ[2][4];
-        acc_to_a(gz[0], gz[1], AZ[0]);
-        acc_to_a(gz[2], gz[3], AZ[1]);
-        bf16* w0 = a.gvout + p0 * C;
-        bf16* w1 = a.gvout + p1 * C;
+      if (!SPEC) {
+        const float m0 = mc[i][0], m1 = mc[i][1];
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
-          float d[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            const bf16* bw = sWT + (8 * n + g) * SP + 16 * ks + 2 * t;
-            mma16816(d, AZ[ks], lds32(bw), lds32(bw + 8));
-          }
-          *reinterpret_cast<uint32_t*>(w0 + 8 * n + 2 * t) = pack2(d[0], d[1]);
-          *reinterpret_cast<uint32_t*>(w1 + 8 * n + 2 * t) = pack2(d[2], d[3]);
+          vb[n][0] += gz[n][0] + gz[n][2];
+          vb[n][1] += gz[n][1] + gz[n][3];
+          vw[n][0] += gz[n][0] * m0 + gz[n][2] * m1;
+          vw[n][1] += gz[n][1] * m0 + gz[n][3] * m1;
         }
+        continue;
       }
+      // g_z_l = g_v GELU'(z_l); v_l
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        uint32_t r[4];
+        ldsm4(r, tz + tile_frag(mt, ks, lane));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float* z = &gz[2 * ks + (q >> 1)][2 * (q & 1)];
+          const float2 v = f2_get(f2(z[0], z[1]) * gelu_grad2(unpack_f2(r[q])));
+          z[0] = v.x;
+          z[1] = v.y;
+        }
+        if (l == 0) {
+          float pw[4], pb[4];
+          lift_coef(th, ks, t, pw, pb);
+          lift_frag(pw, pb, mc[i][0], mc[i][1], r);
+        } else {
+          ldsm4(r, tv + tile_frag(mt, ks, lane));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) r[q] = pack2(gelu2(unpack_f2(r[q])));
+        }
+        stsm4(tv + tile_frag(mt, ks, lane), r[0], r[1], r[2], r[3]);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        vb[n][0] += gz[n][0] + gz[n][2];
+        vb[n][1] += gz[n][1] + gz[n][3];
+      }
+      tile_put(tgv, mt, lane, gz);
+      // gvpw_l = g_z W_l: B[k = o][n = c] = W[o][c] = sWT[c][o]
+      uint32_t AZ[2][4];
+      acc_to_a(gz[0], gz[1], AZ[0]);
+      acc_to_a(gz[2], gz[3], AZ[1]);
+      float d[4][4] = {};
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        uint32_t bw[2][2];
+        ldsm_b(bw, smem_u32(sWT), 8 * n, lane);
+        mma16816(d[n], AZ[0], bw[0][0], bw[0][1]);
+        mma16816(d[n], AZ[1], bw[1][0], bw[1][1]);
+      }
+      tile_put(tz, mt, lane, d);
+      tile_store(smraw + S.sZ, mt, lane, a.gvout + (size_t)row * L * C);
     }
-    if (HEAD == HEAD_LIFT) continue;
+    if (!SPEC) continue;
     __syncthreads();
-    {
-      const int mt2 = warp >> 2, nt = warp & 3;
-      // dW_l tile (o rows 16 mt2.., c cols 8 nt..) += sum_px gz^T v
-      const bf16* pa = sGZT + (16 * mt2 + g) * LP + 2 * t;
-      const bf16* pbv = sVT + (8 * nt + g) * LP + 2 * t;
-      // Xg tile (kxri rows 16 mt2.., o cols 8 nt..) = sum_px TT gz
-      const bf16* ta = sTT + (16 * mt2 + g) * LP + 2 * t;
-      const bf16* pbz = sGZT + (8 * nt + g) * LP + 2 * t;
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-      for (int ks = 0; ks < L / 16; ++ks) {
-        const int k = 16 * ks;
-        uint32_t AF[4];
-        AF[0] = lds32(pa + k);
-        AF[1] = lds32(pa + 8 * LP + k);
-        AF[2] = lds32(pa + k + 8);
-        AF[3] = lds32(pa + 8 * LP + k + 8);
-        mma16816(dW, AF, lds32(pbv + k), lds32(pbv + k + 8));
-        AF[0] = lds32(ta + k);
-        AF[1] = lds32(ta + 8 * LP + k);
-        AF[2] = lds32(ta + k + 8);
-        AF[3] = lds32(ta + 8 * LP + k + 8);
-        mma16816(d, AF, lds32(pbz + k), lds32(pbz + k + 8));
-      }
-      float* xg = reinterpret_cast<float*>(a.Xg + (size_t)row * M * C);
-      const int k0 = 16 * mt2 + g, c0 = 8 * nt + 2 * t;
-      xg[((k0 >> 1) * C + c0) * 2 + (k0 & 1)] = d[0];
-      xg[((k0 >> 1) * C + c0 + 1) * 2 + (k0 & 1)] = d[1];
-      xg[(((k0 + 8) >> 1) * C + c0) * 2 + (k0 & 1)] = d[2];
-      xg[(((k0 + 8) >> 1) * C + c0 + 1) * 2 + (k0 & 1)] = d[3];
-    }
-    if (HEAD == HEAD_PROJ) {
-      // dQ1 tiles (h rows, c cols) += sum_px ghp^T v4; warp -> tiles 4 warp .. 4 warp + 3
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int tile = 4 * warp + q, mh = tile >> 2, nt = tile & 3;
-        const bf16* pa = sGHT + (16 * mh + g) * LP + 2 * t;
-        const bf16* pbv = sV4T + (8 * nt + g) * LP + 2 * t;
-        for (int ks = 0; ks < L / 16; ++ks) {
-          const int k = 16 * ks;
-          uint32_t AF[4];
-          AF[0] = lds32(pa + k);
-          AF[1] = lds32(pa + 8 * LP + k);
-          AF[2] = lds32(pa + k + 8);
-          AF[3] = lds32(pa + 8 * LP + k + 8);
-          mma16816(dQ1[q], AF, lds32(pbv + k), lds32(pbv + k + 8));
-        }
-      }
-    }
+    if (next < a.rows) load_z(next);
+    cp_async_commit();
+    row_dw(tgv, tv, T, warp >> 2, warp & 3, lane, dW);
+    row_dft(smem_u32(sTT), LP, tgv, T, warp, lane, a.Xg + (size_t)row * M * C);
   }
 
-  // ---- per-CTA partials ----
+  // ---- per-CTA partials; over the warps in a fixed order, so that the gradient repeats bit for bit ----
   float* gp = a.gpart + (size_t)blockIdx.x * Dn::N;
-  // vector partials: reduce over g (lanes xor 4, 8, 16), then over warps in a fixed
-  // order (per-warp slots), so that the gradient is bitwise reproducible
-  auto red_g = [&](float v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    v += __shfl_xor_sync(0xffffffffu, v, 8);
-    v += __shfl_xor_sync(0xffffffffu, v, 16);
-    return v;
-  };
-  float* myRed = sRed + warp * NRED;
-  __syncthreads();
+  cp_async_wait<0>();
+  float* mine = sRed + warp * 2 * C;
 #pragma unroll
   for (int n = 0; n < 4; ++n)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const float s0 = red_g(vb[n][e]);
-      const float s1 = red_g(vw[n][e]);
+      const float s0 = red_g(vb[n][e]), s1 = SPEC ? 0.f : red_g(vw[n][e]);
       if (g == 0) {
-        myRed[8 * n + 2 * t + e] = s0;
-        myRed[C + 8 * n + 2 * t + e] = s1;
+        mine[8 * n + 2 * t + e] = s0;
+        mine[C + 8 * n + 2 * t + e] = s1;
       }
     }
-  if (HEAD == HEAD_PROJ) {
+  __syncthreads();
+  for (int i = tid; i < (SPEC ? C : 2 * C); i += THREADS) {
+    float s = 0.f;
+    for (int w = 0; w < THREADS / 32; ++w) s += sRed[w * 2 * C + i];
+    gp[SPEC ? Dn::Wb + l * C + i : i < C ? Dn::Pb + i : Dn::Pw + i - C] = s;
+  }
+  if (SPEC) put_dw(gp + Dn::W + l * C * C, warp >> 2, warp & 3, lane, dW);
+}
+
+// ---------------------------------------------------------------------------
+// HEAD_PROJ: one CTA of sixteen warps per SM.  The hidden layer bounds it: 128 GELUs with their
+// derivatives a pixel (about fifteen FP32 instructions each, taken two at a time).  Two warps share a
+// pixel tile, one half of the hidden channels each, which halves the sums a thread keeps (dq1b, dQ2) and
+// lets sixteen warps fit; they exchange halves of g_v4.  The hidden gradients stay in shared memory,
+// row-major, and are read transposed for dQ1 after the row's one barrier, beside dW, Xg and gvpw.
+// With eight warps, all hidden channels each and two-byte transposing stores: 740 us for 32 masks of
+// 256 x 256; now 446.
+// ---------------------------------------------------------------------------
+constexpr int PROJ_THREADS = 512, PROJ_WARPS = PROJ_THREADS / 32;
+constexpr int PROJ_RED = H + 2 * C;  // a warp's slots: dq1b, dQ2 of its half, dWb of its half, dq2b
+
+struct ProjSmem {
+  size_t sZ, sV, sGz, sGH, sX, sTT, sQ1, sWT, sq, total;
+  __host__ __device__ static constexpr size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
+  __host__ __device__ explicit ProjSmem(int L) {
+    const size_t LP = (size_t)L + 8, tile = (size_t)L * C * 2;
+    size_t o = 0;
+    sZ = o; o += 2 * tile;            // z_3, by parity
+    sV = o; o += 2 * tile;            // z_2, by parity; v_3 takes its place
+    sGz = o; o += tile;               // g_z
+    sX = o; o += PROJ_WARPS * 1024;   // a kilobyte a warp: halves of g_v4, then gvpw tiles
+    sGH = o;                          // [L][H] hidden gradients; at the end, the warps' sums
+    const size_t gh = (size_t)L * H * 2, red = PROJ_WARPS * PROJ_RED * sizeof(float);
+    o += gh > red ? gh : red;
+    sTT = o; o += up16(J * LP * 2);
+    sQ1 = o; o += up16(H * SP * 2);
+    sWT = o; o += up16(C * SP * 2);
+    sq = o; o += 2 * H * sizeof(float);  // q1b, Q2
+    total = o;
+  }
+};
+
+__global__ void __launch_bounds__(PROJ_THREADS, 1) row_bwd_proj_kernel(const RowBwd a) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int L = a.L, LP = L + 8, l = NL - 1, T = L / 16;
+  const ProjSmem S(L);
+  const size_t tile = (size_t)L * C * 2;
+  bf16* sTT = reinterpret_cast<bf16*>(smraw + S.sTT);
+  bf16* sQ1 = reinterpret_cast<bf16*>(smraw + S.sQ1);  // [H][SP]
+  bf16* sWT = reinterpret_cast<bf16*>(smraw + S.sWT);  // [C c][SP]: W[o][c] at [c][o]
+  float* sq = reinterpret_cast<float*>(smraw + S.sq);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int hh = warp & 1, pair = warp >> 1;  // half of the hidden channels; tiles pair, pair + 8
+  const float* th = a.theta;
+  for (int i = tid; i < J * L / 2; i += PROJ_THREADS) {
+    const int k = i / (L / 2), px = 2 * (i % (L / 2));
+    *reinterpret_cast<uint32_t*>(sTT + k * LP + px) = *reinterpret_cast<const uint32_t*>(a.TT + (size_t)k * L + px);
+  }
+  for (int i = tid; i < C * C; i += PROJ_THREADS)
+    sWT[(i % C) * SP + i / C] = __float2bfloat16(th[Off::W + l * C * C + i]);
+  for (int i = tid; i < H * C; i += PROJ_THREADS) sQ1[(i / C) * SP + i % C] = __float2bfloat16(th[Off::Q1 + i]);
+  for (int i = tid; i < H; i += PROJ_THREADS) {
+    sq[i] = th[Off::q1b + i];
+    sq[H + i] = th[Off::Q2 + i];
+  }
+  const uint32_t gh = smem_u32(smraw + S.sGH);
+  auto gh_off = [](int px, int chunk) { return (uint32_t)(px * 2 * H + ((chunk ^ (px & 7)) << 4)); };
+
+  F2 dq1b[8], dq2[8];  // over rows g, g + 8; channels 64 hh + 8 nh + 2 t, + 1
 #pragma unroll
-    for (int nh = 0; nh < 16; ++nh)
+  for (int i = 0; i < 8; ++i) dq1b[i] = dq2[i] = f2(0.f);
+  float vb[2][2] = {};                 // dWb, channels 16 hh + 8 n + 2 t, + 1
+  float dq2b = 0.f;
+  float dW[4] = {0.f, 0.f, 0.f, 0.f};  // warps 8-15: a 16 x 8 tile of dW_l
+  float dQ1[2][4] = {};                // hidden rows 16 pair, columns 8 (2 hh), 8 (2 hh + 1)
+
+  float po[MAXT][2], pt[MAXT][2];  // the next row's outputs and targets
+  auto load_row = [&](int row, int st) {
+    const uint32_t tz = smem_u32(smraw + S.sZ) + st * (uint32_t)tile, tv = smem_u32(smraw + S.sV) + st * (uint32_t)tile;
+    for (int i = tid; i < 4 * L; i += PROJ_THREADS) {
+      cp_async16(tz + tile_off(i >> 2, i & 3), a.zl + (size_t)row * L * C + 8 * i);
+      cp_async16(tv + tile_off(i >> 2, i & 3), a.zlm1 + (size_t)row * L * C + 8 * i);
+    }
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float s0 = red_g(dq1b[nh][e]);
-        const float s1 = red_g(dq2[nh][e]);
-        if (g == 0) {
-          myRed[2 * C + 8 * nh + 2 * t + e] = s0;
-          myRed[2 * C + H + 8 * nh + 2 * t + e] = s1;
+    for (int i = 0; i < MAXT; ++i)
+      if (pair + 8 * i < T) {
+        const size_t p = (size_t)row * L + 16 * (pair + 8 * i) + g;
+        po[i][0] = __ldg(a.out + p);
+        po[i][1] = __ldg(a.out + p + 8);
+        pt[i][0] = __ldg(a.tgt + p);
+        pt[i][1] = __ldg(a.tgt + p + 8);
+      }
+  };
+  if (blockIdx.x < a.rows) load_row(blockIdx.x, 0);
+  cp_async_commit();
+
+  int st = 0;
+  for (int row = blockIdx.x; row < a.rows; row += gridDim.x, st ^= 1) {
+    const float cf = __ldg(a.coef + row / L);
+    float go[MAXT][2];
+#pragma unroll
+    for (int i = 0; i < MAXT; ++i) {
+      go[i][0] = (po[i][0] - pt[i][0]) * cf;
+      go[i][1] = (po[i][1] - pt[i][1]) * cf;
+    }
+    cp_async_wait<0>();
+    __syncthreads();  // this row's inputs; the previous row is done with every tile
+    if (row + (int)gridDim.x < a.rows) load_row(row + gridDim.x, st ^ 1);
+    cp_async_commit();
+    const uint32_t tz = smem_u32(smraw + S.sZ) + st * (uint32_t)tile, tv = smem_u32(smraw + S.sV) + st * (uint32_t)tile,
+                   tg = smem_u32(smraw + S.sGz);
+    float* xch = reinterpret_cast<float*>(smraw + S.sX);
+#pragma unroll 1
+    for (int i = 0; i < MAXT; ++i) {
+      const int mt = pair + 8 * i;
+      if (mt >= T) break;
+      const float go0 = i ? go[1][0] : go[0][0], go1 = i ? go[1][1] : go[0][1];
+      if (t == 0 && hh == 0) dq2b += go0 + go1;
+      uint32_t A[2][4];
+      ldsm4(A[0], tz + tile_frag(mt, 0, lane));
+      ldsm4(A[1], tz + tile_frag(mt, 1, lane));
+      float gz[4][4] = {};
+#pragma unroll
+      for (int kh = 0; kh < 4; ++kh) {  // hidden channels 64 hh + 16 kh .. + 15
+        const int h0 = 64 * hh + 16 * kh;
+        uint32_t AG[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          uint32_t bq[2][2];
+          ldsm_b(bq, smem_u32(sQ1), h0 + 8 * u, lane);
+          const float2 b = *reinterpret_cast<const float2*>(sq + h0 + 8 * u + 2 * t);
+          const float2 qv = *reinterpret_cast<const float2*>(sq + H + h0 + 8 * u + 2 * t);
+          float hc[4] = {b.x, b.y, b.x, b.y};
+          mma16816(hc, A[0], bq[0][0], bq[0][1]);
+          mma16816(hc, A[1], bq[1][0], bq[1][1]);
+          const F2 q = f2(qv.x, qv.y);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            // GELU and its derivative; gh = go Q2, ghp = gh GELU'(hpre)
+            const F2 x = f2(hc[2 * r], hc[2 * r + 1]), x2 = x * x;
+            const F2 tt = tanh2(x * fma2(f2(GK0 * GK1), x2, f2(GK0)));
+            const F2 hx = f2(0.5f) * x, gr_ = f2(r ? go1 : go0);
+            dq2[2 * kh + u] = fma2(gr_, fma2(hx, tt, hx), dq2[2 * kh + u]);
+            const F2 d = fma2(hx * fma2(f2(-1.0f) * tt, tt, f2(1.0f)), fma2(f2(3.0f * GK0 * GK1), x2, f2(GK0)),
+                              fma2(f2(0.5f), tt, f2(0.5f)));
+            const F2 gp = (gr_ * q) * d;
+            dq1b[2 * kh + u] = dq1b[2 * kh + u] + gp;
+            AG[2 * u + r] = pack2(gp);
+          }
+        }
+        stsm4(gh + gh_off(16 * mt + (lane & 15), h0 / 8 + (lane >> 4)), AG[0], AG[1], AG[2], AG[3]);
+        // g_v4 += ghp Q1: B[k = h][n = c], the table read transposed
+#pragma unroll
+        for (int n2 = 0; n2 < 2; ++n2) {
+          uint32_t bq[4];
+          ldsm4t(bq, smem_u32(sQ1) + (uint32_t)((h0 + (lane & 15)) * SP + 8 * (2 * n2 + (lane >> 4))) * 2);
+          mma16816(gz[2 * n2], AG, bq[0], bq[1]);
+          mma16816(gz[2 * n2 + 1], AG, bq[2], bq[3]);
         }
       }
-    float s = dq2b;
-    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
-    if (lane == 0) myRed[2 * C + 2 * H] = s;
-  }
-  __syncthreads();
-  for (int i = tid; i < NRED; i += THREADS) {
-    float s = 0.f;
-    for (int w = 0; w < THREADS / 32; ++w) s += sRed[w * NRED + i];
-    sRed[i] = s;  // slot 0 of warp 0 is read only by this thread
-  }
-  __syncthreads();
-  if constexpr (HEAD == HEAD_LIFT) {
-    for (int i = tid; i < C; i += THREADS) {
-      gp[Dn::Pb + i] = sRed[i];
-      gp[Dn::Pw + i] = sRed[C + i];
-    }
-    return;
-  } else {
-    for (int i = tid; i < C; i += THREADS) gp[Dn::Wb + l * C + i] = sRed[i];
-    {
-      const int mt2 = warp >> 2, nt = warp & 3;
-      const int o = 16 * mt2 + g, c = 8 * nt + 2 * t;
-      float* w = gp + Dn::W + l * C * C;
-      w[o * C + c] = dW[0];
-      w[o * C + c + 1] = dW[1];
-      w[(o + 8) * C + c] = dW[2];
-      w[(o + 8) * C + c + 1] = dW[3];
-    }
-    if (HEAD == HEAD_PROJ) {
-      for (int i = tid; i < H; i += THREADS) {
-        gp[Dn::q1b + i] = sRed[2 * C + i];
-        gp[Dn::Q2 + i] = sRed[2 * C + H + i];
-      }
-      if (tid == 0) gp[Dn::q2b] = sRed[2 * C + 2 * H];
+      // channels 16 (1 - hh) .. + 15 go to the other warp of the pair, 16 hh .. stay
+      float* mine = xch + warp * 256 + lane * 8;
+      const float* other = xch + (warp ^ 1) * 256 + lane * 8;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int tile = 4 * warp + q, mh = tile >> 2, nt = tile & 3;
-        const int h = 16 * mh + g, c = 8 * nt + 2 * t;
-        float* w = gp + Dn::Q1;
-        w[h * C + c] = dQ1[q][0];
-        w[h * C + c + 1] = dQ1[q][1];
-        w[(h + 8) * C + c] = dQ1[q][2];
-        w[(h + 8) * C + c + 1] = dQ1[q][3];
+      for (int n = 0; n < 2; ++n)
+        *reinterpret_cast<float4*>(mine + 4 * n) =
+            hh ? make_float4(gz[n][0], gz[n][1], gz[n][2], gz[n][3])
+               : make_float4(gz[2 + n][0], gz[2 + n][1], gz[2 + n][2], gz[2 + n][3]);
+      // v_3, the same channels
+      {
+        uint32_t r[4];
+        ldsm4(r, tv + tile_frag(mt, hh, lane));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[q] = pack2(gelu2(unpack_f2(r[q])));
+        stsm4(tv + tile_frag(mt, hh, lane), r[0], r[1], r[2], r[3]);
+      }
+      pair_bar(pair);
+      float z[2][4];
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const float4 o = *reinterpret_cast<const float4*>(other + 4 * n);
+        z[n][0] = (hh ? gz[2 + n][0] : gz[n][0]) + o.x;
+        z[n][1] = (hh ? gz[2 + n][1] : gz[n][1]) + o.y;
+        z[n][2] = (hh ? gz[2 + n][2] : gz[n][2]) + o.z;
+        z[n][3] = (hh ? gz[2 + n][3] : gz[n][3]) + o.w;
+        vb[n][0] += z[n][0] + z[n][2];
+        vb[n][1] += z[n][1] + z[n][3];
+      }
+      stsm4(tg + tile_frag(mt, hh, lane), pack2(z[0][0], z[0][1]), pack2(z[0][2], z[0][3]), pack2(z[1][0], z[1][1]),
+            pack2(z[1][2], z[1][3]));
+      pair_bar(pair);  // the exchange is read before it is written again
+    }
+    __syncthreads();
+    if (warp < T) {  // gvpw = g_z W of pixel tile `warp`
+      uint32_t AZ[2][4];
+      ldsm4(AZ[0], tg + tile_frag(warp, 0, lane));
+      ldsm4(AZ[1], tg + tile_frag(warp, 1, lane));
+      float d[4][4] = {};
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        uint32_t bw[2][2];
+        ldsm_b(bw, smem_u32(sWT), 8 * n, lane);
+        mma16816(d[n], AZ[0], bw[0][0], bw[0][1]);
+        mma16816(d[n], AZ[1], bw[1][0], bw[1][1]);
+      }
+      unsigned char* x = smraw + S.sX + warp * 1024;  // as a tile of its own
+      tile_put(smem_u32(x), 0, lane, d);
+      tile_store(x, 0, lane, a.gvout + ((size_t)row * L + 16 * warp) * C);
+    }
+    if (warp < 8) row_dft(smem_u32(sTT), LP, tg, T, warp, lane, a.Xg + (size_t)row * M * C);
+    else row_dw(tg, tv, T, (warp - 8) >> 2, warp & 3, lane, dW);
+    {  // dQ1: hidden rows 16 pair .. + 15 by channels 16 hh .. + 15
+      const int px = (lane & 7) + 8 * (lane >> 4), ch = 2 * pair + ((lane >> 3) & 1);
+#pragma unroll 4
+      for (int ks = 0; ks < T; ++ks) {
+        uint32_t A[4], b[4];
+        ldsm4t(A, gh + gh_off(16 * ks + px, ch));
+        ldsm4t(b, tz + tile_off(16 * ks + (lane & 15), 2 * hh + (lane >> 4)));
+        mma16816(dQ1[0], A, b[0], b[1]);
+        mma16816(dQ1[1], A, b[2], b[3]);
       }
     }
-  }  // HEAD != HEAD_LIFT
+  }
+
+  // ---- per-CTA partials; over the warps in a fixed order, so that the gradient repeats bit for bit ----
+  float* gp = a.gpart + (size_t)blockIdx.x * Dn::N;
+  cp_async_wait<0>();
+  __syncthreads();
+  float* sRed = reinterpret_cast<float*>(smraw + S.sGH);
+  float* red = sRed + warp * PROJ_RED;
+#pragma unroll
+  for (int nh = 0; nh < 8; ++nh) {
+    const float2 b = f2_get(dq1b[nh]), q = f2_get(dq2[nh]);
+    const float s0 = red_g(b.x), s1 = red_g(b.y), s2 = red_g(q.x), s3 = red_g(q.y);
+    if (g == 0) {
+      red[8 * nh + 2 * t] = s0;
+      red[8 * nh + 2 * t + 1] = s1;
+      red[64 + 8 * nh + 2 * t] = s2;
+      red[64 + 8 * nh + 2 * t + 1] = s3;
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float s = red_g(vb[n][e]);
+      if (g == 0) red[H + 8 * n + 2 * t + e] = s;
+    }
+  float sb = dq2b;
+  for (int k = 16; k > 0; k >>= 1) sb += __shfl_xor_sync(0xffffffffu, sb, k);
+  if (lane == 0) red[H + 16] = sb;
+  __syncthreads();
+  for (int i = tid; i < 2 * H + C + 1; i += PROJ_THREADS) {
+    int w, slot, dst;  // first warp of the half, its slot, where it goes
+    if (i < H) {
+      w = i >= 64;
+      slot = i & 63;
+      dst = Dn::q1b + i;
+    } else if (i < 2 * H) {
+      w = i - H >= 64;
+      slot = 64 + (i & 63);
+      dst = Dn::Q2 + i - H;
+    } else if (i < 2 * H + C) {
+      w = i - 2 * H >= 16;
+      slot = H + (i & 15);
+      dst = Dn::Wb + l * C + i - 2 * H;
+    } else {
+      w = 0;
+      slot = H + 16;
+      dst = Dn::q2b;
+    }
+    float s = 0.f;
+    for (; w < PROJ_WARPS; w += 2) s += sRed[w * PROJ_RED + slot];
+    gp[dst] = s;
+  }
+  if (warp >= 8) put_dw(gp + Dn::W + l * C * C, (warp - 8) >> 2, warp & 3, lane, dW);
+  {
+    const int h = 16 * pair + g;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      float* w = gp + Dn::Q1 + h * C + 16 * hh + 8 * n + 2 * t;
+      w[0] = dQ1[n][0];
+      w[1] = dQ1[n][1];
+      w[8 * C] = dQ1[n][2];
+      w[8 * C + 1] = dQ1[n][3];
+    }
+  }
 }
 
 // dense partials -> gradient vector
@@ -1825,8 +1947,9 @@ int backward(litho_fno* f, const float* masks, const float* targets, int B) {
   litho_ctx* ctx = f->ctx;
   const int L = f->L, rows = B * L, grid = f->bwd_grid;
   const float* th = f->theta.as<float>();
-  const BwdSmem sp(L, HEAD_PROJ), ss(L, HEAD_SPEC), sl(L, HEAD_LIFT);
-  LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_PROJ>, sp.total));
+  const BwdSmem ss(L, HEAD_SPEC), sl(L, HEAD_LIFT);
+  const ProjSmem sp(L);
+  LITHO_RET(set_smem(ctx, (const void*)row_bwd_proj_kernel, sp.total));
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_SPEC>, ss.total));
   LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_LIFT>, sl.total));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 3 * NL + 4);
@@ -1847,7 +1970,7 @@ int backward(litho_fno* f, const float* masks, const float* targets, int B) {
     a.gvin = f->gv[cur ^ 1].as<bf16>();
     a.gvout = f->gv[cur].as<bf16>();
     if (l == NL - 1)
-      row_bwd_kernel<HEAD_PROJ><<<grid, THREADS, sp.total, ctx->stream>>>(a);
+      row_bwd_proj_kernel<<<std::min(rows, ctx->sm_count), PROJ_THREADS, sp.total, ctx->stream>>>(a);
     else
       row_bwd_kernel<HEAD_SPEC><<<grid, THREADS, ss.total, ctx->stream>>>(a);
     LITHO_RET(launch_column<true>(f, B, l, Xg, Gg, f->gU.as<float2>()));
