@@ -1508,24 +1508,38 @@ __global__ void reduce_dense_kernel(const float* __restrict__ gpart, int nparts,
   grad[dense_to_param(i)] = s;
 }
 
-// dR[j][kx][c][o] = s_kx sum_b gU_b[j][kx][o] conj(V_b[j][kx][c]); one CTA per (j, kx)
+// dR[j][kx][c][o] = s_kx sum_b gU_b[j][kx][o] conj(V_b[j][kx][c]); one CTA per (j, kx), the operands of
+// DR_MASKS masks at a time in shared memory (one mask between two barriers, its load exposed, took
+// 20 us for 32 masks; now 8)
+constexpr int DR_MASKS = 32;
 __global__ void __launch_bounds__(THREADS) dR_kernel(int L, int B, int layer, const float2* __restrict__ gU,
                                                      const float2* __restrict__ V, float* __restrict__ grad) {
   const int jk = blockIdx.x, tid = threadIdx.x;  // jk = j * M + kx
-  const int kx = jk % M;
-  __shared__ float2 su[C], sv[C];
-  float2 acc[4] = {};
-  for (int b = 0; b < B; ++b) {
-    __syncthreads();
-    if (tid < C) su[tid] = gU[((size_t)b * J * M + jk) * C + tid];
-    else if (tid < 2 * C) sv[tid - C] = V[((size_t)b * J * M + jk) * C + tid - C];
+  const int kx = jk % M, lane = tid & 31, warp = tid >> 5;
+  __shared__ float2 su[DR_MASKS][C], sv[DR_MASKS][C];
+  float2 acc[4] = {};  // c = warp + 8 r, o = lane
+  for (int b0 = 0; b0 < B; b0 += DR_MASKS) {
+    const int nb = min(DR_MASKS, B - b0);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int idx = tid + THREADS * r, c = idx / C, o = idx % C;
-      const float2 u = su[o], v = sv[c];
-      acc[r].x += u.x * v.x + u.y * v.y;
-      acc[r].y += u.y * v.x - u.x * v.y;
+    for (int q = 0; q < DR_MASKS / 8; ++q) {
+      const int b = warp + 8 * q;
+      if (b < nb) {
+        const size_t i = ((size_t)(b0 + b) * J * M + jk) * C + lane;
+        su[b][lane] = __ldg(gU + i);
+        sv[b][lane] = __ldg(V + i);
+      }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int b = 0; b < nb; ++b) {
+      const float2 u = su[b][lane];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float2 v = sv[b][warp + 8 * r];
+        acc[r].x += u.x * v.x + u.y * v.y;
+        acc[r].y += u.y * v.x - u.x * v.y;
+      }
     }
   }
   const float s = (kx == 0 ? 1.0f : 2.0f) / ((float)L * (float)L);
