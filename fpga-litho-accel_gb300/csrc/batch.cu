@@ -16,7 +16,7 @@
 //   window row splits in {r, 2r}, r what the class's tiles take by themselves
 // with CUDA events on the context's stream and keeps the fastest; results are
 // cached by (L, Nx, nk, images, precision, band form, r).  The plan then
-// captures the whole sequence in a CUDA graph (LITHO_BATCH_GRAPH).
+// captures the whole sequence in a CUDA graph (LITHO_BATCH_GRAPH), a branch per class.
 #include "litho_internal.cuh"
 
 #include <algorithm>
@@ -118,16 +118,61 @@ static int run_class(litho_batch_plan* bp, int ci) {
   return run_fi(ctx, p, c.band.as<float2>(), c.tmbuf.as<float>(), c.images);
 }
 
-// Every class with masks, one after another on the context's stream.  (Running the
-// classes as parallel graph branches, plain or staggered so that one class's SOCS meets
-// another's streaming kernels, with the persistent kernels taking tiles from per-class
-// counters, measured slower: the streaming kernels hold ~200 KB of shared memory per
-// SM, so a class's latency-bound SOCS CTAs and another class's streaming CTAs cannot
-// share an SM, and whichever kernel was launched first takes the SMs as they free up.)
+// Every class with masks, one after another on the context's stream.
 static int run_all(litho_batch_plan* bp) {
   for (int ci = 0; ci < (int)bp->classes.size(); ++ci)
     if (bp->classes[ci].count > 0) LITHO_RET(run_class(bp, ci));
   return LITHO_OK;
+}
+
+// The same as branches of the graph being captured on the context's stream, the class with the most
+// pixels first.  A class's chain has latency-bound stages (SOCS, interpolation rows) and ones bound by
+// memory or the FP32 pipe, and the window and image kernels leave room on an SM for another class's
+// CTAs; every buffer a class writes is its own.  50 images of 1024^2 and 10 of 2048^2 with masks of
+// five sizes: 220 us one class after the other, 187 as branches.  Streams of the classes live for the
+// capture alone.
+static int capture_branches(litho_batch_plan* bp) {
+  litho_ctx* ctx = bp->ctx;
+  std::vector<int> order;
+  for (int ci = 0; ci < (int)bp->classes.size(); ++ci)
+    if (bp->classes[ci].count > 0) order.push_back(ci);
+  auto pixels = [&](int ci) { return (size_t)bp->classes[ci].count * bp->classes[ci].L * bp->classes[ci].L; };
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return pixels(a) > pixels(b); });
+  const cudaStream_t home = ctx->stream;
+  cudaEvent_t fork = nullptr;
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> done;
+  int rc = LITHO_OK;
+  auto ok = [&](cudaError_t e) {
+    if (e != cudaSuccess && rc == LITHO_OK) {
+      set_error(ctx, LITHO_ERR_CUDA, "graph branch: %s", cudaGetErrorString(e));
+      rc = LITHO_ERR_CUDA;
+    }
+    return rc == LITHO_OK;
+  };
+  if (order.size() > 1 && ok(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming))) ok(cudaEventRecord(fork, home));
+  for (size_t i = 1; i < order.size() && rc == LITHO_OK; ++i) {
+    cudaStream_t s = nullptr;
+    if (!ok(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking))) break;
+    side.push_back(s);
+    if (!ok(cudaStreamWaitEvent(s, fork, 0))) break;
+  }
+  for (size_t i = 0; i < order.size() && rc == LITHO_OK; ++i) {
+    ctx->stream = i == 0 ? home : side[i - 1];
+    rc = run_class(bp, order[i]);
+  }
+  ctx->stream = home;
+  for (size_t i = 0; i < side.size(); ++i) {  // every fork is joined, also after an error
+    cudaEvent_t e = nullptr;
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) continue;
+    done.push_back(e);
+    ok(cudaEventRecord(e, side[i]));
+    ok(cudaStreamWaitEvent(home, e, 0));
+  }
+  for (cudaEvent_t e : done) cudaEventDestroy(e);
+  if (fork) cudaEventDestroy(fork);
+  for (cudaStream_t s : side) cudaStreamDestroy(s);
+  return rc;
 }
 
 static int time_class(litho_batch_plan* bp, int ci, float* ms, int reps = 3) {
@@ -357,7 +402,7 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       rc = LITHO_ERR_CUDA;
     } else {
-      const int rr = run_all(bp);
+      const int rr = capture_branches(bp);
       const cudaError_t e = cudaStreamEndCapture(ctx->stream, &bp->graph);
       if (rr != LITHO_OK || e != cudaSuccess) rc = rr != LITHO_OK ? rr : LITHO_ERR_CUDA;
       else if (cudaGraphInstantiate(&bp->exec, bp->graph, 0) != cudaSuccess) rc = LITHO_ERR_CUDA;
