@@ -892,7 +892,10 @@ __global__ void __launch_bounds__(IV_THREADS) invvec_kernel(const double* __rest
 // larger than RR_MAXC (the near-zero tail of a rank-deficient TCC), or one whose
 // Gram matrix is not numerically positive definite, is orthonormalised by modified
 // Gram-Schmidt (two passes) instead, without the rotation in the first case.
-// One CTA per cluster: CTA j works only if a cluster starts at j.
+// One CTA per cluster: CTA j works only if a cluster starts at j.  Chains of divisions and roots bound
+// it (some ten FP64 instructions of ~66 cycles each), so nothing but those is left to one thread: the
+// factorisation with a thread per row and a rotation by two reciprocal roots, 24 vectors of the
+// usual quasar source, took 287 -> 204 us at n = 289 and 221 -> 184 at n = 1089.
 constexpr int RR_THREADS = 256, RR_MAXC = 48;
 
 // y_i = (T z)_i for the symmetric tridiagonal T
@@ -951,8 +954,8 @@ __global__ void __launch_bounds__(RR_THREADS) cluster_rr_kernel(const double* __
   __shared__ double red[32];
   __shared__ double H[RR_MAXC][RR_MAXC + 1];
   __shared__ double V[RR_MAXC][RR_MAXC + 1];
+  __shared__ double s_inv[RR_MAXC], s_diag;
   __shared__ int s_order[RR_MAXC];
-  __shared__ int s_ok;
   double tn = 0.0;
   for (int i = threadIdx.x; i < n; i += RR_THREADS)
     tn = fmax(tn, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0));
@@ -976,25 +979,26 @@ __global__ void __launch_bounds__(RR_THREADS) cluster_rr_kernel(const double* __
   for (int pass = 0; ok && pass < 2; ++pass) {
     rr_pairs(d, e, Zc, n, c, false, H);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      s_ok = 1;
-      for (int a = 0; a < c && s_ok; ++a) {  // H <- L (lower), in place
-        double diag = H[a][a];
-        for (int b = 0; b < a; ++b) diag -= H[a][b] * H[a][b];
-        if (!(diag > 1e-24)) {
-          s_ok = 0;
-          break;
-        }
-        H[a][a] = sqrt(diag);
-        for (int r = a + 1; r < c; ++r) {
-          double v = H[r][a];
-          for (int b = 0; b < a; ++b) v -= H[r][b] * H[a][b];
-          H[r][a] = v / H[a][a];
-        }
+    // H <- L (lower), in place, a column at a time with a thread per row; s_inv: 1 / L_aa
+    ok = true;
+    for (int a = 0; a < c && ok; ++a) {
+      const int r = a + (int)threadIdx.x;
+      double v = 0.0;
+      if (r < c) {
+        v = H[r][a];
+        for (int b = 0; b < a; ++b) v = fma(-H[r][b], H[a][b], v);
+        if (r == a) s_diag = v;
       }
+      __syncthreads();
+      const double diag = s_diag;
+      ok = diag > 1e-24;
+      if (ok && r < c) {
+        const double root = sqrt(diag), inv = 1.0 / root;
+        H[r][a] = r == a ? root : v * inv;
+        if (r == a) s_inv[a] = inv;
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    ok = s_ok != 0;
     if (!ok) break;
     // z_i <- L^-1 z_i for every component i (forward substitution)
     for (int i = threadIdx.x; i < n; i += RR_THREADS) {
@@ -1002,7 +1006,7 @@ __global__ void __launch_bounds__(RR_THREADS) cluster_rr_kernel(const double* __
       for (int a = 0; a < c; ++a) {
         double v = Zc[(size_t)a * n + i];
         for (int b = 0; b < a; ++b) v -= H[a][b] * y[b];
-        y[a] = v / H[a][a];
+        y[a] = v * s_inv[a];
       }
       for (int a = 0; a < c; ++a) Zc[(size_t)a * n + i] = y[a];
     }
@@ -1044,19 +1048,18 @@ __global__ void __launch_bounds__(RR_THREADS) cluster_rr_kernel(const double* __
   {
     __shared__ double s_cs[RR_MAXC / 2], s_sn[RR_MAXC / 2];
     __shared__ int s_p[RR_MAXC / 2], s_q[RR_MAXC / 2];
-    __shared__ int s_done;
     const int cp = c + (c & 1), np = cp / 2;
     for (int sweep = 0; sweep < 30; ++sweep) {
-      if (threadIdx.x == 0) {
-        double off = 0.0, dia = 0.0;
-        for (int a = 0; a < c; ++a) {
-          dia += H[a][a] * H[a][a];
-          for (int b = a + 1; b < c; ++b) off += H[a][b] * H[a][b];
-        }
-        s_done = off <= 1e-32 * dia;
+      double off = 0.0, dia = 0.0;
+      for (int i = threadIdx.x; i < c * c; i += RR_THREADS) {
+        const int x = i / c, y = i - x * c;
+        const double v = H[x][y];
+        if (x == y) dia = fma(v, v, dia);
+        else if (x < y) off = fma(v, v, off);
       }
-      __syncthreads();
-      if (s_done) break;
+      off = block_sum<RR_THREADS>(off, red);
+      dia = block_sum<RR_THREADS>(dia, red);
+      if (off <= 1e-32 * dia) break;
       for (int r = 0; r < cp - 1; ++r) {
         if (threadIdx.x < np) {
           const int i = threadIdx.x, j = cp - 1 - i;
@@ -1067,10 +1070,19 @@ __global__ void __launch_bounds__(RR_THREADS) cluster_rr_kernel(const double* __
           if (qq < c) {
             const double apq = H[pp][qq];
             if (apq != 0.0) {
-              const double theta = (H[qq][qq] - H[pp][pp]) / (2.0 * apq);
-              const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-              cs = 1.0 / sqrt(t * t + 1.0);
-              sn = t * cs;
+              const double h = H[qq][qq] - H[pp][pp], g2 = 2.0 * apq, rr = fma(h, h, g2 * g2);
+              if (rr > 1e-280 && rr < 1e280) {
+                // cos 2 phi = |h| / r, sin 2 phi = +-2 apq / r: two reciprocal roots instead of three
+                // divisions and two roots in a chain
+                const double ir = rsqrt(rr), c2 = fma(0.5 * fabs(h), ir, 0.5), rc = rsqrt(c2);
+                cs = c2 * rc;
+                sn = (h >= 0.0 ? 0.5 : -0.5) * g2 * ir * rc;
+              } else {  // the squares leave the range
+                const double theta = h / g2;
+                const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+                cs = 1.0 / sqrt(t * t + 1.0);
+                sn = t * cs;
+              }
             }
           }
           s_p[i] = pp;
