@@ -80,7 +80,9 @@ __global__ void win_sum_kernel(const float2* __restrict__ win_part, int nparts, 
                                float2* __restrict__ wsum) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   const int KX = 2 * Nx + 1, KY = 2 * Ny + 1, KD = KX * KY;
+  early_next();
   if (idx >= KDP) return;
+  early_wait(win_part);
   // several images per thread: their partial loads are in flight together
 #pragma unroll 4
   for (int img = blockIdx.y; img < batch; img += gridDim.y) {
@@ -148,6 +150,8 @@ __global__ void __launch_bounds__(BT_THREADS, 2) band_tcc_kernel(const float2* _
     for (int e = tid; e < tsz / 2; e += blockDim.x) cp_async16(sT + 2 * e, src + 2 * e, 16);
     cp_async_commit();
   }
+  early_next();
+  early_wait(wsum);  // (the table is the kernel set's)
   const bool active = lane < IPW * NL;
   const int sub = active ? lane / NL : 0, j = active ? lane - sub * NL : lane % NL;
   float4* myW = reinterpret_cast<float4*>(sW + (size_t)warp * IPW * KDP);
@@ -297,9 +301,8 @@ int run_band_tcc(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const lit
     const int sms = std::max(1, p.sms > 0 ? p.sms : ctx->sm_count);
     const int ipt = std::max(1, std::min(4, (p.batch * bx) / (4 * sms)));
     const int by = std::max(1, std::min(65535, (p.batch + ipt - 1) / ipt));
-    win_sum_kernel<<<dim3(bx, by), 128, 0, ctx->stream>>>(
-        w.part, w.nparts, w.mskf_r, w.mskf_i, g.Fx, g.Fy, g.Nx, g.Ny, KDP, p.batch, wsum);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
+    LITHO_CUDA_TRY(ctx, launch_early(p.early, win_sum_kernel, dim3(bx, by), 128, 0, ctx->stream, w.part, w.nparts, w.mskf_r,
+                                     w.mskf_i, g.Fx, g.Fy, g.Nx, g.Ny, KDP, p.batch, wsum));
     int most = 0;
     const int ntc = (g.Ny + 1) * nc;
     for (int b = 0; b < ntc; ++b) most = std::max(most, bt_task_shape(b, g.Nx, g.Ny, nc).size);
@@ -320,9 +323,8 @@ int run_band_tcc(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const lit
     per_sm = std::max(1, per_sm);
     const int per_pass = nw * IPW;
     const int groups = std::max(1, std::min((p.batch + per_pass - 1) / per_pass, (per_sm * sms + ntc - 1) / ntc));
-    k<<<dim3(ntc, groups), 32 * nw, smem_for(nw), ctx->stream>>>(ks->band_tab, wsum, KDP, g.Ny, nc, p.batch,
-                                                                 band_part);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
+    LITHO_CUDA_TRY(ctx, launch_early(p.early, k, dim3(ntc, groups), 32 * nw, smem_for(nw), ctx->stream, ks->band_tab, wsum, KDP,
+                                     g.Ny, nc, p.batch, band_part));
   }
   return LITHO_OK;
 }

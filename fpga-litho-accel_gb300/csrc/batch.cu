@@ -109,6 +109,7 @@ static int run_class(litho_batch_plan* bp, int ci) {
   ImgPlan p = make_plan(class_geom(c, band ? default_conv(Nx, Ny) : c.convN), c.count, ctx->sm_count);
   p.kpg = band ? c.ks->nk : std::min(c.kpg, c.ks->nk);
   p.ngroups = band ? c.ks->band_nc : (c.ks->nk + p.kpg - 1) / p.kpg;
+  p.early = true;  // in a graph as well
   WindowSrc w;
   w.part = c.win.as<float2>();
   w.nparts = nparts;

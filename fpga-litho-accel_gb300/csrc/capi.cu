@@ -158,7 +158,6 @@ void* litho_ctx_get_stream(litho_ctx* ctx) { return ctx ? (void*)ctx->stream : n
 
 int litho_ctx_synchronize(litho_ctx* ctx) {
   if (ctx == nullptr) return LITHO_ERR_ARG;
-  LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return tc_check_flag(ctx);
 }
 
@@ -531,8 +530,10 @@ int litho_image_batch(litho_ctx* ctx, const litho_kernel_set* ks, const float* m
     return image_pipeline(ctx, g, batch, masks, ks, images, precision);
   }
   LITHO_RET(host_batch(ctx, g, batch, masks, ks, images, precision, img));
+  // only the mixed form and the copies of rows that aren't whole 16-byte pieces wait with a limit
+  if (precision == LITHO_PREC_MIXED || (Lx & 3) != 0) return tc_check_flag(ctx);
   LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  return tc_check_flag(ctx);
+  return LITHO_OK;
 }
 
 int litho_image(litho_ctx* ctx, const float* mask, int Lx, int Ly, const float* krn_r, const float* krn_i,

@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
   constexpr int CPL = P::CPL, COLS = P::COLS, KS = P::KS;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  early_next();
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm) + warp * WF_ST;
   float* zero = sm + P::BARS;
   float2* sTw = reinterpret_cast<float2*>(zero + P::ZERO);    // [Nx+1][TS]
@@ -505,6 +506,8 @@ __global__ void __launch_bounds__(FF_THREADS, 3) fi_fold_kernel(const float* __r
   constexpr int CPL = ff_cpl(NY), COLS = 32 * CPL, KS = ff_stride(NY);
   extern __shared__ __align__(16) float sK[];  // [rows][KS] coefficients, then [rows] row offsets
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  early_wait(tm);
+  early_wait(coef);
   const int X0 = blockIdx.x * COLS, img = blockIdx.z;
   const int b0 = (int)((long long)nb * blockIdx.y / gridDim.y), b1 = (int)((long long)nb * (blockIdx.y + 1) / gridDim.y);
   const int xl = VEC ? X0 + CPL * lane : X0 + lane;
@@ -618,8 +621,7 @@ static cudaError_t launch_fi_fold_t(cudaStream_t s, const ImgPlan& p, const floa
   auto k = vec ? fi_fold_kernel<NY, true> : fi_fold_kernel<NY, false>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k<<<dim3(ncb, R, p.batch), FF_THREADS, smem, s>>>(tm, g.Lx, g.Ly, g.Fy, g.Ny, coef, nb, images);
-  return cudaGetLastError();
+  return launch_early(p.early, k, dim3(ncb, R, p.batch), FF_THREADS, smem, s, tm, g.Lx, g.Ly, g.Fy, g.Ny, coef, nb, images);
 }
 
 cudaError_t launch_fi_fold(cudaStream_t s, const ImgPlan& p, const float* tm, const float* coef, float* images) {

@@ -455,12 +455,12 @@ static int tc_err_flag(litho_ctx* ctx, int** flag) {
 
 int tc_err_flag_public(litho_ctx* ctx, int** flag) { return tc_err_flag(ctx, flag); }
 
-// Read and clear the device-side timeout flag of the tensor-core kernels
-// (the caller has synchronised the stream).
+// Wait for the context's stream, then read and clear the device-side flag of the bounded waits.
 int tc_check_flag(litho_ctx* ctx) {
-  if (ctx->mx_d.p == nullptr) return LITHO_OK;
   int v = 0;
-  LITHO_CUDA_TRY(ctx, cudaMemcpy(&v, ctx->mx_d.p, sizeof(int), cudaMemcpyDeviceToHost));
+  if (ctx->mx_d.p != nullptr)  // on the context's stream: one wait for the work and the flag
+    LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(&v, ctx->mx_d.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   if (v != 0) {
     LITHO_CUDA_TRY(ctx, cudaMemset(ctx->mx_d.p, 0, 256));
     set_error(ctx, LITHO_ERR_TIMEOUT, "a tensor-core pipeline wait gave up (bounded mbarrier wait)");

@@ -201,8 +201,36 @@ struct ImgPlan {
   int rowBlocks = 1, colSplits = 1;  // window DFT: column blocks, row splits -> nparts
   int kpg = 1, ngroups = 1;          // SOCS kernels per CTA -> ngroups
   int sms = 0;                       // SMs of the device (launch sizing)
+  bool early = false;                // each stage's CTAs start while the stage before it runs (launch_early)
   int nparts() const { return rowBlocks * colSplits; }
 };
+
+// Programmatic dependent launch.  A kernel launched `early` may start once every CTA of the one before
+// it on the stream has called early_next (or ended); what that one writes is there after early_wait,
+// which comes before a kernel's first write and its first read of anything the launches of its call
+// write.  early_wait hands back the pointers read from then on, so that no read moves before it.  Both
+// are nothing in a launch without it.
+__device__ __forceinline__ void early_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename T>
+__device__ __forceinline__ void early_wait(const T* __restrict__& p) {
+  unsigned long long v = reinterpret_cast<unsigned long long>(p);
+  asm volatile("griddepcontrol.wait;" : "+l"(v)::"memory");
+  p = reinterpret_cast<const T*>(v);
+}
+template <typename... P, typename... A>
+cudaError_t launch_early(bool early, void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
 
 ImgPlan make_plan(const ImgGeom& g, int batch, int sm_count);
 
