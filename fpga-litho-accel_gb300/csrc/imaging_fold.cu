@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
         for (int k = 0; k < 4; ++k) {
           const float* q = off[k] >= 0 ? src + k * P::RB + ((base4 + off[k]) & 3) : zero;
 #pragma unroll
-          for (int i = 0; i < CPL; ++i) p[k][i] = lane + 32 * i < ncol ? q[lane + 32 * i] : 0.f;
+          for (int i = 0; i < CPL; ++i) p[k][i] = q[lane + 32 * i];  // (past ncol: left in the ring, dropped below)
         }
         __syncwarp();  // the slot refilled below (the previous row's) has been read by every lane
         issue(lane < 4 ? reinterpret_cast<const int*>(sOff + (b - t0 + WF_AHEAD))[lane] : -1,
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
         reinterpret_cast<float2*>(r + n * COLS)[lane] = make_float2(v[0], v[1]);
       } else {
 #pragma unroll
-        for (int i = 0; i < CPL; ++i) r[n * COLS + lane + 32 * i] = v[i];
+        for (int i = 0; i < CPL; ++i) r[n * COLS + lane + 32 * i] = lane + 32 * i < ncol ? v[i] : 0.f;
       }
     };
 #pragma unroll
