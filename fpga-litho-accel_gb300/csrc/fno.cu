@@ -276,14 +276,26 @@ __global__ void __launch_bounds__(THREADS) lift_dft_kernel(int L, int rows, cons
 // themselves are short, so the operands' way to the registers decides.  The twiddles depend on
 // neither kx nor the mask: column_tables_kernel lays them out once as the fragments a lane holds, one
 // 16-byte load each (gathered from a cosine table they took four loads, four selects and four
-// conversions).  A mask has 8 / G warps of its own: its column goes from global memory straight into
-// fragments, a step ahead of its use, each serving two row tiles, and its mixed modes stay in
-// registers for all rows of the inverse.
-// 64 masks: 142 -> 51 us a launch; 32 masks: forward 84 -> 31, backward 75 -> 36.
+// conversions).  The columns and the table stream through a ring, four steps ahead of their use (a CTA
+// meets the table once, so that its loads are L2's).  A mask has 8 / G warps of its own, its mixed modes
+// stay in their registers for all rows of the inverse.
+// 64 masks: 142 -> 48 us a launch; 32 masks: forward 84 -> 31, backward 75 -> 35 (columns straight from global
+// memory into fragments, a step ahead: 51, 31 and 36).  What is left is mostly the operands' shared-memory reads.
 // ---------------------------------------------------------------------------
 constexpr int COL_G = 4;
+constexpr int COL_ST = 5;          // ring stages, eight rows of the columns each: four of them in flight
+constexpr int CXP = 2 * C + 16;    // padded row of the ring (floats): the two rows of a fragment load miss each other's banks
 constexpr int CP = C + 8;  // padded row of the modes in shared memory: fragment loads of two rows miss each other's banks
 
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ uint32_t tf32r(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
@@ -332,70 +344,75 @@ __global__ void __launch_bounds__(THREADS, 2) column_kernel(int L, int B, const 
                                                             const uint4* __restrict__ fi) {
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* sV = reinterpret_cast<float2*>(smraw);  // [G][J][CP]
-  float2* sR = sV + G * J * CP;                   // BWD mixing: per-warp transposed R blocks
+  float2* sR = sV + G * J * CP;                   // the ring; then, BWD mixing, per-warp transposed R blocks
   constexpr int WPM = THREADS / 32 / G;           // warps of a mask
   constexpr int MT = G == 4 ? 2 : 1, NT = G == 1 ? 2 : 4;  // a warp's DFT_y tiles: MT x NT of 4 x 4
   const int kx = blockIdx.x, b0 = blockIdx.y * G, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, ri = t & 1;
   const int ng = min(G, B - b0);
   const int gi = warp / WPM, sub = warp % WPM;
-  if (gi < ng) {
+  {
     const int mt0 = G == 1 ? sub >> 1 : sub * MT, n0 = G == 1 ? 2 * (sub & 1) : 0;
-    // X[y][c].ri at y = 4 ks + t / 2 (+ 2), c = 8 n + g: a step of K
-    const float* x = reinterpret_cast<const float*>(Xin + (((size_t)(b0 + gi) * L + (t >> 1)) * M + kx) * C + 8 * n0 + g) + ri;
-    const size_t ys = (size_t)M * C * 2;
-    const uint4* af = fd + ((size_t)mt0 * (L / 4)) * 32 + lane;
-    struct Step {
-      float b[2][NT][2];
-      uint4 a[2][MT];
-    };
-    auto load = [&](Step& q, int k2) {  // K steps 2 k2, 2 k2 + 1
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const float* p = x + (size_t)(8 * k2 + 4 * k) * ys;
-#pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          q.b[k][n][0] = __ldg(p + 16 * n);
-          q.b[k][n][1] = __ldg(p + 2 * ys + 16 * n);
-        }
-#pragma unroll
-        for (int m = 0; m < MT; ++m) q.a[k][m] = __ldg(af + ((size_t)m * (L / 4) + 2 * k2 + k) * 32);
-      }
-    };
-    float d[MT][NT][4] = {};
-    auto step = [&](const Step& q) {
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          const uint32_t b0r = tf32r(q.b[k][n][0]), b1r = tf32r(q.b[k][n][1]);
-#pragma unroll
-          for (int m = 0; m < MT; ++m) mma1688(d[m][n], q.a[k][m], b0r, b1r);
-        }
-    };
-    Step q0, q1;
-    load(q0, 0);
+    // steps of eight rows (two K steps) of every mask's column and the table's fragments for them, through
+    // one ring of the CTA
+    constexpr int XS = 8 * CXP;                       // floats of a mask's step
+    constexpr int STEP = G * XS + 2 * 4 * 128;        // and the table's: [K step][row tile][lane] x 16 bytes
+    float* ring = reinterpret_cast<float*>(sV + G * J * CP);
+    const float2* x = Xin + ((size_t)b0 * L * M + kx) * C;
     const int N2 = L / 8;
-    for (int k2 = 0; k2 < N2; k2 += 2) {
-      load(q1, k2 + 1);
-      step(q0);
-      if (k2 + 2 < N2) load(q0, k2 + 2);
-      step(q1);
+    auto copy = [&](int k2) {
+      if (k2 < N2) {
+        float* st = ring + (k2 % COL_ST) * STEP;
+        for (int i = tid; i < 128 * ng; i += THREADS) {  // 16-byte pieces: mask i / 128, its row i / 16 % 8
+          const int m = i >> 7, r = (i >> 4) & 7, q = i & 15;
+          cp_async16(smem_u32(st + m * XS + r * CXP + 4 * q), x + ((size_t)m * L + 8 * k2 + r) * M * C + 2 * q);
+        }
+        const int k = tid >> 7, m = (tid >> 5) & 3;
+        cp_async16(smem_u32(st + G * XS + 4 * tid), fd + ((size_t)m * (L / 4) + 2 * k2 + k) * 32 + lane);
+      }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int k2 = 0; k2 < COL_ST - 1; ++k2) copy(k2);
+    float d[MT][NT][4] = {};
+    for (int k2 = 0; k2 < N2; ++k2) {
+      cp_async_wait<COL_ST - 2>();
+      __syncthreads();  // the step is there; the one before is read
+      copy(k2 + COL_ST - 1);
+      const float* st = ring + (k2 % COL_ST) * STEP;
+      // X[y][c].ri at y = 4 ks + t / 2 (+ 2), c = 8 n + g
+      const float* b = st + gi * XS + (t >> 1) * CXP + 2 * (8 * n0 + g) + ri;
+      const uint4* af = reinterpret_cast<const uint4*>(st + G * XS) + 32 * mt0 + lane;
+      if (gi < ng) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          uint4 A[MT];
+#pragma unroll
+          for (int m = 0; m < MT; ++m) A[m] = af[128 * k + 32 * m];
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            const uint32_t b0r = tf32r(b[4 * k * CXP + 16 * n]), b1r = tf32r(b[(4 * k + 2) * CXP + 16 * n]);
+#pragma unroll
+            for (int m = 0; m < MT; ++m) mma1688(d[m][n], A[m], b0r, b1r);
+          }
+        }
+      }
     }
     // D rows m = 16 mt + g (+8) = 2j + ro, cols c
+    if (gi < ng)
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      const int j = 8 * (mt0 + m) + (g >> 1), ro = g & 1;
-      float* v = reinterpret_cast<float*>(sV + ((size_t)gi * J + j) * CP) + ro;
+      for (int m = 0; m < MT; ++m) {
+        const int j = 8 * (mt0 + m) + (g >> 1), ro = g & 1;
+        float* v = reinterpret_cast<float*>(sV + ((size_t)gi * J + j) * CP) + ro;
 #pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        const int c = 8 * (n0 + n) + 2 * t;
-        v[2 * c] = d[m][n][0];
-        v[2 * c + 2] = d[m][n][1];
-        v[4 * CP * 2 + 2 * c] = d[m][n][2];
-        v[4 * CP * 2 + 2 * c + 2] = d[m][n][3];
+        for (int n = 0; n < NT; ++n) {
+          const int c = 8 * (n0 + n) + 2 * t;
+          v[2 * c] = d[m][n][0];
+          v[2 * c + 2] = d[m][n][1];
+          v[4 * CP * 2 + 2 * c] = d[m][n][2];
+          v[4 * CP * 2 + 2 * c + 2] = d[m][n][3];
+        }
       }
-    }
   }
   __syncthreads();
   if (modes_out)
@@ -423,7 +440,7 @@ __global__ void __launch_bounds__(THREADS, 2) column_kernel(int L, int B, const 
       __syncwarp();
     }
     // FWD: U[o] = s sum_c R[c][o] V[c]; BWD: gV[c] = s sum_o conj(R[c][o]) gU[o], lane = c
-#pragma unroll 4
+#pragma unroll 8
     for (int c = 0; c < C; c += 2) {
       const float2 ra = BWD ? sRt[c * (C + 1) + lane] : Rj[c * C + lane];
       const float2 rb = BWD ? sRt[(c + 1) * (C + 1) + lane] : Rj[(c + 1) * C + lane];
@@ -460,15 +477,24 @@ __global__ void __launch_bounds__(THREADS, 2) column_kernel(int L, int B, const 
       for (int h = 0; h < 2; ++h)
         bf[ks][n][h] = reinterpret_cast<const uint32_t*>(
             sV + ((size_t)gi * J + 4 * ks + (t >> 1) + 2 * h) * CP + 8 * n + g)[ri];
-  for (int mt = sub; mt < L / 8; mt += WPM) {
-    const int y = 8 * mt + (g >> 1), ro = g & 1;  // rows g, g + 8 -> y, y + 4
-    const uint4* af = fi + (size_t)mt * 256 + lane;
+  const int ntile = (L / 8 - sub + WPM - 1) / WPM;
+  uint4 A[2][4];  // half a tile's table fragments, and the next half's
+  auto load_a = [&](uint4* q, int i, int h) {
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) q[ks] = __ldg(fi + (size_t)(sub + WPM * i) * 256 + 32 * (4 * h + ks) + lane);
+  };
+  load_a(A[0], 0, 0);
+  for (int i = 0; i < ntile; ++i) {
+    const int y = 8 * (sub + WPM * i) + (g >> 1), ro = g & 1;  // rows g, g + 8 -> y, y + 4
     float d[4][4] = {};
 #pragma unroll
-    for (int ks = 0; ks < J / 4; ++ks) {
-      const uint4 a = __ldg(af + 32 * ks);
+    for (int h = 0; h < 2; ++h) {
+      if (h == 0) load_a(A[1], i, 1);
+      else if (i + 1 < ntile) load_a(A[0], i + 1, 0);
 #pragma unroll
-      for (int n = 0; n < 4; ++n) mma1688(d[n], a, bf[ks][n][0], bf[ks][n][1]);
+      for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) mma1688(d[n], A[h][ks], bf[4 * h + ks][n][0], bf[4 * h + ks][n][1]);
     }
     // lanes g (re) and g ^ 1 (im) hold channels c, c + 1 of one row: each takes one of the two whole
     float2* go = Gout + (((size_t)(b0 + gi) * L + y) * M + kx) * C + 2 * t + ro;
@@ -483,7 +509,8 @@ __global__ void __launch_bounds__(THREADS, 2) column_kernel(int L, int B, const 
 }
 
 size_t column_smem(int G, bool bwd) {
-  return ((size_t)G * J * CP + (bwd ? (THREADS / 32) * C * (C + 1) : 0)) * sizeof(float2);
+  const size_t rings = (size_t)COL_ST * (G * 8 * CXP + 1024) / 2, r = bwd ? (size_t)(THREADS / 32) * C * (C + 1) : 0;
+  return ((size_t)G * J * CP + std::max(rings, r)) * sizeof(float2);
 }
 
 // ---------------------------------------------------------------------------
@@ -495,7 +522,6 @@ size_t column_smem(int G, bool bwd) {
 __device__ __forceinline__ uint32_t tile_off(int px, int chunk) {
   return (uint32_t)(px * 64 + ((chunk ^ ((px >> 1) & 3)) << 4));
 }
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ldsm4(uint32_t* r, uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -512,14 +538,6 @@ __device__ __forceinline__ void stsm4(uint32_t addr, uint32_t r0, uint32_t r1, u
   asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(r0), "r"(r1),
                "r"(r2), "r"(r3)
                : "memory");
-}
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 // A fragment of pixels 16 mt .. + 15, channels 16 ks .. + 15; also the place of a C-layout pair of n tiles
 // 2 ks, 2 ks + 1 (stsm4) with the lane's row and chunk
