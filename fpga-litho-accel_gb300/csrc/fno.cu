@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(THREADS) lift_dft_kernel(int L, int rows, cons
                                                            const float2* __restrict__ twL, float2* __restrict__ Xf,
                                                            float2* __restrict__ Mrow) {
   extern __shared__ __align__(16) unsigned char smraw[];
+  early_next();
   float2* sTw = reinterpret_cast<float2*>(smraw);
   for (int i = threadIdx.x; i < L; i += THREADS) sTw[i] = twL[i];
   __syncthreads();
@@ -350,6 +351,8 @@ __global__ void __launch_bounds__(THREADS, 2) column_kernel(int L, int B, const 
   const int kx = blockIdx.x, b0 = blockIdx.y * G, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, ri = t & 1;
   const int ng = min(G, B - b0);
+  early_next();
+  early_wait(Xin);
   const int gi = warp / WPM, sub = warp % WPM;
   {
     const int mt0 = G == 1 ? sub >> 1 : sub * MT, n0 = G == 1 ? 2 * (sub & 1) : 0;
@@ -715,6 +718,9 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS) row_fwd_kernel(const RowFwd
   const float q2b = th[Off::q2b];
 
   // the next row's inputs: zin into the tile of its parity, the rest into registers
+  early_next();
+  const bf16* __restrict__ zin = a.zin;
+  const float2* __restrict__ Gy = a.Gy;
   float mr[MAXT][2];
   float2 gr[2];
   auto load_row = [&](int row, int st) {
@@ -728,12 +734,14 @@ __global__ void __launch_bounds__(THREADS, FWD_CTAS) row_fwd_kernel(const RowFwd
         }
       }
     } else {
-      tile_load(smem_u32(smraw + S.sZ) + st * L * C * 2, a.zin + (size_t)row * L * C, L, tid);
+      tile_load(smem_u32(smraw + S.sZ) + st * L * C * 2, zin + (size_t)row * L * C, L, tid);
     }
-    const float2* gp = a.Gy + (size_t)row * M * C;
+    const float2* gp = Gy + (size_t)row * M * C;
     gr[0] = __ldg(gp + tid);
     gr[1] = __ldg(gp + tid + THREADS);
   };
+  early_wait(zin);  // (the prologue reads parameters and tables alone)
+  early_wait(Gy);
   if (blockIdx.x < a.rows) load_row(blockIdx.x, 0);
   cp_async_commit();
 
@@ -903,6 +911,8 @@ size_t row_fwd_smem(int L, bool final_) { return FwdSmem(L, final_).total; }
 constexpr int LOSS_SHARES = 16;
 __global__ void __launch_bounds__(THREADS) loss_part_kernel(int L, const float* __restrict__ out,
                                                             const float* __restrict__ tgt, double2* __restrict__ part) {
+  early_next();
+  early_wait(out);
   const size_t b = blockIdx.x / LOSS_SHARES, n = (size_t)L * L;
   const int sh = blockIdx.x % LOSS_SHARES;
   const float* o = out + b * n;
@@ -931,6 +941,7 @@ __global__ void __launch_bounds__(THREADS) loss_part_kernel(int L, const float* 
 }
 __global__ void loss_kernel(int B, const double2* __restrict__ part, float* __restrict__ loss_b, float* __restrict__ coef) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  early_wait(part);
   if (b >= B) return;
   double a = 0.0, c = 0.0;
 #pragma unroll
@@ -1083,12 +1094,15 @@ __global__ void __launch_bounds__(THREADS, 2) row_bwd_kernel(const RowBwd a) {
   float vw[4][2] = {};                 // dPw (LIFT)
   float dW[4] = {0.f, 0.f, 0.f, 0.f};  // the warp's 16 x 8 tile of dW_l
 
+  early_next();
+  const bf16 *__restrict__ gvin = a.gvin, *__restrict__ zl = a.zl, *__restrict__ zlm1 = a.zlm1;
+  const float2* __restrict__ Gg = a.Gg;
   float mr[MAXT][2];
   float2 gr[2];
   const bool masks = !SPEC || l == 0;
   auto load_row = [&](int row, int st) {  // all but z_l
-    tile_load(smem_u32(smraw + S.sGv) + st * (uint32_t)tile, a.gvin + (size_t)row * L * C, L, tid);
-    if (SPEC && l > 0) tile_load(smem_u32(smraw + S.sV) + st * (uint32_t)tile, a.zlm1 + (size_t)row * L * C, L, tid);
+    tile_load(smem_u32(smraw + S.sGv) + st * (uint32_t)tile, gvin + (size_t)row * L * C, L, tid);
+    if (SPEC && l > 0) tile_load(smem_u32(smraw + S.sV) + st * (uint32_t)tile, zlm1 + (size_t)row * L * C, L, tid);
     if (masks)
 #pragma unroll
       for (int i = 0; i < MAXT; ++i)
@@ -1096,13 +1110,17 @@ __global__ void __launch_bounds__(THREADS, 2) row_bwd_kernel(const RowBwd a) {
           mr[i][0] = __ldg(a.masks + (size_t)row * L + 16 * (warp + 8 * i) + g);
           mr[i][1] = __ldg(a.masks + (size_t)row * L + 16 * (warp + 8 * i) + g + 8);
         }
-    const float2* gp = a.Gg + (size_t)row * M * C;
+    const float2* gp = Gg + (size_t)row * M * C;
     gr[0] = __ldg(gp + tid);
     gr[1] = __ldg(gp + tid + THREADS);
   };
   auto load_z = [&](int row) {
-    if (SPEC) tile_load(smem_u32(smraw + S.sZ), a.zl + (size_t)row * L * C, L, tid);
+    if (SPEC) tile_load(smem_u32(smraw + S.sZ), zl + (size_t)row * L * C, L, tid);
   };
+  early_wait(gvin);  // (the prologue reads parameters and tables alone)
+  early_wait(zl);
+  early_wait(zlm1);
+  early_wait(Gg);
   if (blockIdx.x < a.rows) {
     load_row(blockIdx.x, 0);
     load_z(blockIdx.x);
@@ -1281,6 +1299,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) row_bwd_proj_kernel(const Row
   float* sq = reinterpret_cast<float*>(smraw + S.sq);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int hh = warp & 1, pair = warp >> 1;  // half of the hidden channels; tiles pair, pair + 8
+  early_next();
   const float* th = a.theta;
   for (int i = tid; i < J * L / 2; i += PROJ_THREADS) {
     const int k = i / (L / 2), px = 2 * (i % (L / 2));
@@ -1535,6 +1554,9 @@ __global__ void __launch_bounds__(THREADS) dR_kernel(int L, int B, int layer, co
   const int jk = blockIdx.x, tid = threadIdx.x;  // jk = j * M + kx
   const int kx = jk % M, lane = tid & 31, warp = tid >> 5;
   __shared__ float2 su[DR_MASKS][C], sv[DR_MASKS][C];
+  early_next();
+  early_wait(gU);
+  early_wait(V);
   float2 acc[4] = {};  // c = warp + 8 r, o = lane
   for (int b0 = 0; b0 < B; b0 += DR_MASKS) {
     const int nb = min(DR_MASKS, B - b0);
@@ -1631,9 +1653,11 @@ __global__ void rect_masks_kernel(uint64_t seed, long long first, int L, int nmi
 __global__ void __launch_bounds__(THREADS) band_rows_kernel(int L, int rows, int KB, const float* __restrict__ img,
                                                             const float2* __restrict__ twL, float2* __restrict__ Xb) {
   extern __shared__ __align__(16) unsigned char smraw[];
+  early_next();
   float2* sTw = reinterpret_cast<float2*>(smraw);
   for (int i = threadIdx.x; i < L; i += THREADS) sTw[i] = twL[i];
   __syncthreads();
+  early_wait(img);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = (blockIdx.x * (THREADS / 32) + warp) * DR, n = min(DR, rows - row0);
   if (n <= 0) return;
@@ -1650,6 +1674,8 @@ __global__ void __launch_bounds__(THREADS) band_rows_kernel(int L, int rows, int
 __global__ void __launch_bounds__(THREADS) band_coef_kernel(int L, int KB, int KBy, const float2* __restrict__ Xb,
                                                             const float2* __restrict__ twL, float2* __restrict__ Cb) {
   __shared__ float2 part[THREADS / 16][16];
+  early_next();
+  early_wait(Xb);
   const int b = blockIdx.y, kyi = blockIdx.x, ky = kyi - KBy, kx = threadIdx.x & 15, sh = threadIdx.x >> 4;
   float re = 0.f, im = 0.f;
   if (kx <= KB) {
@@ -1684,6 +1710,8 @@ __global__ void __launch_bounds__(THREADS) band_synth_kernel(int L, int rows, in
   constexpr int MAXI = 256 / 32;
   for (int i = threadIdx.x; i < L; i += THREADS) sTw[i] = twL[i];
   __syncthreads();
+  early_next();
+  early_wait(Cb);
   const int row = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const int b = row / L, y = row % L, nky = 2 * KBy + 1, kx = lane & 15;
@@ -1765,6 +1793,9 @@ __global__ void __launch_bounds__(LOWQ_THREADS) lowq_est_kernel(int L, int Nx, i
   __shared__ float2 sM[33 * 33];
   __shared__ float2 part[5][64];
   __shared__ double en;
+  early_wait(Cm);
+  early_wait(Cb);
+  early_wait(Enew);
   for (int i = tid; i < KD; i += blockDim.x) {
     const int v = i / KX - Ny, u = i % KX - Nx;
     float2 m;
@@ -1875,9 +1906,8 @@ int launch_column(litho_fno* f, int B, int layer, const float2* Xin, float2* Gou
     const size_t smem = column_smem(G, BWD);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<dim3(M, (B + G - 1) / G), THREADS, smem, ctx->stream>>>(f->L, B, f->theta.as<float>(), layer, Xin, Gout, modes_out,
-                                                               f->colF.as<uint4>(), f->colI.as<uint4>());
-    return cudaGetLastError();
+    return launch_early(true, k, dim3(M, (B + G - 1) / G), THREADS, smem, ctx->stream, f->L, B, f->theta.as<float>(), layer,
+                        Xin, Gout, modes_out, f->colF.as<uint4>(), f->colI.as<uint4>());
   };
   const int want = 3 * ctx->sm_count / 2;
   cudaError_t e;
@@ -1919,9 +1949,8 @@ int launch_band_coef(litho_fno* f, int KB, int KBy, int batch, const float2* X, 
   litho_ctx* ctx = f->ctx;
   const int nky = 2 * KBy + 1;
   for (int b = 0; b < batch; b += 65535) {
-    band_coef_kernel<<<dim3(nky, std::min(65535, batch - b)), THREADS, 0, ctx->stream>>>(
-        f->L, KB, KBy, X + (size_t)b * f->L * 16, f->twL.as<float2>(), Cb + (size_t)b * nky * 16);
-    LITHO_CUDA_TRY(ctx, cudaGetLastError());
+    LITHO_CUDA_TRY(ctx, launch_early(true, band_coef_kernel, dim3(nky, std::min(65535, batch - b)), THREADS, 0, ctx->stream, f->L,
+                                     KB, KBy, X + (size_t)b * f->L * 16, f->twL.as<float2>(), Cb + (size_t)b * nky * 16));
   }
   return LITHO_OK;
 }
@@ -1931,7 +1960,10 @@ int set_smem(litho_ctx* ctx, const void* fn, size_t bytes) {
   return LITHO_OK;
 }
 
-// forward pass over B masks; train keeps z_l and V_l for the backward pass
+// forward pass over B masks; train keeps z_l and V_l for the backward pass.  From the second kernel on
+// each is launched early, here and in the passes below: it loads its tables and weights while the one
+// before it ends, and waits before it touches anything a pass writes (64 masks of 256 x 256, predict:
+// 1,000 -> 959 us; 32, loss and gradients: 1,910 -> 1,847).
 int forward(litho_fno* f, const float* masks, int B, bool train, float* images, float2* Mrow = nullptr) {
   litho_ctx* ctx = f->ctx;
   const int L = f->L, rows = B * L;
@@ -1957,11 +1989,11 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
     a.out = images;
     a.Ttab = f->Ttab.as<bf16>(); a.TT = f->TT.as<bf16>();
     if (l == 0)
-      row_fwd_kernel<FWD_FIRST><<<grid, THREADS, row_fwd_smem(L, false), ctx->stream>>>(a);
+      LITHO_CUDA_TRY(ctx, launch_early(true, row_fwd_kernel<FWD_FIRST>, dim3(grid), THREADS, row_fwd_smem(L, false), ctx->stream, a));
     else if (l < NL - 1)
-      row_fwd_kernel<FWD_MID><<<grid, THREADS, row_fwd_smem(L, false), ctx->stream>>>(a);
+      LITHO_CUDA_TRY(ctx, launch_early(true, row_fwd_kernel<FWD_MID>, dim3(grid), THREADS, row_fwd_smem(L, false), ctx->stream, a));
     else
-      row_fwd_kernel<FWD_LAST><<<grid, THREADS, row_fwd_smem(L, true), ctx->stream>>>(a);
+      LITHO_CUDA_TRY(ctx, launch_early(true, row_fwd_kernel<FWD_LAST>, dim3(grid), THREADS, row_fwd_smem(L, true), ctx->stream, a));
   }
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
@@ -1969,9 +2001,11 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
 
 cudaError_t launch_loss(litho_fno* f, const float* targets, int B) {
   cudaStream_t s = f->ctx->stream;
-  loss_part_kernel<<<(unsigned)B * LOSS_SHARES, THREADS, 0, s>>>(f->L, f->out.as<float>(), targets, f->lossp.as<double2>());
-  loss_kernel<<<(B + 31) / 32, 32, 0, s>>>(B, f->lossp.as<double2>(), f->lossb.as<float>(), f->coef.as<float>());
-  return cudaGetLastError();
+  const cudaError_t e = launch_early(true, loss_part_kernel, dim3((unsigned)B * LOSS_SHARES), THREADS, 0, s, f->L,
+                                     f->out.as<float>(), targets, f->lossp.as<double2>());
+  if (e != cudaSuccess) return e;
+  return launch_early(true, loss_kernel, dim3((B + 31) / 32), 32, 0, s, B, f->lossp.as<double2>(), f->lossb.as<float>(),
+                      f->coef.as<float>());
 }
 
 // loss (device, per mask) + gradient into f->grad
@@ -2004,15 +2038,15 @@ int backward(litho_fno* f, const float* masks, const float* targets, int B) {
     if (l == NL - 1)
       row_bwd_proj_kernel<<<std::min(rows, ctx->sm_count), PROJ_THREADS, sp.total, ctx->stream>>>(a);
     else
-      row_bwd_kernel<HEAD_SPEC><<<grid, THREADS, ss.total, ctx->stream>>>(a);
+      LITHO_CUDA_TRY(ctx, launch_early(true, row_bwd_kernel<HEAD_SPEC>, dim3(grid), THREADS, ss.total, ctx->stream, a));
     LITHO_RET(launch_column<true>(f, B, l, Xg, Gg, f->gU.as<float2>()));
-    dR_kernel<<<J * M, THREADS, 0, ctx->stream>>>(L, B, l, f->gU.as<float2>(), f->Vs[l].as<float2>(),
-                                                  f->grad.as<float>());
+    LITHO_CUDA_TRY(ctx, launch_early(true, dR_kernel, dim3(J * M), THREADS, 0, ctx->stream, L, B, l, f->gU.as<float2>(),
+                                     f->Vs[l].as<float2>(), f->grad.as<float>()));
     cur ^= 1;
   }
   a.layer = 0;
   a.gvin = f->gv[cur ^ 1].as<bf16>();
-  row_bwd_kernel<HEAD_LIFT><<<grid, THREADS, sl.total, ctx->stream>>>(a);
+  LITHO_CUDA_TRY(ctx, launch_early(true, row_bwd_kernel<HEAD_LIFT>, dim3(grid), THREADS, sl.total, ctx->stream, a));
   reduce_dense_kernel<<<(Dn::N + 255) / 256, 256, 0, ctx->stream>>>(f->gpart.as<float>(), grid,
                                                                     f->grad.as<float>());
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
@@ -2028,11 +2062,11 @@ int project(litho_fno* f, int Nx, int Ny, float* images, int batch) {
   LITHO_RET(f->Enew.ensure(ctx, (size_t)rows * sizeof(float)));
   LITHO_RET(f->Cb.ensure(ctx, (size_t)batch * (2 * KBy + 1) * 16 * sizeof(float2)));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 3);
-  band_rows_kernel<<<dft_blocks(rows), THREADS, rows_dft_smem(L), ctx->stream>>>(L, rows, KB, images, f->twL.as<float2>(),
-                                                                                f->Xb.as<float2>());
+  LITHO_CUDA_TRY(ctx, launch_early(true, band_rows_kernel, dim3(dft_blocks(rows)), THREADS, rows_dft_smem(L), ctx->stream, L,
+                                   rows, KB, images, f->twL.as<float2>(), f->Xb.as<float2>()));
   LITHO_RET(launch_band_coef(f, KB, KBy, batch, f->Xb.as<float2>(), f->Cb.as<float2>()));
-  band_synth_kernel<<<(rows + 7) / 8, THREADS, 0, ctx->stream>>>(L, rows, KB, KBy, f->Cb.as<float2>(), f->twL.as<float2>(),
-                                                                 images, f->Eres.as<float>(), f->Enew.as<float>());
+  LITHO_CUDA_TRY(ctx, launch_early(true, band_synth_kernel, dim3((rows + 7) / 8), THREADS, 0, ctx->stream, L, rows, KB, KBy,
+                                   f->Cb.as<float2>(), f->twL.as<float2>(), images, f->Eres.as<float>(), f->Enew.as<float>()));
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
 }
@@ -2048,8 +2082,9 @@ int predict(litho_fno* f, const litho_kernel_set* ks, const float* masks, int ba
   LITHO_RET(project(f, ks->Nx, ks->Ny, images, batch));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 2);
   LITHO_RET(launch_band_coef(f, ks->Nx, ks->Ny, batch, f->Mrow.as<float2>(), f->Cm.as<float2>()));
-  lowq_est_kernel<<<batch, LOWQ_THREADS, 0, ctx->stream>>>(L, ks->Nx, ks->Ny, f->Cm.as<float2>(), f->Cb.as<float2>(), ks->krn,
-                                                  ks->scales, ks->nk, f->Enew.as<float>(), f->est_alpha, est);
+  LITHO_CUDA_TRY(ctx, launch_early(true, lowq_est_kernel, dim3(batch), LOWQ_THREADS, 0, ctx->stream, L, ks->Nx, ks->Ny,
+                                   f->Cm.as<float2>(), f->Cb.as<float2>(), ks->krn, ks->scales, ks->nk, f->Enew.as<float>(),
+                                   f->est_alpha, est));
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
 }
