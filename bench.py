@@ -8,8 +8,8 @@ eigensolver for a quasar source (4 poles at 45/135/225/315 deg, sigma 0.7-0.9,
 ~2000 lit points), NA 0.8, lambda 193 nm, defocus 0.  B=1024 masks are 4 GiB in
 and 4 GiB out per step, far larger than the 129 MB L2, so no flush is needed.
 Smaller steps pay a fixed per-step cost (the previous step's image writes still
-dirty in L2, kernel ramps, tails and launch gaps) over fewer masks: 256 masks per
-step run at ~0.9 of the 1024-mask throughput, 64 masks at ~0.75.
+dirty in L2, kernel ramps and tails) over fewer masks: 256 masks per step run at
+~0.9 of the 1024-mask throughput, 64 masks at ~0.64.
 
   value : images/s with masks resident in HBM (litho_image_batch on device
           pointers), timed with CUDA events over K steps on the library's stream.
@@ -43,13 +43,13 @@ sys.path.insert(0, os.path.join(ROOT, "fpga-litho-accel_gb300"))
 
 METRIC = "aerial images/s at 1024^2 K=24: mixed/batched/surrogate vs plain GPU at stated rel-L2"
 L_SIZE, K_KERNELS, NA, WAVELENGTH, DEFOCUS = 1024, 24, 0.8, 193.0, 0.0
-# DRAM bytes (read + write) per mask of the mixed form's two HBM-bound kernels, from an
-# ncu capture of one launch of each on 48 masks of this workload (the traffic scales with
-# the masks).  The FI kernel's figure is what DRAM saw during its launch: part of its
-# image writes is still in L2 when it ends and drains during the next launch.
-TRAFFIC_PER_IMAGE = {("mixed", "win_dft"): (201.65e6 + 3.31e6) / 48,
-                     ("mixed", "fi_out"): (13.07e6 + 140.29e6) / 48}
-TRAFFIC_KERNEL = {"win_dft": "win_dft_tc", "fi_out": "fi_tc"}
+# DRAM bytes (read + write) per mask of the two HBM-bound kernels (both forms run them at
+# this support), from an ncu capture of one launch of each on 48 masks of this workload (the
+# traffic scales with the masks).  The FI kernel's figure is what DRAM saw during its launch:
+# part of its image writes is still in L2 when it ends and drains during the next launch.
+TRAFFIC_PER_IMAGE = {(form, stage): b / 48 for form in ("mixed", "plain")
+                     for stage, b in (("win_dft", 201.46e6 + 3.90e6), ("fi_out", 6.55e6 + 139.85e6))}
+TRAFFIC_KERNEL = {"win_dft": "win_fold", "fi_out": "fi_fold"}
 WORKLOAD = ("1024x1024 float32 Manhattan masks (L/S + contacts, ~50% density), K=24 SOCS kernels from a "
             "~2000-point quasar source (sigma 0.7-0.9), NA 0.8, 193 nm; fixed kernels, batch of masks per step")
 
@@ -140,7 +140,7 @@ def bench_config(nx, npts, batch, form):
     gib = batch * 4 * L_SIZE * L_SIZE / 2 ** 30
     return {"workload": WORKLOAD, "L": L_SIZE, "K": K_KERNELS, "Nx": nx, "source_points": npts,
             "batch_per_step": batch, "form": form,
-            "forms": "mixed = split-BF16 tcgen05 TCC + FP64 eigensolve + split-TF32 tcgen05 DFTs; "
+            "forms": "mixed = split-BF16 tcgen05 TCC + FP64 eigensolve + folded FP32 DFTs; "
                      "plain = FP64 TCC + FP64 eigensolve + FP32 CUDA-core DFTs; both FP32 FFTs",
             "l2": f"inputs larger than L2 ({gib:g} GiB in + {gib:g} GiB out per step), no flush"}
 
@@ -619,8 +619,7 @@ def main():
     value = job_images_per_s(ws, B, args.steps, ms / 1e3)
     value_o = job_images_per_s(ws, B, args.steps, ms_o / 1e3)
     launches = sum(n for _, n in st_v.values())
-    # the same masks as 8-bit grey levels / 255 (the reference's PNG-mask convention): no tile of
-    # these is exact in TF32, so the mixed window DFT runs its residual products on every tile
+    # the same masks as 8-bit grey levels / 255 (the reference's PNG-mask convention)
     grey = grey_levels(masks)
     for _ in range(3):
         step("mixed", grey)
@@ -686,7 +685,7 @@ def main():
                      "stage_ms_per_step_serial": {s: st_o[s][0] / ksteps for s in names}}}
     line = {"metric": METRIC, "value": value, "unit": "images/s", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "tf32x3/f32" if head == "mixed" else "f32", "data": "synthetic",
+            "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": bench_config(nx, npts, B, head),
             "gpu_launches": int(launches),
             "forms": forms,

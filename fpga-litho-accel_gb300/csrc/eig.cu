@@ -24,13 +24,14 @@
 //                           shared memory;
 //      cluster_rr_kernel    inside each cluster of close eigenvalues (a symmetric
 //                           source gives exact degenerate pairs) the vectors are
-//                           orthonormalised (Gram-Schmidt, twice) and rotated by
+//                           orthonormalised (Cholesky QR, twice) and rotated by
 //                           a Rayleigh-Ritz step on the cluster's subspace
 //                           (Jacobi eigendecomposition of Z^T T Z);
 //   5. backtransform_kernel y = H_0 H_1 ... H_{n-2} z;
 //   6. output_kernel        scales[i] = lambda_i (descending) and
 //                           krn[i][j] = y_i[n-1-j] (litho.cpp:626-634 reversal).
-// No kernel waits on another; every step is a separate launch on the stream.
+// No kernel waits on another; every step is a separate launch on the stream (tridiag_kernel's CTAs wait
+// on one another inside their cooperative launch, each time with a limit).
 #include "litho_internal.cuh"
 #include "tc_common.cuh"
 
