@@ -12,7 +12,7 @@
 // bound by the FP32 pipe and by shared-memory reads), so up to Ny = 8 the 4 bytes per pixel of
 // HBM bound both: 1024 masks of 1024^2 (4 GiB each way) measured 1172 -> 639 us (6.7 TB/s) for the
 // window and 1299 -> 639 us for the image, 40 grey masks of 777 x 913 (rows at any alignment)
-// 90 -> 44 and 51 -> 35 us.  At Ny = 16 the FMAs bound the image (44 of 2048^2: 195 us, 3.8 TB/s).
+// 90 -> 34 and 51 -> 30 us.  At Ny = 16 the FMAs bound the image (44 of 2048^2: 195 us, 3.8 TB/s).
 // Scalar FMAs: packed (f32x2) ones gave no higher rate here and cost register moves.
 #include "litho_internal.cuh"
 #include "fold.hpp"
