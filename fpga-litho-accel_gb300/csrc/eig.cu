@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(256) her2_kernel(double2* __restrict__ A, int 
 // ---------------------------------------------------------------------------
 constexpr int TD_WARPS = 8, TD_THREADS = 32 * (TD_WARPS + 1);
 constexpr int TD_MAX_ROWS = 16;
+constexpr size_t TD_MAX_SMEM = 224 * 1024;
 
 size_t tridiag_smem(int n, int G) {
   return ((size_t)((n + G - 1) / G) * n + 3 * (size_t)n) * sizeof(double2);
@@ -1406,7 +1407,7 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
     const int iv_launches = iv_in_smem ? 1 : (nk + IV_CHUNK - 1) / IV_CHUNK;
     const int G = std::min(n, ctx->sm_count);
     const size_t td_smem = tridiag_smem(n, G);
-    const bool coop = n > 1 && td_smem <= 224 * 1024 && (n + G - 1) / G <= TD_MAX_ROWS;
+    const bool coop = n > 1 && td_smem <= TD_MAX_SMEM && (n + G - 1) / G <= TD_MAX_ROWS;
     StageScope sc(ctx, LITHO_STAGE_EIG, (coop ? 1 : 2 * n) + 4 + (wy_blocks > 0 ? 1 : 0) + iv_launches);
     hermitize_kernel<<<dim3((n + 127) / 128, n), 128, 0, ctx->stream>>>(static_cast<const double2*>(dtcc), A, n);
     LITHO_CUDA_TRY(ctx, cudaGetLastError());
@@ -1416,8 +1417,9 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
       LITHO_RET(tc_err_flag_public(ctx, &err));
       unsigned* count = reinterpret_cast<unsigned*>(td_part + 2 * G);
       LITHO_CUDA_TRY(ctx, cudaMemsetAsync(count, 0, sizeof(unsigned), ctx->stream));
+      // the limit, not this matrix's size: the attribute is shared by every thread that solves
       LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)td_smem));
+                                               (int)TD_MAX_SMEM));
       const double2* Ac = A;
       double2 *xg = td_vec, *rowbuf = td_vec + 2 * (size_t)n;
       int nn_ = n;
@@ -1458,7 +1460,7 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
     const int bc = std::max(1, std::min({BK_CMAX, ctx->sm_count * 4 / 5 / nk, (n + 31) / 32}));
     const size_t bt_smem = backtransform_smem(n, bc);
     LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(backtransform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)bt_smem));
+                                             (int)backtransform_smem(8192, 1)));  // the largest (every thread's)
     LITHO_CUDA_TRY(ctx, launch_clusters(backtransform_kernel, nk, bc, WY_THREADS, bt_smem, ctx->stream, cvpack, n, cTg,
                                         (const double*)Z, Y));
     LITHO_CUDA_TRY(ctx, cudaGetLastError());
