@@ -36,15 +36,17 @@ __device__ __forceinline__ int4 fold_offsets(int b, int Lx, int Ly, int Fy) {
 // ---------------------------------------------------------------------------
 // window DFT
 // ---------------------------------------------------------------------------
-// Template support: 2NY+1 sums per column.  Four columns per lane up to NY = 8 (68 accumulator
-// registers); two above (NY = 16: 66).
-constexpr int wf_cpl(int NY) { return NY <= 8 ? 4 : 2; }
+// Template support: 2NY+1 sums per column.  Four columns per lane, so that a coefficient read (a broadcast
+// takes shared memory a wavefront per word) serves four: 68 accumulator registers at NY = 8, in two CTAs of
+// eight warps per SM; 132 at NY = 16, in two of four warps with a deeper ring.  (Two columns per lane and eight
+// warps above NY = 8: 16 masks of 1999 x 2001 254 us, now 227; 200 of 1280^2 1,050, now 957; 100 of
+// 1100^2 487, now 438; 10 of 2048^2 147, now 130; one 55.7, now 60.)
+constexpr int wf_cpl(int) { return 4; }
 constexpr int wf_stride(int NY) { return 2 * NY; }
-constexpr int WF_WARPS = 8, WF_THREADS = 32 * WF_WARPS;
-constexpr int WF_ST = 4;  // ring stages: three base rows (6 KB) of every warp in flight
-constexpr int WF_AHEAD = (WF_ST - 1) * WF_WARPS;
+constexpr int wf_warps(int NY) { return NY <= 8 ? 8 : 4; }
+constexpr int wf_st(int NY) { return NY <= 8 ? 4 : 8; }  // ring stages: three, seven base rows (2 KB each) of every warp in flight
 // base rows whose coefficients and row offsets are staged at a time
-constexpr int wf_stage(int NY) { return 40 * 1024 / (wf_stride(NY) * 4 + 16) / WF_WARPS * WF_WARPS; }
+constexpr int wf_stage(int NY) { return (NY <= 8 ? 40 : 18) * 1024 / (wf_stride(NY) * 4 + 16) / 8 * 8; }
 
 static int wf_ny(int Ny) { return Ny <= 2 ? 2 : Ny <= 4 ? 4 : Ny <= 8 ? 8 : Ny <= 12 ? 12 : Ny <= 16 ? 16 : -1; }
 
@@ -60,13 +62,14 @@ __global__ void wf_coef_kernel(float* __restrict__ coef, int nb, int NY, int Ny,
 template <int NY>
 struct WinFold {
   static constexpr int CPL = wf_cpl(NY), COLS = 32 * CPL, KS = wf_stride(NY), NR = 2 * NY + 1;
+  static constexpr int WARPS = wf_warps(NY), THREADS = 32 * WARPS, ST = wf_st(NY), AHEAD = (ST - 1) * WARPS;
   static constexpr int RB = COLS + 4;       // ring row (floats): the columns and one granule of misalignment
-  static constexpr int RING = WF_WARPS * WF_ST * 4 * RB;
+  static constexpr int RING = WARPS * ST * 4 * RB;
   static constexpr int RS = COLS + 4;       // row stride of the summed row sums (floats)
   static constexpr int TS = COLS + 2;       // row stride of the column twiddles (float2)
   static constexpr int ZERO = RB + 4;       // a row of zeros, padded to 16 bytes
-  static constexpr int RED = WF_WARPS * NR * COLS;  // floats of the warps' sums
-  static constexpr int BARS = WF_WARPS * WF_ST * 2;  // floats of the ring's barriers
+  static constexpr int RED = WARPS * NR * COLS;  // floats of the warps' sums
+  static constexpr int BARS = WARPS * ST * 2;  // floats of the ring's barriers
 };
 
 template <int NY>
@@ -74,7 +77,7 @@ static size_t win_fold_smem(int Nx, int rows) {
   using P = WinFold<NY>;
   const size_t tw = (size_t)(Nx + 1) * P::TS * 2;
   const int st = std::min(rows, wf_stage(NY));
-  const size_t loop = (size_t)P::RING + (size_t)(st + WF_AHEAD) * 4 + (size_t)st * P::KS;
+  const size_t loop = (size_t)P::RING + (size_t)(st + P::AHEAD) * 4 + (size_t)st * P::KS;
   const size_t sums = (size_t)P::RED + (size_t)P::NR * P::RS;
   return (P::BARS + P::ZERO + tw + std::max(loop, sums)) * sizeof(float);
 }
@@ -121,7 +124,7 @@ struct WinSet {
 };
 
 template <int NY, bool VEC>
-__global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_constant__ WinSet G, int Fx, int Fy, int Nx,
+__global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __grid_constant__ WinSet G, int Fx, int Fy, int Nx,
                                                                  int Ny, float2* __restrict__ win_part, int nparts,
                                                                  int stall, int* err) {
   using P = WinFold<NY>;
@@ -129,14 +132,14 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   early_next();
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm) + warp * WF_ST;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm) + warp * P::ST;
   float* zero = sm + P::BARS;
   float2* sTw = reinterpret_cast<float2*>(zero + P::ZERO);    // [Nx+1][TS]
   float* sK = zero + P::ZERO + 2 * (Nx + 1) * P::TS;          // ring, row offsets, coefficients; then the warps' sums
-  int4* sOff = reinterpret_cast<int4*>(sK + P::RING);         // [rows + WF_AHEAD]
+  int4* sOff = reinterpret_cast<int4*>(sK + P::RING);         // [rows + P::AHEAD]
   const int srows = min(G.rows, wf_stage(NY));
-  float* sCoef = sK + P::RING + 4 * (srows + WF_AHEAD);       // [rows][KS]
-  float* ring = sK + warp * (WF_ST * 4 * P::RB);
+  float* sCoef = sK + P::RING + 4 * (srows + P::AHEAD);       // [rows][KS]
+  float* ring = sK + warp * (P::ST * 4 * P::RB);
   int sz, img, cb, rs, b0, b1;
   win_tile(G.T, blockIdx.x, 1, sz, img, cb, rs, b0, b1);
   const int Lx = G.Lx[sz], Ly = G.Ly[sz];
@@ -193,21 +196,21 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
   int b = b0 + warp;
   if constexpr (VEC) {
 #pragma unroll
-    for (int k = 0; k < WF_ST - 1; ++k) {
-      const int bk = b + k * WF_WARPS;
+    for (int k = 0; k < P::ST - 1; ++k) {
+      const int bk = b + k * P::WARPS;
       issue_vec(bk < b1 ? fold_offsets(bk, Lx, Ly, Fy) : make_int4(-1, -1, -1, -1), k);
     }
   } else {
     if (lane == 0) {
-      for (int i = 0; i < WF_ST; ++i) tc::mbar_init(&bar[i], 4);  // one arrival per row
+      for (int i = 0; i < P::ST; ++i) tc::mbar_init(&bar[i], 4);  // one arrival per row
       tc::fence_mbar_init();
     }
     __syncwarp();
 #pragma unroll
-    for (int k = 0; k < WF_ST - 1; ++k) issue(offset_of(b + k * WF_WARPS), k);
-    for (int e = tid; e < P::ZERO; e += WF_THREADS) zero[e] = 0.f;
+    for (int k = 0; k < P::ST - 1; ++k) issue(offset_of(b + k * P::WARPS), k);
+    for (int e = tid; e < P::ZERO; e += P::THREADS) zero[e] = 0.f;
   }
-  for (int e = tid; e < (Nx + 1) * COLS; e += WF_THREADS) {
+  for (int e = tid; e < (Nx + 1) * COLS; e += P::THREADS) {
     const int u = e / COLS, x = e - u * COLS;
     sTw[u * P::TS + x] = x < ncol ? __ldg(twF + (size_t)u * Lx + X0 + x) : make_float2(0.f, 0.f);
   }
@@ -217,15 +220,15 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
     const int t1 = min(b1, t0 + wf_stage(NY));
     if (t0 > b0) __syncthreads();
     const float4* src = reinterpret_cast<const float4*>(coef + (size_t)t0 * KS);
-    for (int e = tid; e < (t1 - t0) * (KS / 4); e += WF_THREADS) reinterpret_cast<float4*>(sCoef)[e] = __ldg(src + e);
-    for (int e = tid; e < t1 - t0 + WF_AHEAD; e += WF_THREADS)
+    for (int e = tid; e < (t1 - t0) * (KS / 4); e += P::THREADS) reinterpret_cast<float4*>(sCoef)[e] = __ldg(src + e);
+    for (int e = tid; e < t1 - t0 + P::AHEAD; e += P::THREADS)
       sOff[e] = t0 + e < b1 ? fold_offsets(t0 + e, Lx, Ly, Fy) : make_int4(-1, -1, -1, -1);
     __syncthreads();
-    for (; b < t1; b += WF_WARPS) {
+    for (; b < t1; b += P::WARPS) {
       float p[4][CPL];
       const float* src = ring + st * (4 * P::RB);
       if constexpr (VEC) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(WF_ST - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(P::ST - 2) : "memory");
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           if constexpr (CPL == 4) {
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
             p[k][1] = v.y;
           }
         }
-        issue_vec(sOff[b - t0 + WF_AHEAD], st == 0 ? WF_ST - 1 : st - 1);  // the previous row's slot
+        issue_vec(sOff[b - t0 + P::AHEAD], st == 0 ? P::ST - 1 : st - 1);  // the previous row's slot
       } else {
         const int4 o4 = sOff[b - t0];
         const int off[4] = {o4.x, o4.y, o4.z, o4.w};
@@ -254,10 +257,10 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
           for (int i = 0; i < CPL; ++i) p[k][i] = q[lane + 32 * i];  // (past ncol: left in the ring, dropped below)
         }
         __syncwarp();  // the slot refilled below (the previous row's) has been read by every lane
-        issue(lane < 4 ? reinterpret_cast<const int*>(sOff + (b - t0 + WF_AHEAD))[lane] : -1,
-              st == 0 ? WF_ST - 1 : st - 1);
+        issue(lane < 4 ? reinterpret_cast<const int*>(sOff + (b - t0 + P::AHEAD))[lane] : -1,
+              st == 0 ? P::ST - 1 : st - 1);
       }
-      if (++st == WF_ST) {
+      if (++st == P::ST) {
         st = 0;
         ph ^= 1;
       }
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
   } else {
     for (; flight > 0; --flight) {
       if (!__all_sync(0xffffffffu, tc::mbar_wait(&bar[st], ph, ok ? 1000u : 200u))) ok = false;
-      if (++st == WF_ST) {
+      if (++st == P::ST) {
         st = 0;
         ph ^= 1;
       }
@@ -322,11 +325,11 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
     for (int n = 1; n <= NY; ++n) put(NY + n, s[n - 1]);
   }
   __syncthreads();
-  for (int e = tid; e < P::NR * (COLS / 4); e += WF_THREADS) {  // the warps' sums in order
+  for (int e = tid; e < P::NR * (COLS / 4); e += P::THREADS) {  // the warps' sums in order
     const int j = e / (COLS / 4), x = 4 * (e - j * (COLS / 4));
     float4 t = *reinterpret_cast<const float4*>(red + j * COLS + x);
 #pragma unroll
-    for (int w = 1; w < WF_WARPS; ++w) {
+    for (int w = 1; w < P::WARPS; ++w) {
       const float4 a = *reinterpret_cast<const float4*>(red + (size_t)w * P::NR * COLS + j * COLS + x);
       t.x += a.x;
       t.y += a.y;
@@ -343,14 +346,14 @@ __global__ void __launch_bounds__(WF_THREADS, 2) win_fold_kernel(const __grid_co
   constexpr int UT = 3;
   const int KY = 2 * Ny + 1, NU = Nx + 1, UG = (NU + UT - 1) / UT, NP = (Ny + 1) * UG;
   int Q = 8;
-  while (Q > 1 && NP * Q > WF_THREADS) Q >>= 1;
+  while (Q > 1 && NP * Q > P::THREADS) Q >>= 1;
   const float scale = 1.0f / ((float)Fx * (float)Fy);
   float2* parts = win_part + (size_t)(G.T.img0[sz] + img) * nparts * KY * NU;
   const int used = G.T.rows[sz] * G.T.ncs[sz];
   if (cb == 0 && rs == 0)
-    for (int e = tid; e < (nparts - used) * KY * NU; e += WF_THREADS) parts[(size_t)used * KY * NU + e] = make_float2(0.f, 0.f);
+    for (int e = tid; e < (nparts - used) * KY * NU; e += P::THREADS) parts[(size_t)used * KY * NU + e] = make_float2(0.f, 0.f);
   float2* out = parts + (size_t)(cb * G.T.ncs[sz] + rs) * KY * NU;
-  for (int base = 0; base < NP * Q; base += WF_THREADS) {  // uniform bound: whole warps shuffle
+  for (int base = 0; base < NP * Q; base += P::THREADS) {  // uniform bound: whole warps shuffle
     const int t = base + tid, q = t % Q, pr = min(t / Q, NP - 1), v = pr / UG, u0 = (pr - v * UG) * UT;
     const float* C = sC + v * P::RS;
     const float* S = sC + (NY + v) * P::RS;  // v = 0: any row, times zero
@@ -414,8 +417,8 @@ static int fold_splits(long long units, int nb, int warps, int most, long long s
 // (or two splits): one mask of 1024^2 takes 22 us in the two stages with 32, 44 us with 256.
 int win_fold_splits(const ImgGeom& g, int ncb, long long tiles, int sm_count) {
   const int nb = fold_nbase(g.Ly, g.Fy);
-  const int most = std::max(1, std::min(nb / WF_WARPS, std::max(2, 32 / ncb)));  // a base row per warp at least
-  return fold_splits(tiles, nb, WF_WARPS, most, 2LL * sm_count, 8);
+  const int warps = wf_warps(wf_ny(g.Ny)), most = std::max(1, std::min(nb / warps, std::max(2, 32 / ncb)));  // a base row per warp at least
+  return fold_splits(tiles, nb, warps, most, 2LL * sm_count, g.Ny > 8 ? 24 : 8);
 }
 
 // column blocks and row splits of a window DFT
@@ -440,7 +443,7 @@ static cudaError_t launch_win_fold_t(cudaStream_t s, const WinSet& G, const ImgG
   auto k = vec ? win_fold_kernel<NY, true> : win_fold_kernel<NY, false>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k<<<G.T.tile0[G.T.n], WF_THREADS, smem, s>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, win_part, nparts, stall, err);
+  k<<<G.T.tile0[G.T.n], WinFold<NY>::THREADS, smem, s>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, win_part, nparts, stall, err);
   return cudaGetLastError();
 }
 
