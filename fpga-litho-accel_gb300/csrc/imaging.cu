@@ -1155,6 +1155,10 @@ int image_pipeline(litho_ctx* ctx, const ImgGeom& g, int batch, const float* mas
   const bool tc = precision == LITHO_PREC_MIXED && fi_tc_serves(g);
   const bool band = use_band_tcc(ctx, ks, batch);
   ImgPlan p = make_plan(g, batch, ctx->sm_count);
+  // (the stall hook is the folded kernel's)
+  const bool win_tc = precision == LITHO_PREC_MIXED && ctx->test_stall_chunk < 0 && win_tc_serves(g, batch) &&
+                      (reinterpret_cast<uintptr_t>(masks) & 15) == 0;
+  if (win_tc) win_tc_plan(p);
   if (band) {
     p.ngroups = ks->band_nc;
     p.kpg = g.nk;
@@ -1169,7 +1173,13 @@ int image_pipeline(litho_ctx* ctx, const ImgGeom& g, int batch, const float* mas
   if (band) LITHO_RET(ctx->band_w.ensure(ctx, band_wsum_bytes(g, batch)));
   if (!tc) LITHO_RET(ctx->tm.ensure(ctx, (size_t)batch * (4 * g.Ny + 1) * g.Lx * sizeof(float)));
   const WinPart part{p, masks, 0};
-  LITHO_RET(run_win_dft(ctx, &part, 1, ctx->win_part.as<float2>(), p.nparts(), precision));
+  if (win_tc) {
+    const float2* twF = nullptr;  // the interpolation rows read it before they wait: made before this stage
+    LITHO_RET(fi_twiddles(ctx, g, &twF));
+    LITHO_RET(run_win_dft_tc(ctx, p, masks, ctx->win_part.as<float2>()));
+  } else {
+    LITHO_RET(run_win_dft(ctx, &part, 1, ctx->win_part.as<float2>(), p.nparts(), precision));
+  }
   WindowSrc w;
   w.part = ctx->win_part.as<float2>();
   w.nparts = p.nparts();

@@ -1,6 +1,6 @@
-// Mixed-precision interpolation output above Ny = 8: the image contraction on the
-// 5th-generation tensor cores (tcgen05, kind::tf32) with split operands and FP32
-// accumulation in TMEM.  The rest of the mixed form is the FP32 path's.
+// Mixed-precision contractions above Ny = 8 on the 5th-generation tensor cores (tcgen05,
+// kind::tf32) with split operands and FP32 accumulation in TMEM: the interpolation's, and the
+// window's of large batches.  The rest of the mixed form is the FP32 path's.
 //
 // Split products.  Every operand X is written as X = Xh + Xl with
 // Xh = round_tf32(X) and Xl = X - Xh (exact in FP32); the contraction computes
@@ -22,6 +22,7 @@
 //                     image is written exactly once).
 #include "litho_internal.cuh"
 #include "tc_common.cuh"
+#include "win_tiles.hpp"
 
 #include <cstring>
 
@@ -36,6 +37,46 @@ using namespace tc;
 // ---------------------------------------------------------------------------
 // operand tables (built once per geometry, cached on the context)
 // ---------------------------------------------------------------------------
+// twT[j][x] (NB rows): j <= Nx cos(2 pi j x'/Fx); Nx < j <= 2Nx -sin(2 pi (j-Nx) x'/Fx); else 0
+__global__ void twT_init_kernel(float* __restrict__ hi, float* __restrict__ lo, int Lx, int Fx, int Nx, int NB) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y;
+  if (x >= Lx || j >= NB) return;
+  const long long xp = (long long)x + (Fx - Lx) / 2 - Fx / 2;
+  double v = 0.0;
+  if (j <= 2 * Nx) {
+    const int u = j <= Nx ? j : j - Nx;
+    long long m = ((long long)u * xp) % Fx;
+    if (m < 0) m += Fx;
+    double s, c;
+    sincospi(2.0 * (double)m / (double)Fx, &s, &c);
+    v = j <= Nx ? c : -s;
+  }
+  const float h = tf32_round((float)v);
+  hi[(size_t)j * Lx + x] = h;
+  lo[(size_t)j * Lx + x] = (float)(v - (double)h);
+}
+
+// ytab[v][y] = e^{-2 pi i v y'/Fy} (v = 0..Ny), y' = y + (Fy - Ly)/2 - Fy/2: the row
+// twiddles of the window DFT's epilogue
+// yt[v][y] = e^{-2 pi i v y' / Fy} for the rows y < Ly, rows padded to Lyp (a multiple
+// of 128) with zeros, so that a 128-row tile reads whole rows of it.
+__global__ void ytab_init_kernel(float2* __restrict__ yt, int Ly, int Lyp, int Fy) {
+  const int y = blockIdx.x * blockDim.x + threadIdx.x;
+  const int v = blockIdx.y;
+  if (y >= Lyp) return;
+  float2 t = make_float2(0.f, 0.f);
+  if (y < Ly) {
+    const long long oyc = (long long)(Fy - Ly) / 2 - Fy / 2;
+    long long m = ((long long)v * (y + oyc)) % Fy;
+    if (m < 0) m += Fy;
+    float sn, cs;
+    sincospif(2.0f * (float)m / (float)Fy, &sn, &cs);
+    t = make_float2(cs, -sn);
+  }
+  yt[(size_t)v * Lyp + y] = t;
+}
+
 // CyT[Y][r] (KP columns): r < 2Ny -> 2cos(2 pi (r+1) y'/Fy); 2Ny <= r < 4Ny ->
 // -2sin(2 pi (r-2Ny+1) y'/Fy); else 0.  The fy = 0 (DC) row is not a column: the
 // FI epilogue adds T0[X] in FP32, so 4Ny rows fill the K blocks exactly when Ny is
@@ -57,6 +98,441 @@ __global__ void cyT_init_kernel(float* __restrict__ hi, float* __restrict__ lo, 
   const float h = tf32_round((float)v);
   hi[(size_t)Y * KP + r] = h;
   lo[(size_t)Y * KP + r] = (float)(v - (double)h);
+}
+
+// ---------------------------------------------------------------------------
+// window DFT on the tensor cores (win_tc_serves)
+// ---------------------------------------------------------------------------
+
+// Persistent window DFT: one CTA per SM streams its tiles (image, 128-row block,
+// column range) through one TMA ring; the TMEM accumulator is double-buffered so
+// a tile's row-DFT epilogue (its own four warps) overlaps the next tile's loads
+// and MMAs.  Roles (448 threads):
+//   warps 0-7   check each landed mask tile for TF32-exactness (warp vote); only
+//               a tile with a residual is split in place (hi, then lo)
+//   warp 8      TMA producer (one lane), warp 9 MMA issuer (one lane)
+//   warps 10-13 epilogue: TMEM -> registers -> shared -> row DFT -> partials
+// Per stage s and running chunk q (parity (q / S) & 1; every role keeps s and the
+// parity as running counters, since a division by the launch-time S on the
+// per-chunk path measurably slows the ring):
+//   producer  : [wait empty[s]] -> TMA mask tile + twiddle [hi; lo] tile -> full[s]
+//   consumers : wait full[s]; vote residual (nzflag); if any: Ah = round_tf32(A) in
+//               place; arrive ready[s]; if residual: wait hidone[s], write Al,
+//               arrive ready2[s]
+//   MMA lane  : [tile start: wait accempty[buf]]; wait ready[s]; Ah*[Bh; Bl] as one
+//               N = 2 NBH MMA per K step (the epilogue adds the two column halves);
+//               if residual: commit hidone[s], wait ready2[s], Al*Bh; commit empty[s];
+//               [tile end: commit accfull[buf]]
+//   epilogue  : wait accfull[buf]; TMEM -> sR (hi + lo halves); arrive accempty[buf];
+//               row DFT with one thread per output pair (+v, -v)
+// hidone/ready2 complete only on chunks with a residual, so their parities are
+// tracked per stage in bit masks that both sides flip identically.
+//
+// The ring is as deep as shared memory allows: under full load a mask tile takes
+// ~3 us from TMA issue to landing, so the bytes in flight per SM, not the work per
+// tile, set the throughput.  Hence the twiddle tile carries only the 2Nx+1 used
+// rows of each half (NBH = 2Nx+1 rounded up to 8), the epilogue keeps only the 2Nx+1
+// used accumulator columns in shared memory and reads the row twiddles from their
+// table (through L1), and the stage count S is chosen at launch: four stages (128 KB of
+// mask in flight) up to Nx = 16.
+template <int NBH>
+struct WinTC {
+  // a stage carries a 64-column chunk as two 32-column K blocks: each pipeline round
+  // trip (land, check, MMA, release) then moves 32 KB of mask, which halves the
+  // per-chunk handshakes that bound this ring
+  static constexpr int KB = 2;                       // K blocks (32 columns each) per stage
+  static constexpr uint32_t A_KB = 128 * 128;        // 128 rows x 32 fp32 (split in place: hi, then lo)
+  static constexpr uint32_t A_B = KB * A_KB;
+  static constexpr uint32_t B_KB = 2 * NBH * 128;    // [hi NBH rows; lo NBH rows] x 32 fp32
+  static constexpr uint32_t B_B = KB * B_KB;
+  static constexpr uint32_t STAGE_B = A_B + B_B;     // a multiple of 2048: every stage is 1024-aligned
+  // one accumulator holds A*Bh in columns [0, NBH) and A*Bl in [NBH, 2 NBH): one
+  // N = 2 NBH MMA reads the mask tile once for both products
+  static constexpr uint32_t NCOL = 2 * NBH <= 32 ? 32 : (2 * NBH <= 64 ? 64 : 128);
+  static constexpr int NLO = (NBH + 15) / 16 * 16;  // N of the residual pass Al*Bh (>= NBH, multiple of 16)
+};
+constexpr int WP_THREADS = 448;  // warps 0-7 split, 8 TMA, 9 MMA, 10-13 epilogue
+constexpr int WP_CONS = 256;     // consumer threads
+// padded row strides of the epilogue buffers: multiples of 4 floats so the row DFT
+// reads 16-byte vectors, and 33 / 65 float4 slots apart so the threads of a warp
+// (different u, different |v|) land in different bank groups
+constexpr int WP_RSR = 132;      // sR rows (fp32)
+constexpr int WP_MAX_STAGES = 12;
+constexpr int WP_TQ = 8;         // tile ring: tiles the producer may publish ahead of the slowest role
+constexpr size_t WP_SMEM_CAP = 227 * 1024;
+
+// epilogue buffer: sR [2Nx+1][RSR] fp32 (a multiple of 16 bytes)
+static inline size_t win_epi_bytes(int Nx) { return (size_t)(2 * Nx + 1) * WP_RSR * 4; }
+// The masks' and twiddles' tensor maps, the row twiddles and the tiles of one mask size.
+struct WinGeo {
+  CUtensorMap mM[1];  // masks [img][Ly][Lx]
+  CUtensorMap mB[1];  // twiddles [hi; lo] x Lx
+  const float2* ytab[1];
+  WinTiles T;                  // widths, row blocks, splits, first images and tiles (win_tiles.hpp)
+};
+
+// mbarriers and flags after the epilogue buffers (S <= WP_MAX_STAGES): 5 per stage, 5 more,
+// two per tile-ring slot; the TMEM slot, abort flag, per-stage ints, tile ring and the two
+// groups' current tiles
+static inline size_t win_bar_bytes(int S) {
+  return (size_t)(5 * S + 5 + 2 * WP_TQ) * 8 + 16 + 8 * (size_t)S + 4 * WP_TQ + 8;
+}
+
+template <int NBH>
+__global__ void __launch_bounds__(WP_THREADS, 1) win_dft_tc_kernel(const __grid_constant__ WinGeo G, int Fx, int Fy,
+                                                                   int Nx, int Ny, int S,
+                                                                   float2* __restrict__ win_part, int* __restrict__ err) {
+  using P = WinTC<NBH>;
+  early_next();
+  extern __shared__ unsigned char smraw[];
+  unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
+  constexpr int RS = WP_RSR;
+  const int KXw = 2 * Nx + 1;                                          // used accumulator columns
+  float* sR = reinterpret_cast<float*>(sm + (size_t)S * P::STAGE_B);  // [KXw][RS]
+  uint64_t* full = reinterpret_cast<uint64_t*>(sR + KXw * RS);
+  uint64_t* ready = full + S;
+  uint64_t* hidone = ready + S;
+  uint64_t* ready2 = hidone + S;
+  uint64_t* empty = ready2 + S;
+  uint64_t* accfull = empty + S;
+  uint64_t* accempty = accfull + 2;
+  uint64_t* done = accempty + 2;
+  uint64_t* tqf = done + 1;       // [WP_TQ] tile-ring slot published (producer)
+  uint64_t* tqe = tqf + WP_TQ;    // [WP_TQ] slot read by all three reading roles
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(tqe + WP_TQ);
+  volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
+  int* last_issued = reinterpret_cast<int*>(tslot + 2);  // [S]
+  int* nzflag = last_issued + S;                          // [S]
+  volatile int* tq = nzflag + S;                          // [WP_TQ] tile index, -1 = no more tiles
+  volatile int* gtile = tq + WP_TQ;                       // [2] consumers' / epilogue's current tile
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int T = G.T.tile0[G.T.n];
+
+  if (warp == 0) tmem_alloc(tslot, 2 * P::NCOL);
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&ready[s], WP_CONS / 32);  // one arrival per consumer warp
+      mbar_init(&hidone[s], 1);
+      mbar_init(&ready2[s], WP_CONS / 32);
+      mbar_init(&empty[s], 1);
+      last_issued[s] = -1;
+      nzflag[s] = 0;
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&accfull[b], 1);
+      mbar_init(&accempty[b], 128);
+    }
+    mbar_init(done, 1);
+    for (int j = 0; j < WP_TQ; ++j) {
+      mbar_init(&tqf[j], 1);
+      mbar_init(&tqe[j], 3);  // the consumers' leader, the MMA lane, the epilogue's leader
+    }
+    *abort = 0;
+    fence_mbar_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tslot;
+
+  // Tiles come through a ring of WP_TQ slots: the producer takes the next tile of its
+  // sequence (blockIdx.x + k gridDim.x) and publishes it; the MMA lane and one leader
+  // thread of the consumer and epilogue groups read it (a named barrier hands the
+  // leader's copy to its group, so a group never splits at a barrier) and release the
+  // slot.  The end of the sequence is published as -1, so every role stops on the same
+  // tile.
+  auto ring_read = [&](int seq, int& t) {  // false: the wait gave up (abort is set)
+    const int j = seq & (WP_TQ - 1);
+    if (!mbar_wait_ab(&tqf[j], (uint32_t)(seq / WP_TQ) & 1u, abort)) {
+      *abort = 1;
+      t = -1;
+      return false;
+    }
+    t = tq[j];
+    mbar_arrive(&tqe[j]);
+    return true;
+  };
+
+  auto sA = [&](int s) { return sm + (size_t)s * P::STAGE_B; };
+  auto sBh = [&](int s) { return sm + (size_t)s * P::STAGE_B + P::A_B; };  // [Bh; Bl], 2 NBH rows
+  // tile t -> (geometry, image, row block, column split) and its chunk range (chunks of
+  // 32 KB columns)
+  auto decode = [&](int t, int& g, int& img, int& rb, int& cs, int& c0, int& c1) {
+    win_tile(G.T, t, 32 * P::KB, g, img, rb, cs, c0, c1);
+  };
+
+  if (warp == 8) {
+    if (lane == 0) {  // TMA producer
+      int q = 0, s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int seq = 0; ok; ++seq) {
+        const int j = seq & (WP_TQ - 1);
+        if (seq >= WP_TQ && !mbar_wait_ab(&tqe[j], (uint32_t)(seq / WP_TQ - 1) & 1u, abort)) {
+          *abort = 1;
+          break;
+        }
+        int t = (int)blockIdx.x + seq * (int)gridDim.x;
+        if (t >= T) t = -1;
+        tq[j] = t;
+        mbar_arrive(&tqf[j]);  // release: the slot's tile index is visible to the readers
+        if (t < 0) break;
+        int g, img, rb, cs, c0, c1;
+        decode(t, g, img, rb, cs, c0, c1);
+        for (int c = c0; c < c1; ++c, ++q) {
+          if (q >= S && !mbar_wait_ab(&empty[s], ph ^ 1u, abort)) {
+            *abort = 1;
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(&full[s], P::STAGE_B);
+#pragma unroll
+          for (int kb = 0; kb < P::KB; ++kb) {
+            tma_load_3d(sA(s) + kb * P::A_KB, &G.mM[g], &full[s], 32 * (P::KB * c + kb), 128 * rb, img);
+            tma_load_2d(sBh(s) + kb * P::B_KB, &G.mB[g], &full[s], 32 * (P::KB * c + kb), 0);
+          }
+          last_issued[s] = q;
+          if (++s == S) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+      }
+    }
+  } else if (warp == 9) {
+    if (lane == 0) {  // MMA issuer
+      constexpr uint32_t IDESC2 = idesc_tf32(128, 2 * NBH);  // A x [Bh; Bl]
+      // Al x Bh over the first NLO twiddle rows: the hi rows, plus (when NBH is not
+      // a multiple of 16) a few lo rows whose Al*Bl terms only add accuracy
+      constexpr uint32_t IDESC1 = idesc_tf32(128, P::NLO);
+      uint32_t ph2 = 0;  // per-stage parity of hidone / ready2
+      int tl = 0, s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int seq = 0; ok; ++seq, ++tl) {
+        int t;
+        if (!ring_read(seq, t) || t < 0) break;
+        int g, img, rb, cs, c0, c1;
+        decode(t, g, img, rb, cs, c0, c1);
+        const int buf = tl & 1;
+        if (tl >= 2 && !mbar_wait_ab(&accempty[buf], (uint32_t)((tl - 2) >> 1) & 1u, abort)) {
+          *abort = 1;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t acc = tmem + (uint32_t)buf * P::NCOL;
+        for (int c = c0; c < c1; ++c) {
+          if (!mbar_wait_ab(&ready[s], ph, abort)) {
+            *abort = 1;
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const bool two = *reinterpret_cast<volatile int*>(&nzflag[s]) != 0;
+          nzflag[s] = 0;  // every consumer read it before arriving on ready[s]
+#pragma unroll
+          for (int kb = 0; kb < P::KB; ++kb) {
+            const uint64_t da = desc_sw128(sA(s) + kb * P::A_KB), dbh = desc_sw128(sBh(s) + kb * P::B_KB);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+              const uint32_t off = kk * 32;
+              mma_tf32(acc, desc_add(da, off), desc_add(dbh, off), IDESC2, (c != c0 || kb != 0 || kk != 0) ? 1u : 0u);
+            }
+          }
+          if (two) {
+            mma_commit(&hidone[s]);
+            if (!mbar_wait_ab(&ready2[s], (ph2 >> s) & 1u, abort)) {
+              *abort = 1;
+              ok = false;
+              break;
+            }
+            ph2 ^= 1u << s;
+            tc_fence_after();
+#pragma unroll
+            for (int kb = 0; kb < P::KB; ++kb) {
+              const uint64_t da = desc_sw128(sA(s) + kb * P::A_KB), dbh = desc_sw128(sBh(s) + kb * P::B_KB);
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) {
+                const uint32_t off = kk * 32;
+                mma_tf32(acc, desc_add(da, off), desc_add(dbh, off), IDESC1, 1u);
+              }
+            }
+          }
+          mma_commit(&empty[s]);
+          if (++s == S) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+        if (ok) mma_commit(&accfull[buf]);  // arrives when this tile's MMAs have completed
+      }
+      mma_commit(done);  // arrives once everything issued above has completed
+    }
+  } else if (warp < 8) {  // warps 0-7: check / split the landed tiles in place
+    uint32_t ph2 = 0, ph = 0;
+    int s = 0;
+    // a wait that gives up flags the error and the thread carries on through the
+    // named barriers with the others (later waits return at once): a thread that
+    // left alone would strand the rest at the next barrier
+    for (int seq = 0;; ++seq) {
+      if (tid == 0) {
+        int t;
+        ring_read(seq, t);
+        gtile[0] = t;
+      }
+      named_bar(1, WP_CONS);
+      const int t = gtile[0];
+      named_bar(1, WP_CONS);  // every consumer holds t before the leader may overwrite it
+      if (t < 0) break;
+      int g, img, rb, cs, c0, c1;
+      decode(t, g, img, rb, cs, c0, c1);
+      for (int c = c0; c < c1; ++c) {
+        if (!mbar_wait_ab(&full[s], ph, abort)) *abort = 1;
+        float4* a = reinterpret_cast<float4*>(sA(s));
+        float4 v[4 * P::KB];
+        // x is exact in TF32 (x == round_tf32(x)) iff its low 13 mantissa bits are zero
+        uint32_t low = 0;
+#pragma unroll
+        for (int i = 0; i < 4 * P::KB; ++i) {
+          v[i] = a[tid + WP_CONS * i];
+          low |= __float_as_uint(v[i].x) | __float_as_uint(v[i].y) | __float_as_uint(v[i].z) | __float_as_uint(v[i].w);
+        }
+        const bool nz = (low & 0x1FFFu) != 0u;
+        if (__any_sync(0xffffffffu, nz) && lane == 0) atomicOr(&nzflag[s], 1);
+        named_bar(1, WP_CONS);
+        const bool two = *reinterpret_cast<volatile int*>(&nzflag[s]) != 0;
+        if (two) {  // write Ah = round_tf32(A) in place; exact tiles are used as landed
+#pragma unroll
+          for (int i = 0; i < 4 * P::KB; ++i)
+            a[tid + WP_CONS * i] =
+                make_float4(tf32_round(v[i].x), tf32_round(v[i].y), tf32_round(v[i].z), tf32_round(v[i].w));
+          fence_proxy_async();
+        }
+        // release: the warp's reads of nzflag and its Ah stores precede its one arrival
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ready[s]);
+        if (two) {
+          if (!mbar_wait_ab(&hidone[s], (ph2 >> s) & 1u, abort)) *abort = 1;
+          ph2 ^= 1u << s;
+#pragma unroll
+          for (int i = 0; i < 4 * P::KB; ++i)
+            a[tid + WP_CONS * i] = make_float4(v[i].x - tf32_round(v[i].x), v[i].y - tf32_round(v[i].y),
+                                               v[i].z - tf32_round(v[i].z), v[i].w - tf32_round(v[i].w));
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ready2[s]);
+        }
+        if (++s == S) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+    }
+  } else {  // warps 10-13: epilogue
+    const int etid = tid - 320, quarter = warp & 3;
+    const int row = 32 * quarter + lane;
+    const int KY = 2 * Ny + 1, NU = Nx + 1;
+    const float inv_ff = 1.0f / ((float)Fx * (float)Fy);
+    int tl = 0;
+    for (int seq = 0;; ++seq, ++tl) {
+      if (etid == 0) {
+        int t;
+        ring_read(seq, t);
+        gtile[1] = t;
+      }
+      named_bar(2, 128);
+      const int t = gtile[1];
+      named_bar(2, 128);  // every epilogue thread holds t before the leader may overwrite it
+      if (t < 0) break;
+      int g, img, rb, cs, c0, c1;
+      decode(t, g, img, rb, cs, c0, c1);
+      const int buf = tl & 1;
+      // on a wait that gives up: flag it and carry on with the group (see above)
+      if (!mbar_wait_ab(&accfull[buf], (uint32_t)(tl >> 1) & 1u, abort)) *abort = 1;
+      tc_fence_after();
+      const uint32_t trow = tmem + (uint32_t)buf * P::NCOL + ((uint32_t)(32 * quarter) << 16);
+      // sR[j] = (A Bh)[j] + (A Bl)[j]: 2 NBH columns in 8-column loads, one wait
+      {
+        uint32_t v[2 * NBH];
+#pragma unroll
+        for (int g = 0; g < 2 * NBH / 8; ++g) tmem_ld8_async(trow + 8u * g, &v[8 * g]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < NBH; ++j)
+          if (j < KXw) sR[j * RS + row] = __uint_as_float(v[j]) + __uint_as_float(v[NBH + j]);
+      }
+      tc_fence_before();
+      mbar_arrive(&accempty[buf]);  // the MMA lane may refill this accumulator
+      const int y0 = 128 * rb;
+      named_bar(2, 128);
+      const int rows = G.T.rows[g], ncs = G.T.ncs[g];
+      const int nps = rows * ncs;
+      float2* out = win_part + ((size_t)(G.T.img0[g] + img) * nps + (rb * ncs + cs)) * KY * NU;
+      // one thread per (|v|, u): four row sums give both outputs +v and -v
+      //   S1 = sum c tx, S2 = sum s ty, S3 = sum c ty, S4 = sum s tx
+      //   (+v): (S1 - S2, S3 + S4)    (-v): (S1 + S2, S4 - S3)
+      // with c, s the cos / -sin accumulator columns of u (s = 0 for u = 0)
+      for (int pq = etid; pq < (Ny + 1) * NU; pq += 128) {
+        const int av = pq / NU, u = pq - av * NU;
+        const float4* rc = reinterpret_cast<const float4*>(sR + u * RS);
+        const float4* rs = reinterpret_cast<const float4*>(sR + (Nx + u) * RS);
+        // the tile's row twiddles of |v| (zero past Ly), two rows per vector, from L1
+        const float4* rt = reinterpret_cast<const float4*>(G.ytab[g] + (size_t)av * (128 * rows) + y0);
+        float s1 = 0.f, s2 = 0.f, s3 = 0.f, s4 = 0.f;
+        if (u == 0) {
+#pragma unroll 4
+          for (int r4 = 0; r4 < 32; ++r4) {
+            const float4 c = rc[r4], ta = __ldg(rt + 2 * r4), tb = __ldg(rt + 2 * r4 + 1);
+            s1 = fmaf(c.x, ta.x, s1);
+            s3 = fmaf(c.x, ta.y, s3);
+            s1 = fmaf(c.y, ta.z, s1);
+            s3 = fmaf(c.y, ta.w, s3);
+            s1 = fmaf(c.z, tb.x, s1);
+            s3 = fmaf(c.z, tb.y, s3);
+            s1 = fmaf(c.w, tb.z, s1);
+            s3 = fmaf(c.w, tb.w, s3);
+          }
+        } else {
+#pragma unroll 4
+          for (int r4 = 0; r4 < 32; ++r4) {
+            const float4 c = rc[r4], sn = rs[r4], ta = __ldg(rt + 2 * r4), tb = __ldg(rt + 2 * r4 + 1);
+            s1 = fmaf(c.x, ta.x, s1);
+            s2 = fmaf(sn.x, ta.y, s2);
+            s3 = fmaf(c.x, ta.y, s3);
+            s4 = fmaf(sn.x, ta.x, s4);
+            s1 = fmaf(c.y, ta.z, s1);
+            s2 = fmaf(sn.y, ta.w, s2);
+            s3 = fmaf(c.y, ta.w, s3);
+            s4 = fmaf(sn.y, ta.z, s4);
+            s1 = fmaf(c.z, tb.x, s1);
+            s2 = fmaf(sn.z, tb.y, s2);
+            s3 = fmaf(c.z, tb.y, s3);
+            s4 = fmaf(sn.z, tb.x, s4);
+            s1 = fmaf(c.w, tb.z, s1);
+            s2 = fmaf(sn.w, tb.w, s2);
+            s3 = fmaf(c.w, tb.w, s3);
+            s4 = fmaf(sn.w, tb.z, s4);
+          }
+        }
+        out[(Ny + av) * NU + u] = make_float2((s1 - s2) * inv_ff, (s3 + s4) * inv_ff);
+        if (av > 0) out[(Ny - av) * NU + u] = make_float2((s1 + s2) * inv_ff, (s4 - s3) * inv_ff);
+      }
+      named_bar(2, 128);  // sR is free for the next tile
+    }
+  }
+  // the MMA lane always commits `done`; everyone waits for the tensor cores to drain
+  if (!mbar_wait(done, 0)) *abort = 1;
+  __syncthreads();
+  if (*abort) {
+    if (tid == 256)  // warp 8 lane 0: wait for the last load of every stage
+      for (int s = 0; s < S; ++s)
+        if (last_issued[s] >= 0) mbar_wait(&full[s], (uint32_t)(last_issued[s] / S) & 1u, 200u);
+    if (tid == 0) atomicExch(err, 1);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 2 * P::NCOL);
 }
 
 // ---------------------------------------------------------------------------
@@ -436,6 +912,11 @@ static int make_map(litho_ctx* ctx, CUtensorMap* m, const void* base, int rank, 
   return LITHO_OK;
 }
 
+// twiddle rows of each half of the window DFT's B tile: 2Nx+1 rounded up to 8
+static int nb_for(int Nx) {
+  const int nj = 2 * Nx + 1;
+  return nj <= 40 ? (nj + 7) / 8 * 8 : -1;
+}
 static int kblk_for(int Ny) { return std::max(1, (4 * Ny + 31) / 32); }  // 4Ny K rows (the DC row is separate)
 
 // The mixed form takes the contraction on the tensor cores where it is the faster of the two:
@@ -481,6 +962,91 @@ static int cached_table(litho_ctx* ctx, std::tuple<int, int, int, int> key, size
   }
   *out = it->second.as<float>();
   return LITHO_OK;
+}
+
+// Column twiddles (hi/lo TF32 rows) and epilogue row twiddles of one window geometry,
+// cached in the context and built on first use on the context's stream.
+template <int NBH>
+static int win_tc_tables(litho_ctx* ctx, const ImgGeom& g, float** twh, float** yt) {
+  bool fresh = false;
+  float* tw = nullptr;
+  LITHO_RET(cached_table(ctx, std::make_tuple(g.Lx, g.Fx, g.Nx, -NBH), (size_t)2 * NBH * g.Lx * sizeof(float),
+                         &fresh, &tw));
+  if (fresh) {
+    StageScope sc(ctx, LITHO_STAGE_UPLOAD);
+    twT_init_kernel<<<dim3((g.Lx + 127) / 128, NBH), 128, 0, ctx->stream>>>(tw, tw + (size_t)NBH * g.Lx, g.Lx, g.Fx,
+                                                                            g.Nx, NBH);
+    LITHO_CUDA_TRY(ctx, cudaGetLastError());
+  }
+  // row twiddles of the epilogue, rows padded to a multiple of 128, cached per (Ly, Fy, Ny)
+  const int Lyp = (g.Ly + 127) / 128 * 128;
+  LITHO_RET(cached_table(ctx, std::make_tuple(g.Ly, g.Fy, g.Ny, -3001), (size_t)(g.Ny + 1) * Lyp * sizeof(float2),
+                         &fresh, yt));
+  if (fresh) {
+    StageScope sc(ctx, LITHO_STAGE_UPLOAD);
+    ytab_init_kernel<<<dim3(Lyp / 128, g.Ny + 1), 128, 0, ctx->stream>>>(reinterpret_cast<float2*>(*yt), g.Ly,
+                                                                          Lyp, g.Fy);
+    LITHO_CUDA_TRY(ctx, cudaGetLastError());
+  }
+  *twh = tw;
+  return LITHO_OK;
+}
+
+template <int NBH>
+static int launch_win_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part, int* err) {
+  WinGeo G;
+  std::memset(&G, 0, sizeof(G));
+  const ImgGeom& g = p.g;
+  float *twh = nullptr, *yt = nullptr;
+  LITHO_RET(win_tc_tables<NBH>(ctx, g, &twh, &yt));
+  LITHO_RET(make_map(ctx, &G.mM[0], masks, 3, g.Lx, g.Ly, p.batch, 128));
+  LITHO_RET(make_map(ctx, &G.mB[0], twh, 2, g.Lx, 2 * NBH, 1, 2 * NBH));  // hi rows, then lo rows
+  G.ytab[0] = reinterpret_cast<const float2*>(yt);
+  G.T.n = 1;
+  G.T.Lx[0] = g.Lx;
+  G.T.rows[0] = p.rowBlocks;
+  G.T.ncs[0] = p.colSplits;
+  const int tiles = p.rowBlocks * p.batch * p.colSplits;
+  G.T.tile0[1] = tiles;
+  // as many ring stages as shared memory holds
+  using P = WinTC<NBH>;
+  const size_t fixed = 1024 + win_epi_bytes(g.Nx) + win_bar_bytes(WP_MAX_STAGES);
+  const int S = (int)std::min<size_t>(WP_MAX_STAGES, (WP_SMEM_CAP - fixed) / P::STAGE_B);
+  const size_t smem = 1024 + (size_t)S * P::STAGE_B + win_epi_bytes(g.Nx) + win_bar_bytes(S);
+  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(win_dft_tc_kernel<NBH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem));
+  const int grid = std::min(tiles, ctx->sm_count);  // persistent: one CTA per SM
+  StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
+  win_dft_tc_kernel<NBH><<<grid, WP_THREADS, smem, ctx->stream>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, S, win_part, err);
+  LITHO_CUDA_TRY(ctx, cudaGetLastError());
+  return LITHO_OK;
+}
+
+// The mixed form takes the window of large batches on the tensor cores above Ny = 8: there the folded
+// kernel is bound by its coefficient reads and the ends of its tiles, and masks whose values are exact in
+// TF32 (binary ones) need no residual products.  us a call, here and folded: 78 masks of 1626 x 1268 450 and
+// 467, 64 of 2048^2 502 and 529, 200 of 1280^2 872 and 957; below 2^27 pixels, 100 of 1100^2 448 and 438,
+// 16 of 1500^2 186 and 139, 10 of 2048^2 175 and 130.
+bool win_tc_serves(const ImgGeom& g, int batch) {
+  return (g.Lx % 4) == 0 && g.Ny > 8 && nb_for(g.Nx) > 0 && (long long)batch * g.Lx * g.Ly >= (1ll << 27);
+}
+
+// p's partials: 128-row blocks
+void win_tc_plan(ImgPlan& p) {
+  p.rowBlocks = (p.g.Ly + 127) / 128;
+  p.colSplits = 1;
+}
+
+int run_win_dft_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part) {
+  int* err = nullptr;
+  LITHO_RET(tc_err_flag(ctx, &err));
+  switch (nb_for(p.g.Nx)) {
+    case 8: return launch_win_tc<8>(ctx, p, masks, win_part, err);
+    case 16: return launch_win_tc<16>(ctx, p, masks, win_part, err);
+    case 24: return launch_win_tc<24>(ctx, p, masks, win_part, err);
+    case 32: return launch_win_tc<32>(ctx, p, masks, win_part, err);
+    default: return launch_win_tc<40>(ctx, p, masks, win_part, err);
+  }
 }
 
 template <int KBLK, int BN>

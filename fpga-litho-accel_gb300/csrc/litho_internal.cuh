@@ -308,6 +308,9 @@ bool use_band_tcc(const litho_ctx* ctx, const litho_kernel_set* ks, int batch);
 // mixed precision interpolation (imaging_tc.cu): whether it serves a geometry of the mixed form
 // (elsewhere the folded FP32 kernel does), and its launches
 bool fi_tc_serves(const ImgGeom& g);
+bool win_tc_serves(const ImgGeom& g, int batch);
+void win_tc_plan(ImgPlan& p);
+int run_win_dft_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part);
 int run_fi_tc(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tmT, float* images);
 struct FiTcBufs {
   float *tmh, *tml, *t0;
