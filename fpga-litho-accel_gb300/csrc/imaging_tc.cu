@@ -1,6 +1,6 @@
-// Mixed-precision contractions above Ny = 8 on the 5th-generation tensor cores (tcgen05,
-// kind::tf32) with split operands and FP32 accumulation in TMEM: the interpolation's, and the
-// window's of large batches.  The rest of the mixed form is the FP32 path's.
+// Mixed-precision contractions on the 5th-generation tensor cores (tcgen05, kind::tf32) with
+// split operands and FP32 accumulation in TMEM: the interpolation's above Ny = 8 and the
+// window's of some large batches.  The rest of the mixed form is the FP32 path's.
 //
 // Split products.  Every operand X is written as X = Xh + Xl with
 // Xh = round_tf32(X) and Xl = X - Xh (exact in FP32); the contraction computes
@@ -1022,13 +1022,18 @@ static int launch_win_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, f
   return LITHO_OK;
 }
 
-// The mixed form takes the window of large batches on the tensor cores above Ny = 8: there the folded
-// kernel is bound by its coefficient reads and the ends of its tiles, and masks whose values are exact in
-// TF32 (binary ones) need no residual products.  us a call, here and folded: 78 masks of 1626 x 1268 450 and
-// 467, 64 of 2048^2 502 and 529, 200 of 1280^2 872 and 957; below 2^27 pixels, 100 of 1100^2 448 and 438,
-// 16 of 1500^2 186 and 139, 10 of 2048^2 175 and 130.
+// The mixed form takes the window of large batches on the tensor cores where the folded kernel falls
+// short of the memory's rate: above Ny = 8 it is bound by its coefficient reads and the ends of its
+// tiles, and where masks fill less than four fifths of their period's rows, many of the four rows it
+// folds are outside and the same work serves fewer pixels.  (Masks whose values are exact in TF32, binary
+// ones, need no residual products here.)  us a call, here and folded: 64 of 2048^2 502 and 529, 200
+// of 1280^2 872 and 957, below 2^27 pixels 100 of 1100^2 448 and 438, 16 of 1500^2 186 and 139; 385 of
+// 604 x 1536 in 1024 rows 717 and 794, 600 of 300 x 2048 in 512 588 and 700, below 2^26 pixels 60 of
+// 604 x 1536 174 and 160.
 bool win_tc_serves(const ImgGeom& g, int batch) {
-  return (g.Lx % 4) == 0 && g.Ny > 8 && nb_for(g.Nx) > 0 && (long long)batch * g.Lx * g.Ly >= (1ll << 27);
+  const bool sparse = 5ll * g.Ly < 4ll * g.Fy;
+  return (g.Lx % 4) == 0 && (g.Ny > 8 || sparse) && nb_for(g.Nx) > 0 &&
+         (long long)batch * g.Lx * g.Ly >= (sparse ? 1ll << 26 : 1ll << 27);
 }
 
 // p's partials: 128-row blocks

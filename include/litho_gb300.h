@@ -54,10 +54,10 @@ extern "C" {
  * LITHO_PREC_FP32  : window DFT, FFTs, intensity sum and interpolation in FP32
  *                    on the CUDA cores (the plain path).
  * LITHO_PREC_MIXED : for supports Ny > 8 the interpolation (intensity band ->
- *                    image), and the window DFT of large batches, on the tensor
- *                    cores with split-operand TF32 products and FP32
- *                    accumulation; everything else as above, whose kernels
- *                    reach the memory's rate in FP32.                          */
+ *                    image), and the window DFT of large batches where that is
+ *                    faster, on the tensor cores with split-operand TF32 products
+ *                    and FP32 accumulation; everything else as above, whose
+ *                    kernels reach the memory's rate in FP32.                  */
 #define LITHO_PREC_FP32  0
 #define LITHO_PREC_MIXED 1
 
