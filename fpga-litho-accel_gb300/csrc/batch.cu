@@ -15,12 +15,13 @@
 //   kernels per CTA in {2, 3, 4, 6, 8, 12} (the SOCS tile), and
 //   window row splits in {r, 2r}, r what the class's tiles take by themselves
 // with CUDA events on the context's stream and keeps the fastest; results are
-// cached by (L, Nx, nk, images, precision, band form, r).  The plan then
+// cached by (L, Nx, Ny, nk, images, precision, band form, r).  The plan then
 // captures the whole sequence in a CUDA graph (LITHO_BATCH_GRAPH), a branch per class.
 #include "litho_internal.cuh"
 
 #include <algorithm>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -43,17 +44,18 @@ struct ClassRun {
 };
 
 struct TuneKey {
-  int L, Nx, nk, count, prec, band, splits0;
+  int L, Nx, Ny, nk, count, prec, band, splits0;
   bool operator<(const TuneKey& o) const {
-    return std::tie(L, Nx, nk, count, prec, band, splits0) <
-           std::tie(o.L, o.Nx, o.nk, o.count, o.prec, o.band, o.splits0);
+    return std::tie(L, Nx, Ny, nk, count, prec, band, splits0) <
+           std::tie(o.L, o.Nx, o.Ny, o.nk, o.count, o.prec, o.band, o.splits0);
   }
 };
 struct TuneVal {
   int convN, kpg, colSplits;
   double ms;
 };
-static std::map<TuneKey, TuneVal> g_tune_cache;  // shared by all contexts of the process
+static std::map<TuneKey, TuneVal> g_tune_cache;  // shared by all contexts of the process, under g_tune_mu
+static std::mutex g_tune_mu;
 
 }  // namespace litho
 
@@ -202,14 +204,17 @@ static int tune_class(litho_batch_plan* bp, int ci) {
   ClassRun& c = bp->classes[ci];
   const bool band_ok = band_tcc_available(bp->ctx, c.ks);
   const int method = band_ok ? (bp->ctx->band_method == LITHO_BAND_TCC ? 2 : 1) : 0;
-  const TuneKey key{c.L, c.ks->Nx, c.ks->nk, c.count, bp->precision, method, c.splits0};
-  auto it = g_tune_cache.find(key);
-  if (it != g_tune_cache.end()) {
-    c.convN = it->second.convN;
-    c.kpg = it->second.kpg;
-    c.colSplits = it->second.colSplits;
-    c.tuned_ms = it->second.ms;
-    return LITHO_OK;
+  const TuneKey key{c.L, c.ks->Nx, c.ks->Ny, c.ks->nk, c.count, bp->precision, method, c.splits0};
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tune_cache.find(key);
+    if (it != g_tune_cache.end()) {
+      c.convN = it->second.convN;
+      c.kpg = it->second.kpg;
+      c.colSplits = it->second.colSplits;
+      c.tuned_ms = it->second.ms;
+      return LITHO_OK;
+    }
   }
   // band forms: conv grids of the FFT form, and 0 for the TCC band where the kernel set
   // has a table (with LITHO_BAND_TCC the TCC band alone)
@@ -262,6 +267,7 @@ static int tune_class(litho_batch_plan* bp, int ci) {
   c.kpg = best.kpg;
   c.colSplits = best.colSplits;
   c.tuned_ms = best.ms;
+  std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune_cache[key] = best;
   return LITHO_OK;
 }
