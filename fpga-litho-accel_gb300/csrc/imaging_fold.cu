@@ -108,7 +108,8 @@ __device__ __forceinline__ void wf_copy(float* dst, const void* src, int bytes, 
 // reads them back.  Otherwise lanes 0-3 issue a bulk copy of one row each, the ring holds whole
 // 16-byte granules and the lanes read their columns (lane + 32 i) past each row's misalignment;
 // every wait is bounded: a warp whose copies do not land in a second issues no more, waits for what
-// it has in flight and sets *err.  (Measured, window stage: 256 aligned masks of 1024^2
+// it has in flight, sets *err and makes its sums NaN, so that the images show it too; while *err is
+// set, warps issue nothing and end the same way.  (Measured, window stage: 256 aligned masks of 1024^2
 // 198 us with cp.async, 206 with bulk copies; 44 of 2048^2 184 and 231; 40 ragged 913 x 777 masks
 // 54 and 49, and 138 with plain loads.)
 // The masks of up to WIN_MAX_SIZES sizes that share the period and the kernel support are one
@@ -302,7 +303,11 @@ __global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __
         ph ^= 1;
       }
     }
-    if (!ok && lane == 0) atomicExch(err, 1);
+    if (!ok) {
+      if (lane == 0) atomicExch(err, 1);
+#pragma unroll
+      for (int i = 0; i < CPL; ++i) c[0][i] = __int_as_float(0x7fffffff);  // W[0][.], and every image that it is in
+    }
   }
   __syncthreads();  // ring, offsets and coefficients are read: their memory takes the warps' sums
   float* red = sK;                 // [warps][NR][COLS]

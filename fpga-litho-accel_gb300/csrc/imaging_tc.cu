@@ -944,7 +944,7 @@ int tc_check_flag(litho_ctx* ctx) {
   LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   if (v != 0) {
     LITHO_CUDA_TRY(ctx, cudaMemset(ctx->mx_d.p, 0, 256));
-    set_error(ctx, LITHO_ERR_TIMEOUT, "a tensor-core pipeline wait gave up (bounded mbarrier wait)");
+    set_error(ctx, LITHO_ERR_TIMEOUT, "a device-side wait gave up (bounded at about a second)");
     return LITHO_ERR_TIMEOUT;
   }
   return LITHO_OK;

@@ -45,14 +45,31 @@ extern "C" {
 #define LITHO_ERR_NOMEM        5  /* device or pinned allocation failed */
 #define LITHO_ERR_IO           6  /* file read/write failed (BIN / JSON helpers) */
 #define LITHO_ERR_UNSUPPORTED  7  /* size or mode outside what the library implements */
-#define LITHO_ERR_TIMEOUT      8  /* a bounded device-side wait gave up */
+#define LITHO_ERR_TIMEOUT      8  /* a bounded device-side wait gave up (below) */
+
+/* Bounded waits.  Kernels that wait for their own asynchronous copies, or for one
+ * another's CTAs inside one launch, do so for about a second at most; after that
+ * they leave, and a flag on the context is set.  A call on host pointers that can
+ * meet such a wait returns LITHO_ERR_TIMEOUT itself.  For device pointers and for
+ * litho_batch_plan_run the next litho_ctx_synchronize on the context does (it also
+ * clears the flag); a program that waits on its own stream alone has to call it to
+ * see the error.  What a call wrote is undefined then; where the window DFT's
+ * copies are what was lost, its images are NaN, and so are those of the context's
+ * further calls with such copies until the flag is cleared.  The calls concerned:
+ * LITHO_PREC_MIXED; LITHO_PREC_FP32 where a mask's rows are not whole 16-byte
+ * pieces (Lx % 4 != 0, or masks that do not start on 16 bytes; the flagless
+ * litho_image_noalloc shows it by NaN alone); litho_calc_kernels up to about
+ * tccSize 1200; the split-BF16 TCC. */
 
 #define LITHO_MEM_HOST   0
 #define LITHO_MEM_DEVICE 1
 
 /* Arithmetic of the imaging pipeline.
  * LITHO_PREC_FP32  : window DFT, FFTs, intensity sum and interpolation in FP32
- *                    on the CUDA cores (the plain path).
+ *                    on the CUDA cores (the plain path).  Rows that are not
+ *                    whole 16-byte pieces are read by whole 16-byte granules: up
+ *                    to 12 bytes before and after the masks, which any CUDA
+ *                    allocation covers, are read too and dropped.
  * LITHO_PREC_MIXED : for supports Ny > 8 the interpolation (intensity band ->
  *                    image), and the window DFT of large batches where that is
  *                    faster, on the tensor cores with split-operand TF32 products
@@ -132,7 +149,7 @@ int litho_ctx_stage_times(litho_ctx* ctx, double* ms, long long* launches, int r
  * takes the kernel's bulk-copy form, the one that waits).  The waits then give up
  * after their limit (about one second), the kernel waits for what is in flight and
  * leaves, and the call (or the next litho_ctx_synchronize, for device pointers)
- * returns LITHO_ERR_TIMEOUT; the images of that call are undefined.  -1, the
+ * returns LITHO_ERR_TIMEOUT; the images of that call are NaN.  -1, the
  * default, turns the hook off.  The value is read when a window DFT is launched
  * (and baked into a batch plan's graph when the plan is created).  For tests of
  * the error path only. */
@@ -254,7 +271,8 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
 /* device slot of item i's mask (mLy x mLx float32) and image (L x L float32) */
 float* litho_batch_plan_mask(litho_batch_plan* plan, int i);
 float* litho_batch_plan_image(litho_batch_plan* plan, int i);
-/* image every item: one graph launch (or the plain launch sequence) on the context's stream */
+/* image every item: one graph launch (or the plain launch sequence) on the context's stream; a bounded
+ * wait that gives up is reported by the next litho_ctx_synchronize (LITHO_ERR_TIMEOUT) */
 int litho_batch_plan_run(litho_batch_plan* plan);
 /* JSON description of the tuned choices per size class; returns the length written */
 int litho_batch_plan_describe(const litho_batch_plan* plan, char* buf, int cap);
