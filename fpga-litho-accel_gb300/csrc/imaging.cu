@@ -1060,9 +1060,11 @@ int run_fft_mask(litho_ctx* ctx, const float* mask, int Lx, int Ly, float* mskf_
 // scratch (used by the allocation-free entry point in noalloc.cu).  Launches
 // only; it allocates nothing and records nothing on a context.
 // ---------------------------------------------------------------------------
+// kernels interleaved; also, the flag of the window's bounded waits starts every call at zero
 __global__ void pack_planes_kernel(const float* __restrict__ kr, const float* __restrict__ ki, int n,
-                                   float2* __restrict__ out) {
+                                   float2* __restrict__ out, int* __restrict__ err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *err = 0;
   if (i < n) out[i] = make_float2(kr[i], ki[i]);
 }
 
@@ -1128,7 +1130,7 @@ cudaError_t image_pipeline_noctx(cudaStream_t s, const ImgPlan& p, const float* 
   float* fcoef = reinterpret_cast<float*>(scratch + off[7]);
   const int KD = (2 * g.Nx + 1) * (2 * g.Ny + 1), ND = 2 * g.Nx + 1;
   cudaError_t e;
-  pack_planes_kernel<<<(g.nk * KD + 255) / 256, 256, 0, s>>>(krn_r, krn_i, g.nk * KD, krn);
+  pack_planes_kernel<<<(g.nk * KD + 255) / 256, 256, 0, s>>>(krn_r, krn_i, g.nk * KD, krn, err);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(sc, scales, g.nk * sizeof(float), cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
   twF_init_kernel<<<dim3((g.Lx + 127) / 128, ND), 128, 0, s>>>(twF, g.Lx, g.Fx, ND);

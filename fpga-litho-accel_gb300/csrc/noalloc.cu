@@ -21,10 +21,12 @@
 // call this entry point again on that device, since the cached address would
 // then name memory of a context that no longer exists.
 // All calls on a device share the array and it keeps the previous call's
-// contents: every region is fully written before it is read in a call, so
-// nothing has to start at zero, but calls whose work overlaps on the GPU
-// (different streams, or different host threads) race on the array and must be
-// serialised by the caller.
+// contents: every region is fully written before it is read in a call (the flag
+// of the window's bounded waits is its first word, cleared by each call), so
+// nothing has to start at zero.  A wait that gives up (a copy that does not land
+// in a second) makes the image NaN; the status cannot tell, as nothing waits for
+// the work here.  Calls whose work overlaps on the GPU (different streams, or
+// different host threads) race on the array and must be serialised by the caller.
 #include "litho_internal.cuh"
 
 #include <mutex>
