@@ -309,7 +309,7 @@ int run_band_tcc(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const lit
     const int IPW = 32 / (2 * g.Nx);
     decltype(&band_tcc_kernel<1>) k = band_kernel_for(g.Nx);
     auto smem_for = [&](int nw) { return ((size_t)most + (size_t)nw * IPW * KDP) * sizeof(float2); };
-    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_for(BT_WARPS)));
+    LITHO_CUDA_TRY(ctx, allow_smem(k));
     // warps per CTA: the largest that still gives every SM a CTA (small batches take
     // smaller CTAs, so that the tasks spread over the whole GPU)
     int nw = 2;

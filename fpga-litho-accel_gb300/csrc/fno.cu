@@ -1904,7 +1904,7 @@ int launch_column(litho_fno* f, int B, int layer, const float2* Xin, float2* Gou
   litho_ctx* ctx = f->ctx;
   auto go = [&](auto* k, int G) {
     const size_t smem = column_smem(G, BWD);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k);
     if (e != cudaSuccess) return e;
     return launch_early(true, k, dim3(M, (B + G - 1) / G), THREADS, smem, ctx->stream, f->L, B, f->theta.as<float>(), layer,
                         Xin, Gout, modes_out, f->colF.as<uint4>(), f->colI.as<uint4>());
@@ -1955,11 +1955,6 @@ int launch_band_coef(litho_fno* f, int KB, int KBy, int batch, const float2* X, 
   return LITHO_OK;
 }
 
-int set_smem(litho_ctx* ctx, const void* fn, size_t bytes) {
-  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return LITHO_OK;
-}
-
 // forward pass over B masks; train keeps z_l and V_l for the backward pass.  From the second kernel on
 // each is launched early, here and in the passes below: it loads its tables and weights while the one
 // before it ends, and waits before it touches anything a pass writes (64 masks of 256 x 256, predict:
@@ -1968,9 +1963,9 @@ int forward(litho_fno* f, const float* masks, int B, bool train, float* images, 
   litho_ctx* ctx = f->ctx;
   const int L = f->L, rows = B * L;
   const float* th = f->theta.as<float>();
-  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<FWD_FIRST>, row_fwd_smem(L, false)));
-  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<FWD_MID>, row_fwd_smem(L, false)));
-  LITHO_RET(set_smem(ctx, (const void*)row_fwd_kernel<FWD_LAST>, row_fwd_smem(L, true)));
+  LITHO_CUDA_TRY(ctx, allow_smem(row_fwd_kernel<FWD_FIRST>));
+  LITHO_CUDA_TRY(ctx, allow_smem(row_fwd_kernel<FWD_MID>));
+  LITHO_CUDA_TRY(ctx, allow_smem(row_fwd_kernel<FWD_LAST>));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 2 * NL + 1);
   lift_dft_kernel<<<dft_blocks(rows), THREADS, rows_dft_smem(L), ctx->stream>>>(L, rows, th, masks, f->twL.as<float2>(),
                                                                                f->Xf.as<float2>(), Mrow);
@@ -2015,9 +2010,9 @@ int backward(litho_fno* f, const float* masks, const float* targets, int B) {
   const float* th = f->theta.as<float>();
   const BwdSmem ss(L, HEAD_SPEC), sl(L, HEAD_LIFT);
   const ProjSmem sp(L);
-  LITHO_RET(set_smem(ctx, (const void*)row_bwd_proj_kernel, sp.total));
-  LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_SPEC>, ss.total));
-  LITHO_RET(set_smem(ctx, (const void*)row_bwd_kernel<HEAD_LIFT>, sl.total));
+  LITHO_CUDA_TRY(ctx, allow_smem(row_bwd_proj_kernel));
+  LITHO_CUDA_TRY(ctx, allow_smem(row_bwd_kernel<HEAD_SPEC>));
+  LITHO_CUDA_TRY(ctx, allow_smem(row_bwd_kernel<HEAD_LIFT>));
   StageScope sc(ctx, LITHO_STAGE_SURROGATE, 3 * NL + 4);
   LITHO_CUDA_TRY(ctx, launch_loss(f, targets, B));
   LITHO_CUDA_TRY(ctx, cudaMemsetAsync(f->gpart.p, 0, (size_t)grid * Dn::N * sizeof(float), ctx->stream));

@@ -712,7 +712,7 @@ static cudaError_t launch_fi_rows_t(cudaStream_t s, const ImgPlan& p, const floa
                       (pre ? pre * raw + 16 : 0);
   auto k = pre == 2 ? fi_rows_kernel<MAXD, KMAJ, KPC, 2> : pre == 1 ? fi_rows_kernel<MAXD, KMAJ, KPC, 1>
                                                                     : fi_rows_kernel<MAXD, KMAJ, KPC, 0>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   // column blocks over the x' < 0 half; as many image groups as keep every CTA resident
   // at once (a second partial wave would double the time of the CTAs in it), each CTA
@@ -975,7 +975,7 @@ static int launch_socs_t(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, c
     smem = ((size_t)(2 * g.Ny + 1) * (N + 1) + N / 2 + KD) * sizeof(float2);
     k = socs_kernel<N>;
   }
-  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LITHO_CUDA_TRY(ctx, allow_smem(k));
   dim3 grid(p.ngroups, p.batch);
   StageScope sc(ctx, LITHO_STAGE_SOCS);
   LITHO_CUDA_TRY(ctx, launch_early(p.early, k, grid, N == 128 ? S128_THREADS : SOCS_THREADS, smem, ctx->stream, w.part,
@@ -1037,7 +1037,7 @@ static int run_fft_rows(litho_ctx* ctx, const float* in_r, const float2* in_c, i
   const int TR = fm_rows_per_cta(F), logF = 31 - __builtin_clz((unsigned)F);
   const size_t smem = ((size_t)TR * fm_stride(F) + F / 2) * sizeof(float2);
   auto k = logF >= 3 ? fft_rows_centred_kernel<3> : logF == 2 ? fft_rows_centred_kernel<2> : fft_rows_centred_kernel<1>;
-  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LITHO_CUDA_TRY(ctx, allow_smem(k));
   k<<<(nrows + TR - 1) / TR, FM_THREADS, smem, ctx->stream>>>(in_r, nullptr, in_c, nrows, len, logF, TR, scale, out_c,
                                                              out_r, out_i, ldo);
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
@@ -1106,7 +1106,7 @@ static cudaError_t noctx_socs_t(cudaStream_t s, const ImgPlan& p, const float2* 
     smem = ((size_t)(2 * g.Ny + 1) * (N + 1) + N / 2 + KD) * sizeof(float2);
     k = socs_kernel<N>;
   }
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   k<<<dim3(p.ngroups, p.batch), N == 128 ? S128_THREADS : SOCS_THREADS, smem, s>>>(win_part, p.nparts(), nullptr,
                                                                                  nullptr, g.Fx, g.Fy, g.Nx,

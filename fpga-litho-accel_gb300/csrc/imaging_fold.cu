@@ -446,7 +446,7 @@ static cudaError_t launch_win_fold_t(cudaStream_t s, const WinSet& G, const ImgG
                                      int nparts, int stall, int* err) {
   const size_t smem = win_fold_smem<NY>(g.Nx, G.rows);
   auto k = vec ? win_fold_kernel<NY, true> : win_fold_kernel<NY, false>;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   k<<<G.T.tile0[G.T.n], WinFold<NY>::THREADS, smem, s>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, win_part, nparts, stall, err);
   return cudaGetLastError();
@@ -627,7 +627,7 @@ static cudaError_t launch_fi_fold_t(cudaStream_t s, const ImgPlan& p, const floa
   const size_t smem = (size_t)std::min((nb + R - 1) / R, ff_stage(NY)) * (ff_stride(NY) * sizeof(float) + sizeof(int4));
   const bool vec = (g.Lx & 3) == 0 && ((reinterpret_cast<uintptr_t>(tm) | reinterpret_cast<uintptr_t>(images)) & 15) == 0;
   auto k = vec ? fi_fold_kernel<NY, true> : fi_fold_kernel<NY, false>;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   return launch_early(p.early, k, dim3(ncb, R, p.batch), FF_THREADS, smem, s, tm, g.Lx, g.Ly, g.Fy, g.Ny, coef, nb, images);
 }

@@ -159,7 +159,7 @@ constexpr int WP_CONS = 256;     // consumer threads
 constexpr int WP_RSR = 132;      // sR rows (fp32)
 constexpr int WP_MAX_STAGES = 12;
 constexpr int WP_TQ = 8;         // tile ring: tiles the producer may publish ahead of the slowest role
-constexpr size_t WP_SMEM_CAP = 227 * 1024;
+constexpr size_t WP_SMEM_CAP = SMEM_MOST;
 
 // epilogue buffer: sR [2Nx+1][RSR] fp32 (a multiple of 16 bytes)
 static inline size_t win_epi_bytes(int Nx) { return (size_t)(2 * Nx + 1) * WP_RSR * 4; }
@@ -1013,8 +1013,7 @@ static int launch_win_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, f
   const size_t fixed = 1024 + win_epi_bytes(g.Nx) + win_bar_bytes(WP_MAX_STAGES);
   const int S = (int)std::min<size_t>(WP_MAX_STAGES, (WP_SMEM_CAP - fixed) / P::STAGE_B);
   const size_t smem = 1024 + (size_t)S * P::STAGE_B + win_epi_bytes(g.Nx) + win_bar_bytes(S);
-  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(win_dft_tc_kernel<NBH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
+  LITHO_CUDA_TRY(ctx, allow_smem(win_dft_tc_kernel<NBH>));
   const int grid = std::min(tiles, ctx->sm_count);  // persistent: one CTA per SM
   StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
   win_dft_tc_kernel<NBH><<<grid, WP_THREADS, smem, ctx->stream>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, S, win_part, err);
@@ -1067,8 +1066,7 @@ static int launch_fi_tc(litho_ctx* ctx, const ImgPlan& p, const float* cyh, cons
   LITHO_RET(make_map(ctx, &mO, images, 3, g.Lx, g.Ly, p.batch, 32));  // one warp's 32-row store
   static_assert(FiTC<KBLK, BN>::SMEM <= 227 * 1024, "FI tiles exceed the shared memory of one CTA");
   const size_t smem = FiTC<KBLK, BN>::SMEM;
-  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(fi_tc_kernel<KBLK, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
+  LITHO_CUDA_TRY(ctx, allow_smem(fi_tc_kernel<KBLK, BN>));
   // persistent: one CTA per SM over all (row band, image, column tile) tiles
   const int ntile = (g.Lx + BN - 1) / BN, rows = (g.Ly + 127) / 128;
   const int ntiles = rows * p.batch * ntile;

@@ -232,6 +232,16 @@ cudaError_t launch_early(bool early, void (*k)(P...), dim3 grid, int threads, si
   return cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
+// Lets a kernel ask for all the dynamic shared memory there is beside its own `fixed` bytes of static.
+// The limit is an attribute of the kernel, which every thread of the process shares: set to what one
+// launch needs, it would refuse the larger launch that another thread has between its own setting and
+// its launch.
+constexpr int SMEM_MOST = 227 * 1024;
+template <typename... P>
+cudaError_t allow_smem(void (*k)(P...), int fixed = 0) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST - fixed);
+}
+
 ImgPlan make_plan(const ImgGeom& g, int batch, int sm_count);
 
 // SOCS conv grid used by the imaging entry points: pow2 >= 4 max(Nx, Ny) + 1, at least 32.

@@ -435,8 +435,7 @@ static int run_gemm(litho_ctx* ctx, const __nv_bfloat16* Ah, const __nv_bfloat16
   LITHO_RET(map_bf16(ctx, &mBh, Ah, Kp, n, BN, BK));  // B = A's first n rows
   LITHO_RET(map_bf16(ctx, &mBl, Al, Kp, n, BN, BK));
   static_assert(P::SMEM <= 227 * 1024, "GEMM stages exceed the shared memory of one CTA");
-  LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(gemm_bf16x3_kernel<BN, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)P::SMEM));
+  LITHO_CUDA_TRY(ctx, allow_smem(gemm_bf16x3_kernel<BN, BK>));
   gemm_bf16x3_kernel<BN, BK><<<t->ctas, GB_THREADS, P::SMEM, ctx->stream>>>(
       mAh, mAl, mBh, mBl, t->segs, t->seg_begin, t->tiles, 2 * n, n, C, ldc, t->part.as<float>(), err);
   LITHO_CUDA_TRY(ctx, cudaGetLastError());

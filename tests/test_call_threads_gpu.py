@@ -50,15 +50,6 @@ def _surrogate(side, B):
     return make
 
 
-def _solve(n):
-    def make(ctx):
-        rng = np.random.default_rng(n)
-        q = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
-        got = []
-        return lambda: got.__setitem__(slice(None), [ctx.calc_kernels(q + q.conj().T, 4)[0]]), lambda: np.stack(got)
-    return make
-
-
 def _sets():
     import litho_gb300 as L
     return {
@@ -70,11 +61,10 @@ def _sets():
         "ragged": (400, [_imager(6, 6, B, 303, 411, L.PREC_FP32, L.BAND_FFT) for B in (1, 30, 200)]),
         "spectra": (60, [_spectrum(s) for s in (60, 500, 1000, 2000)]),
         "surrogates": (60, [_surrogate(64, 3), _surrogate(128, 2), _surrogate(256, 1)]),
-        "solves": (40, [_solve(n) for n in (65, 130, 20, 260)]),
     }
 
 
-@pytest.mark.parametrize("name", ["batches", "supports", "large", "ragged", "spectra", "surrogates", "solves"])
+@pytest.mark.parametrize("name", ["batches", "supports", "large", "ragged", "spectra", "surrogates"])
 def test_calls_at_once(name):
     import litho_gb300 as L
     rounds, makers = _sets()[name]
