@@ -1366,7 +1366,7 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
   // Z (nk*n double); inverse-iteration scratch (large n only: IV_CHUNK * 6n double);
   // Y (nk*n double2)
   const size_t iv_smem = (size_t)5 * n * sizeof(double) + n;
-  const bool iv_in_smem = iv_smem <= 200 * 1024;
+  const bool iv_in_smem = iv_smem <= 200 * 1024;  // (the solver kernels' own static shared memory: under 8 KB)
   constexpr int IV_CHUNK = 64;
   const size_t iv_scratch = iv_in_smem ? 0 : (size_t)IV_CHUNK * 6 * n * sizeof(double);
   const size_t vpack_bytes = (size_t)n * (n - 1) / 2 * sizeof(double2) + sizeof(double2);
@@ -1417,9 +1417,7 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
       LITHO_RET(tc_err_flag_public(ctx, &err));
       unsigned* count = reinterpret_cast<unsigned*>(td_part + 2 * G);
       LITHO_CUDA_TRY(ctx, cudaMemsetAsync(count, 0, sizeof(unsigned), ctx->stream));
-      // the limit, not this matrix's size: the attribute is shared by every thread that solves
-      LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)TD_MAX_SMEM));
+      LITHO_CUDA_TRY(ctx, allow_smem(tridiag_kernel, SMEM_MOST - (int)TD_MAX_SMEM));
       const double2* Ac = A;
       double2 *xg = td_vec, *rowbuf = td_vec + 2 * (size_t)n;
       int nn_ = n;
@@ -1443,8 +1441,7 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
     LITHO_CUDA_TRY(ctx, launch_clusters(multisect_kernel, nk, nk * MS_CMAX <= ctx->sm_count ? MS_CMAX : 1, MS_THREADS, 0,
                                         ctx->stream, (const double*)d, (const double*)e, (const double*)e2, n, ev));
     if (iv_in_smem) {
-      LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(invvec_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)iv_smem));
+      LITHO_CUDA_TRY(ctx, allow_smem(invvec_kernel<true>, 1024));
       invvec_kernel<true><<<nk, IV_THREADS, iv_smem, ctx->stream>>>(d, e, n, 0, ev, Z, nullptr);
     } else {
       for (int j0 = 0; j0 < nk; j0 += IV_CHUNK)
@@ -1459,8 +1456,7 @@ extern "C" int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize
     // of five, 783 on six and 710 on four)
     const int bc = std::max(1, std::min({BK_CMAX, ctx->sm_count * 4 / 5 / nk, (n + 31) / 32}));
     const size_t bt_smem = backtransform_smem(n, bc);
-    LITHO_CUDA_TRY(ctx, cudaFuncSetAttribute(backtransform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)backtransform_smem(8192, 1)));  // the largest (every thread's)
+    LITHO_CUDA_TRY(ctx, allow_smem(backtransform_kernel, 8 * 1024));
     LITHO_CUDA_TRY(ctx, launch_clusters(backtransform_kernel, nk, bc, WY_THREADS, bt_smem, ctx->stream, cvpack, n, cTg,
                                         (const double*)Z, Y));
     LITHO_CUDA_TRY(ctx, cudaGetLastError());
