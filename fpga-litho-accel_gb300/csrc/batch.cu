@@ -95,6 +95,8 @@ static int run_class(litho_batch_plan* bp, int ci) {
   std::stable_sort(sb.begin(), sb.end(), [](const SubBatch* a, const SubBatch* b) {
     return (size_t)a->count * a->mLx * a->mLy > (size_t)b->count * b->mLx * b->mLy;
   });
+  const float2* twF = nullptr;  // the interpolation rows read it before they wait: made before this stage
+  LITHO_RET(fi_twiddles(ctx, class_geom(c, c.convN), &twF));
   std::vector<WinPart> parts;
   int nparts = 1;
   for (const SubBatch* s : sb) {
