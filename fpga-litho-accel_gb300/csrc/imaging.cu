@@ -1157,8 +1157,7 @@ int image_pipeline(litho_ctx* ctx, const ImgGeom& g, int batch, const float* mas
   const bool tc = precision == LITHO_PREC_MIXED && fi_tc_serves(g);
   const bool band = use_band_tcc(ctx, ks, batch);
   ImgPlan p = make_plan(g, batch, ctx->sm_count);
-  // (the stall hook is the folded kernel's)
-  const bool win_tc = precision == LITHO_PREC_MIXED && ctx->test_stall_chunk < 0 && win_tc_serves(g, batch) &&
+  const bool win_tc = precision == LITHO_PREC_MIXED && win_tc_serves(g, batch) &&
                       (reinterpret_cast<uintptr_t>(masks) & 15) == 0;
   if (win_tc) win_tc_plan(p);
   if (band) {

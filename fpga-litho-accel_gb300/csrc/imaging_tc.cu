@@ -181,7 +181,8 @@ static inline size_t win_bar_bytes(int S) {
 template <int NBH>
 __global__ void __launch_bounds__(WP_THREADS, 1) win_dft_tc_kernel(const __grid_constant__ WinGeo G, int Fx, int Fy,
                                                                    int Nx, int Ny, int S,
-                                                                   float2* __restrict__ win_part, int* __restrict__ err) {
+                                                                   float2* __restrict__ win_part, int* __restrict__ err,
+                                                                   int stall_at) {
   using P = WinTC<NBH>;
   early_next();
   extern __shared__ unsigned char smraw[];
@@ -281,6 +282,10 @@ __global__ void __launch_bounds__(WP_THREADS, 1) win_dft_tc_kernel(const __grid_
         int g, img, rb, cs, c0, c1;
         decode(t, g, img, rb, cs, c0, c1);
         for (int c = c0; c < c1; ++c, ++q) {
+          if (q == stall_at) {  // error-path test hook: the producer is lost here
+            ok = false;
+            break;
+          }
           if (q >= S && !mbar_wait_ab(&empty[s], ph ^ 1u, abort)) {
             *abort = 1;
             ok = false;
@@ -529,6 +534,14 @@ __global__ void __launch_bounds__(WP_THREADS, 1) win_dft_tc_kernel(const __grid_
       for (int s = 0; s < S; ++s)
         if (last_issued[s] >= 0) mbar_wait(&full[s], (uint32_t)(last_issued[s] / S) & 1u, 200u);
     if (tid == 0) atomicExch(err, 1);
+    // W[0][0] of the CTA's tiles, reached or not: every image that they are of comes out NaN
+    for (int t = (int)blockIdx.x + tid * (int)gridDim.x; t < T; t += WP_THREADS * (int)gridDim.x) {
+      int g, img, rb, cs, c0, c1;
+      decode(t, g, img, rb, cs, c0, c1);
+      const int ncs = G.T.ncs[g], nps = G.T.rows[g] * ncs;
+      win_part[((size_t)(G.T.img0[g] + img) * nps + (rb * ncs + cs)) * (2 * Ny + 1) * (Nx + 1) + Ny * (Nx + 1)] =
+          make_float2(__int_as_float(0x7fffffff), 0.f);
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -1016,7 +1029,8 @@ static int launch_win_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, f
   LITHO_CUDA_TRY(ctx, allow_smem(win_dft_tc_kernel<NBH>));
   const int grid = std::min(tiles, ctx->sm_count);  // persistent: one CTA per SM
   StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
-  win_dft_tc_kernel<NBH><<<grid, WP_THREADS, smem, ctx->stream>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, S, win_part, err);
+  win_dft_tc_kernel<NBH><<<grid, WP_THREADS, smem, ctx->stream>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, S, win_part, err,
+                                                                  ctx->test_stall_chunk);
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
 }

@@ -156,7 +156,7 @@ struct litho_ctx {
   std::map<std::tuple<int, int, int, int>, std::shared_ptr<void>> gemm_tables;
   int tcc_force_bn = 0, tcc_force_bk = 64, tcc_force_sched = 0;  // litho_tcc_gemm_shape: bn > 0 bypasses the tuner
   // error-path test hook (litho_ctx_set_test_stall): >= 0 stops the copies of a mixed call's
-  // window DFT after that many steps of every warp; -1 = off
+  // window DFT after that many steps of every warp (folded) or CTA (tensor cores); -1 = off
   int test_stall_chunk = -1;
 };
 

@@ -311,8 +311,8 @@ class Context:
         self._check(_lib.litho_ctx_enable_timing(self.h, 1 if on else 0))
 
     def set_test_stall(self, chunk: int):
-        """Error-path test hook (litho_ctx_set_test_stall): chunk >= 0 makes the mixed window
-        DFT's TMA producer stop at that chunk, so the call returns LITHO_ERR_TIMEOUT; -1 = off."""
+        """Error-path test hook (litho_ctx_set_test_stall): chunk >= 0 makes the copies of a mixed
+        call's window DFT stop after that many steps, so the call returns LITHO_ERR_TIMEOUT; -1 = off."""
         self._check(_lib.litho_ctx_set_test_stall(self.h, int(chunk)))
 
     def set_band_method(self, method: int):

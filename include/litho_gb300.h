@@ -146,7 +146,8 @@ int litho_ctx_stage_times(litho_ctx* ctx, double* ms, long long* launches, int r
  * (common/file_io.cpp:137-150, litho.cpp:246-248).  chunk >= 0 makes every warp of
  * the window DFT of a LITHO_PREC_MIXED call stop issuing bulk copies after that
  * many steps of its share of the work, as if the rest had been lost (the call
- * takes the kernel's bulk-copy form, the one that waits).  The waits then give up
+ * takes the kernel's bulk-copy form, the one that waits; a window on the tensor
+ * cores stops every CTA's loads at that 64-column chunk of its share).  The waits then give up
  * after their limit (about one second), the kernel waits for what is in flight and
  * leaves, and the call (or the next litho_ctx_synchronize, for device pointers)
  * returns LITHO_ERR_TIMEOUT; the images of that call are NaN.  -1, the
