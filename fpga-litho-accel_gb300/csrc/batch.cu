@@ -36,8 +36,11 @@ struct ClassRun {
   int L = 0;
   const litho_kernel_set* ks = nullptr;
   int count = 0, maxBlocks = 0, tiles = 0;  // tiles: of one row split
+  long long pixels = 0, filled = 0, rows = 0;  // of the masks; mask rows and image rows
+  int tcRows = 0;                              // 128-row blocks of the tallest mask (tensor-core window)
+  bool tc = false;                             // window on the tensor cores first (plan_win_tc)
   float* images = nullptr;
-  DevBuf win, band, tmbuf, wsum;
+  DevBuf win, band, tmbuf, wsum, form;
   int convN = 0, kpg = 1, colSplits = 1, splits0 = 1;  // convN == 0: the TCC band (band_tcc.cu)
   double tuned_ms = -1.0;
   int candidates = 0;
@@ -81,6 +84,19 @@ static int default_conv(int Nx, int Ny) {
   return n < 32 ? 32 : n;
 }
 
+// Whether a class of a mixed plan asks the tensor cores for its window first.  They serve masks whose
+// values TF32 holds (binary ones) faster than the folded kernel above Ny = 8, where that one is bound by
+// its coefficient reads, and where masks fill half of their period's rows or less, so that half of the
+// rows it folds are outside; other masks they leave to it (win_dft_tc_kernel), which costs 4 to 12 us, as
+// much as there is to gain below these sizes.  us a run of a tuned plan: binary masks folded, and with the
+// tensor cores asked first; then grey ones.  64 of 2048^2 486, 464; 486, 495 (643 where no mask
+// is left).  40 of 2048^2 346, 330; 346, 354.  100 of 1024^2 in 2048^2 549, 507; 549, 561.  30 of them 189, 187;
+// 190, 198.  Up to Ny = 8: 100 of 512^2 in 1024^2 132, 123; 132, 136.  400 of them 409, 389; 409, 414.  1000 of
+// 256^2 in 512^2 258, 241; 258, 264.  256 of 768^2 in 1024^2 317, 314; 317, 324.
+static bool plan_win_tc(const ClassRun& c) {
+  return c.ks->Ny > 8 ? c.pixels >= 1ll << 26 : 2 * c.filled <= c.rows && c.pixels >= 3ll << 23;
+}
+
 // enqueue one class on the context's stream: windows of its sub-batches, SOCS,
 // interpolation
 static int run_class(litho_batch_plan* bp, int ci) {
@@ -97,18 +113,23 @@ static int run_class(litho_batch_plan* bp, int ci) {
   });
   const float2* twF = nullptr;  // the interpolation rows read it before they wait: made before this stage
   LITHO_RET(fi_twiddles(ctx, class_geom(c, c.convN), &twF));
-  std::vector<WinPart> parts;
-  int nparts = 1;
+  std::vector<WinPart> parts, tc;
+  int nparts = c.tc ? c.tcRows : 1;
   for (const SubBatch* s : sb) {
     const ImgGeom gw{s->mLx, s->mLy, c.L, c.L, Nx, Ny, c.ks->nk, c.convN};
     ImgPlan pw = make_plan(gw, s->count, ctx->sm_count);
     pw.colSplits = c.colSplits;
     nparts = std::max(nparts, pw.nparts());
     parts.push_back(WinPart{pw, s->masks, s->first_in_class});
+    win_tc_plan(pw);
+    tc.push_back(WinPart{pw, s->masks, s->first_in_class});
   }
-  for (size_t i = 0; i < parts.size(); i += WIN_MAX_SIZES)
-    LITHO_RET(run_win_dft(ctx, parts.data() + i, (int)std::min<size_t>(WIN_MAX_SIZES, parts.size() - i),
-                          c.win.as<float2>(), nparts, bp->precision));
+  int* form = c.tc ? c.form.as<int>() : nullptr;
+  for (size_t i = 0; i < parts.size(); i += WIN_MAX_SIZES) {
+    const int n = (int)std::min<size_t>(WIN_MAX_SIZES, parts.size() - i);
+    if (form) LITHO_RET(run_win_dft_tc(ctx, tc.data() + i, n, c.win.as<float2>(), nparts, form));
+    LITHO_RET(run_win_dft(ctx, parts.data() + i, n, c.win.as<float2>(), nparts, bp->precision, form));
+  }
   const bool band = c.convN == 0;
   ImgPlan p = make_plan(class_geom(c, band ? default_conv(Nx, Ny) : c.convN), c.count, ctx->sm_count);
   p.kpg = band ? c.ks->nk : std::min(c.kpg, c.ks->nk);
@@ -231,7 +252,8 @@ static int tune_class(litho_batch_plan* bp, int ci) {
   for (int k : {2, 3, 4, 6, 8, 12})
     if (k <= c.ks->nk) kpgs.push_back(k);
   if (kpgs.empty()) kpgs.push_back(1);
-  const std::vector<int> splits{c.splits0, 2 * c.splits0};
+  std::vector<int> splits{c.splits0};
+  if (!c.tc) splits.push_back(2 * c.splits0);  // (the masks are zero here: the tensor cores do them)
   // the best candidate of each band form (FFT grids, TCC band) ...
   TuneVal best_fft{convs[0], kpgs[0], 1, 1e30}, best_tcc{0, kpgs[0], 1, 1e30};
   for (int cn : convs)
@@ -343,6 +365,10 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
     const int blocks = make_plan(gw, s.count, ctx->sm_count).rowBlocks;
     c.maxBlocks = std::max(c.maxBlocks, blocks);
     c.tiles += blocks * s.count;
+    c.pixels += (long long)s.count * s.mLx * s.mLy;
+    c.filled += (long long)s.count * s.mLy;
+    c.rows += (long long)s.count * c.L;
+    c.tcRows = std::max(c.tcRows, (s.mLy + 127) / 128);
   }
   for (auto& c : bp->classes) image_floats += (size_t)c.count * c.L * c.L;
   int rc = bp->mask_pool.ensure(ctx, mask_floats * sizeof(float));
@@ -382,7 +408,12 @@ int litho_batch_plan_create(litho_ctx* ctx, const litho_kernel_set* const* sets,
     // row splits of the window DFTs: as one launch of the class's tiles would take, or twice as many
     c.splits0 = win_fold_splits(class_geom(c, c.convN), c.maxBlocks, c.tiles, ctx->sm_count);
     c.colSplits = c.splits0;
-    rc = c.win.ensure(ctx, (size_t)c.count * c.maxBlocks * 2 * c.splits0 * KY * (Nx + 1) * sizeof(float2));
+    if (precision == LITHO_PREC_MIXED && plan_win_tc(c)) {
+      c.tc = true;
+      rc = c.form.ensure(ctx, 256);
+    }
+    const int most = std::max(c.maxBlocks * 2 * c.splits0, c.tcRows);
+    if (rc == LITHO_OK) rc = c.win.ensure(ctx, (size_t)c.count * most * KY * (Nx + 1) * sizeof(float2));
     const int groups = std::max(c.ks->nk, c.ks->band_nc);  // the FFT form's kernel groups or the band chunks
     if (rc == LITHO_OK) rc = c.band.ensure(ctx, (size_t)c.count * groups * KY * (4 * Nx + 1) * sizeof(float2));
     const ImgGeom g = class_geom(c, c.convN);
@@ -498,6 +529,7 @@ int litho_batch_plan_destroy(litho_batch_plan* bp) {
     c.band.release();
     c.tmbuf.release();
     c.wsum.release();
+    c.form.release();
   }
   bp->mask_pool.release();
   bp->image_pool.release();

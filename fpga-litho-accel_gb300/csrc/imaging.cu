@@ -929,7 +929,7 @@ static int fold_table(litho_ctx* ctx, const ImgGeom& g, int kind, size_t floats,
   return LITHO_OK;
 }
 
-int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int precision) {
+int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int precision, const int* form) {
   const ImgGeom& g0 = parts[0].plan.g;
   if (g0.Nx > 16 || g0.Ny > 16) {
     set_error(ctx, LITHO_ERR_UNSUPPORTED, "window DFT supports Nx, Ny <= 16 (got %d, %d)", g0.Nx, g0.Ny);
@@ -954,7 +954,7 @@ int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, i
   LITHO_RET(tc_err_flag_public(ctx, &err));
   StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
   LITHO_CUDA_TRY(ctx, launch_win_fold(ctx->stream, parts, n, coef, twF, win_part, nparts,
-                                      precision == LITHO_PREC_MIXED ? ctx->test_stall_chunk : -1, err));
+                                      precision == LITHO_PREC_MIXED ? ctx->test_stall_chunk : -1, err, form));
   return LITHO_OK;
 }
 
@@ -1140,7 +1140,7 @@ cudaError_t image_pipeline_noctx(cudaStream_t s, const ImgPlan& p, const float* 
   const WinPart part{p, mask, 0};
   const float* wc = wcoef;
   const float2* wt = twF;
-  if ((e = launch_win_fold(s, &part, 1, &wc, &wt, win_part, p.nparts(), -1, err)) != cudaSuccess) return e;
+  if ((e = launch_win_fold(s, &part, 1, &wc, &wt, win_part, p.nparts(), -1, err, nullptr)) != cudaSuccess) return e;
   switch (g.convN) {
     case 32: e = noctx_socs_t<32>(s, p, win_part, krn, sc, band_part); break;
     case 64: e = noctx_socs_t<64>(s, p, win_part, krn, sc, band_part); break;
@@ -1177,9 +1177,9 @@ int image_pipeline(litho_ctx* ctx, const ImgGeom& g, int batch, const float* mas
   if (win_tc) {
     const float2* twF = nullptr;  // the interpolation rows read it before they wait: made before this stage
     LITHO_RET(fi_twiddles(ctx, g, &twF));
-    LITHO_RET(run_win_dft_tc(ctx, p, masks, ctx->win_part.as<float2>()));
+    LITHO_RET(run_win_dft_tc(ctx, &part, 1, ctx->win_part.as<float2>(), p.nparts(), nullptr));
   } else {
-    LITHO_RET(run_win_dft(ctx, &part, 1, ctx->win_part.as<float2>(), p.nparts(), precision));
+    LITHO_RET(run_win_dft(ctx, &part, 1, ctx->win_part.as<float2>(), p.nparts(), precision, nullptr));
   }
   WindowSrc w;
   w.part = ctx->win_part.as<float2>();

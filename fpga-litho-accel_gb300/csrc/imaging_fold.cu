@@ -127,12 +127,16 @@ struct WinSet {
 template <int NY, bool VEC>
 __global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __grid_constant__ WinSet G, int Fx, int Fy, int Nx,
                                                                  int Ny, float2* __restrict__ win_part, int nparts,
-                                                                 int stall, int* err) {
+                                                                 int stall, int* err, const int* __restrict__ form) {
   using P = WinFold<NY>;
   constexpr int CPL = P::CPL, COLS = P::COLS, KS = P::KS;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   early_next();
+  if (form != nullptr) {  // (launched early, then)
+    early_wait(form);
+    if (*form == 0) return;  // the tensor cores have done these masks
+  }
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm) + warp * P::ST;
   float* zero = sm + P::BARS;
   float2* sTw = reinterpret_cast<float2*>(zero + P::ZERO);    // [Nx+1][TS]
@@ -443,19 +447,21 @@ cudaError_t win_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef) {
 
 template <int NY>
 static cudaError_t launch_win_fold_t(cudaStream_t s, const WinSet& G, const ImgGeom& g, bool vec, float2* win_part,
-                                     int nparts, int stall, int* err) {
+                                     int nparts, int stall, int* err, const int* __restrict__ form) {
   const size_t smem = win_fold_smem<NY>(g.Nx, G.rows);
   auto k = vec ? win_fold_kernel<NY, true> : win_fold_kernel<NY, false>;
   const cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
-  k<<<G.T.tile0[G.T.n], WinFold<NY>::THREADS, smem, s>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, win_part, nparts, stall, err);
-  return cudaGetLastError();
+  return launch_early(form != nullptr, k, dim3((unsigned)G.T.tile0[G.T.n]), WinFold<NY>::THREADS, smem, s, G, g.Fx, g.Fy, g.Nx,
+                      g.Ny, win_part, nparts, stall, err, form);
 }
 
 // n <= WIN_MAX_SIZES mask sizes of one period and support, nparts partials per image; err: the
-// timeout flag; stall >= 0: the error-path test hook
+// timeout flag; stall >= 0: the error-path test hook; form: nullptr, or a device word that says whether
+// the launch has masks to do (run_win_dft_tc)
 cudaError_t launch_win_fold(cudaStream_t s, const WinPart* parts, int n, const float* const* coef,
-                            const float2* const* twF, float2* win_part, int nparts, int stall, int* err) {
+                            const float2* const* twF, float2* win_part, int nparts, int stall, int* err,
+                            const int* __restrict__ form) {
   const ImgGeom& g0 = parts[0].plan.g;
   WinSet G = {};
   G.T.n = n;
@@ -477,11 +483,11 @@ cudaError_t launch_win_fold(cudaStream_t s, const WinPart* parts, int n, const f
     vec = vec && (p.g.Lx & 3) == 0 && (reinterpret_cast<uintptr_t>(parts[i].masks) & 15) == 0;
   }
   switch (wf_ny(g0.Ny)) {
-    case 2: return launch_win_fold_t<2>(s, G, g0, vec, win_part, nparts, stall, err);
-    case 4: return launch_win_fold_t<4>(s, G, g0, vec, win_part, nparts, stall, err);
-    case 8: return launch_win_fold_t<8>(s, G, g0, vec, win_part, nparts, stall, err);
-    case 12: return launch_win_fold_t<12>(s, G, g0, vec, win_part, nparts, stall, err);
-    default: return launch_win_fold_t<16>(s, G, g0, vec, win_part, nparts, stall, err);
+    case 2: return launch_win_fold_t<2>(s, G, g0, vec, win_part, nparts, stall, err, form);
+    case 4: return launch_win_fold_t<4>(s, G, g0, vec, win_part, nparts, stall, err, form);
+    case 8: return launch_win_fold_t<8>(s, G, g0, vec, win_part, nparts, stall, err, form);
+    case 12: return launch_win_fold_t<12>(s, G, g0, vec, win_part, nparts, stall, err, form);
+    default: return launch_win_fold_t<16>(s, G, g0, vec, win_part, nparts, stall, err, form);
   }
 }
 

@@ -163,11 +163,14 @@ constexpr size_t WP_SMEM_CAP = SMEM_MOST;
 
 // epilogue buffer: sR [2Nx+1][RSR] fp32 (a multiple of 16 bytes)
 static inline size_t win_epi_bytes(int Nx) { return (size_t)(2 * Nx + 1) * WP_RSR * 4; }
-// The masks' and twiddles' tensor maps, the row twiddles and the tiles of one mask size.
+// The mask sizes of one launch (they share the period, the kernels and the partial array): per size the
+// masks' and twiddles' tensor maps, the row twiddles, the masks and their pixels.
 struct WinGeo {
-  CUtensorMap mM[1];  // masks [img][Ly][Lx]
-  CUtensorMap mB[1];  // twiddles [hi; lo] x Lx
-  const float2* ytab[1];
+  CUtensorMap mM[WIN_MAX_SIZES];  // masks [img][Ly][Lx]
+  CUtensorMap mB[WIN_MAX_SIZES];  // twiddles [hi; lo] x Lx
+  const float2* ytab[WIN_MAX_SIZES];
+  const float* masks[WIN_MAX_SIZES];
+  long long px[WIN_MAX_SIZES];
   WinTiles T;                  // widths, row blocks, splits, first images and tiles (win_tiles.hpp)
 };
 
@@ -181,10 +184,26 @@ static inline size_t win_bar_bytes(int S) {
 template <int NBH>
 __global__ void __launch_bounds__(WP_THREADS, 1) win_dft_tc_kernel(const __grid_constant__ WinGeo G, int Fx, int Fy,
                                                                    int Nx, int Ny, int S,
-                                                                   float2* __restrict__ win_part, int* __restrict__ err,
-                                                                   int stall_at) {
+                                                                   float2* __restrict__ win_part, int nparts,
+                                                                   int* __restrict__ err, int stall_at,
+                                                                   int* __restrict__ form) {
   using P = WinTC<NBH>;
   early_next();
+  // With `form`, a launch of the folded kernel follows that does what this one leaves.  Masks with a value
+  // that TF32 does not hold take twice the time here (their tiles are split in place and multiplied once
+  // more), so a launch whose samples show one leaves its masks to it.  Every CTA looks at the same pixels.
+  if (form != nullptr) {
+    uint32_t low = 0;
+    for (int g = 0; g < G.T.n; ++g) {  // two runs of 32 pixels a warp, spread over the size's masks
+      const float* m = G.masks[g] + min((long long)(threadIdx.x & 31), G.px[g] - 1);
+      const long long step = max(0ll, G.px[g] - 32) / (2 * (WP_THREADS / 32));
+      const int i = 2 * (threadIdx.x >> 5);
+      low |= __float_as_uint(__ldg(m + step * i)) | __float_as_uint(__ldg(m + step * (i + 1)));
+    }
+    const int grey = __syncthreads_or((low & 0x1FFFu) != 0u);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *form = grey;
+    if (grey) return;
+  }
   extern __shared__ unsigned char smraw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
   constexpr int RS = WP_RSR;
@@ -472,8 +491,11 @@ __global__ void __launch_bounds__(WP_THREADS, 1) win_dft_tc_kernel(const __grid_
       const int y0 = 128 * rb;
       named_bar(2, 128);
       const int rows = G.T.rows[g], ncs = G.T.ncs[g];
-      const int nps = rows * ncs;
-      float2* out = win_part + ((size_t)(G.T.img0[g] + img) * nps + (rb * ncs + cs)) * KY * NU;
+      float2* parts = win_part + (size_t)(G.T.img0[g] + img) * nparts * KY * NU;
+      float2* out = parts + (size_t)(rb * ncs + cs) * KY * NU;
+      if (rb == 0 && cs == 0)  // the partials that the image's size does not use
+        for (int e = etid; e < (nparts - rows * ncs) * KY * NU; e += 128)
+          parts[(size_t)rows * ncs * KY * NU + e] = make_float2(0.f, 0.f);
       // one thread per (|v|, u): four row sums give both outputs +v and -v
       //   S1 = sum c tx, S2 = sum s ty, S3 = sum c ty, S4 = sum s tx
       //   (+v): (S1 - S2, S3 + S4)    (-v): (S1 + S2, S4 - S3)
@@ -538,8 +560,8 @@ __global__ void __launch_bounds__(WP_THREADS, 1) win_dft_tc_kernel(const __grid_
     for (int t = (int)blockIdx.x + tid * (int)gridDim.x; t < T; t += WP_THREADS * (int)gridDim.x) {
       int g, img, rb, cs, c0, c1;
       decode(t, g, img, rb, cs, c0, c1);
-      const int ncs = G.T.ncs[g], nps = G.T.rows[g] * ncs;
-      win_part[((size_t)(G.T.img0[g] + img) * nps + (rb * ncs + cs)) * (2 * Ny + 1) * (Nx + 1) + Ny * (Nx + 1)] =
+      const size_t part = (size_t)(G.T.img0[g] + img) * nparts + (rb * G.T.ncs[g] + cs);
+      win_part[part * (2 * Ny + 1) * (Nx + 1) + Ny * (Nx + 1)] =
           make_float2(__int_as_float(0x7fffffff), 0.f);
     }
   }
@@ -1006,21 +1028,28 @@ static int win_tc_tables(litho_ctx* ctx, const ImgGeom& g, float** twh, float** 
 }
 
 template <int NBH>
-static int launch_win_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part, int* err) {
+static int launch_win_tc(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int* err, int* form) {
   WinGeo G;
   std::memset(&G, 0, sizeof(G));
-  const ImgGeom& g = p.g;
-  float *twh = nullptr, *yt = nullptr;
-  LITHO_RET(win_tc_tables<NBH>(ctx, g, &twh, &yt));
-  LITHO_RET(make_map(ctx, &G.mM[0], masks, 3, g.Lx, g.Ly, p.batch, 128));
-  LITHO_RET(make_map(ctx, &G.mB[0], twh, 2, g.Lx, 2 * NBH, 1, 2 * NBH));  // hi rows, then lo rows
-  G.ytab[0] = reinterpret_cast<const float2*>(yt);
-  G.T.n = 1;
-  G.T.Lx[0] = g.Lx;
-  G.T.rows[0] = p.rowBlocks;
-  G.T.ncs[0] = p.colSplits;
-  const int tiles = p.rowBlocks * p.batch * p.colSplits;
-  G.T.tile0[1] = tiles;
+  G.T.n = n;
+  for (int i = 0; i < n; ++i) {
+    const ImgPlan& p = parts[i].plan;
+    const ImgGeom& g = p.g;
+    float *twh = nullptr, *yt = nullptr;
+    LITHO_RET(win_tc_tables<NBH>(ctx, g, &twh, &yt));
+    LITHO_RET(make_map(ctx, &G.mM[i], parts[i].masks, 3, g.Lx, g.Ly, p.batch, 128));
+    LITHO_RET(make_map(ctx, &G.mB[i], twh, 2, g.Lx, 2 * NBH, 1, 2 * NBH));  // hi rows, then lo rows
+    G.ytab[i] = reinterpret_cast<const float2*>(yt);
+    G.masks[i] = parts[i].masks;
+    G.px[i] = (long long)p.batch * g.Lx * g.Ly;
+    G.T.Lx[i] = g.Lx;
+    G.T.rows[i] = p.rowBlocks;
+    G.T.ncs[i] = p.colSplits;
+    G.T.img0[i] = parts[i].img0;
+    G.T.tile0[i + 1] = G.T.tile0[i] + p.rowBlocks * p.batch * p.colSplits;
+  }
+  const int tiles = G.T.tile0[n];
+  const ImgGeom& g = parts[0].plan.g;
   // as many ring stages as shared memory holds
   using P = WinTC<NBH>;
   const size_t fixed = 1024 + win_epi_bytes(g.Nx) + win_bar_bytes(WP_MAX_STAGES);
@@ -1029,8 +1058,8 @@ static int launch_win_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, f
   LITHO_CUDA_TRY(ctx, allow_smem(win_dft_tc_kernel<NBH>));
   const int grid = std::min(tiles, ctx->sm_count);  // persistent: one CTA per SM
   StageScope sc(ctx, LITHO_STAGE_WIN_DFT);
-  win_dft_tc_kernel<NBH><<<grid, WP_THREADS, smem, ctx->stream>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, S, win_part, err,
-                                                                  ctx->test_stall_chunk);
+  win_dft_tc_kernel<NBH><<<grid, WP_THREADS, smem, ctx->stream>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, S, win_part, nparts, err,
+                                                                  ctx->test_stall_chunk, form);
   LITHO_CUDA_TRY(ctx, cudaGetLastError());
   return LITHO_OK;
 }
@@ -1055,15 +1084,27 @@ void win_tc_plan(ImgPlan& p) {
   p.colSplits = 1;
 }
 
-int run_win_dft_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part) {
+// up to WIN_MAX_SIZES mask sizes that share the period, the kernels and the partial array, nparts partials
+// per image; form: nullptr, or a device word that says afterwards whether the masks are left to the
+// folded kernel
+int run_win_dft_tc(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int* form) {
+  const ImgGeom& g0 = parts[0].plan.g;
+  for (int i = 0; i < n; ++i) {
+    const ImgGeom& g = parts[i].plan.g;
+    if (n > WIN_MAX_SIZES || g.Fx != g0.Fx || g.Fy != g0.Fy || g.Nx != g0.Nx || g.Ny != g0.Ny ||
+        parts[i].plan.nparts() > nparts) {
+      set_error(ctx, LITHO_ERR_ARG, "window DFT mask sizes of one launch must share the period and the kernels");
+      return LITHO_ERR_ARG;
+    }
+  }
   int* err = nullptr;
   LITHO_RET(tc_err_flag(ctx, &err));
-  switch (nb_for(p.g.Nx)) {
-    case 8: return launch_win_tc<8>(ctx, p, masks, win_part, err);
-    case 16: return launch_win_tc<16>(ctx, p, masks, win_part, err);
-    case 24: return launch_win_tc<24>(ctx, p, masks, win_part, err);
-    case 32: return launch_win_tc<32>(ctx, p, masks, win_part, err);
-    default: return launch_win_tc<40>(ctx, p, masks, win_part, err);
+  switch (nb_for(g0.Nx)) {
+    case 8: return launch_win_tc<8>(ctx, parts, n, win_part, nparts, err, form);
+    case 16: return launch_win_tc<16>(ctx, parts, n, win_part, nparts, err, form);
+    case 24: return launch_win_tc<24>(ctx, parts, n, win_part, nparts, err, form);
+    case 32: return launch_win_tc<32>(ctx, parts, n, win_part, nparts, err, form);
+    default: return launch_win_tc<40>(ctx, parts, n, win_part, nparts, err, form);
   }
 }
 

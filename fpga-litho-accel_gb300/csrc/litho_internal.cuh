@@ -277,14 +277,15 @@ struct WinPart {
   int img0;
 };
 cudaError_t launch_win_fold(cudaStream_t s, const WinPart* parts, int n, const float* const* coef,
-                            const float2* const* twF, float2* win_part, int nparts, int stall, int* err);
+                            const float2* const* twF, float2* win_part, int nparts, int stall, int* err,
+                            const int* form);
 size_t fi_fold_coef_floats(const ImgGeom& g);
 cudaError_t fi_fold_coefs(cudaStream_t s, const ImgGeom& g, float* coef);
 cudaError_t launch_fi_fold(cudaStream_t s, const ImgPlan& p, const float* tm, const float* coef, float* images);
 
 // window DFT of up to WIN_MAX_SIZES mask sizes, nparts partials per image; precision: whether the
-// error-path test hook acts
-int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int precision);
+// error-path test hook acts; form: nullptr, or what run_win_dft_tc wrote just before
+int run_win_dft(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int precision, const int* form);
 int run_socs(litho_ctx* ctx, const ImgPlan& p, const WindowSrc& w, const float2* krn,
              const float* scales, float2* band_part, float* tmpImgp);
 int run_tmp_join(litho_ctx* ctx, const float* part, int ngroups, int n, float* tmpImgp);
@@ -320,7 +321,7 @@ bool use_band_tcc(const litho_ctx* ctx, const litho_kernel_set* ks, int batch);
 bool fi_tc_serves(const ImgGeom& g);
 bool win_tc_serves(const ImgGeom& g, int batch);
 void win_tc_plan(ImgPlan& p);
-int run_win_dft_tc(litho_ctx* ctx, const ImgPlan& p, const float* masks, float2* win_part);
+int run_win_dft_tc(litho_ctx* ctx, const WinPart* parts, int n, float2* win_part, int nparts, int* form);
 int run_fi_tc(litho_ctx* ctx, const ImgPlan& p, const float2* band_part, float* tmT, float* images);
 struct FiTcBufs {
   float *tmh, *tml, *t0;
