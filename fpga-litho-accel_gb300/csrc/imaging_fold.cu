@@ -41,7 +41,7 @@ __device__ __forceinline__ int4 fold_offsets(int b, int Lx, int Ly, int Fy) {
 // eight warps per SM; 132 at NY = 16, in two of four warps with a deeper ring.  (Two columns per lane and eight
 // warps above NY = 8: 16 masks of 1999 x 2001 254 us, now 227; 200 of 1280^2 1,050, now 957; 100 of
 // 1100^2 487, now 438; 10 of 2048^2 147, now 130; one 55.7, now 60.)
-constexpr int wf_cpl(int) { return 4; }
+constexpr int WF_CPL = 4;
 constexpr int wf_stride(int NY) { return 2 * NY; }
 constexpr int wf_warps(int NY) { return NY <= 8 ? 8 : 4; }
 constexpr int wf_st(int NY) { return NY <= 8 ? 4 : 8; }  // ring stages: three, seven base rows (2 KB each) of every warp in flight
@@ -61,7 +61,7 @@ __global__ void wf_coef_kernel(float* __restrict__ coef, int nb, int NY, int Ny,
 
 template <int NY>
 struct WinFold {
-  static constexpr int CPL = wf_cpl(NY), COLS = 32 * CPL, KS = wf_stride(NY), NR = 2 * NY + 1;
+  static constexpr int CPL = WF_CPL, COLS = 32 * CPL, KS = wf_stride(NY), NR = 2 * NY + 1;
   static constexpr int WARPS = wf_warps(NY), THREADS = 32 * WARPS, ST = wf_st(NY), AHEAD = (ST - 1) * WARPS;
   static constexpr int RB = COLS + 4;       // ring row (floats): the columns and one granule of misalignment
   static constexpr int RING = WARPS * ST * 4 * RB;
@@ -82,13 +82,9 @@ static size_t win_fold_smem(int Nx, int rows) {
   return (P::BARS + P::ZERO + tw + std::max(loop, sums)) * sizeof(float);
 }
 
-template <int BYTES>
-__device__ __forceinline__ void wf_copy_lane(float* dst, const void* src, bool ok) {  // zeros where !ok
-  const unsigned d = tc::smem_u32(dst);
-  if constexpr (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+__device__ __forceinline__ void wf_copy_lane(float* dst, const void* src, bool ok) {  // 16 bytes, zeros where !ok
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0)
+               : "memory");
 }
 // bulk copy global -> shared (16-byte aligned, whole 16 bytes), counted on an mbarrier
 __device__ __forceinline__ void wf_copy(float* dst, const void* src, int bytes, uint64_t* bar) {
@@ -98,9 +94,9 @@ __device__ __forceinline__ void wf_copy(float* dst, const void* src, int bytes, 
                : "memory");
 }
 
-// One CTA per (column block of 32 CPL columns, share of the base rows, image).  Row sums
+// One CTA per (column block of 128 columns, share of the base rows, image).  Row sums
 // C_n = sum_y m cos(2 pi n y'/Fy), S_n = sum_y m sin of every column: warp w takes the base rows
-// b0 + w, b0 + w + 8, ..; their four mask rows stream through the warp's own ring (rows and columns
+// b0 + w, b0 + w + WARPS, ..; their four mask rows stream through the warp's own ring (rows and columns
 // outside the mask as zeros), a lane folds its CPL columns and adds them into its 2NY+1 sums with
 // one broadcast load per four coefficients.  The warps' sums are then added in order and summed
 // over the columns with the column twiddles.
@@ -161,7 +157,7 @@ __global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __
     const float* base = M + (in ? CPL * lane : 0);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      wf_copy_lane<4 * CPL>(dst + k * P::RB, base + (off[k] >= 0 ? off[k] : 0), off[k] >= 0 && in);
+      wf_copy_lane(dst + k * P::RB, base + (off[k] >= 0 ? off[k] : 0), off[k] >= 0 && in);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   bool ok = VEC || __all_sync(0xffffffffu, *reinterpret_cast<volatile int*>(err) == 0);  // after a timeout, end quickly
@@ -236,17 +232,11 @@ __global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __
         asm volatile("cp.async.wait_group %0;" ::"n"(P::ST - 2) : "memory");
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          if constexpr (CPL == 4) {
-            const float4 v = *reinterpret_cast<const float4*>(src + k * P::RB + 4 * lane);
-            p[k][0] = v.x;
-            p[k][1] = v.y;
-            p[k][2] = v.z;
-            p[k][3] = v.w;
-          } else {
-            const float2 v = *reinterpret_cast<const float2*>(src + k * P::RB + 2 * lane);
-            p[k][0] = v.x;
-            p[k][1] = v.y;
-          }
+          const float4 v = *reinterpret_cast<const float4*>(src + k * P::RB + 4 * lane);
+          p[k][0] = v.x;
+          p[k][1] = v.y;
+          p[k][2] = v.z;
+          p[k][3] = v.w;
         }
         issue_vec(sOff[b - t0 + P::AHEAD], st == 0 ? P::ST - 1 : st - 1);  // the previous row's slot
       } else {
@@ -319,10 +309,8 @@ __global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __
   {
     float* r = red + (size_t)warp * P::NR * COLS;
     auto put = [&](int n, const float(&v)[CPL]) {
-      if constexpr (VEC && CPL == 4) {
+      if constexpr (VEC) {
         reinterpret_cast<float4*>(r + n * COLS)[lane] = make_float4(v[0], v[1], v[2], v[3]);
-      } else if constexpr (VEC) {
-        reinterpret_cast<float2*>(r + n * COLS)[lane] = make_float2(v[0], v[1]);
       } else {
 #pragma unroll
         for (int i = 0; i < CPL; ++i) r[n * COLS + lane + 32 * i] = lane + 32 * i < ncol ? v[i] : 0.f;
@@ -432,7 +420,7 @@ int win_fold_splits(const ImgGeom& g, int ncb, long long tiles, int sm_count) {
 
 // column blocks and row splits of a window DFT
 void win_fold_plan(ImgPlan& p, int sm_count) {
-  const int cols = 32 * wf_cpl(wf_ny(p.g.Ny));
+  const int cols = 32 * WF_CPL;
   p.rowBlocks = (p.g.Lx + cols - 1) / cols;
   p.colSplits = win_fold_splits(p.g, p.rowBlocks, (long long)p.rowBlocks * p.batch, sm_count);
 }
