@@ -35,6 +35,10 @@ namespace litho {
 // registers, forward FFT of the intensity, band output.  socs_kernel<N> uses the
 // warp-shuffle transforms of fft_warp.cuh and serves the 32 x 32 grid; the 64 and
 // 128 grids have their own kernels on the lane-group transforms of fft_lane8.cuh.
+// The groups' bands are stored last group first.  Kernels come by falling weight, and the
+// interpolation rows add the bands in the stored order: the first group's, as large as all the
+// others', is rounded once then, and not for each of them (calcSOCS of 512 x 512 with ten groups:
+// 2.07e-7 from 64 bits in the mean of twelve masks, and 1.83e-7).
 // ---------------------------------------------------------------------------
 constexpr int SOCS_THREADS = 256;
 
@@ -150,7 +154,7 @@ __global__ void __launch_bounds__(SOCS_THREADS) socs_kernel(
   __syncthreads();
   const int BW = 4 * Nx + 1;
   const float inv = 1.0f / ((float)N * (float)N);
-  float2* band = band_part + ((size_t)img * ngroups + g) * KY * BW;
+  float2* band = band_part + ((size_t)img * ngroups + (ngroups - 1 - g)) * KY * BW;
   for (int fy = warp; fy <= 2 * Ny; fy += 8) {
     float2 x[J];
 #pragma unroll
@@ -301,7 +305,7 @@ __global__ void __launch_bounds__(SOCS_THREADS) socs64_kernel(
   __syncthreads();
   const int BW = 4 * Nx + 1;
   const float inv = 1.0f / ((float)N * (float)N);
-  float2* band = band_part + ((size_t)img * ngroups + g) * KY * BW;
+  float2* band = band_part + ((size_t)img * ngroups + (ngroups - 1 - g)) * KY * BW;
   {
     const int fy = 8 * q + warp;
     const bool act = fy <= 2 * Ny;
@@ -464,7 +468,7 @@ __global__ void __launch_bounds__(S128_THREADS) socs128_kernel(
   __syncthreads();
   const int BW = 4 * Nx + 1;
   const float inv = 1.0f / ((float)N * (float)N);
-  float2* band = band_part + ((size_t)img * ngroups + g) * KY * BW;
+  float2* band = band_part + ((size_t)img * ngroups + (ngroups - 1 - g)) * KY * BW;
   for (int r0 = 0; r0 < KY; r0 += 32) {
     const int fy = r0 + sl;
     const bool act = fy <= 2 * Ny;
