@@ -105,9 +105,9 @@ __device__ __forceinline__ void wf_copy(float* dst, const void* src, int bytes, 
 // 16-byte granules and the lanes read their columns (lane + 32 i) past each row's misalignment;
 // every wait is bounded: a warp whose copies do not land in a second issues no more, waits for what
 // it has in flight, sets *err and makes its sums NaN, so that the images show it too; while *err is
-// set, warps issue nothing and end the same way.  (Measured, window stage: 256 aligned masks of 1024^2
-// 198 us with cp.async, 206 with bulk copies; 44 of 2048^2 184 and 231; 40 ragged 913 x 777 masks
-// 54 and 49, and 138 with plain loads.)
+// set, warps issue nothing and end the same way.  (Measured, window stage: 256 masks of 1024^2
+// 186 us with cp.async, 222 with bulk copies (the same masks off by four bytes); 44 of 2048^2, Ny = 16, 167
+// and 257; 40 ragged 913 x 777 masks, which have no aligned rows, 37.)
 // The masks of up to WIN_MAX_SIZES sizes that share the period and the kernel support are one
 // launch: its CTAs are the tiles of win_tiles.hpp (per size: image, column block, share of the
 // base rows).  An image has nparts partials; those its size does not use are left zero.

@@ -1,6 +1,6 @@
 // Mixed-precision contractions on the 5th-generation tensor cores (tcgen05, kind::tf32) with
 // split operands and FP32 accumulation in TMEM: the interpolation's above Ny = 8 and the
-// window's of some large batches.  The rest of the mixed form is the FP32 path's.
+// window's of some large batches and plan classes.  The rest of the mixed form is the FP32 path's.
 //
 // Split products.  Every operand X is written as X = Xh + Xl with
 // Xh = round_tf32(X) and Xl = X - Xh (exact in FP32); the contraction computes
@@ -958,6 +958,9 @@ static int kblk_for(int Ny) { return std::max(1, (4 * Ny + 31) / 32); }  // 4Ny 
 // above Ny = 8, where the folded FP32 kernel is bound by its FMAs (44 images of 2048^2, Ny = 16:
 // 137 us here, 195 us folded).  Up to Ny = 8 the folded kernel reaches the rate of the stores
 // (1024 images of 1024^2, Ny = 8: 639 us, against 707 us here) and its rows need no split.
+// us a call over the batch above Ny = 8, here and folded: 1, 4, 16, 44 of 2048^2 (Ny = 16) 62, 79, 159, 371 and
+// 62, 85, 188, 428; 1, 8, 64 of 1280^2 (Ny = 10) 43, 58, 229 and 39, 62, 267; one of 1500 x 1200 43 and 39: a
+// single image below 2048^2 would be faster folded.
 bool fi_tc_serves(const ImgGeom& g) { return (g.Lx % 4) == 0 && g.Ny > 8 && kblk_for(g.Ny) == 2; }
 
 static int tc_err_flag(litho_ctx* ctx, int** flag) {
@@ -1067,11 +1070,14 @@ static int launch_win_tc(litho_ctx* ctx, const WinPart* parts, int n, float2* wi
 // The mixed form takes the window of large batches on the tensor cores where the folded kernel falls
 // short of the memory's rate: above Ny = 8 it is bound by its coefficient reads and the ends of its
 // tiles, and where masks fill less than four fifths of their period's rows, many of the four rows it
-// folds are outside and the same work serves fewer pixels.  (Masks whose values are exact in TF32, binary
-// ones, need no residual products here.)  us a call, here and folded: 64 of 2048^2 502 and 529, 200
-// of 1280^2 872 and 957, below 2^27 pixels 100 of 1100^2 448 and 438, 16 of 1500^2 186 and 139; 385 of
-// 604 x 1536 in 1024 rows 717 and 794, 600 of 300 x 2048 in 512 588 and 700, below 2^26 pixels 60 of
-// 604 x 1536 174 and 160.
+// folds are outside and the same work serves fewer pixels.  us a call, here and folded, of binary masks: 64
+// of 2048^2 482 and 499, 200 of 1280^2 649 and 737, 100 of 1100^2 245 and 282 (rows of 2048), below 2^27
+// pixels 16 of 1500^2 186 and 139; 385 of 604 x 1536 in 1024 rows 519 and 563, 600 of 300 x 2048 in 512
+// 528 and 624, 110 of 600 x 1020 129 and 133, below 2^26 pixels 60 of 604 x 1536 174 and 160.
+// Binary masks are exact in TF32 and need no residual products.  Grey ones do, and take longer here than
+// folded (which takes what it takes for binary ones): 64 of 2048^2 659, 200 of 1280^2 873, 385 of 604 x 1536
+// 774, 600 of 300 x 2048 880, 110 of 600 x 1020 174.  A call takes this form all the same: it does not know
+// its masks, and looking at them first (as plans do, plan_win_tc) would cost the binary ones 5 us.
 bool win_tc_serves(const ImgGeom& g, int batch) {
   const bool sparse = 5ll * g.Ly < 4ll * g.Fy;
   return (g.Lx % 4) == 0 && (g.Ny > 8 || sparse) && nb_for(g.Nx) > 0 &&

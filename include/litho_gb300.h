@@ -71,10 +71,11 @@ extern "C" {
  *                    to 12 bytes before and after the masks, which any CUDA
  *                    allocation covers, are read too and dropped.
  * LITHO_PREC_MIXED : for supports Ny > 8 the interpolation (intensity band ->
- *                    image), and the window DFT of large batches where that is
- *                    faster, on the tensor cores with split-operand TF32 products
- *                    and FP32 accumulation; everything else as above, whose
- *                    kernels reach the memory's rate in FP32.                  */
+ *                    image), and the window DFT of large batches and plan classes
+ *                    where that is faster for binary masks, on the tensor cores
+ *                    with split-operand TF32 products and FP32 accumulation;
+ *                    everything else as above, whose kernels reach the memory's
+ *                    rate in FP32.                                             */
 #define LITHO_PREC_FP32  0
 #define LITHO_PREC_MIXED 1
 
@@ -392,7 +393,8 @@ int litho_calc_tcc_medium(litho_ctx* ctx, const float* src, int srcSize, float o
  * Top-nk eigenpairs of the Hermitian tcc (interleaved float64, upper triangle
  * used as zheevr 'U').  scales descending (float32, and optionally float64);
  * kernel i is eigenvector i stored reversed: krn[i][j] = v_i[n-1-j].
- * krn64 (optional): nk*tccSize interleaved float64 kernels. */
+ * krn64 (optional): nk*tccSize interleaved float64 kernels.
+ * The eigenvalue counts hold for matrices of norm 1e-75 to 1e75. */
 int litho_calc_kernels(litho_ctx* ctx, const double* tcc, int tccSize, int nk,
                        float* krn_r, float* krn_i, float* scales,
                        double* krn64, double* scales64, int mem);
