@@ -120,7 +120,7 @@ struct WinSet {
   int rows;                           // most base rows of a tile
 };
 
-template <int NY, bool VEC>
+template <int NY, bool VEC, bool ASK>
 __global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __grid_constant__ WinSet G, int Fx, int Fy, int Nx,
                                                                  int Ny, float2* __restrict__ win_part, int nparts,
                                                                  int stall, int* err, const int* __restrict__ form) {
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(32 * wf_warps(NY), 2) win_fold_kernel(const __
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   early_next();
-  if (form != nullptr) {  // (launched early, then)
+  if constexpr (ASK) {  // launched early after win_dft_tc_kernel
     early_wait(form);
     if (*form == 0) return;  // the tensor cores have done these masks
   }
@@ -437,16 +437,21 @@ template <int NY>
 static cudaError_t launch_win_fold_t(cudaStream_t s, const WinSet& G, const ImgGeom& g, bool vec, float2* win_part,
                                      int nparts, int stall, int* err, const int* __restrict__ form) {
   const size_t smem = win_fold_smem<NY>(g.Nx, G.rows);
-  auto k = vec ? win_fold_kernel<NY, true> : win_fold_kernel<NY, false>;
+  const bool ask = vec && form != nullptr;  // (its own kernel: the test alone cost one image of 256^2 0.6 us)
+  auto k = ask ? win_fold_kernel<NY, true, true> : vec ? win_fold_kernel<NY, true, false> : win_fold_kernel<NY, false, false>;
   const cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
-  return launch_early(form != nullptr, k, dim3((unsigned)G.T.tile0[G.T.n]), WinFold<NY>::THREADS, smem, s, G, g.Fx, g.Fy, g.Nx,
-                      g.Ny, win_part, nparts, stall, err, form);
+  const int tiles = G.T.tile0[G.T.n];
+  if (ask)
+    return launch_early(true, k, dim3((unsigned)tiles), WinFold<NY>::THREADS, smem, s, G, g.Fx, g.Fy, g.Nx, g.Ny, win_part,
+                        nparts, stall, err, form);
+  k<<<tiles, WinFold<NY>::THREADS, smem, s>>>(G, g.Fx, g.Fy, g.Nx, g.Ny, win_part, nparts, stall, err, nullptr);
+  return cudaGetLastError();
 }
 
 // n <= WIN_MAX_SIZES mask sizes of one period and support, nparts partials per image; err: the
 // timeout flag; stall >= 0: the error-path test hook; form: nullptr, or a device word that says whether
-// the launch has masks to do (run_win_dft_tc)
+// the launch has masks to do (run_win_dft_tc; not asked with the hook, which stalls both kernels)
 cudaError_t launch_win_fold(cudaStream_t s, const WinPart* parts, int n, const float* const* coef,
                             const float2* const* twF, float2* win_part, int nparts, int stall, int* err,
                             const int* __restrict__ form) {
