@@ -39,7 +39,8 @@ def test_producer_lost(grey):
             names = [e.name for e in prof.events() if "win_" in e.name]
             if names:
                 break
-        assert names and all("win_dft_tc" in name for name in names)
+        if [e for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]:  # there are activity records
+            assert names and all("win_dft_tc" in name for name in names)
         ctx.set_test_stall(-1)
         again = ctx.image_batch(ks, masks, precision=L.PREC_MIXED)
         ctx.synchronize()
